@@ -33,6 +33,7 @@ EXPORTS = (
     "ditto_b200_gemm_relu_gemm_static_scratch",
     "ditto_b200_multi_head_attention",
     "ditto_b200_ffn",
+    "ditto_b200_ffn_ws",
     "ditto_b200_workspace_bytes",
     "ditto_b200_mlp_cluster_slots",
     "ditto_b200_selftest_umma",
@@ -85,6 +86,8 @@ def load():
     lib.ditto_b200_multi_head_attention.restype = i
     lib.ditto_b200_ffn.argtypes = [vp, vp, vp, vp, vp, vp, i, i, i, i, i, i, i, i, i, vp, vp]
     lib.ditto_b200_ffn.restype = i
+    lib.ditto_b200_ffn_ws.argtypes = [vp, vp, vp, vp, vp, vp, i, i, i, i, i, i, i, i, i, vp, sz, vp, vp]
+    lib.ditto_b200_ffn_ws.restype = i
     lib.ditto_b200_workspace_bytes.argtypes = [i, i, i, i, i, i, i]
     lib.ditto_b200_workspace_bytes.restype = sz
     lib.ditto_b200_mlp_cluster_slots.argtypes = [i, i]

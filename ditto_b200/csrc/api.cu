@@ -244,9 +244,9 @@ int ditto_b200_gemm_relu_gemm_static_scratch(const void* x, const void* w1, cons
                                                epilogue, status_word, static_cast<cudaStream_t>(stream));
 }
 
-int ditto_b200_ffn(const void* x, const void* w1, const void* b1, const void* w2, const void* b2, void* y, int batch,
-                   int M, int N, int K, int L, int dtype, int w_layout, int act1, int act2, int* status_word,
-                   void* stream) {
+int ditto_b200_ffn_ws(const void* x, const void* w1, const void* b1, const void* w2, const void* b2, void* y, int batch,
+                      int M, int N, int K, int L, int dtype, int w_layout, int act1, int act2, void* workspace, size_t ws_bytes,
+                      int* status_word, void* stream) {
   if (!x || !w1 || !w2 || !y) return DITTO_ERR_INVALID_ARG;
   if (batch <= 0 || M <= 0 || N <= 0 || K <= 0 || L <= 0) return DITTO_ERR_INVALID_ARG;
   if (!aligned16(x) || !aligned16(w1) || !aligned16(w2) || !aligned16(y)) return DITTO_ERR_INVALID_ARG;
@@ -256,8 +256,14 @@ int ditto_b200_ffn(const void* x, const void* w1, const void* b1, const void* w2
   if (act1 < 0 || act1 > 2 || act2 < 0 || act2 > 2) return DITTO_ERR_INVALID_ARG;
   if (M % 16 || N % 16 || K % 16 || L % 16) return DITTO_ERR_INVALID_ARG;
   return ditto_b200::launch_mlp_chain(x, w1, w2, y, batch, M, N, K, L, dtype == DITTO_DTYPE_BF16, w_layout, act1, act2,
-                                      b1, b2, ditto_b200::kMlpAuto, nullptr, 0, status_word,
+                                      b1, b2, ditto_b200::kMlpAuto, workspace, ws_bytes, status_word,
                                       static_cast<cudaStream_t>(stream));
+}
+
+int ditto_b200_ffn(const void* x, const void* w1, const void* b1, const void* w2, const void* b2, void* y, int batch,
+                   int M, int N, int K, int L, int dtype, int w_layout, int act1, int act2, int* status_word,
+                   void* stream) {
+  return ditto_b200_ffn_ws(x, w1, b1, w2, b2, y, batch, M, N, K, L, dtype, w_layout, act1, act2, nullptr, 0, status_word, stream);
 }
 
 size_t ditto_b200_workspace_bytes(int op, int batch, int M, int N, int K, int L, int dtype) {

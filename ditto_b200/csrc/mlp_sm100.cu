@@ -41,6 +41,7 @@
 #include "../../include/ditto_b200.h"
 #include "host_util.cuh"
 #include "mlp_common.cuh"
+#include "mlp_flow_sm100.cuh"
 #include "sm100_ptx.cuh"
 
 // Optional timeline capture for tuning (compiled in only with -DDITTO_TRACE): the first CTA stores
@@ -713,6 +714,8 @@ static int resolve_variant(int variant, int N, int K, int L, int w_layout) {
 
 size_t mlp_workspace_bytes(int batch, int M, int N, int K, int L, bool bf16, int w_layout, int variant) {
   int slots = 0;
+  if (variant == kMlpAuto && mlp_flow_supported(N, K, L))
+    return mlp_flow_pair_slots(bf16, &slots) == DITTO_OK ? mlp_flow_workspace_bytes(batch, M, N, L, mlp_flow_plan(batch, M, N, K, L, slots)) : 0;
   switch (resolve_variant(variant, N, K, L, w_layout)) {
     case kMlpWide:
       if (!mlp_wide_supported(N, K, L) || mlp_wide_cluster_slots(bf16, &slots) != DITTO_OK) return 0;
@@ -732,6 +735,14 @@ int launch_mlp_chain(const void* x, const void* w1, const void* w2, void* y, int
   // With few row blocks -- or a last wave that would leave most of the device idle -- some row blocks are
   // shared by several clusters, if the caller provided the scratch memory that form needs.
   int slots = 0, rc = 0;
+  // With scratch memory for a ring of hidden tiles the two GEMMs run as one flow of 2-SM tiles: measured faster than
+  // the cluster kernels at every size.  Without it (or with too little) the hidden layer stays inside a cluster.
+  if (variant == kMlpAuto && workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && mlp_flow_supported(N, K, L)) {
+    if ((rc = mlp_flow_pair_slots(bf16, &slots)) != DITTO_OK) return rc;
+    const FlowPlan plan = mlp_flow_plan(batch, M, N, K, L, slots);
+    if (ws_bytes >= mlp_flow_workspace_bytes(batch, M, N, L, plan))
+      return launch_mlp_flow(x, w1, w2, y, batch, M, N, K, L, bf16, w_layout, act1, act2, b1, b2, plan, workspace, status, stream);
+  }
   switch (resolve_variant(variant, N, K, L, w_layout)) {
     case kMlpWide: {
       if (!mlp_wide_supported(N, K, L)) return DITTO_ERR_UNSUPPORTED;

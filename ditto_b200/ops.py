@@ -144,29 +144,29 @@ def multi_head_attention(qkv, num_heads, out=None, scale=1.0, flags=0):
 
 
 _VARIANT_BITS = {"auto": 0, "pair": 0x200, "quad": 0x400, "wide": 0x800}
-_workspaces = {}
 
 
-def _workspace(device, nbytes):
-    """A scratch buffer of at least `nbytes` on `device`, kept and grown per device (the C ABI itself
-    allocates nothing: scratch memory is the caller's, and this module is that caller)."""
-    key = device.index if device.index is not None else torch.cuda.current_device()
-    buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = _workspaces[key] = torch.empty(nbytes, dtype=torch.uint8, device=f"cuda:{key}")
-    return buf
+def _scratch(lib, op, batch, M, N, K, L, dtype, device):
+    """(tensor, pointer, bytes) of the scratch memory a call runs fastest with (the C ABI itself allocates nothing).
+    Taken from the caching allocator per call: in stream order, so calls on several streams and threads and
+    captured graphs each have their own."""
+    need = lib.ditto_b200_workspace_bytes(op, batch, M, N, K, L, _DTYPE_CODE[dtype])
+    if not need:
+        return None, None, 0
+    buf = torch.empty(need, dtype=torch.uint8, device=device)
+    return buf, buf.data_ptr(), need
 
 
 def gemm_relu_gemm(x, w1, w2, out=None, activation="relu", weight_layout="IO", variant="auto", workspace="auto"):
-    """out = act(x @ w1) @ w2 with the hidden activations kept on chip.
+    """out = act(x @ w1) @ w2 in one kernel, the hidden activations in a ring that stays in L2 or inside a cluster.
 
     x [batch, M, K] or [M, K]; w1 [batch, K, L] / [K, L]; w2 [batch, L, N] / [L, N] when
     weight_layout == "IO" ([in, out]); "OI" takes the transposed [out, in] weights of
     nn/functional/linear.py.  activation: "relu" or "identity".  variant: "auto" (by shape), "pair"
     (eight-CTA clusters of CTA pairs, 2-SM MMAs), "quad" (four-CTA clusters, 128-wide hidden chunks) or "wide"
     (four-CTA clusters, 256-wide hidden chunks).  workspace: "auto" (this
-    module keeps a scratch buffer of ditto_b200_workspace_bytes() per device), None (no scratch: every row
-    block is computed by one cluster) or a uint8 CUDA tensor.
+    call takes ditto_b200_workspace_bytes() of scratch memory from the caching allocator), None (no scratch: the
+    hidden layer stays inside a cluster, which is slower) or a uint8 CUDA tensor.
     """
     global launch_count
     _check_tensor(x, "x")
@@ -210,11 +210,8 @@ def gemm_relu_gemm(x, w1, w2, out=None, activation="relu", weight_layout="IO", v
             _check_tensor(workspace, "workspace", torch.uint8)
             ws_ptr, ws_bytes = workspace.data_ptr(), workspace.numel()
         elif isinstance(workspace, str) and workspace == "auto":
-            need = lib.ditto_b200_workspace_bytes(_lib.OP_GEMM_RELU_GEMM | _VARIANT_BITS[variant], batch, M, N, K, L,
-                                                  _DTYPE_CODE[x.dtype])
-            if need:
-                buf = _workspace(x.device, need)
-                ws_ptr, ws_bytes = buf.data_ptr(), buf.numel()
+            _buf, ws_ptr, ws_bytes = _scratch(lib, _lib.OP_GEMM_RELU_GEMM | _VARIANT_BITS[variant], batch, M, N, K, L,
+                                              x.dtype, x.device)
         elif workspace is not None:
             raise TypeError("workspace must be 'auto', None or a uint8 CUDA tensor")
         stream = torch.cuda.current_stream().cuda_stream
@@ -231,7 +228,7 @@ _ACT_CODE = {"identity": 0, "relu": 1, "gelu": 2}
 
 
 def ffn(x, w1, b1, w2, b2, out=None, act1="relu", act2="relu", weight_layout="OI"):
-    """Position-wise feed-forward block out = act2(act1(x @ W1 + b1) @ W2 + b2), hidden layer on chip.
+    """Position-wise feed-forward block out = act2(act1(x @ W1 + b1) @ W2 + b2) in one kernel.
 
     Defaults follow the reference's PositionwiseFeedForward (nn/model/transformer.py:21-34): weights
     stored [out, in] like nn/functional/linear.py, ReLU after both linears.  x [M, K] or [batch, M, K];
@@ -273,10 +270,11 @@ def ffn(x, w1, b1, w2, b2, out=None, act1="relu", act2="relu", weight_layout="OI
     lib = _lib.load()
     with _on_device(x.device):
         stream = torch.cuda.current_stream().cuda_stream
-        rc = lib.ditto_b200_ffn(x3.data_ptr(), w13.data_ptr(), b1.data_ptr() if b1 is not None else None, w23.data_ptr(),
+        _buf, ws_ptr, ws_bytes = _scratch(lib, _lib.OP_GEMM_RELU_GEMM, batch, M, N, K, L, x.dtype, x.device)
+        rc = lib.ditto_b200_ffn_ws(x3.data_ptr(), w13.data_ptr(), b1.data_ptr() if b1 is not None else None, w23.data_ptr(),
                                 b2.data_ptr() if b2 is not None else None, out3.data_ptr(), batch, M, N, K, L,
                                 _DTYPE_CODE[x.dtype], 1 if weight_layout == "OI" else 0, _ACT_CODE[act1], _ACT_CODE[act2],
-                                _status_ptr(x.device), stream)
+                                ws_ptr, ws_bytes, _status_ptr(x.device), stream)
     _lib.check(rc, "ditto_b200_ffn")
     launch_count += 1
     return out

@@ -73,7 +73,7 @@ int ditto_b200_bmm_softmax_bmm(const void* q, const void* k, const void* v, void
 int ditto_b200_multi_head_attention(const void* qkv, void* out, int batch, int M, int heads, int head_dim, int dtype,
                                     float scale, int flags, int* status_word, void* stream);
 
-/* Fused MLP chain  y = act(X W1) W2 with the hidden activations kept on chip, replacing the
+/* Fused MLP chain  y = act(X W1) W2 in one kernel, replacing the
  * module built from BatchGemmReluGemm (python_test/auto_tensorize/test_hyper_fusion_cpu.py:24-96,
  * evaluation/cpu/bmm_relu_bmm.py:56-125) and, with epilogue 0, BatchGemmGemm
  * (benchmark/chimera/cuda/bmm_bmm_cuda.py:69-150).
@@ -82,9 +82,10 @@ int ditto_b200_multi_head_attention(const void* qkv, void* out, int batch, int M
  *   epilogue 0: identity between the GEMMs; 1: ReLU; | DITTO_EPILOGUE_PAIR_MMA / _QUAD_MMA / _WIDE_MMA
  *   forces one of the kernels (same results up to fp32 summation order; default: by shape)
  *   workspace / ws_bytes: optional scratch memory (ditto_b200_workspace_bytes; contents irrelevant on entry,
- *   undefined on return).  With few row blocks several clusters share a row block, each takes a range of the
- *   hidden dimension and the fp32 partials of Y are added through the scratch memory in a fixed order (the
- *   hidden activations still never leave the chip).  NULL or too small: one cluster per row block.
+ *   undefined on return).  With it the hidden activations pass through a ring of a few row blocks (at most about
+ *   64 MB, rewritten while it is in L2) between the tiles of the two GEMMs, the fastest form at every size; a
+ *   forced cluster kernel uses it to share row blocks between clusters when there are few.  NULL or too small:
+ *   the hidden activations stay inside a cluster, one cluster per row block.
  * Shapes: N <= 128 and K <= 128 (any multiples of 16, either weight layout): the reference's own shape family;
  * otherwise L % 128 == 0, K % 64 == 0, N in {256, 512, 768, 1024}, or -- on the default kernel -- L % 64 == 0,
  * K % 16 == 0 and N any multiple of 256 up to 16384 (results wider than 1024 columns are computed in column
@@ -128,6 +129,13 @@ int ditto_b200_gemm_relu_gemm_static_scratch(const void* x, const void* w1, cons
 int ditto_b200_ffn(const void* x, const void* w1, const void* b1, const void* w2, const void* b2, void* y, int batch,
                    int M, int N, int K, int L, int dtype, int w_layout, int act1, int act2, int* status_word,
                    void* stream);
+
+/* ditto_b200_ffn with scratch memory (ditto_b200_workspace_bytes with DITTO_OP_GEMM_RELU_GEMM; contents irrelevant on
+ * entry, undefined on return): the hidden layer then passes through a small ring in it that stays in L2, which
+ * is the faster form at every size.  NULL or too small: as ditto_b200_ffn. */
+int ditto_b200_ffn_ws(const void* x, const void* w1, const void* b1, const void* w2, const void* b2, void* y, int batch,
+                      int M, int N, int K, int L, int dtype, int w_layout, int act1, int act2, void* workspace,
+                      size_t ws_bytes, int* status_word, void* stream);
 
 /* Scratch bytes with which the op runs fastest at this shape on the current device (0 when none; every call
  * also works without).  `op` may be or-ed with DITTO_EPILOGUE_PAIR_MMA / DITTO_EPILOGUE_QUAD_MMA / DITTO_EPILOGUE_WIDE_MMA to ask for the
