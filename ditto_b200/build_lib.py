@@ -14,6 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libditto_b200.so")
+FASTCALL_PATH = os.path.join(LIB_DIR, "_fastcall.so")     # the operators' call path (csrc/fastcall.cpp)
 SOURCES = ["api.cu", "host_util.cu", "attention_sm100.cu", "attention_persistent_sm100.cu", "mlp_sm100.cu", "mlp_wide_sm100.cu", "mlp_pair_sm100.cu", "mlp_flow_sm100.cu", "selftest_sm100.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -29,12 +30,24 @@ def _nvcc():
 
 
 def _stale():
-    if not os.path.exists(LIB_PATH):
+    if not os.path.exists(LIB_PATH) or not os.path.exists(FASTCALL_PATH):
         return True
-    t = os.path.getmtime(LIB_PATH)
+    t = min(os.path.getmtime(LIB_PATH), os.path.getmtime(FASTCALL_PATH))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
     deps.append(os.path.join(HERE, "..", "include", "ditto_b200.h"))
     return any(os.path.getmtime(d) > t for d in deps if os.path.isfile(d))
+
+
+def _fastcall_command():
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    inc = [f"-I{p}" for p in cpp_extension.include_paths()]
+    inc += [f"-I{sysconfig.get_paths()['include']}", f"-I{os.path.join(os.path.dirname(os.path.dirname(_nvcc())), 'include')}"]
+    return ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *inc, os.path.join(CSRC, "fastcall.cpp"), "-o", FASTCALL_PATH, f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
+            "-ltorch_cuda", "-ltorch_python"]
 
 
 def build(force=False, verbose=False):
@@ -51,12 +64,13 @@ def build(force=False, verbose=False):
             cmd.insert(1, "-Xptxas=-v")
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
         objs.append(obj)
+    procs.append(("fastcall.cpp", subprocess.Popen(_fastcall_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
     for src, p in procs:
         out, _ = p.communicate()
         if verbose and out:
             print(out)
         if p.returncode != 0:
-            raise RuntimeError(f"nvcc failed on {src}:\n{out}")
+            raise RuntimeError(f"compiling {src} failed:\n{out}")
     link = [_nvcc(), "-shared", "-o", LIB_PATH, *objs, "-lcudart"]
     r = subprocess.run(link, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:

@@ -3,6 +3,11 @@
 PyTorch supplies device memory and the stream; all arithmetic happens in the hand-written
 sm_100a kernels of libditto_b200.so.  There is no CPU path: tensors must live on a CUDA device.
 """
+import ctypes
+import importlib.machinery
+import importlib.util
+import os
+
 import torch
 
 from . import _lib
@@ -50,6 +55,35 @@ def _status_ptr(device):
     return p
 
 
+# The call path in native code (csrc/fastcall.cpp), set up by the first checked call on a device: it handles the
+# straight case -- everything valid, on the current device -- and answers None for all others, which then take the
+# checked path below and its error messages.
+_fast = None
+
+
+def _enable_fast(device):
+    global _fast
+    if _fast is None:
+        path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "_fastcall.so")
+        if not os.path.exists(path):
+            raise ImportError(f"{path} not found: build it with `python -m ditto_b200.build_lib`")
+        loader = importlib.machinery.ExtensionFileLoader("_fastcall", path)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastcall", path, loader=loader))
+        loader.exec_module(mod)
+        lib = _lib.load()
+        mod.bind(*(ctypes.cast(fn, ctypes.c_void_p).value for fn in (
+            lib.ditto_b200_bmm_softmax_bmm, lib.ditto_b200_multi_head_attention, lib.ditto_b200_gemm_relu_gemm,
+            lib.ditto_b200_ffn_ws, lib.ditto_b200_workspace_bytes)))
+        _fast = mod
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    if index not in _fast_devices:
+        _fast.status(index, _status_ptr(device))
+        _fast_devices.add(index)
+
+
+_fast_devices = set()
+
+
 def device_status(device=None, reset=True):
     """Synchronise and return the device-side status word (0 = no bounded wait has expired)."""
     dev = torch.device(device) if device is not None else torch.device("cuda", torch.cuda.current_device())
@@ -78,6 +112,11 @@ def bmm_softmax_bmm(query, key, value, out=None, scale=1.0, key_layout="KL", fla
     scale = 1 gives the reference's exp / row-sum semantics.
     """
     global launch_count
+    if _fast is not None:
+        r = _fast.softmax(query, key, value, out, scale, key_layout, flags)
+        if r is not None:
+            launch_count += 1
+            return r
     _check_tensor(query, "query")
     if query.dtype not in _DTYPE_CODE:
         raise TypeError(f"query dtype {query.dtype} not supported (float16 / bfloat16)")
@@ -110,6 +149,7 @@ def bmm_softmax_bmm(query, key, value, out=None, scale=1.0, key_layout="KL", fla
                                             batch, M, N, K, L, _DTYPE_CODE[query.dtype], klay, float(scale),
                                             int(flags), None, 0, _status_ptr(query.device), stream)
     _lib.check(rc, "ditto_b200_bmm_softmax_bmm")
+    _enable_fast(query.device)
     launch_count += 1
     return out
 
@@ -119,6 +159,11 @@ def multi_head_attention(qkv, num_heads, out=None, scale=1.0, flags=0):
     hidden = num_heads * head_dim; returns [batch, M, hidden].  The head split / merge of
     nn/module/self_attention.py:46-73 is folded into the kernel's addressing (no reshape passes)."""
     global launch_count
+    if _fast is not None:
+        r = _fast.mha(qkv, num_heads, out, scale, flags)
+        if r is not None:
+            launch_count += 1
+            return r
     _check_tensor(qkv, "qkv")
     if qkv.dtype not in _DTYPE_CODE:
         raise TypeError(f"qkv dtype {qkv.dtype} not supported (float16 / bfloat16)")
@@ -139,6 +184,7 @@ def multi_head_attention(qkv, num_heads, out=None, scale=1.0, flags=0):
                                                  _DTYPE_CODE[qkv.dtype], float(scale), int(flags),
                                                  _status_ptr(qkv.device), stream)
     _lib.check(rc, "ditto_b200_multi_head_attention")
+    _enable_fast(qkv.device)
     launch_count += 1
     return out
 
@@ -169,6 +215,11 @@ def gemm_relu_gemm(x, w1, w2, out=None, activation="relu", weight_layout="IO", v
     hidden layer stays inside a cluster, which is slower) or a uint8 CUDA tensor.
     """
     global launch_count
+    if _fast is not None and variant == "auto" and (workspace is None or isinstance(workspace, str) and workspace == "auto"):
+        r = _fast.gemm(x, w1, w2, out, activation, weight_layout, workspace is not None)
+        if r is not None:
+            launch_count += 1
+            return r
     _check_tensor(x, "x")
     if x.dtype not in _DTYPE_CODE:
         raise TypeError(f"x dtype {x.dtype} not supported (float16 / bfloat16)")
@@ -220,6 +271,7 @@ def gemm_relu_gemm(x, w1, w2, out=None, activation="relu", weight_layout="IO", v
                                            (1 if activation == "relu" else 0) | _VARIANT_BITS[variant], ws_ptr, ws_bytes,
                                            _status_ptr(x.device), stream)
     _lib.check(rc, "ditto_b200_gemm_relu_gemm")
+    _enable_fast(x.device)
     launch_count += 1
     return out
 
@@ -234,6 +286,11 @@ def ffn(x, w1, b1, w2, b2, out=None, act1="relu", act2="relu", weight_layout="OI
     stored [out, in] like nn/functional/linear.py, ReLU after both linears.  x [M, K] or [batch, M, K];
     w1 [L, K], w2 [N, L] ("OI") or [K, L], [L, N] ("IO"); b1 [L], b2 [N] or None."""
     global launch_count
+    if _fast is not None:
+        r = _fast.ffn(x, w1, b1, w2, b2, out, act1, act2, weight_layout)
+        if r is not None:
+            launch_count += 1
+            return r
     _check_tensor(x, "x")
     if x.dtype not in _DTYPE_CODE:
         raise TypeError(f"x dtype {x.dtype} not supported (float16 / bfloat16)")
@@ -276,5 +333,6 @@ def ffn(x, w1, b1, w2, b2, out=None, act1="relu", act2="relu", weight_layout="OI
                                 _DTYPE_CODE[x.dtype], 1 if weight_layout == "OI" else 0, _ACT_CODE[act1], _ACT_CODE[act2],
                                 ws_ptr, ws_bytes, _status_ptr(x.device), stream)
     _lib.check(rc, "ditto_b200_ffn")
+    _enable_fast(x.device)
     launch_count += 1
     return out
