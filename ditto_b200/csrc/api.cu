@@ -43,6 +43,16 @@ int make_map_3d(CUtensorMap* map, bool bf16, const void* base, uint64_t cols, ui
   return ditto_b200::make_tensor_map(map, bf16, base, 3, dims, strides, box);
 }
 
+// CTAs that share an item's keys: as the caller's flags say, else by shape unless they name another tiling.
+int parts_for(int flags, bool any, long long batch, int M, int L, int d, int mode = 0) {
+  const int asked = (flags & DITTO_FLAG_SPLIT_MASK) / DITTO_FLAG_SPLIT_UNIT, blocks = (L + 127) / 128;
+  if (!any || (asked == 0 && batch > 4096)) return 1;
+  if (asked == 0) return ditto_b200::attention_parts(static_cast<int>(batch), M, L, d, mode);
+  int parts = 1 << (asked - 1);
+  while (parts > blocks) parts /= 2;
+  return parts;
+}
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace
@@ -103,9 +113,11 @@ int ditto_b200_bmm_softmax_bmm(const void* q, const void* k, const void* v, void
 #endif
   // head dimensions up to 64 with few key blocks per item take the persistent kernel (it hides the
   // per-item start-up, which long sequences amortise anyway) unless a flag asks for a specific tiling
-  const bool persistent = d == 64 && L <= kPersistentMaxKeys &&
-                          !(flags & (DITTO_FLAG_ONE_TILE | DITTO_FLAG_TWO_TILES | DITTO_FLAG_P_VIA_SMEM));
-  cudaError_t e = persistent
+  const bool any = !(flags & (DITTO_FLAG_ONE_TILE | DITTO_FLAG_TWO_TILES | DITTO_FLAG_P_VIA_SMEM));
+  const bool persistent = any && d == 64 && L <= kPersistentMaxKeys;
+  const int parts = parts_for(flags, any, batch, M, L, d);
+  cudaError_t e = parts > 1 ? ditto_b200::launch_attention_split(p, batch, d, bf16, 0, parts, static_cast<cudaStream_t>(stream))
+                  : persistent
                       ? ditto_b200::launch_attention_persistent(p, batch, bf16, 0, static_cast<cudaStream_t>(stream))
                       : ditto_b200::launch_attention(p, batch, d, bf16, nt, psmem, 0, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail("bmm_softmax_bmm launch", e);
@@ -146,8 +158,12 @@ int ditto_b200_multi_head_attention(const void* qkv, void* out, int batch, int M
   p.out_ld = hidden;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = status_word;
-  const bool persistent = d == 64 && M <= kPersistentMaxKeys && !(flags & (DITTO_FLAG_ONE_TILE | DITTO_FLAG_TWO_TILES));
-  cudaError_t e = persistent ? ditto_b200::launch_attention_persistent(p, batch * heads, bf16, 0,
+  const bool any = !(flags & (DITTO_FLAG_ONE_TILE | DITTO_FLAG_TWO_TILES));
+  const bool persistent = any && d == 64 && M <= kPersistentMaxKeys;
+  const int parts = parts_for(flags, any, batch * heads, M, M, d);
+  cudaError_t e = parts > 1 ? ditto_b200::launch_attention_split(p, batch * heads, d, bf16, 0, parts,
+                                                                 static_cast<cudaStream_t>(stream))
+                  : persistent ? ditto_b200::launch_attention_persistent(p, batch * heads, bf16, 0,
                                                                        static_cast<cudaStream_t>(stream))
                              : ditto_b200::launch_attention(p, batch * heads, d, bf16, nt, false, 0,
                                                             static_cast<cudaStream_t>(stream));
@@ -207,7 +223,9 @@ int ditto_b200_gemm_relu_gemm(const void* x, const void* w1, const void* w2, voi
     p.status = status_word;
     const int nt = (dk == 64 || M <= 128) ? 1 : 2;
     const int mode = act == 1 ? 1 : 2;
-    cudaError_t e = (dk == 64 && L <= kPersistentMaxKeys) ? ditto_b200::launch_attention_persistent(p, batch, bf16, mode, static_cast<cudaStream_t>(stream))
+    const int parts = parts_for(0, true, batch, M, L, dk, mode);
+    cudaError_t e = parts > 1 ? ditto_b200::launch_attention_split(p, batch, dk, bf16, mode, parts, static_cast<cudaStream_t>(stream))
+                    : (dk == 64 && L <= kPersistentMaxKeys) ? ditto_b200::launch_attention_persistent(p, batch, bf16, mode, static_cast<cudaStream_t>(stream))
                              : ditto_b200::launch_attention(p, batch, dk, bf16, nt, false, mode,
                                                             static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail("gemm_relu_gemm launch", e);

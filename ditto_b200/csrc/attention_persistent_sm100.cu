@@ -122,6 +122,11 @@ __global__ void __launch_bounds__(kThreads, 2) attention_persistent_kernel(const
     tmem_alloc(&bar->tmem_base, kTmemCols);
     tmem_relinquish();
   }
+  if (warp == 4 && lane == 0) {                        // parameters, not memory of the kernel ahead: ready early
+    tma_prefetch_desc(&p.map_q);
+    tma_prefetch_desc(&p.map_k);
+    tma_prefetch_desc(&p.map_v);
+  }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -135,9 +140,6 @@ __global__ void __launch_bounds__(kThreads, 2) attention_persistent_kernel(const
   if (warp == 4) {
     // ------------------------------------------------------------ TMA producer (one thread)
     if (lane == 0) {
-      tma_prefetch_desc(&p.map_q);
-      tma_prefetch_desc(&p.map_k);
-      tma_prefetch_desc(&p.map_v);
       bool ok = true;
       int g = 0;                                   // K/V blocks loaded so far, over all items
       int it = 0;

@@ -87,8 +87,8 @@ template <int D, int NT, bool PSMEM>
 constexpr bool kSeparateP = (NT == 1 && D == 64 && !PSMEM);
 
 // Instances whose CTAs walk several work items (the others are launched with one CTA per item).
-template <int D, int NT, bool PSMEM>
-constexpr bool kLoopItems = (D == 128 && !kSeparateP<D, NT, PSMEM>);
+template <int D, int NT, bool PSMEM, bool SPLIT>
+constexpr bool kLoopItems = (D == 128 && !kSeparateP<D, NT, PSMEM> && !SPLIT);
 
 template <int D, int NT, bool PSMEM>
 struct Smem {
@@ -132,7 +132,10 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 // MODE selects the element-wise stage between the two GEMMs: kModeSoftmax (online softmax and final
 // normalisation), kModeRelu / kModeIdentity (P = act(S) rounded to the input type, no scale, no
 // normalisation) -- the small-N form of the GEMM -> ReLU -> GEMM and plain GEMM -> GEMM chains.
-template <bool BF16, int D, int NT, bool PSMEM, int MODE>
+//
+// SPLIT: the CTAs of a cluster share one item (NT = 1), each taking a contiguous part of its K/V blocks, and combine
+// their (max, sum, O) through distributed shared memory -- see the epilogue.
+template <bool BF16, int D, int NT, bool PSMEM, int MODE, bool SPLIT>
 __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 : 1)
     attention_kernel(const __grid_constant__ AttnParams p) {
   using SM = Smem<D, NT, PSMEM>;
@@ -163,14 +166,17 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
   const int tiles = (p.M + NT * kBM - 1) / (NT * kBM);
   // The loop is a compile-time property of the instance (head dimension 128; see the launcher): with one item
   // per CTA known at compile time the other instances keep the code -- and the registers -- of a single pass.
-  constexpr bool kLoop = kLoopItems<D, NT, PSMEM>;
+  constexpr bool kLoop = kLoopItems<D, NT, PSMEM, SPLIT>;
+  // the CTAs of a cluster are consecutive: rank r of `parts` takes K/V blocks [r * n / parts, (r + 1) * n / parts)
+  const int part = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
+  const int parts = SPLIT ? p.parts : 1;
   const int my_items = kLoop ? (p.items - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x) : 1;
   struct Item {
     int slice, seq, head_col, m0;
   };
   auto decode = [&](int k) -> Item {
     Item it;
-    const int id = static_cast<int>(blockIdx.x) + k * static_cast<int>(gridDim.x);
+    const int id = SPLIT ? static_cast<int>(blockIdx.x) / parts : static_cast<int>(blockIdx.x) + k * static_cast<int>(gridDim.x);
     it.slice = id / tiles;
     // Packed multi-head input: slice = (sequence, head); rows come from the sequence, columns from
     // the head.  Plain batched input has heads == 1 and zero column offsets.
@@ -179,7 +185,9 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
     it.m0 = (id % tiles) * (NT * kBM);
     return it;
   };
-  const int nkv = (p.L + kBN - 1) / kBN;        // the last block may be partial: TMA zero-fills rows >= L
+  const int nkv_all = (p.L + kBN - 1) / kBN;    // the last block may be partial: TMA zero-fills rows >= L
+  const int j0 = SPLIT ? part * nkv_all / parts : 0;            // first K/V block of this CTA
+  const int nkv = SPLIT ? (part + 1) * nkv_all / parts - j0 : nkv_all;
   const int ksteps_d = p.d / 16;                // head dimension actually used by S = Q K^T (<= D / 16)
 
   if (threadIdx.x == 0) {
@@ -206,6 +214,11 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
     tmem_alloc(&bar->tmem_base, kTmemCols);
     tmem_relinquish();
   }
+  if (warp == kProducerWarp && lane == 0) {             // parameters, not memory of the kernel ahead: ready early
+    tma_prefetch_desc(&p.map_q);
+    tma_prefetch_desc(&p.map_k);
+    tma_prefetch_desc(&p.map_v);
+  }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -222,13 +235,11 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
   }
 #endif
 
+  bool ok = true;                           // every role's own: no bounded wait of this warp has expired
+  [[maybe_unused]] float row_m = 0.f, row_l = 0.f;   // SPLIT: this part's maximum and sum of the thread's row
   if (warp == kProducerWarp) {
     // ------------------------------------------------------------ TMA producer (one thread)
     if (lane == 0) {
-      tma_prefetch_desc(&p.map_q);
-      tma_prefetch_desc(&p.map_k);
-      tma_prefetch_desc(&p.map_v);
-      bool ok = true;
       int armed_k[4] = {-1, -1, -1, -1}, armed_v[4] = {-1, -1, -1, -1};  // parity of the newest armed phase
       int g = 0;                            // K/V blocks loaded so far, over all items: ring stage g % kStages
       for (int k = 0; k < my_items && ok; ++k) {
@@ -259,11 +270,11 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
             if (p.k_transposed) {
               // K given as [slice, D, L]: boxes of 64 kv-columns x D rows (MN-major operand)
               for (int a = 0; a < kBN / 64; ++a)
-                tma_load_3d(dst + a * (D * 128), &p.map_k, &bar->k_full[s], j * kBN + a * 64, 0, it.slice);
+                tma_load_3d(dst + a * (D * 128), &p.map_k, &bar->k_full[s], (j0 + j) * kBN + a * 64, 0, it.slice);
             } else {
               for (int a = 0; a < kAtoms; ++a)
                 tma_load_3d(dst + a * (kBN * 128), &p.map_k, &bar->k_full[s], p.k_col0 + it.head_col + a * 64,
-                            j * kBN, it.seq);
+                            (j0 + j) * kBN, it.seq);
             }
           }
           if (j == 0 && k > 0) {
@@ -279,11 +290,11 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
             if (p.v_transposed) {
               // V given as [slice, dv, L]: boxes of 64 kv-columns x D rows (K-major operand of P*V)
               for (int a = 0; a < kBN / 64; ++a)
-                tma_load_3d(dst + a * (D * 128), &p.map_v, &bar->v_full[s], j * kBN + a * 64, 0, it.slice);
+                tma_load_3d(dst + a * (D * 128), &p.map_v, &bar->v_full[s], (j0 + j) * kBN + a * 64, 0, it.slice);
             } else {
               for (int a = 0; a < kAtoms; ++a)
                 tma_load_3d(dst + a * (kBN * 128), &p.map_v, &bar->v_full[s], p.v_col0 + it.head_col + a * 64,
-                            j * kBN, it.seq);
+                            (j0 + j) * kBN, it.seq);
             }
           }
         }
@@ -351,10 +362,10 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
       }
     };
     auto wait = [&](uint64_t* b, uint32_t parity, uint32_t code) {
-      bool ok = mbar_wait(b, parity, abort_word, code);
-      ok = __all_sync(0xffffffffu, ok);
+      bool r = mbar_wait(b, parity, abort_word, code);
+      r = __all_sync(0xffffffffu, r);
       tc_fence_after_sync();
-      return ok;
+      return r;
     };
 
     // With a single K/V stage the release cannot wait for the next iteration's first MMA
@@ -363,7 +374,7 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
     // The CTA's K/V blocks form one sequence G = 0 .. my_items * nkv - 1 (block j = G % nkv of item G / nkv):
     // ring stages, barrier phases and the look-ahead waits follow G, whatever item a block belongs to.
     const int total_blocks = my_items * nkv;
-    bool ok = wait(&bar->k_full[0], 0, 0x301);
+    ok = wait(&bar->k_full[0], 0, 0x301);
     for (int t = 0; t < NT && ok; ++t) {
       ok = wait(&bar->q_full[t], 0, 0x300 + t);
       if (!ok) break;
@@ -486,7 +497,6 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
     const uint32_t o_col = lane_base + kColO + t * D;
     const uint32_t p_col = kSep ? lane_base + kColP : s_col;   // P overwrites S unless it has its own columns
     const float c = p.scale_log2;
-    bool ok = true;
 
     uint32_t par = 0;                       // parity of the K/V blocks of all items so far: the phase of s_full / p_part
 
@@ -509,7 +519,7 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
 
       float m_new = m;
       if constexpr (MODE == kModeSoftmax) {
-        if (j == nkv - 1 && (p.L % kBN) != 0) {
+        if (j0 + j == nkv_all - 1 && (p.L % kBN) != 0) {
           // partial last block: K rows >= L were zero-filled, their scores must not count
           const int valid = p.L % kBN;
 #pragma unroll
@@ -563,7 +573,8 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
       }
 
       if ((warp & 3) == 0) DITTO_STAMP(t * 256, k * nkv + j, 2);
-      const float mc = m * c;
+      // a part whose scores so far are all -inf contributes nothing (another part may have finite ones)
+      const float mc = SPLIT && m == -INFINITY ? 0.f : m * c;
       float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
       for (int part = 0; part < 2; ++part) {
@@ -638,7 +649,10 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
     if (!ok) break;
     tc_fence_after_sync();
     if ((warp & 3) == 0) DITTO_STAMP(t * 256, k * nkv + nkv - 1, 12);
-    {
+    if constexpr (SPLIT) {
+      row_m = m;
+      row_l = l;
+    } else {
       const Item it = decode(k);
       const float inv = MODE == kModeSoftmax ? 1.0f / l : 1.0f;
       // O leaves tensor memory whole (normalised and rounded: D / 2 registers), so that the accumulator is
@@ -684,6 +698,82 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
     }
   }
 
+  if constexpr (SPLIT) {
+    // Combine the parts.  Every CTA publishes its rows' (max, sum), scales its O by
+    // 2^(max - overall max) / overall sum and hands D / parts columns of it to each CTA of the cluster, which adds
+    // what it was given and writes those columns of the result: a reduce-scatter, so the exchange (D * 512 bytes in
+    // and out of every CTA) and the write-out are spread over the cluster.  Parts are added in rank order.
+    // The incoming pieces go to the K ring, idle since the last P*V of this CTA (first cluster barrier); laid out
+    // [source][16-byte piece][row], a warp's store or load covers 512 contiguous bytes.  Both barriers are reached
+    // by every thread whether its waits expired or not.
+    float2* ml = reinterpret_cast<float2*>(smem + SM::kOffStage);
+    if (warp < 4 && MODE == kModeSoftmax) ml[threadIdx.x] = make_float2(row_m, row_l);
+    __syncwarp();
+    cluster_sync_all();
+    const int cols = D / parts;                        // columns of the result that one CTA adds up: 8 to 64
+    const int cols_log2 = 31 - __clz(cols);
+    if (warp < 4) {
+      const int row = static_cast<int>(threadIdx.x);
+      float f = 1.f;
+      if constexpr (MODE == kModeSoftmax) {
+        const uint32_t at = smem_u32(ml + row);
+        float mv[8], lv[8], top = -INFINITY;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          if (r < parts) {
+            ld_cluster_v2(map_to_cta(at, r), mv[r], lv[r]);
+            top = fmaxf(top, mv[r]);
+          }
+        }
+        float total = 0.f;
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+          if (r < parts) total = fmaf(lv[r], ex2_approx((mv[r] - top) * p.scale_log2), total);
+        f = ex2_approx((row_m - top) * p.scale_log2) / total;
+      }
+      const uint32_t o_col = tmem_base + (static_cast<uint32_t>(warp * 32) << 16) + kColO;
+      const uint32_t in0 = smem_u32(smem + SM::kOffK) + (part * (cols / 4) * kBM + row) * 16;
+      // compact: these instructions run once per launch, and fetching them shows
+#pragma unroll 1
+      for (int h = 0; h < D; h += 32) {
+        uint32_t o[32];
+        tmem_ld_x32_wait(o_col + h, o);                // warp-collective
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int col = h + 4 * q;
+          st_cluster_v4(map_to_cta(in0 + (col & (cols - 1)) * (kBM * 4), col >> cols_log2), __uint_as_float(o[4 * q]) * f,
+                        __uint_as_float(o[4 * q + 1]) * f, __uint_as_float(o[4 * q + 2]) * f,
+                        __uint_as_float(o[4 * q + 3]) * f);
+        }
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();
+    if (warp < 4) {
+      const Item it = decode(0);
+      const int row = static_cast<int>(threadIdx.x);
+      const float4* in = reinterpret_cast<const float4*>(smem + SM::kOffK) + row;
+      if (it.m0 + row < p.M) {
+        uint8_t* dst = reinterpret_cast<uint8_t*>(p.out) +
+                       ((static_cast<size_t>(it.seq) * p.M + it.m0 + row) * p.out_ld + it.head_col) * 2;
+#pragma unroll 1
+        for (int c8 = 0; c8 < cols / 8; ++c8) {
+          const int col = part * cols + 8 * c8;        // widths are multiples of 16: whole 16-byte pieces
+          if (col >= p.dv) break;
+          float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+#pragma unroll 2
+          for (int r = 0; r < parts; ++r) {
+            const float4 u = in[(r * (cols / 4) + 2 * c8) * kBM], v = in[(r * (cols / 4) + 2 * c8 + 1) * kBM];
+            a.x += u.x; a.y += u.y; a.z += u.z; a.w += u.w;
+            b.x += v.x; b.y += v.y; b.z += v.z; b.w += v.w;
+          }
+          *reinterpret_cast<uint4*>(dst + col * 2) =
+              make_uint4(pack2<BF16>(a.x, a.y), pack2<BF16>(a.z, a.w), pack2<BF16>(b.x, b.y), pack2<BF16>(b.z, b.w));
+        }
+      }
+    }
+  }
+
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) DITTO_STAMP(512, 0, 9);
@@ -694,10 +784,10 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
 }
 
 // ------------------------------------------------------------------ launcher
-template <bool BF16, int D, int NT, bool PSMEM, int MODE>
-static cudaError_t launch_one(const AttnParams& p, int batch, cudaStream_t stream) {
+template <bool BF16, int D, int NT, bool PSMEM, int MODE, bool SPLIT>
+static cudaError_t launch_one(const AttnParams& p, int batch, int parts, cudaStream_t stream) {
   using SM = Smem<D, NT, PSMEM>;
-  auto kern = attention_kernel<BF16, D, NT, PSMEM, MODE>;
+  auto kern = attention_kernel<BF16, D, NT, PSMEM, MODE, SPLIT>;
   // the function attributes are set once per device (this instantiation's static)
   static std::atomic<unsigned long long> configured{0};
   static std::atomic<int> places[64];      // CTAs of this kernel the device holds at once
@@ -721,23 +811,28 @@ static cudaError_t launch_one(const AttnParams& p, int batch, cudaStream_t strea
     configured.fetch_or(1ull << dev, std::memory_order_release);
   }
   cudaLaunchConfig_t cfg = {};
-  // one CTA per place the device has (or per item, if there are fewer), or one CTA per item
+  // one CTA per place the device has (or per item, if there are fewer), one CTA per item, or one cluster per item
   AttnParams q = p;
   q.items = ((p.M + NT * kBM - 1) / (NT * kBM)) * batch;
+  q.parts = parts;
   // The work loop pays where an item is long enough for its fixed cost to show and short enough for it to
   // matter: measured at head dimension 128 (S = 512: -5 %, 2048: -1 % per item); at 64, where the exponentials
   // set the pace, one CTA per item was faster (S = 2048: 109 against 119 us), so those launches keep it.
-  constexpr bool loop = kLoopItems<D, NT, PSMEM>;
-  const int grid = loop ? std::min(q.items, places[dev].load(std::memory_order_relaxed)) : q.items;
+  constexpr bool loop = kLoopItems<D, NT, PSMEM, SPLIT>;
+  const int grid = loop ? std::min(q.items, places[dev].load(std::memory_order_relaxed)) : q.items * parts;
   cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
   cfg.blockDim = dim3(threads_for(NT), 1, 1);
   cfg.dynamicSmemBytes = SM::kBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see grid_dependency_wait in the kernel
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(parts);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = SPLIT ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, q);
 }
 
@@ -745,7 +840,7 @@ cudaError_t launch_attention(const AttnParams& p, int batch, int d, bool bf16, i
                              cudaStream_t stream) {
 #define DITTO_DISPATCH(BF, DD, NN, PS, MO) \
   if (bf16 == BF && d == DD && nt == NN && psmem == PS && mode == MO) \
-    return launch_one<BF, DD, NN, PS, MO>(p, batch, stream);
+    return launch_one<BF, DD, NN, PS, MO, false>(p, batch, 1, stream);
 #define DITTO_DISPATCH_SHAPES(PS, MO)  \
   DITTO_DISPATCH(false, 64, 1, PS, MO) \
   DITTO_DISPATCH(false, 64, 2, PS, MO) \
@@ -762,6 +857,87 @@ cudaError_t launch_attention(const AttnParams& p, int batch, int d, bool bf16, i
 #undef DITTO_DISPATCH_SHAPES
 #undef DITTO_DISPATCH
   return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_attention_split(const AttnParams& p, int batch, int d, bool bf16, int mode, int parts, cudaStream_t stream) {
+  const int blocks = (p.L + kBN - 1) / kBN;
+  const long long ctas = static_cast<long long>((p.M + kBM - 1) / kBM) * batch * parts;
+  if ((parts != 2 && parts != 4 && parts != 8) || parts > blocks || ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
+#define DITTO_DISPATCH(BF, DD, MO)              \
+  if (bf16 == BF && d == DD && mode == MO) \
+    return launch_one<BF, DD, 1, false, MO, true>(p, batch, parts, stream);
+#define DITTO_DISPATCH_SHAPES(MO)  \
+  DITTO_DISPATCH(false, 64, MO)  \
+  DITTO_DISPATCH(false, 128, MO) \
+  DITTO_DISPATCH(true, 64, MO)   \
+  DITTO_DISPATCH(true, 128, MO)
+  DITTO_DISPATCH_SHAPES(kModeSoftmax)
+  DITTO_DISPATCH_SHAPES(kModeRelu)
+  DITTO_DISPATCH_SHAPES(kModeIdentity)
+#undef DITTO_DISPATCH_SHAPES
+#undef DITTO_DISPATCH
+  return cudaErrorInvalidValue;
+}
+
+// Clusters of `parts` CTAs the device holds at once.
+template <int D>
+static int split_places(int lg) {
+  static std::atomic<int> places[64][4];                // 0: not looked up yet; else clusters + 1
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int n = places[dev][lg].load(std::memory_order_relaxed);
+  if (n == 0) {
+    using SM = Smem<D, 1, false>;
+    auto kern = attention_kernel<false, D, 1, false, kModeSoftmax, true>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1024, 1, 1);
+    cfg.blockDim = dim3(threads_for(1), 1, 1);
+    cfg.dynamicSmemBytes = SM::kBytes;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1u << lg;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int count = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::kBytes) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&count, kern, &cfg) != cudaSuccess)
+      return 0;
+    n = std::max(0, count) + 1;
+    places[dev][lg].store(n, std::memory_order_relaxed);
+  }
+  return n - 1;
+}
+
+// The split pays when a launch is one wave of few, long items: a launch lasts as long as its longest CTA.  With more
+// clusters than the device holds at once a second wave costs more than the split saves, so those are left alone.
+// Times of one launch (us, back to back in a graph) as fixed + per 128-key block, fitted to 62 shapes of 1 to 384
+// items and 2 to 64 blocks, fp16; a chain without a softmax takes about 0.6 of the time per block.  Measured, whole ->
+// chosen parts: head dimension 64: 1 x 16 rows, 8192 keys 78 -> 14.7; 8 tiles, 1024 keys 13.7 -> 7.5; 64 tiles, 8192 keys
+// 80 -> 34; 48 tiles, 512 keys 9.0 -> 8.6; 128: 16 tiles, 2048 keys 32.7 -> 13.2; 48 tiles, 512 keys 12.9 -> 9.7.
+int attention_parts(int batch, int M, int L, int d, int mode) {
+  constexpr int kSms = 148;
+  const long long items = static_cast<long long>((M + kBM - 1) / kBM) * batch;
+  const int blocks = (L + kBN - 1) / kBN;
+  if (items > kSms || blocks < 2) return 1;
+  const double f = mode == kModeSoftmax ? 1.0 : 0.6;
+  const double whole = d == 64 ? 4.2 + 1.16 * f * blocks : M <= kBM ? 4.1 + 1.5 * f * blocks : 5.8 + 1.7 * f * blocks;
+  int best = 1;
+  double best_t = 0.96 * whole;                         // a gain that is sure
+  for (int lg = 1; lg <= 3 && (1 << lg) <= blocks; ++lg) {
+    const int parts = 1 << lg, own = (blocks + parts - 1) / parts;
+    if (items * parts > 2 * kSms || items > (d == 64 ? split_places<64>(lg) : split_places<128>(lg))) break;
+    const bool crowded = items * parts > kSms;          // two CTAs on some SMs
+    const double t = d == 128 ? 6.6 + 1.6 * f * own
+                     : crowded ? 7.7 + 1.6 * f * own : 5.8 + (items * parts > 100 ? 0.6 : 0.0) + 1.16 * f * own;
+    if (t < best_t) {
+      best = parts;
+      best_t = t;
+    }
+  }
+  return best;
 }
 
 }  // namespace ditto_b200

@@ -22,6 +22,7 @@ struct AttnParams {
   int q_col0, k_col0, v_col0;  // first column of Q / K / V inside the packed row (0 when not packed)
   int out_ld;         // elements between output rows (D when not packed)
   int items;          // work items of the launch: slices x tiles of NT x 128 query rows (filled in by the launcher)
+  int parts;          // CTAs of a cluster that share an item's keys (filled in by the launcher)
   float scale_log2;   // softmax scale * log2(e)
   int* status;        // device word receiving a non-zero code if a bounded wait expired; may be null
   long long* trace;   // timeline buffer of -DDITTO_TRACE builds (null otherwise)
@@ -31,6 +32,13 @@ struct AttnParams {
 // (softmax mode only); mode 0 softmax, 1 ReLU, 2 identity between the two GEMMs.
 cudaError_t launch_attention(const AttnParams& p, int batch, int d, bool bf16, int nt, bool psmem, int mode,
                              cudaStream_t stream);
+
+// One 128-row tile per cluster of `parts` (2, 4 or 8, at most the number of 128-key blocks) CTAs that divide the keys
+// between them and combine on chip.
+cudaError_t launch_attention_split(const AttnParams& p, int batch, int d, bool bf16, int mode, int parts, cudaStream_t stream);
+
+// The number of parts that is expected to be fastest for a shape (1: no split).
+int attention_parts(int batch, int M, int L, int d, int mode);
 
 // Persistent variant for head dimensions up to 64 (attention_persistent_sm100.cu): two CTAs per SM walk the
 // (slice, tile) work items.  mode as above.

@@ -49,6 +49,8 @@ extern "C" {
 #define DITTO_FLAG_P_VIA_SMEM 1   /* stage the probabilities through shared memory instead of TMEM */
 #define DITTO_FLAG_ONE_TILE 2     /* one 128-row query tile per CTA, one CTA per tile (no persistent work loop) */
 #define DITTO_FLAG_TWO_TILES 4    /* two query tiles per CTA even where one is the default (N = K = 64) */
+#define DITTO_FLAG_SPLIT_UNIT 256  /* 1, 2, 3, 4 of these: 1, 2, 4, 8 CTAs share a tile's keys (at most one per 128 keys) */
+#define DITTO_FLAG_SPLIT_MASK (7 * DITTO_FLAG_SPLIT_UNIT)   /* not set: by shape.  Ignored beside the flags above */
 
 /* Fused attention chain  out = softmax(scale * Q K^T) V, replacing the module TVM builds from
  * BatchGemmSoftmaxGemmMMA (python/ditto/auto_compute/nn/functional/bmm_chain.py:5-104) under
