@@ -27,6 +27,7 @@ FLAG_SPLIT_UNIT = 256     # 1, 2, 3, 4 of these: 1, 2, 4, 8 CTAs share a tile's 
 EPILOGUE_PAIR_MMA = 0x200
 EPILOGUE_QUAD_MMA = 0x400
 EPILOGUE_WIDE_MMA = 0x800
+EPILOGUE_FLOW_MMA = 0x1000
 
 EXPORTS = (
     "ditto_b200_bmm_softmax_bmm",

@@ -179,7 +179,7 @@ int ditto_b200_gemm_relu_gemm(const void* x, const void* w1, const void* w2, voi
   if (!aligned16(x) || !aligned16(w1) || !aligned16(w2) || !aligned16(y)) return DITTO_ERR_INVALID_ARG;
   if (dtype != DITTO_DTYPE_FP16 && dtype != DITTO_DTYPE_BF16) return DITTO_ERR_UNSUPPORTED;
   if (w_layout != 0 && w_layout != 1) return DITTO_ERR_INVALID_ARG;
-  constexpr int kVariantMask = DITTO_EPILOGUE_PAIR_MMA | DITTO_EPILOGUE_QUAD_MMA | DITTO_EPILOGUE_WIDE_MMA;
+  constexpr int kVariantMask = DITTO_EPILOGUE_PAIR_MMA | DITTO_EPILOGUE_QUAD_MMA | DITTO_EPILOGUE_WIDE_MMA | DITTO_EPILOGUE_FLOW_MMA;
   const int variant_bits = epilogue & kVariantMask;
   const int act = epilogue & ~kVariantMask;
   if (act != 0 && act != 1) return DITTO_ERR_INVALID_ARG;
@@ -242,6 +242,7 @@ int ditto_b200_gemm_relu_gemm(const void* x, const void* w1, const void* w2, voi
   const int variant = variant_bits == DITTO_EPILOGUE_PAIR_MMA   ? ditto_b200::kMlpPair
                       : variant_bits == DITTO_EPILOGUE_QUAD_MMA ? ditto_b200::kMlpQuad
                       : variant_bits == DITTO_EPILOGUE_WIDE_MMA ? ditto_b200::kMlpWide
+                      : variant_bits == DITTO_EPILOGUE_FLOW_MMA ? ditto_b200::kMlpFlow
                                                                 : ditto_b200::kMlpAuto;
   return ditto_b200::launch_mlp_chain(x, w1, w2, y, batch, M, N, K, L, dtype == DITTO_DTYPE_BF16, w_layout, act, 0,
                                       nullptr, nullptr, variant, workspace, ws_bytes, status_word,
@@ -294,6 +295,7 @@ size_t ditto_b200_workspace_bytes(int op, int batch, int M, int N, int K, int L,
   const int variant = (op & DITTO_EPILOGUE_PAIR_MMA)   ? ditto_b200::kMlpPair
                       : (op & DITTO_EPILOGUE_QUAD_MMA) ? ditto_b200::kMlpQuad
                       : (op & DITTO_EPILOGUE_WIDE_MMA) ? ditto_b200::kMlpWide
+                      : (op & DITTO_EPILOGUE_FLOW_MMA) ? ditto_b200::kMlpFlow
                                                        : ditto_b200::kMlpAuto;
   size_t a = ditto_b200::mlp_workspace_bytes(batch, M, N, K, L, dtype == DITTO_DTYPE_BF16, 0, variant);
   size_t b = ditto_b200::mlp_workspace_bytes(batch, M, N, K, L, dtype == DITTO_DTYPE_BF16, 1, variant);

@@ -42,6 +42,7 @@
 #include "host_util.cuh"
 #include "mlp_common.cuh"
 #include "mlp_flow_sm100.cuh"
+#include "mlp_tiles_sm100.cuh"
 #include "sm100_ptx.cuh"
 
 // Optional timeline capture for tuning (compiled in only with -DDITTO_TRACE): the first CTA stores
@@ -714,8 +715,10 @@ static int resolve_variant(int variant, int N, int K, int L, int w_layout) {
 
 size_t mlp_workspace_bytes(int batch, int M, int N, int K, int L, bool bf16, int w_layout, int variant) {
   int slots = 0;
-  if (variant == kMlpAuto && mlp_flow_supported(N, K, L))
+  if (variant == kMlpAuto && mlp_flow_supported(N, K, L) && mlp_tiles_faster(batch, M, N, K, L)) return mlp_tiles_workspace_bytes(batch, M, L);
+  if ((variant == kMlpAuto || variant == kMlpFlow) && mlp_flow_supported(N, K, L))
     return mlp_flow_pair_slots(bf16, &slots) == DITTO_OK ? mlp_flow_workspace_bytes(batch, M, N, L, mlp_flow_plan(batch, M, N, K, L, slots)) : 0;
+  if (variant == kMlpFlow) return 0;
   switch (resolve_variant(variant, N, K, L, w_layout)) {
     case kMlpWide:
       if (!mlp_wide_supported(N, K, L) || mlp_wide_cluster_slots(bf16, &slots) != DITTO_OK) return 0;
@@ -735,14 +738,18 @@ int launch_mlp_chain(const void* x, const void* w1, const void* w2, void* y, int
   // With few row blocks -- or a last wave that would leave most of the device idle -- some row blocks are
   // shared by several clusters, if the caller provided the scratch memory that form needs.
   int slots = 0, rc = 0;
-  // With scratch memory for a ring of hidden tiles the two GEMMs run as one flow of 2-SM tiles: measured faster than
-  // the cluster kernels at every size.  Without it (or with too little) the hidden layer stays inside a cluster.
-  if (variant == kMlpAuto && workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && mlp_flow_supported(N, K, L)) {
+  // With scratch memory for the hidden layer small calls run as two launches over tiles, with scratch memory for a ring of
+  // hidden tiles large ones run as one flow of 2-SM tiles: measured faster than the cluster kernels at every size.
+  // Without it (or with too little) the hidden layer stays inside a cluster.
+  if ((variant == kMlpAuto || variant == kMlpFlow) && workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && mlp_flow_supported(N, K, L)) {
+    if (variant == kMlpAuto && mlp_tiles_faster(batch, M, N, K, L) && ws_bytes >= mlp_tiles_workspace_bytes(batch, M, L))
+      return launch_mlp_tiles(x, w1, w2, y, batch, M, N, K, L, bf16, w_layout, act1, act2, b1, b2, mlp_tiles_plan(batch, M, N, K, L), workspace, status, stream);
     if ((rc = mlp_flow_pair_slots(bf16, &slots)) != DITTO_OK) return rc;
     const FlowPlan plan = mlp_flow_plan(batch, M, N, K, L, slots);
     if (ws_bytes >= mlp_flow_workspace_bytes(batch, M, N, L, plan))
       return launch_mlp_flow(x, w1, w2, y, batch, M, N, K, L, bf16, w_layout, act1, act2, b1, b2, plan, workspace, status, stream);
   }
+  if (variant == kMlpFlow) return mlp_flow_supported(N, K, L) ? DITTO_ERR_WORKSPACE : DITTO_ERR_UNSUPPORTED;
   switch (resolve_variant(variant, N, K, L, w_layout)) {
     case kMlpWide: {
       if (!mlp_wide_supported(N, K, L)) return DITTO_ERR_UNSUPPORTED;

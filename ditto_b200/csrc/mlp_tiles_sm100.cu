@@ -1,0 +1,461 @@
+// GEMM -> activation -> GEMM for sm_100a as two launches of one tile kernel, D = act(A B + bias), with the hidden
+// layer in scratch memory (it stays in L2).
+//
+// For calls of few tiles the flow kernel (mlp_flow_sm100.cu) is a chain of waits: its two GEMMs hand over tile by
+// tile inside one launch (8 k clocks from a hidden tile to the GEMM2 tile that reads it), a split tile's partials
+// make a round trip through global memory (9 k clocks and more), and a counter reset runs in front.  Two plain
+// launches cost less: the second one's CTAs are set up, and have their first weights in shared memory, before the
+// first one ends (programmatic dependent launch), and a reduction that would leave SMs idle is divided between the CTAs of a
+// cluster, which combine through distributed shared memory.
+//
+// A CTA computes one tile of 128 x bn (cta_group::1 MMAs, one accumulator in tensor memory) over its share of the
+// reduction.  Roles: warps 0-3 epilogue, 4 and 5 TMA producers (A and B operands), 6 MMA issuer.  Operand stages hold
+// one k-step of 64; with a ring of 96 KB two CTAs share an SM, so that one's epilogue runs under the other's MMAs,
+// with 192 KB a lone CTA has enough bytes in flight to be fed at the L2 rate.
+//
+// What bounds it: operand bytes out of L2 -- 16 KB + bn * 128 B a k-step against the 87 B/clk per SM that TMA loads
+// deliver on all SMs at once: 376 clocks at bn = 128 (256 of tensor work), 565 at 256 (512) -- and, in short calls,
+// two chains of launch, first load, epilogue.
+#include <cuda.h>
+
+#include <algorithm>
+#include <atomic>
+#include <cstring>
+
+#include "../../include/ditto_b200.h"
+#include "host_util.cuh"
+#include "mlp_common.cuh"
+#include "mlp_tiles_sm100.cuh"
+#include "sm100_ptx.cuh"
+
+namespace ditto_b200 {
+
+namespace {
+
+constexpr int kRows = 128;
+constexpr int kATile = 16 * 1024;                // 128 rows x 64
+constexpr int kMaxStages = 8;
+constexpr int kWarpA = 4, kWarpB = 5, kWarpMma = 6;
+constexpr int kThreads = 7 * 32;
+constexpr uint32_t kTmemCols = 256;              // two CTAs an SM
+
+struct TilesParams {
+  CUtensorMap map_a;        // A (K, M, batch), box 64 x 128 x 1
+  CUtensorMap map_b;        // [out, in]: (K, N, batch), box 64 x bn x 1;  [in, out]: (64, K, N / 64, batch), box 64 x 64 x bn / 64 x 1
+  void* out;                // [batch, M, N]
+  const void* bias;         // [batch, N] or null
+  int M, N;
+  int bn, blocks_per_batch, blocks;     // 128-row blocks
+  int steps;                // k-steps of 64
+  int chunks;               // GEMM2: 256-column chunks of the hidden layer, taken in the order below (0: in order)
+  int parts, stages, stage_bytes;
+  int oi;
+  int early_b;              // B is not written by the kernel ahead: its loads need not wait for that
+  int* status;
+};
+
+struct TilesBars {
+  uint64_t full[kMaxStages], empty[kMaxStages];
+  uint64_t acc_full;
+  uint32_t tmem_base;
+  uint32_t abort_word;
+};
+static_assert(sizeof(TilesBars) <= 256, "barrier block too large");
+
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z, int w) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(w)
+      : "memory");
+}
+
+// First column of k-step k.  GEMM2 adds the hidden columns in the order the four-CTA kernel adds them -- 64-column units
+// dealt out over four 256-column chunks: unit e of round i is quarter e / cr of chunk 4 i + e % cr (cr chunks in the
+// round) -- so that a tile whose reduction is not split has the same bits in all forms of the chain.
+__device__ __forceinline__ int step_col(int k, int chunks) {
+  if (chunks == 0) return k * 64;
+  const int i = k >> 4, e = k & 15;
+  const int cr = min(4, chunks - 4 * i);
+  const int qt = cr == 4 ? e >> 2 : e / cr;
+  return (4 * i + (e - qt * cr)) * 256 + qt * 64;
+}
+
+// N accumulator columns + bias -> activation -> packed words; 16-byte bias loads where the vector's alignment allows.
+template <bool BF16, int ACT, bool BIAS, int N>
+__device__ __forceinline__ void finish(const uint32_t (&v)[N], const uint32_t* bias, uint32_t (&w)[N / 2]) {
+  if constexpr (BIAS) {
+    if ((reinterpret_cast<uintptr_t>(bias) & 15) == 0) act_pack_fixed<BF16, ACT, true, N, true>(v, bias, w);
+    else act_pack_fixed<BF16, ACT, true, N>(v, bias, w);
+  } else {
+    act_pack_fixed<BF16, ACT, false, N>(v, nullptr, w);
+  }
+}
+
+}  // namespace
+
+template <bool BF16, int ACT, bool BIAS>
+__global__ void __launch_bounds__(kThreads, 2) mlp_tiles_kernel(const __grid_constant__ TilesParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  // the CTAs of a cluster round up by the same amount: offsets match across the cluster
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  TilesBars* bar = reinterpret_cast<TilesBars*>(smem + p.stages * p.stage_bytes);
+  volatile uint32_t* abort_word = &bar->abort_word;
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  // clusters are consecutive CTAs; row blocks innermost, so that neighbours share weights
+  const int part = static_cast<int>(cluster_ctarank());
+  const int tile = static_cast<int>(blockIdx.x) / p.parts;
+  const int n = tile / p.blocks, rb = tile - n * p.blocks;
+  const int b = rb / p.blocks_per_batch;
+  const int row0 = (rb - b * p.blocks_per_batch) * kRows;
+  const int col0 = n * p.bn;
+  const int k0 = p.steps * part / p.parts, k1 = p.steps * (part + 1) / p.parts;   // parts <= steps: never empty
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(&bar->full[s], 1);
+      mbar_init(&bar->empty[s], 1);
+    }
+    mbar_init(&bar->acc_full, 1);
+    bar->abort_word = 0;
+    fence_mbar_init();
+  }
+  if (warp == 0) {
+    tmem_alloc(&bar->tmem_base, kTmemCols);
+    tmem_relinquish();
+  }
+  if (warp == kWarpA && lane == 0) {
+    tma_prefetch_desc(&p.map_a);
+    tma_prefetch_desc(&p.map_b);
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = bar->tmem_base;
+
+  bool ok = true;
+  if (warp == kWarpB) {
+    // ------------------------------------------------------------ B operand (weights)
+    if (p.early_b == 0) grid_dependency_wait();
+    if (lane == 0) {
+      int st = 0;
+      uint32_t ph = 1;
+      for (int k = k0; k < k1; ++k) {
+        ok = mbar_wait(&bar->empty[st], ph, abort_word, 0x110);
+        if (!ok) break;
+        uint8_t* dst = smem + st * p.stage_bytes + kATile;
+        const int kc = step_col(k, p.chunks);
+        if (p.oi) tma_load_3d(dst, &p.map_b, &bar->full[st], kc, col0, b);
+        else tma_load_4d(dst, &p.map_b, &bar->full[st], 0, kc, col0 >> 6, b);
+        if (++st == p.stages) { st = 0; ph ^= 1; }
+      }
+    }
+    __syncwarp();
+    if (p.early_b != 0) grid_dependency_wait();
+    grid_launch_dependents();
+  } else {
+    grid_dependency_wait();
+    grid_launch_dependents();
+    if (warp == kWarpA) {
+      // ---------------------------------------------------------- A operand; arms the stage for both
+      if (lane == 0) {
+        asm volatile("fence.proxy.async.global;" ::: "memory");   // A may be the kernel ahead's ordinary stores
+        int st = 0;
+        uint32_t ph = 1;
+        for (int k = k0; k < k1; ++k) {
+          ok = mbar_wait(&bar->empty[st], ph, abort_word, 0x100);
+          if (!ok) break;
+          mbar_arrive_expect_tx(&bar->full[st], static_cast<uint32_t>(p.stage_bytes));
+          tma_load_3d(smem + st * p.stage_bytes, &p.map_a, &bar->full[st], step_col(k, p.chunks), row0, b);
+          if (++st == p.stages) { st = 0; ph ^= 1; }
+        }
+      }
+      __syncwarp();
+    } else if (warp == kWarpMma) {
+      // ---------------------------------------------------------- MMA issuer (converged warp)
+      const uint32_t issuer = elect_one();
+      const uint32_t ring = smem_u32(smem);
+      const uint32_t idesc = umma_idesc_f16(BF16, kRows, p.bn, false, p.oi == 0);
+      int st = 0;
+      uint32_t ph = 0;
+      for (int k = k0; k < k1; ++k) {
+        ok = mbar_wait(&bar->full[st], ph, abort_word, 0x200);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after_sync();
+        const uint32_t sa = ring + st * p.stage_bytes, sb = sa + kATile;
+        const uint64_t da = umma_desc_sw128(sa, 16, 1024);
+        const uint64_t db = p.oi ? umma_desc_sw128(sb, 16, 1024) : umma_desc_sw128(sb, 8192, 1024);
+        const uint32_t step_b = p.oi ? 32u >> 4 : 2048u >> 4;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          umma_ss_elected(tmem_base, da + ((i * 32) >> 4), db + i * step_b, idesc, (k > k0 || i > 0) ? 1u : 0u, issuer);
+        umma_commit_elected(&bar->empty[st], issuer);
+        if (++st == p.stages) { st = 0; ph ^= 1; }
+      }
+      if (ok) umma_commit_elected(&bar->acc_full, issuer);
+    } else {
+      // ---------------------------------------------------------- epilogue
+      ok = mbar_wait(&bar->acc_full, 0, abort_word, 0x300);
+      ok = __all_sync(0xffffffffu, ok);
+      tc_fence_after_sync();
+      if (ok && p.parts == 1) {
+        // 32 columns at a time, turned around in 2 KB of the (now idle) ring per warp -- 64-byte rows of four 16-byte
+        // pieces, swizzled: no bank conflicts -- so that a store instruction writes 64 contiguous bytes of eight rows
+        const uint32_t acc = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+        uint8_t* stage = smem + warp * 2048;
+        const int row = row0 + warp * 32;
+        uint8_t* to = static_cast<uint8_t*>(p.out) + (static_cast<size_t>(b) * p.M + row + (lane >> 2)) * p.N * 2 + (lane & 3) * 16;
+        const int cols = min(p.bn, p.N - col0);          // N is a multiple of 64
+#pragma unroll 1
+        for (int c = 0; c < cols; c += 32) {
+          uint32_t v[32], w[16];
+          tmem_ld_x32_wait(acc + c, v);
+          finish<BF16, ACT, BIAS>(v, BIAS ? reinterpret_cast<const uint32_t*>(p.bias) + (static_cast<size_t>(b) * p.N + col0 + c) / 2 : nullptr, w);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<uint4*>(stage + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) =
+                make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int rr = 8 * i + (lane >> 2);
+            const uint4 t = *reinterpret_cast<const uint4*>(stage + rr * 64 + (((lane & 3) ^ ((rr >> 1) & 3)) << 4));
+            if (row + rr < p.M) *reinterpret_cast<uint4*>(to + static_cast<size_t>(8 * i) * p.N * 2 + (col0 + c) * 2) = t;
+          }
+          __syncwarp();
+        }
+      }
+    }
+  }
+
+  if (p.parts > 1) {
+    // The CTAs of the cluster hold partial sums of the same tile.  Each hands bn / parts columns of its own to every
+    // CTA (into its ring, idle since the last MMA: first barrier), adds what it was given in rank order and finishes
+    // those columns.  Laid out [source][four columns][row], a warp's store or load covers 512 contiguous bytes.  Every
+    // thread reaches both barriers whether its waits expired or not.
+    __syncwarp();
+    cluster_sync_all();
+    const int cols = p.bn / p.parts;                     // 16, 32 or 64
+    const int row = static_cast<int>(threadIdx.x);
+    if (warp < 4) {
+      const int cols_log2 = 31 - __clz(cols);
+      const uint32_t in0 = smem_u32(smem) + (part * (cols / 4) * kRows + row) * 16;
+      const uint32_t acc = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+#pragma unroll 1
+      for (int h = 0; h < p.bn; h += 32) {
+        uint32_t v[32];
+        tmem_ld_x32_wait(acc + h, v);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int col = h + 4 * q;
+          st_cluster_v4(map_to_cta(in0 + (col & (cols - 1)) * (kRows * 4), col >> cols_log2), __uint_as_float(v[4 * q]),
+                        __uint_as_float(v[4 * q + 1]), __uint_as_float(v[4 * q + 2]), __uint_as_float(v[4 * q + 3]));
+        }
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();
+    if (warp < 4 && row0 + row < p.M) {
+      const float4* in = reinterpret_cast<const float4*>(smem) + row;
+      uint8_t* to = static_cast<uint8_t*>(p.out) + (static_cast<size_t>(b) * p.M + row0 + row) * p.N * 2;
+#pragma unroll 1
+      for (int c = 0; c < cols; c += 16) {
+        const int col = col0 + part * cols + c;
+        if (col >= p.N) break;
+        float sum[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) sum[j] = 0.f;
+#pragma unroll 2
+        for (int r = 0; r < p.parts; ++r) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float4 t = in[(r * (cols / 4) + c / 4 + q) * kRows];
+            sum[4 * q] += t.x; sum[4 * q + 1] += t.y; sum[4 * q + 2] += t.z; sum[4 * q + 3] += t.w;
+          }
+        }
+        uint32_t v[16], w[8];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(sum[j]);
+        finish<BF16, ACT, BIAS>(v, BIAS ? reinterpret_cast<const uint32_t*>(p.bias) + (static_cast<size_t>(b) * p.N + col) / 2 : nullptr, w);
+        *reinterpret_cast<uint4*>(to + col * 2) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(to + col * 2 + 16) = make_uint4(w[4], w[5], w[6], w[7]);
+      }
+    }
+  }
+
+  // After a wait has given up, copies this CTA issued may still be in flight; they complete within microseconds.
+  if (*abort_word != 0u) {
+    for (int t = 0; t < 64; ++t) __nanosleep(1000);
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    tmem_dealloc(tmem_base, kTmemCols);
+    if (lane == 0 && bar->abort_word != 0 && p.status != nullptr) atomicCAS(p.status, 0, static_cast<int>(bar->abort_word));
+  }
+}
+
+// ------------------------------------------------------------------ host side
+namespace {
+
+constexpr int kBarBytes = 256, kSlack = 1024;
+constexpr int kRingLone = 192 * 1024, kRingShared = 96 * 1024;
+
+template <bool BF16, int ACT, bool BIAS>
+cudaError_t launch_one(const TilesParams& p, int ctas, cudaStream_t stream) {
+  auto kern = mlp_tiles_kernel<BF16, ACT, BIAS>;
+  static std::atomic<unsigned long long> configured{0};
+  int dev = 0;
+  cudaError_t e = current_device_checked(&dev);
+  if (e != cudaSuccess) return e;
+  if (!device_configured(configured, dev)) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingLone + kBarBytes + kSlack);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+    mark_device_configured(configured, dev);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(ctas), 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = static_cast<size_t>(p.stages) * p.stage_bytes + kBarBytes + kSlack;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(p.parts);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.parts > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, p);
+}
+
+// D [batch, M, N] = act(A [batch, M, K] * B + bias)
+int launch_gemm(const void* a, const void* w, void* out, const void* bias, int batch, int M, int N, int K, bool bf16,
+                int w_layout, int act, bool second, const TilesGemm& g, int* status, cudaStream_t stream) {
+  TilesParams p;
+  std::memset(&p, 0, sizeof(p));
+  const uint64_t uM = M, uN = N, uK = K, ub = batch;
+  auto map3 = [&](CUtensorMap* m, const void* base, uint64_t rows, uint32_t box_rows) {
+    const uint64_t dims[3] = {uK, rows, ub}, strides[2] = {uK * 2, rows * uK * 2};
+    const uint32_t box[3] = {64, box_rows, 1};
+    return make_tensor_map(m, bf16, base, 3, dims, strides, box);
+  };
+  int rc = map3(&p.map_a, a, uM, kRows);
+  if (rc) return rc;
+  if (w_layout == 1) {
+    rc = map3(&p.map_b, w, uN, static_cast<uint32_t>(g.bn));
+  } else {
+    // [K, N] seen as (64 columns, K, N / 64, batch): one box brings the swizzle atoms of an MN-major operand tile
+    const uint64_t dims[4] = {64, uK, uN / 64, ub}, strides[3] = {uN * 2, 128, uK * uN * 2};
+    const uint32_t box[4] = {64, 64, static_cast<uint32_t>(g.bn / 64), 1};
+    rc = make_tensor_map(&p.map_b, bf16, w, 4, dims, strides, box);
+  }
+  if (rc) return rc;
+  p.out = out;
+  p.bias = bias;
+  p.M = M;
+  p.N = N;
+  p.bn = g.bn;
+  p.blocks_per_batch = (M + kRows - 1) / kRows;
+  p.blocks = batch * p.blocks_per_batch;
+  p.chunks = second ? (K + 255) / 256 : 0;
+  p.steps = second ? 4 * p.chunks : (K + 63) / 64;      // (units past the hidden size read as zero)
+  p.parts = g.parts;
+  p.stage_bytes = kATile + g.bn * 128;
+  p.stages = std::min(kMaxStages, (g.per_sm == 2 ? kRingShared : kRingLone) / p.stage_bytes);
+  p.oi = w_layout == 1;
+  p.early_b = second ? 1 : 0;
+  p.status = status;
+  const long long ctas = static_cast<long long>(p.blocks) * ((N + g.bn - 1) / g.bn) * g.parts;
+  if (ctas > 0x7fffffffLL) return DITTO_ERR_UNSUPPORTED;
+  cudaError_t e = cudaErrorInvalidValue;
+#define DITTO_TILES(BF, AC, BI) \
+  if (bf16 == BF && act == AC && (bias != nullptr) == BI) e = launch_one<BF, AC, BI>(p, static_cast<int>(ctas), stream);
+#define DITTO_TILES_ACTS(BF, BI) DITTO_TILES(BF, 0, BI) DITTO_TILES(BF, 1, BI) DITTO_TILES(BF, 2, BI)
+  DITTO_TILES_ACTS(false, false)
+  DITTO_TILES_ACTS(false, true)
+  DITTO_TILES_ACTS(true, false)
+  DITTO_TILES_ACTS(true, true)
+#undef DITTO_TILES_ACTS
+#undef DITTO_TILES
+  return e == cudaSuccess ? DITTO_OK : cuda_fail("mlp tile kernel launch", e);
+}
+
+}  // namespace
+
+size_t mlp_tiles_workspace_bytes(int batch, int M, int L) { return static_cast<size_t>(batch) * M * L * 2; }
+
+namespace {
+
+// Modelled time (us, without a launch's fixed part) of D [M, N] over `steps` k-steps.  Waves of tiles: a step on an SM
+// with a full set of CTAs, and one of a lone CTA, which is longer where too few bytes are in flight (bn = 64; a 96 KB
+// ring).  The constants are fitted to 390 timings (13 shapes of 16 to 16384 rows, each with 10 to 20 ways to cut either
+// GEMM); the cut it picks is on average 1.3 % slower than the best one timed.
+double tiles_time(long long blocks, int N, int steps, const TilesGemm& g) {
+  const double shared = 0.109 + 0.00059 * g.bn;
+  const double lone = std::max(g.per_sm == 1 ? 0.382 - 0.00333 * g.bn : -0.066 + 0.00242 * g.bn, shared);
+  const double own = (steps + g.parts - 1) / g.parts, ends = 1.77 + 0.0067 * g.bn;
+  const long long ctas = blocks * ((N + g.bn - 1) / g.bn) * g.parts, places = 148LL * g.per_sm;
+  const long long full = ctas / places, rest = ctas % places;
+  double t = g.parts > 1 ? 0.975 + 0.162 * g.parts : 0.0;
+  if (g.per_sm == 1) return t + static_cast<double>(full + (rest > 0)) * (own * lone + ends);
+  if (full > 0) t += static_cast<double>(full) * 2.0 * own * shared + ends;
+  if (rest > 0) t += own * (lone + (2.0 * shared - lone) * std::min(1.0, std::max<long long>(0, rest - 148) / 74.0)) + ends;
+  return t;
+}
+
+// (A reduction over 1024 or less is not split, as in the flow kernel: the result has the bits of the cluster kernels.)
+TilesGemm best_gemm(long long blocks, int N, int steps, double* time) {
+  TilesGemm best = {128, 1, 2};
+  *time = tiles_time(blocks, N, steps, best);
+  for (int bn = 64; bn <= 256; bn += 64)
+    for (int parts = 1; parts <= (bn == 128 ? 8 : bn == 64 ? 4 : 1) && (parts == 1 || steps > 16); parts *= 2)
+      for (int per_sm = 1; per_sm <= 2; ++per_sm) {
+        const long long ctas = blocks * ((N + bn - 1) / bn) * parts;
+        // all clusters at once; alone on their SMs, large ones leave part of a GPC unused
+        if (parts > 1 && ctas > (per_sm == 2 ? 296 : parts == 2 ? 148 : 112)) continue;
+        const TilesGemm g = {bn, parts, per_sm};
+        const double t = tiles_time(blocks, N, steps, g);
+        if (t < *time) {
+          best = g;
+          *time = t;
+        }
+      }
+  return best;
+}
+
+}  // namespace
+
+// Where two launches are the faster form.  The flow kernel's waits cost it about 10 us a call, and it is 20 % faster
+// per operation once its pairs are busy: measured, flow -> tiles, 16 x 1024 -> 4096 -> 1024 24.3 -> 12.9 us, 512 x 768 24.4 ->
+// 16.6, 2048 x 1024 (34 GFLOP) 40.8 -> 33.0, 4096 x 768 (39) 52.3 -> 45.9; 1024 x 2048 (69) 67.0 -> 67.6, 16384 x 512 (69)
+// 67 -> 74, 3328 x 1280 (87) 75 -> 82.  The hidden layer has to stay in L2 beside the operands.
+bool mlp_tiles_faster(int batch, int M, int N, int K, int L) {
+  return 2.0 * batch * M * static_cast<double>(L) * (static_cast<double>(K) + N) <= 4.8e10 &&
+         mlp_tiles_workspace_bytes(batch, M, L) <= (static_cast<size_t>(48) << 20);
+}
+
+TilesPlan mlp_tiles_plan(int batch, int M, int N, int K, int L) {
+  const long long blocks = static_cast<long long>(batch) * ((M + kRows - 1) / kRows);
+  TilesPlan plan;
+  double t1, t2;
+  plan.g1 = best_gemm(blocks, L, (K + 63) / 64, &t1);
+  plan.g2 = best_gemm(blocks, N, 4 * ((L + 255) / 256), &t2);
+  return plan;
+}
+
+int launch_mlp_tiles(const void* x, const void* w1, const void* w2, void* y, int batch, int M, int N, int K, int L,
+                     bool bf16, int w_layout, int act1, int act2, const void* b1, const void* b2, const TilesPlan& plan,
+                     void* workspace, int* status, cudaStream_t stream) {
+  if (workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 15)) return DITTO_ERR_WORKSPACE;
+  int rc = launch_gemm(x, w1, workspace, b1, batch, M, L, K, bf16, w_layout, act1, false, plan.g1, status, stream);
+  // The second launch starts when every CTA of the first is past its own dependency wait: whatever wrote the weights
+  // is complete by then, and the first launch does not write them.
+  return rc ? rc : launch_gemm(workspace, w2, y, b2, batch, M, N, L, bf16, w_layout, act2, true, plan.g2, status, stream);
+}
+
+}  // namespace ditto_b200

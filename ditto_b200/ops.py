@@ -189,7 +189,7 @@ def multi_head_attention(qkv, num_heads, out=None, scale=1.0, flags=0):
     return out
 
 
-_VARIANT_BITS = {"auto": 0, "pair": 0x200, "quad": 0x400, "wide": 0x800}
+_VARIANT_BITS = {"auto": 0, "pair": 0x200, "quad": 0x400, "wide": 0x800, "flow": 0x1000}
 
 
 def _scratch(lib, op, batch, M, N, K, L, dtype, device):
@@ -204,13 +204,13 @@ def _scratch(lib, op, batch, M, N, K, L, dtype, device):
 
 
 def gemm_relu_gemm(x, w1, w2, out=None, activation="relu", weight_layout="IO", variant="auto", workspace="auto"):
-    """out = act(x @ w1) @ w2 in one kernel, the hidden activations in a ring that stays in L2 or inside a cluster.
+    """out = act(x @ w1) @ w2, fused: the hidden activations stay in L2 (scratch memory) or inside a cluster.
 
     x [batch, M, K] or [M, K]; w1 [batch, K, L] / [K, L]; w2 [batch, L, N] / [L, N] when
     weight_layout == "IO" ([in, out]); "OI" takes the transposed [out, in] weights of
     nn/functional/linear.py.  activation: "relu" or "identity".  variant: "auto" (by shape), "pair"
-    (eight-CTA clusters of CTA pairs, 2-SM MMAs), "quad" (four-CTA clusters, 128-wide hidden chunks) or "wide"
-    (four-CTA clusters, 256-wide hidden chunks).  workspace: "auto" (this
+    (eight-CTA clusters of CTA pairs, 2-SM MMAs), "quad" (four-CTA clusters, 128-wide hidden chunks), "wide"
+    (four-CTA clusters, 256-wide hidden chunks) or "flow" (one flow of 2-SM tiles over both GEMMs).  workspace: "auto" (this
     call takes ditto_b200_workspace_bytes() of scratch memory from the caching allocator), None (no scratch: the
     hidden layer stays inside a cluster, which is slower) or a uint8 CUDA tensor.
     """
@@ -280,7 +280,7 @@ _ACT_CODE = {"identity": 0, "relu": 1, "gelu": 2}
 
 
 def ffn(x, w1, b1, w2, b2, out=None, act1="relu", act2="relu", weight_layout="OI"):
-    """Position-wise feed-forward block out = act2(act1(x @ W1 + b1) @ W2 + b2) in one kernel.
+    """Position-wise feed-forward block out = act2(act1(x @ W1 + b1) @ W2 + b2), fused.
 
     Defaults follow the reference's PositionwiseFeedForward (nn/model/transformer.py:21-34): weights
     stored [out, in] like nn/functional/linear.py, ReLU after both linears.  x [M, K] or [batch, M, K];

@@ -41,6 +41,7 @@ extern "C" {
 #define DITTO_EPILOGUE_PAIR_MMA 0x200 /* eight-CTA clusters of CTA pairs, 2-SM MMAs */
 #define DITTO_EPILOGUE_QUAD_MMA 0x400 /* four-CTA clusters, single-SM MMAs, 128-wide hidden chunks */
 #define DITTO_EPILOGUE_WIDE_MMA 0x800 /* four-CTA clusters, single-SM MMAs, 256-wide hidden chunks */
+#define DITTO_EPILOGUE_FLOW_MMA 0x1000 /* one flow of 2-SM tiles, hidden tiles through a ring of scratch memory (needed) */
 
 #define DITTO_OP_BMM_SOFTMAX_BMM 0
 #define DITTO_OP_GEMM_RELU_GEMM 1

@@ -1,0 +1,90 @@
+"""The MLP chain's two forms with scratch memory at the sizes where each can go wrong, against float32 products (bounds as
+in the random-shape sweeps): the tile kernel, which small calls take, in all its tile widths, reduction splits and
+epilogues, and the flow kernel, asked for by name at the shapes that small calls no longer bring to it."""
+import pytest
+import torch
+
+from ditto_b200 import _lib, ops
+from tests.test_gpu_mlp_flow import SHAPES
+from tests.test_gpu_random_shapes import _act, _assert_close
+
+pytestmark = pytest.mark.gpu
+
+
+def _operands(cuda, batch, M, N, K, L, dtype, seed):
+    g = torch.Generator(device=cuda).manual_seed(seed)
+    x = torch.randn(batch, M, K, device=cuda, generator=g).to(dtype)
+    w1 = (torch.randn(batch, K, L, device=cuda, generator=g) * K ** -0.5).to(dtype)
+    w2 = (torch.randn(batch, L, N, device=cuda, generator=g) * L ** -0.5).to(dtype)
+    return g, x, w1, w2
+
+
+@pytest.mark.parametrize("layout", ["IO", "OI"])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_flow_kernel_by_name(cuda, dtype, layout):
+    # the last two are large enough for "auto" to take it
+    for batch, M, N, K, L in SHAPES + ((1, 3344, 1280, 1280, 5120), (1, 16400, 512, 512, 2048)):
+        _, x, w1, w2 = _operands(cuda, batch, M, N, K, L, dtype, 41)
+        a1, a2 = (w1, w2) if layout == "IO" else (w1.transpose(1, 2).contiguous(), w2.transpose(1, 2).contiguous())
+        for act in ("relu", "identity"):
+            out = ops.gemm_relu_gemm(x, a1, a2, activation=act, weight_layout=layout, variant="flow")
+            ref = _act(x.float() @ w1.float(), act).to(dtype).float() @ w2.float()
+            _assert_close(out, ref, dtype, (act, batch, M, N, K, L, str(dtype), layout), cuda)
+
+
+@pytest.mark.parametrize("acts", [("gelu", "identity"), ("relu", "relu"), ("relu", "identity"), ("gelu", "relu")])
+def test_flow_kernel_epilogues(cuda, acts):
+    batch, M, N, K, L = 1, 3344, 1280, 1280, 5120
+    g, x, w1, w2 = _operands(cuda, batch, M, N, K, L, torch.bfloat16, 42)
+    b1 = (torch.randn(1, L, device=cuda, generator=g) * 0.5).bfloat16()
+    b2 = (torch.randn(1, N, device=cuda, generator=g) * 0.5).bfloat16()
+    out = ops.ffn(x, w1, b1, w2, b2, act1=acts[0], act2=acts[1], weight_layout="IO")
+    h = _act(x.float() @ w1.float() + b1.float()[:, None], acts[0]).bfloat16().float()
+    _assert_close(out, _act(h @ w2.float() + b2.float()[:, None], acts[1]), torch.bfloat16, acts, cuda)
+
+
+# one k-step in either GEMM; clusters of four and eight; a last tile wider than what is left of the result (256, 192 and
+# 128 columns); two CTAs per SM over several waves; a K tail; batches with partial row blocks
+@pytest.mark.parametrize("shape", [(1, 16, 256, 16, 64), (1, 16, 1024, 1024, 4096), (1, 144, 256, 4096, 128),
+                                   (1, 512, 768, 768, 3072), (1, 2064, 1024, 1024, 4096), (1, 8208, 256, 272, 1088),
+                                   (1, 4096, 768, 768, 3072), (5, 80, 512, 144, 576), (1, 1040, 2048, 512, 2112)])
+@pytest.mark.parametrize("layout", ["IO", "OI"])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_tile_kernel(cuda, shape, layout, dtype):
+    batch, M, N, K, L = shape
+    g, x, w1, w2 = _operands(cuda, batch, M, N, K, L, dtype, 43)
+    a1, a2 = (w1, w2) if layout == "IO" else (w1.transpose(1, 2).contiguous(), w2.transpose(1, 2).contiguous())
+    assert _lib.load().ditto_b200_workspace_bytes(_lib.OP_GEMM_RELU_GEMM, batch, M, N, K, L, 0) == batch * M * L * 2
+    out = ops.gemm_relu_gemm(x, a1, a2, weight_layout=layout)
+    ref = torch.relu(x.float() @ w1.float()).to(dtype).float() @ w2.float()
+    _assert_close(out, ref, dtype, ("chain",) + shape, cuda)
+    assert torch.equal(out, ops.gemm_relu_gemm(x, a1, a2, weight_layout=layout))
+    # biases at addresses that allow 16-byte loads and at such that do not, and one bias missing
+    bias = (torch.randn(batch * (L + N) + 2, device=cuda, generator=g) * 0.5).to(dtype)
+    for b1, b2 in ((bias[:batch * L], bias[batch * L:batch * (L + N)]), (bias[2:2 + batch * L], None),
+                   (None, bias[2:2 + batch * N])):
+        out = ops.ffn(x, a1, b1, a2, b2, act1="gelu", act2="relu", weight_layout=layout)
+        h = x.float() @ w1.float() + (0 if b1 is None else b1.float().view(batch, 1, L))
+        y = _act(h, "gelu").to(dtype).float() @ w2.float() + (0 if b2 is None else b2.float().view(batch, 1, N))
+        _assert_close(out, _act(y, "relu"), dtype, ("ffn",) + shape, cuda)
+
+
+def test_tile_kernel_streams_and_changed_weights(cuda):
+    """The second launch reads its weights ahead of the first one's end: a weight written by the work just ahead in the
+    stream is the one that is used, and calls on two streams have hidden layers of their own."""
+    _, x, w1, w2 = _operands(cuda, 1, 512, 768, 768, 3072, torch.bfloat16, 44)
+    want = [ops.gemm_relu_gemm(x * s, w1 * s, w2 * s) for s in (1.0, 2.0, 0.5)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    got = []
+    for _ in range(10):
+        for st in streams:
+            with torch.cuda.stream(st):
+                a, u, v = torch.empty_like(x), torch.empty_like(w1), torch.empty_like(w2)
+                for i, s in enumerate((1.0, 2.0, 0.5)):
+                    torch.mul(x, s, out=a), torch.mul(w1, s, out=u), torch.mul(w2, s, out=v)
+                    got.append((ops.gemm_relu_gemm(a, u, v), want[i]))
+    torch.cuda.synchronize()
+    assert ops.device_status(cuda) == 0
+    for g, w in got:
+        assert torch.equal(g, w)
