@@ -23,6 +23,7 @@ OP_GEMM_RELU_GEMM = 1
 FLAG_P_VIA_SMEM = 1
 FLAG_ONE_TILE = 2
 FLAG_TWO_TILES = 4
+FLAG_NARROW = 8
 FLAG_SPLIT_UNIT = 256     # 1, 2, 3, 4 of these: 1, 2, 4, 8 CTAs share a tile's keys
 EPILOGUE_PAIR_MMA = 0x200
 EPILOGUE_QUAD_MMA = 0x400

@@ -53,6 +53,13 @@ int parts_for(int flags, bool any, long long batch, int M, int L, int d, int mod
   return parts;
 }
 
+// The kernel with 64-key blocks (head dimensions up to 64): where the caller asks for it, or by shape.
+bool narrow_for(int flags, bool any, long long batch, int M, int L, int d, int mode = 0) {
+  if (!any || d != 64) return false;
+  if (flags & DITTO_FLAG_NARROW) return true;
+  return !(flags & DITTO_FLAG_SPLIT_MASK) && ditto_b200::attention_narrow_pays(static_cast<int>(batch), M, L, mode);
+}
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace
@@ -85,6 +92,10 @@ int ditto_b200_bmm_softmax_bmm(const void* q, const void* k, const void* v, void
   if (d == 64 && !(flags & (DITTO_FLAG_TWO_TILES | DITTO_FLAG_P_VIA_SMEM))) nt = 1;
   const bool psmem = (flags & DITTO_FLAG_P_VIA_SMEM) != 0;
 
+  const bool any = !(flags & (DITTO_FLAG_ONE_TILE | DITTO_FLAG_TWO_TILES | DITTO_FLAG_P_VIA_SMEM));
+  const bool narrow = narrow_for(flags, any, batch, M, L, d);
+  const uint32_t kv_rows = narrow ? 64 : 128;
+
   ditto_b200::AttnParams p;
   std::memset(&p, 0, sizeof(p));
   const uint64_t uK = K, uM = M, uL = L, ub = batch;
@@ -93,10 +104,10 @@ int ditto_b200_bmm_softmax_bmm(const void* q, const void* k, const void* v, void
   if (k_layout == 0)
     rc = make_map_3d(&p.map_k, bf16, k, uL, uK, ub, uL, uK * uL, 64, d);
   else
-    rc = make_map_3d(&p.map_k, bf16, k, uK, uL, ub, uK, uL * uK, 64, 128);
+    rc = make_map_3d(&p.map_k, bf16, k, uK, uL, ub, uK, uL * uK, 64, kv_rows);
   if (rc) return rc;
   const uint64_t uN = N;
-  rc = make_map_3d(&p.map_v, bf16, v, uN, uL, ub, uN, uL * uN, 64, 128);
+  rc = make_map_3d(&p.map_v, bf16, v, uN, uL, ub, uN, uL * uN, 64, kv_rows);
   if (rc) return rc;
   p.out = out;
   p.M = M;
@@ -113,10 +124,10 @@ int ditto_b200_bmm_softmax_bmm(const void* q, const void* k, const void* v, void
 #endif
   // head dimensions up to 64 with few key blocks per item take the persistent kernel (it hides the
   // per-item start-up, which long sequences amortise anyway) unless a flag asks for a specific tiling
-  const bool any = !(flags & (DITTO_FLAG_ONE_TILE | DITTO_FLAG_TWO_TILES | DITTO_FLAG_P_VIA_SMEM));
   const bool persistent = any && d == 64 && L <= kPersistentMaxKeys;
   const int parts = parts_for(flags, any, batch, M, L, d);
-  cudaError_t e = parts > 1 ? ditto_b200::launch_attention_split(p, batch, d, bf16, 0, parts, static_cast<cudaStream_t>(stream))
+  cudaError_t e = narrow      ? ditto_b200::launch_attention_narrow(p, batch, bf16, 0, static_cast<cudaStream_t>(stream))
+                  : parts > 1 ? ditto_b200::launch_attention_split(p, batch, d, bf16, 0, parts, static_cast<cudaStream_t>(stream))
                   : persistent
                       ? ditto_b200::launch_attention_persistent(p, batch, bf16, 0, static_cast<cudaStream_t>(stream))
                       : ditto_b200::launch_attention(p, batch, d, bf16, nt, psmem, 0, static_cast<cudaStream_t>(stream));
@@ -137,6 +148,8 @@ int ditto_b200_multi_head_attention(const void* qkv, void* out, int batch, int M
   const int d = head_dim <= 64 ? 64 : 128, hidden = heads * head_dim;
   int nt = (M > 128 && !(flags & DITTO_FLAG_ONE_TILE)) ? 2 : 1;
   if (d == 64 && !(flags & DITTO_FLAG_TWO_TILES)) nt = 1;
+  const bool any = !(flags & (DITTO_FLAG_ONE_TILE | DITTO_FLAG_TWO_TILES));
+  const bool narrow = narrow_for(flags, any, static_cast<long long>(batch) * heads, M, M, d);
   ditto_b200::AttnParams p;
   std::memset(&p, 0, sizeof(p));
   // one tensor map over the packed [batch*M, 3*hidden] matrix serves Q, K and V: the head split and
@@ -144,7 +157,8 @@ int ditto_b200_multi_head_attention(const void* qkv, void* out, int batch, int M
   int rc = make_map_3d(&p.map_q, bf16, qkv, 3ull * hidden, M, batch, 3ull * hidden, 3ull * hidden * M, 64, 128);
   if (rc) return rc;
   p.map_k = p.map_q;
-  p.map_v = p.map_q;
+  if (narrow && (rc = make_map_3d(&p.map_k, bf16, qkv, 3ull * hidden, M, batch, 3ull * hidden, 3ull * hidden * M, 64, 64)) != 0) return rc;
+  p.map_v = p.map_k;
   p.out = out;
   p.M = M;
   p.L = M;
@@ -158,10 +172,10 @@ int ditto_b200_multi_head_attention(const void* qkv, void* out, int batch, int M
   p.out_ld = hidden;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = status_word;
-  const bool any = !(flags & (DITTO_FLAG_ONE_TILE | DITTO_FLAG_TWO_TILES));
   const bool persistent = any && d == 64 && M <= kPersistentMaxKeys;
   const int parts = parts_for(flags, any, batch * heads, M, M, d);
-  cudaError_t e = parts > 1 ? ditto_b200::launch_attention_split(p, batch * heads, d, bf16, 0, parts,
+  cudaError_t e = narrow      ? ditto_b200::launch_attention_narrow(p, batch * heads, bf16, 0, static_cast<cudaStream_t>(stream))
+                  : parts > 1 ? ditto_b200::launch_attention_split(p, batch * heads, d, bf16, 0, parts,
                                                                  static_cast<cudaStream_t>(stream))
                   : persistent ? ditto_b200::launch_attention_persistent(p, batch * heads, bf16, 0,
                                                                        static_cast<cudaStream_t>(stream))
@@ -194,6 +208,9 @@ int ditto_b200_gemm_relu_gemm(const void* x, const void* w1, const void* w2, voi
     const int dk = (K <= 64 && N <= 64) ? 64 : 128;
     ditto_b200::AttnParams p;
     std::memset(&p, 0, sizeof(p));
+    const int mode = act == 1 ? 1 : 2;
+    const bool narrow = narrow_for(0, true, batch, M, L, dk, mode);
+    const uint32_t kv_rows = narrow ? 64 : 128;
     const uint64_t uK = K, uM = M, uL = L, ub = batch;
     int rc = make_map_3d(&p.map_q, bf16, x, uK, uM, ub, uK, uM * uK, 64, 128);
     if (rc) return rc;
@@ -202,10 +219,10 @@ int ditto_b200_gemm_relu_gemm(const void* x, const void* w1, const void* w2, voi
       // [in, out] weights: w1 [K, L] is the reference's transposed-K form, w2 [L, N] the usual V
       rc = make_map_3d(&p.map_k, bf16, w1, uL, uK, ub, uL, uK * uL, 64, dk);
       if (rc) return rc;
-      rc = make_map_3d(&p.map_v, bf16, w2, uN, uL, ub, uN, uL * uN, 64, 128);
+      rc = make_map_3d(&p.map_v, bf16, w2, uN, uL, ub, uN, uL * uN, 64, kv_rows);
     } else {
       // [out, in] weights: w1 [L, K] is K in rows-of-keys form, w2 [N, L] a transposed V (K-major operand of GEMM2)
-      rc = make_map_3d(&p.map_k, bf16, w1, uK, uL, ub, uK, uL * uK, 64, 128);
+      rc = make_map_3d(&p.map_k, bf16, w1, uK, uL, ub, uK, uL * uK, 64, kv_rows);
       if (rc) return rc;
       rc = make_map_3d(&p.map_v, bf16, w2, uL, uN, ub, uL, uN * uL, 64, dk);
     }
@@ -222,9 +239,9 @@ int ditto_b200_gemm_relu_gemm(const void* x, const void* w1, const void* w2, voi
     p.scale_log2 = 1.0f;
     p.status = status_word;
     const int nt = (dk == 64 || M <= 128) ? 1 : 2;
-    const int mode = act == 1 ? 1 : 2;
     const int parts = parts_for(0, true, batch, M, L, dk, mode);
-    cudaError_t e = parts > 1 ? ditto_b200::launch_attention_split(p, batch, dk, bf16, mode, parts, static_cast<cudaStream_t>(stream))
+    cudaError_t e = narrow      ? ditto_b200::launch_attention_narrow(p, batch, bf16, mode, static_cast<cudaStream_t>(stream))
+                    : parts > 1 ? ditto_b200::launch_attention_split(p, batch, dk, bf16, mode, parts, static_cast<cudaStream_t>(stream))
                     : (dk == 64 && L <= kPersistentMaxKeys) ? ditto_b200::launch_attention_persistent(p, batch, bf16, mode, static_cast<cudaStream_t>(stream))
                              : ditto_b200::launch_attention(p, batch, dk, bf16, nt, false, mode,
                                                             static_cast<cudaStream_t>(stream));
@@ -286,12 +303,11 @@ int ditto_b200_ffn(const void* x, const void* w1, const void* b1, const void* w2
 }
 
 size_t ditto_b200_workspace_bytes(int op, int batch, int M, int N, int K, int L, int dtype) {
-  // The attention chain keeps everything on chip.  The MLP chain does too, except that with few row blocks
-  // it runs faster when several clusters share a row block and combine fp32 partials of Y through scratch
-  // memory (the hidden activations still never leave the chip); the call works without it.
+  // The attention chain keeps everything on chip.  The MLP chain runs fastest with its hidden layer, or a ring of
+  // hidden tiles, in scratch memory that stays in L2; without it the hidden layer stays inside a cluster.
   if ((op & 0xff) != DITTO_OP_GEMM_RELU_GEMM || batch <= 0 || M <= 0 || N <= 0 || K <= 0 || L <= 0) return 0;
   if (N <= 128 && K <= 128) return 0;
-  // `op` may carry DITTO_EPILOGUE_PAIR_MMA / DITTO_EPILOGUE_QUAD_MMA like the call's `epilogue` argument
+  // `op` may carry a kernel's DITTO_EPILOGUE_* bit like the call's `epilogue` argument
   const int variant = (op & DITTO_EPILOGUE_PAIR_MMA)   ? ditto_b200::kMlpPair
                       : (op & DITTO_EPILOGUE_QUAD_MMA) ? ditto_b200::kMlpQuad
                       : (op & DITTO_EPILOGUE_WIDE_MMA) ? ditto_b200::kMlpWide

@@ -37,6 +37,12 @@ cudaError_t launch_attention(const AttnParams& p, int batch, int d, bool bf16, i
 // between them and combine on chip.
 cudaError_t launch_attention_split(const AttnParams& p, int batch, int d, bool bf16, int mode, int parts, cudaStream_t stream);
 
+// Head dimensions up to 64 and many items (attention_narrow_sm100.cu): a small CTA an item, 64-key blocks (map_k / map_v
+// boxes of 64 rows).  mode as above.
+cudaError_t launch_attention_narrow(const AttnParams& p, int batch, bool bf16, int mode, cudaStream_t stream);
+// Whether it is expected to be the fastest form for a shape.
+bool attention_narrow_pays(int batch, int M, int L, int mode);
+
 // The number of parts that is expected to be fastest for a shape (1: no split).
 int attention_parts(int batch, int M, int L, int d, int mode);
 

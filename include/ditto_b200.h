@@ -50,6 +50,7 @@ extern "C" {
 #define DITTO_FLAG_P_VIA_SMEM 1   /* stage the probabilities through shared memory instead of TMEM */
 #define DITTO_FLAG_ONE_TILE 2     /* one 128-row query tile per CTA, one CTA per tile (no persistent work loop) */
 #define DITTO_FLAG_TWO_TILES 4    /* two query tiles per CTA even where one is the default (N = K = 64) */
+#define DITTO_FLAG_NARROW 8       /* 64-key blocks, a small CTA per tile (N, K <= 64; ignored beside the flags above) */
 #define DITTO_FLAG_SPLIT_UNIT 256  /* 1, 2, 3, 4 of these: 1, 2, 4, 8 CTAs share a tile's keys (at most one per 128 keys) */
 #define DITTO_FLAG_SPLIT_MASK (7 * DITTO_FLAG_SPLIT_UNIT)   /* not set: by shape.  Ignored beside the flags above */
 
@@ -82,7 +83,7 @@ int ditto_b200_multi_head_attention(const void* qkv, void* out, int batch, int M
  * (benchmark/chimera/cuda/bmm_bmm_cuda.py:69-150).
  *   x [batch, M, K]; w1 [batch, K, L]; w2 [batch, L, N]; y [batch, M, N]
  *   w_layout 0: weights as above ([in, out]); 1: [out, in] as in nn/functional/linear.py:4-41
- *   epilogue 0: identity between the GEMMs; 1: ReLU; | DITTO_EPILOGUE_PAIR_MMA / _QUAD_MMA / _WIDE_MMA
+ *   epilogue 0: identity between the GEMMs; 1: ReLU; | DITTO_EPILOGUE_PAIR_MMA / _QUAD_MMA / _WIDE_MMA / _FLOW_MMA
  *   forces one of the kernels (same results up to fp32 summation order; default: by shape)
  *   workspace / ws_bytes: optional scratch memory (ditto_b200_workspace_bytes; contents irrelevant on entry,
  *   undefined on return).  With it the hidden activations pass through a ring of a few row blocks (at most about
@@ -134,14 +135,14 @@ int ditto_b200_ffn(const void* x, const void* w1, const void* b1, const void* w2
                    void* stream);
 
 /* ditto_b200_ffn with scratch memory (ditto_b200_workspace_bytes with DITTO_OP_GEMM_RELU_GEMM; contents irrelevant on
- * entry, undefined on return): the hidden layer then passes through a small ring in it that stays in L2, which
- * is the faster form at every size.  NULL or too small: as ditto_b200_ffn. */
+ * entry, undefined on return): the hidden layer, or a ring of its tiles, then stays in L2 there, which is the
+ * faster form at every size.  NULL or too small: as ditto_b200_ffn. */
 int ditto_b200_ffn_ws(const void* x, const void* w1, const void* b1, const void* w2, const void* b2, void* y, int batch,
                       int M, int N, int K, int L, int dtype, int w_layout, int act1, int act2, void* workspace,
                       size_t ws_bytes, int* status_word, void* stream);
 
 /* Scratch bytes with which the op runs fastest at this shape on the current device (0 when none; every call
- * also works without).  `op` may be or-ed with DITTO_EPILOGUE_PAIR_MMA / DITTO_EPILOGUE_QUAD_MMA / DITTO_EPILOGUE_WIDE_MMA to ask for the
+ * also works without).  `op` may be or-ed with DITTO_EPILOGUE_PAIR_MMA / _QUAD_MMA / _WIDE_MMA / _FLOW_MMA to ask for the
  * kernel that the same bits in `epilogue` select. */
 size_t ditto_b200_workspace_bytes(int op, int batch, int M, int N, int K, int L, int dtype);
 

@@ -1,0 +1,90 @@
+"""The attention kernel with 64-key blocks (head dimensions up to 64), against float64 products of the same 16-bit operands:
+one to many blocks, partial last blocks, row tails, widths below 64, both layouts and types, packed heads, the chains
+without a softmax, growing maxima and scores of -inf; and large calls, which take it by themselves."""
+import pytest
+import torch
+
+from ditto_b200 import _lib, ops
+from tests.test_gpu_attention_split import _close, _reference
+
+pytestmark = pytest.mark.gpu
+
+NARROW = _lib.FLAG_NARROW
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("b,M,N,K,L,layout", [
+    (3, 128, 64, 64, 64, "LK"),        # one block
+    (2, 144, 64, 64, 16, "KL"),        # a block of 16 keys, a row tail
+    (3, 16, 64, 64, 128, "LK"),        # two blocks: no stage is refilled
+    (2, 208, 64, 64, 208, "KL"),       # four, the last of 16 keys
+    (1, 272, 48, 16, 1168, "LK"),      # widths below 64
+    (2, 128, 16, 64, 320, "KL"),
+    (40, 2048, 64, 64, 80, "LK"),      # more CTAs than the device holds at once
+])
+def test_shapes(dtype, b, M, N, K, L, layout):
+    g = torch.Generator(device="cuda").manual_seed(b * M + L)
+    q = torch.randn(b, M, K, generator=g, device="cuda").to(dtype)
+    k = torch.randn(b, L, K, generator=g, device="cuda").to(dtype)
+    v = torch.randn(b, L, N, generator=g, device="cuda").to(dtype)
+    keys = k if layout == "LK" else k.transpose(1, 2).contiguous()
+    out = ops.bmm_softmax_bmm(q, keys, v, scale=2 * K ** -0.5, key_layout=layout, flags=NARROW)
+    assert ops.device_status() == 0
+    _close(out, _reference(q, k, v, 2 * K ** -0.5), dtype)
+    assert torch.equal(out, ops.bmm_softmax_bmm(q, keys, v, scale=2 * K ** -0.5, key_layout=layout, flags=NARROW))
+
+
+def test_growing_maxima_and_infinite_scores():
+    g = torch.Generator(device="cuda").manual_seed(6)
+    b, M, d, L = 1, 128, 64, 512
+    q = (torch.rand(b, M, d, generator=g, device="cuda") + 0.5).bfloat16()
+    v = torch.randn(b, L, d, generator=g, device="cuda").bfloat16()
+    k = torch.randn(b, L, d, generator=g, device="cuda").bfloat16()
+    k = (k.float() * (1 + torch.arange(L, device="cuda")[None, :, None] / 40)).bfloat16()      # the maximum grows past the rescale threshold
+    _close(ops.bmm_softmax_bmm(q, k, v, scale=0.5, key_layout="LK", flags=NARROW), _reference(q, k, v, 0.5), torch.bfloat16)
+    for lo, hi in ((0, 64), (128, 512)):               # q is positive: scores of -inf for whole blocks, the first or the last
+        ki = k.clone()
+        ki[:, lo:hi] = float("-inf")
+        rest = [i for i in range(L) if not lo <= i < hi]
+        _close(ops.bmm_softmax_bmm(q, ki, v, scale=0.25, key_layout="LK", flags=NARROW),
+               _reference(q, k[:, rest], v[:, rest], 0.25), torch.bfloat16)
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("heads,d,M", [(4, 64, 1040), (3, 48, 80)])
+def test_packed_heads(heads, d, M):
+    g = torch.Generator(device="cuda").manual_seed(M)
+    qkv = torch.randn(2, M, 3 * heads * d, generator=g, device="cuda").half()
+    out = ops.multi_head_attention(qkv, heads, scale=d ** -0.5, flags=NARROW)
+    assert ops.device_status() == 0
+    for i in range(2):
+        q, k, v = (t.reshape(M, heads, d).transpose(0, 1) for t in qkv[i].chunk(3, dim=-1))
+        _close(out[i], _reference(q, k, v, d ** -0.5).transpose(0, 1).reshape(M, heads * d), torch.float16)
+
+
+@pytest.mark.parametrize("act", ["identity", "relu"])
+@pytest.mark.parametrize("layout", ["IO", "OI"])
+@pytest.mark.parametrize("b,M,N,K,L", [(600, 144, 64, 64, 208), (300, 512, 32, 48, 256), (320, 16, 64, 64, 64)])
+def test_many_items_of_a_chain(act, layout, b, M, N, K, L):
+    g = torch.Generator(device="cuda").manual_seed(M + L)
+    x = torch.randn(b, M, K, generator=g, device="cuda").half()
+    w1 = (torch.randn(b, K, L, generator=g, device="cuda") * K ** -0.5).half()
+    w2 = (torch.randn(b, L, N, generator=g, device="cuda") * L ** -0.5).half()
+    h = x.float() @ w1.float()
+    want = ((h.relu() if act == "relu" else h).half().float() @ w2.float()).double()
+    ws = (w1, w2) if layout == "IO" else (w1.transpose(1, 2).contiguous(), w2.transpose(1, 2).contiguous())
+    out = ops.gemm_relu_gemm(x, *ws, activation=act, weight_layout=layout)
+    assert ops.device_status() == 0
+    _close(out, want, torch.float16)
+
+
+@pytest.mark.parametrize("b,M,L", [(20, 2048, 2048), (320, 128, 512), (150, 512, 208), (60, 2048, 2064)])
+def test_many_items(b, M, L):
+    g = torch.Generator(device="cuda").manual_seed(b)
+    q = torch.randn(b, M, 64, generator=g, device="cuda").half()
+    k = torch.randn(b, L, 64, generator=g, device="cuda").half()
+    v = torch.randn(b, L, 64, generator=g, device="cuda").half()
+    out = ops.bmm_softmax_bmm(q, k, v, scale=0.125, key_layout="LK")
+    assert ops.device_status() == 0
+    for i in range(0, b, 7):
+        _close(out[i:i + 1], _reference(q[i:i + 1], k[i:i + 1], v[i:i + 1], 0.125), torch.float16)
