@@ -19,6 +19,7 @@
 
 #include "mlp_common.cuh"
 #include "sm100_ptx.cuh"
+#include "softmax_step.cuh"
 
 namespace ditto_b200 {
 
@@ -171,7 +172,8 @@ __global__ void __launch_bounds__(kThreads, 4) attention_narrow_kernel(const __g
     // ------------------------------------------------------------ softmax and write-out
     const uint32_t s_col = tmem_base + (static_cast<uint32_t>(warp * 32) << 16), o_col = s_col + kColO;
     const float c = p.scale_log2;
-    float m = -INFINITY, l = 0.f;
+    RowReference ref;
+    float l = 0.f;
     bool ok = true;
     for (int g = 0; g < nkv; ++g) {
       ok = mbar_wait(&bar->s_full, g & 1, abort_word, 0x800);
@@ -197,11 +199,10 @@ __global__ void __launch_bounds__(kThreads, 4) attention_narrow_kernel(const __g
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) mx[u] = fmaxf(mx[u], mx[u + 4]);
-        const float m_new = fmaxf(fmaxf(m, mx[0]), fmaxf(fmaxf(mx[1], mx[2]), mx[3]));
+        const float m_new = fmaxf(fmaxf(ref.m, mx[0]), fmaxf(fmaxf(mx[1], mx[2]), mx[3]));
         // lazy rescale, as in attention_sm100.cu; s_full(g) implies that P*V(g - 1) is done, so O is quiescent
-        const bool need = (m_new - m) * c > kRescaleThreshold;
-        if (__any_sync(0xffffffffu, need)) {
-          const float f = ex2_approx((m - m_new) * c);
+        if (__any_sync(0xffffffffu, ref.asks(m_new, c, kRescaleThreshold))) {
+          const float f = ref.move(m_new, c);
           if (g > 0) {
 #pragma unroll 1
             for (int cc = 0; cc < kD; cc += 16) {
@@ -214,11 +215,9 @@ __global__ void __launch_bounds__(kThreads, 4) attention_narrow_kernel(const __g
             tmem_wait_st();
           }
           l *= f;
-          m = m_new;
+          ref.subtract(sv);
         }
       }
-      // (blocks without one finite score so far contribute nothing: the first ones of a row, half as long as elsewhere)
-      const float mc = m == -INFINITY ? 0.f : m * c;
       float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -227,8 +226,8 @@ __global__ void __launch_bounds__(kThreads, 4) attention_narrow_kernel(const __g
         for (int i = 0; i < 16; ++i) {
           float p0 = __uint_as_float(sv[32 * h + 2 * i]), p1 = __uint_as_float(sv[32 * h + 2 * i + 1]);
           if constexpr (MODE == kModeSoftmax) {
-            p0 = ex2_approx(fmaf(p0, c, -mc));
-            p1 = ex2_approx(fmaf(p1, c, -mc));
+            p0 = ex2_approx(fmaf(p0, c, -ref.mc));
+            p1 = ex2_approx(fmaf(p1, c, -ref.mc));
             sum0 += p0;
             sum1 += p1;
           } else if constexpr (MODE == kModeRelu) {

@@ -1,0 +1,50 @@
+// The running maximum of a softmax row, as the attention kernels use it.
+#pragma once
+#include <cstdint>
+
+#include "sm100_ptx.cuh"
+
+namespace ditto_b200 {
+
+// Up to this |m * c| the exponent of a score s is one fused multiply-add, s * c - mc: rounding mc = m * c moves all of a row's
+// exponents by at most 2^-13, which is below the rounding of the 16-bit probabilities.
+constexpr float kFusedReference = 4096.0f;
+
+// m is the (possibly stale) maximum that a row's exponentials refer to, c = scale * log2(e): a score's weight is
+// ex2(fmaf(s, c, -mc)), at most 2^(rescale threshold).
+//
+// Rows whose reference is large -- -inf as long as there is no finite score, or a mask of the type's lowest value that fills all
+// blocks so far -- have it subtracted from their scores instead (mc = 0): the rounding error of m * c alone could be an
+// exponent beyond the range (it is 2^101 at the lowest float32), and the infinity that comes of it, or the NaN of
+// (-inf) - (-inf), stays in the row's sum however small the row's weight becomes later.  Such rows join the vote on
+// rescaling at every block; where there are none it costs a block nothing.
+struct RowReference {
+  float m = -INFINITY, mc = 0.0f;
+  bool large = true;
+
+  // Whether this row asks its warp to rescale, given the maximum up to and including the present block.
+  __device__ __forceinline__ bool asks(float m_new, float c, float threshold) const {
+    return large || (m_new - m) * c > threshold;
+  }
+  // Moves the reference to m_new and returns the factor for what the row has accumulated.  A row whose reference stays gets
+  // exactly 1: a warp rescales together, and without a finite score yet the difference is NaN.
+  __device__ __forceinline__ float move(float m_new, float c) {
+    const float f = m_new == m ? 1.0f : ex2_approx((m - m_new) * c);
+    m = m_new;
+    mc = m * c;
+    large = !(fabsf(mc) <= kFusedReference);
+    return f;
+  }
+  // Behind move, by the whole warp: the present block's scores of rows with a large reference.
+  template <int N>
+  __device__ __forceinline__ void subtract(uint32_t (&s)[N]) {
+    if (__any_sync(0xffffffffu, large)) {
+      const float ref = large && m != -INFINITY ? m : 0.0f;      // (scores of -inf stay what they are)
+#pragma unroll
+      for (int i = 0; i < N; ++i) s[i] = __float_as_uint(__uint_as_float(s[i]) - ref);
+      if (large) mc = 0.0f;
+    }
+  }
+};
+
+}  // namespace ditto_b200

@@ -1,0 +1,59 @@
+"""Rows of one warp that differ in where their scores are -inf or near the lowest float32, against float64: every form of the
+attention kernel has to give the softmax over the keys that are left, wherever its blocks and parts begin.
+
+The mask travels in one column of the head: q there is a for the rows that are masked and 0 for the others, k there is b for the
+keys that are masked and 0 for the others, so a masked score is a * b plus a few units."""
+import pytest
+import torch
+
+from ditto_b200 import _lib, ops
+from tests.test_gpu_attention_split import _close, _reference
+
+pytestmark = pytest.mark.gpu
+
+FORMS = {"narrow": _lib.FLAG_NARROW}
+# masked keys of 512: less than a block, whole blocks at the start, in the middle and at the end, whole parts, all but a few
+MASKED = ((0, 64), (0, 128), (64, 192), (128, 256), (256, 384), (0, 256), (256, 512), (0, 496), (16, 512))
+# a, b, type: a product that overflows float32 to -inf; the lowest values of the two types; large ones that a float32 can tell apart
+VALUES = ((1e30, -1e30, torch.bfloat16), (1.0, torch.finfo(torch.bfloat16).min, torch.bfloat16), (1.0, -1e30, torch.bfloat16),
+          (1.0, torch.finfo(torch.float16).min, torch.float16))
+
+
+@pytest.mark.parametrize("a,b,dtype", VALUES)
+@pytest.mark.parametrize("form,d", [(f, d) for f in FORMS for d in (64, 128) if d == 64 or f != "narrow"])
+def test_rows_masked_apart(form, d, a, b, dtype):
+    g = torch.Generator(device="cuda").manual_seed(11)
+    M, L = 160, 512
+    for scale in (d ** -0.5, 2.0):
+        q = torch.randn(1, M, d, generator=g, device="cuda")
+        k = torch.randn(1, L, d, generator=g, device="cuda")
+        if scale > 1:
+            q *= 0.25
+        v = torch.randn(1, L, d, generator=g, device="cuda").to(dtype)
+        masked_rows = torch.arange(M, device="cuda") % 3 == 1
+        q[:, :, 5] = torch.where(masked_rows, a, 0.0)
+        q = q.to(dtype)
+        for lo, hi in MASKED:
+            kk = k.clone()
+            kk[:, :, 5] = 0.0
+            kk[:, lo:hi, 5] = b
+            kk = kk.to(dtype)
+            out = ops.bmm_softmax_bmm(q, kk, v, scale=scale, key_layout="LK", flags=FORMS[form])
+            _close(out, _reference(q, kk, v, scale), dtype)
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("form,d", [(f, d) for f in FORMS for d in (64, 128) if d == 64 or f != "narrow"])
+def test_row_without_a_finite_score(form, d):
+    """0 / 0 as in torch.softmax -- in that row alone."""
+    g = torch.Generator(device="cuda").manual_seed(12)
+    q = torch.randn(1, 128, d, generator=g, device="cuda")
+    k = torch.randn(1, 512, d, generator=g, device="cuda")
+    q[:, :, 5] = torch.where(torch.arange(128, device="cuda") == 40, 1e30, 0.0)
+    k[:, :, 5] = -1e30
+    q, k = q.bfloat16(), k.bfloat16()
+    v = torch.randn(1, 512, d, generator=g, device="cuda").bfloat16()
+    out = ops.bmm_softmax_bmm(q, k, v, scale=0.125, key_layout="LK", flags=FORMS[form])
+    assert out[:, 40].isnan().all()
+    keep = [i for i in range(128) if i != 40]
+    _close(out[:, keep], _reference(q[:, keep], k, v, 0.125), torch.bfloat16)
