@@ -37,7 +37,14 @@ constexpr int kSmemBytes = kOffBar + 128 + 1024;
 constexpr int kThreads = 160;
 constexpr uint32_t kTmemCols = 128;
 constexpr uint32_t kColO = 64;
-constexpr float kRescaleThreshold = 8.0f;  // log2 units, as in attention_sm100.cu
+// How far (log2 units) a row's maximum may run ahead of its reference.  The largest weights decide a row's rounding error: one that
+// the reference was taken from is exactly 1, one above a stale reference is rounded like any other.  With blocks half as
+// long as in the other kernels the reference is stale more often, so it has to follow more closely: nearly always at the
+// second block (with the first, the other kernels' first block), within 5 later (8 there).  Error against float64, other
+// kernels / this one with 8 throughout / this one: 2.88e-4 / 2.90e-4 / 2.88e-4 for fp16 rows of 512 keys at
+// scale d^-0.5, 2.19e-4 / 2.28e-4 / 2.15e-4 unscaled; 144 keys at 0.35, simulated, 2.33e-4 / 2.60e-4 / 2.29e-4.
+// The price is about one rescale an item, 56.4 -> 58.2 us for 2048 items of 512 keys.
+constexpr float kRescaleThreshold = 5.0f, kSecondBlockThreshold = 1.0f;
 constexpr int kModeSoftmax = 0, kModeRelu = 1;
 
 struct NBars {
@@ -201,7 +208,7 @@ __global__ void __launch_bounds__(kThreads, 4) attention_narrow_kernel(const __g
         for (int u = 0; u < 4; ++u) mx[u] = fmaxf(mx[u], mx[u + 4]);
         const float m_new = fmaxf(fmaxf(ref.m, mx[0]), fmaxf(fmaxf(mx[1], mx[2]), mx[3]));
         // lazy rescale, as in attention_sm100.cu; s_full(g) implies that P*V(g - 1) is done, so O is quiescent
-        if (__any_sync(0xffffffffu, ref.asks(m_new, c, kRescaleThreshold))) {
+        if (__any_sync(0xffffffffu, ref.asks(m_new, c, g == 1 ? kSecondBlockThreshold : kRescaleThreshold))) {
           const float f = ref.move(m_new, c);
           if (g > 0) {
 #pragma unroll 1
@@ -324,19 +331,20 @@ cudaError_t launch_attention_narrow(const AttnParams& p, int batch, bool bf16, i
   return bf16 ? launch_n<true, 2>(p, items, stream) : launch_n<false, 2>(p, items, stream);
 }
 
-// Where the lines lie: up to four 128-key blocks an item this is the faster form as soon as most SMs have one, up to eight
-// with more items than the other kernels hold at once (296); for longer items the other kernels' 128-key blocks cost less
-// (1.6 us for two a SM against 2 x 1.0), and it pays again once a launch is three waves of those or more.  Measured, us,
-// others -> this kernel: 2048 items of 512 keys 70 -> 57; 1200 of 208 30 -> 23.8; 1000 of 128 17.6 -> 13.7; 640 of 64 14.1 -> 8.6;
-// 384 of 512 21.2 -> 18.3; 144 of 512 10.6 -> 10.2; 350 of 1024 34.8 -> 32.5; 1024 of 8192 381 -> 357; and left alone: 48 of 512
-// 9.0 -> 9.8, 128 of 2048 23.8 -> 30.4, 384 of 2048 51.7 -> 56.8, 320 of 8192 179 -> 209.  A chain without a softmax has less
-// between the hand-overs: it gains with one or two blocks and many items only (600 x 208 rows and keys 19.4 -> 18.0, 640 of 64
-// 9.4 -> 7.4; 640 of 1024 would go 40 -> 43, 144 of 512 7.4 -> 8.6).
+// Where the lines lie: up to three 128-key blocks an item this is the faster form as soon as most SMs have one, with four as
+// soon as some SMs have two, up to eight with more items than the other kernels hold at once (296) and a half-full wave of
+// them; for longer items the other kernels' 128-key blocks cost less (1.6 us for two a SM against 2 x 1.0), and it pays again
+// once a launch is three waves of those or more.  Measured, us, others -> this kernel: 2048 items of 512 keys 74.8 -> 63.2; 1200
+// of 208 30.0 -> 25.0; 1000 of 128 17.5 -> 14.4; 640 of 64 13.9 -> 8.8; 384 of 512 20.7 -> 18.4; 180 of 512 12.0 -> 12.0; 110 of 208
+// 7.5 -> 7.1; 400 of 1024 36.2 -> 32.2; 1024 of 8192 393 -> 368; and left alone: 48 of 512 9.0 -> 9.8, 144 of 512 10.4 -> 10.6,
+// 320 of 1024 30.2 -> 31.8, 128 of 2048 23.8 -> 30.4, 384 of 2048 51.7 -> 56.8, 320 of 8192 179 -> 209.  A chain without a softmax
+// has less between the hand-overs: it gains with one or two blocks and many items only (600 x 208 rows and keys 19.4 -> 18.0,
+// 640 of 64 9.4 -> 7.4; 640 of 1024 would go 40 -> 43, 144 of 512 7.4 -> 8.6).
 bool attention_narrow_pays(int batch, int M, int L, int mode) {
   const long long items = static_cast<long long>((M + kBM - 1) / kBM) * batch;
   const int blocks = (L + 127) / 128;
   if (mode != kModeSoftmax) return blocks <= 2 && items > 296;
-  return items > (blocks <= 4 ? 100 : blocks <= 8 ? 296 : 887);
+  return items > (blocks <= 3 ? 100 : blocks == 4 ? 148 : blocks <= 8 ? 349 : 887);
 }
 
 }  // namespace ditto_b200
