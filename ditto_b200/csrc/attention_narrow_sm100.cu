@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(kThreads, 4) attention_narrow_kernel(const __g
     // ------------------------------------------------------------ softmax and write-out
     const uint32_t s_col = tmem_base + (static_cast<uint32_t>(warp * 32) << 16), o_col = s_col + kColO;
     const float c = p.scale_log2;
-    RowReference ref;
+    RowReference ref(c);
     float l = 0.f;
     bool ok = true;
     for (int g = 0; g < nkv; ++g) {
@@ -225,6 +225,7 @@ __global__ void __launch_bounds__(kThreads, 4) attention_narrow_kernel(const __g
           ref.subtract(sv);
         }
       }
+      const float mc = ref.offset(c);
       float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -233,8 +234,8 @@ __global__ void __launch_bounds__(kThreads, 4) attention_narrow_kernel(const __g
         for (int i = 0; i < 16; ++i) {
           float p0 = __uint_as_float(sv[32 * h + 2 * i]), p1 = __uint_as_float(sv[32 * h + 2 * i + 1]);
           if constexpr (MODE == kModeSoftmax) {
-            p0 = ex2_approx(fmaf(p0, c, -ref.mc));
-            p1 = ex2_approx(fmaf(p1, c, -ref.mc));
+            p0 = ex2_approx(fmaf(p0, c, -mc));
+            p1 = ex2_approx(fmaf(p1, c, -mc));
             sum0 += p0;
             sum1 += p1;
           } else if constexpr (MODE == kModeRelu) {

@@ -43,6 +43,7 @@
 #include <cuda_fp16.h>
 
 #include "sm100_ptx.cuh"
+#include "softmax_step.cuh"
 
 // 1: the softmax evaluates its exponentials two at a time on packed 16-bit arguments (see ex2_packed)
 #ifndef DITTO_PACKED_EX2
@@ -501,7 +502,8 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
     uint32_t par = 0;                       // parity of the K/V blocks of all items so far: the phase of s_full / p_part
 
     for (int k = 0; k < my_items && ok; ++k) {
-    float m = -INFINITY, l = 0.f;
+    std::conditional_t<SPLIT, RowReference, PlainReference> ref(c);
+    float l = 0.f;
     for (int j = 0; j < nkv; ++j, par ^= 1u) {
       ok = mbar_wait(&bar->s_full[t], par, abort_word, 0x800 + j);
       ok = __all_sync(0xffffffffu, ok);
@@ -517,7 +519,7 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
       }
       if ((warp & 3) == 0) DITTO_STAMP(t * 256, k * nkv + j, 1);
 
-      float m_new = m;
+      float m_new = ref.m;
       if constexpr (MODE == kModeSoftmax) {
         if (j0 + j == nkv_all - 1 && (p.L % kBN) != 0) {
           // partial last block: K rows >= L were zero-filled, their scores must not count
@@ -538,7 +540,7 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
         for (int u = 0; u < 8; ++u) mx[u] = fmaxf(mx[u], mx[u + 8]);
 #pragma unroll
         for (int u = 0; u < 4; ++u) mx[u] = fmaxf(mx[u], mx[u + 4]);
-        m_new = fmaxf(fmaxf(m, mx[0]), fmaxf(fmaxf(mx[1], mx[2]), mx[3]));
+        m_new = fmaxf(fmaxf(ref.m, mx[0]), fmaxf(fmaxf(mx[1], mx[2]), mx[3]));
       }
       if constexpr (kSep) {
         if (j > 0) {
@@ -552,9 +554,9 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
       }
       // Lazy rescale: keep the stale maximum while the true one is within
       // 2^kRescaleThreshold of it; the final division by l cancels the difference.
-      const bool need = MODE == kModeSoftmax && (m_new - m) * c > kRescaleThreshold;
+      const bool need = MODE == kModeSoftmax && ref.asks(m_new, c, kRescaleThreshold);
       if (MODE == kModeSoftmax && __any_sync(0xffffffffu, need)) {
-        const float f = ex2_approx((m - m_new) * c);
+        const float f = ref.move(m_new, c);
         if (j > 0) {
           // s_full(j) was committed after P*V(j-1) by the same thread and a commit covers every
           // earlier MMA, so the accumulator is quiescent here.
@@ -569,12 +571,11 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
           tmem_wait_st();
         }
         l *= f;
-        m = m_new;
+        ref.subtract(sv);
       }
 
       if ((warp & 3) == 0) DITTO_STAMP(t * 256, k * nkv + j, 2);
-      // a part whose scores so far are all -inf contributes nothing (another part may have finite ones)
-      const float mc = SPLIT && m == -INFINITY ? 0.f : m * c;
+      const float mc = ref.offset(c);
       float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
       for (int part = 0; part < 2; ++part) {
@@ -650,7 +651,7 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
     tc_fence_after_sync();
     if ((warp & 3) == 0) DITTO_STAMP(t * 256, k * nkv + nkv - 1, 12);
     if constexpr (SPLIT) {
-      row_m = m;
+      row_m = ref.m;
       row_l = l;
     } else {
       const Item it = decode(k);
