@@ -20,6 +20,7 @@
 #include <cuda_fp16.h>
 
 #include "sm100_ptx.cuh"
+#include "softmax_step.cuh"
 
 // 1: the softmax evaluates its exponentials two at a time on packed 16-bit arguments (see ex2_packed)
 #ifndef DITTO_PACKED_EX2
@@ -275,7 +276,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_persistent_kernel(const
       const int seq = slice / p.heads;
       const int head_col = (slice % p.heads) * p.d;
       const int m0 = (item % tiles) * kBM;
-      float m = -INFINITY, l = 0.f;
+      PlainReference ref(c);
+      float l = 0.f;
       for (int j = 0; j < nkv; ++j, ++g) {
         ok = mbar_wait(&bar->s_full, g & 1, abort_word, 0x800);
         ok = __all_sync(0xffffffffu, ok);
@@ -287,7 +289,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_persistent_kernel(const
         tc_fence_before_sync();
         mbar_arrive(&bar->s_taken);                // the S columns may be overwritten by the next S
 
-        float m_new = m;
+        float m_new = ref.m;
         if constexpr (MODE == kModeSoftmax) {
           if (j == nkv - 1 && (p.L % kBN) != 0) {
             const int valid = p.L % kBN;           // partial last block: zero-filled K rows must not count
@@ -307,7 +309,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_persistent_kernel(const
           for (int u = 0; u < 8; ++u) mx[u] = fmaxf(mx[u], mx[u + 8]);
 #pragma unroll
           for (int u = 0; u < 4; ++u) mx[u] = fmaxf(mx[u], mx[u + 4]);
-          m_new = fmaxf(fmaxf(m, mx[0]), fmaxf(fmaxf(mx[1], mx[2]), mx[3]));
+          m_new = fmaxf(fmaxf(ref.m, mx[0]), fmaxf(fmaxf(mx[1], mx[2]), mx[3]));
         }
         DITTO_STAMP(1024 + it * 16 + j);
         if (g > 0) {
@@ -318,9 +320,9 @@ __global__ void __launch_bounds__(kThreads, 2) attention_persistent_kernel(const
           tc_fence_after_sync();
         }
         DITTO_STAMP(it * 16 + 8 + j);
-        const bool need = MODE == kModeSoftmax && (m_new - m) * c > kRescaleThreshold;
+        const bool need = MODE == kModeSoftmax && ref.asks(m_new, c, kRescaleThreshold);
         if (MODE == kModeSoftmax && __any_sync(0xffffffffu, need)) {
-          const float f = ex2_approx((m - m_new) * c);
+          const float f = ref.move(m_new, c);
           if (j > 0) {
 #pragma unroll
             for (int cc = 0; cc < kD; cc += 32) {
@@ -333,9 +335,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_persistent_kernel(const
             tmem_wait_st();
           }
           l *= f;
-          m = m_new;
         }
-        const float mc = m * c;
+        const float mc = ref.offset(c);
         float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
         for (int part = 0; part < 2; ++part) {

@@ -11,7 +11,9 @@ from tests.test_gpu_attention_split import _close, _reference
 
 pytestmark = pytest.mark.gpu
 
-FORMS = {"narrow": _lib.FLAG_NARROW, "split 2": 2 * _lib.FLAG_SPLIT_UNIT, "split 4": 3 * _lib.FLAG_SPLIT_UNIT}
+FORMS = {"narrow": _lib.FLAG_NARROW, "split 2": 2 * _lib.FLAG_SPLIT_UNIT, "split 4": 3 * _lib.FLAG_SPLIT_UNIT,
+         "whole": _lib.FLAG_SPLIT_UNIT, "one tile": _lib.FLAG_ONE_TILE, "two tiles": _lib.FLAG_TWO_TILES,
+         "P via smem": _lib.FLAG_P_VIA_SMEM}
 # masked keys of 512: less than a block, whole blocks at the start, in the middle and at the end, whole parts, all but a few
 MASKED = ((0, 64), (0, 128), (64, 192), (128, 256), (256, 384), (0, 256), (256, 512), (0, 496), (16, 512))
 # a, b, type: a product that overflows float32 to -inf; the lowest values of the two types; large ones that a float32 can tell apart
