@@ -88,6 +88,16 @@ bool shape_is(const at::Tensor& t, int64_t a, int64_t b, int64_t c) {
   return t.dim() == 3 && t.size(0) == a && t.size(1) == b && t.size(2) == c;
 }
 
+// Lets other Python threads run: around allocations and launches, which can block (a full launch queue, cudaMalloc, a queue that
+// waits for a Python host callback).  Everything taken from Python objects -- addresses, shapes, texts -- is read before.
+struct WithoutLock {
+  PyThreadState* state = PyEval_SaveThread();
+  WithoutLock() = default;
+  WithoutLock(const WithoutLock&) = delete;
+  WithoutLock& operator=(const WithoutLock&) = delete;
+  ~WithoutLock() { PyEval_RestoreThread(state); }
+};
+
 // Runs `body` and returns what it returns; None for nullptr or an exception.
 template <class F>
 PyObject* guarded(F body) {
@@ -100,19 +110,34 @@ PyObject* guarded(F body) {
   Py_RETURN_NONE;
 }
 
-// The result: `given` if it is a tensor of the right shape, else a new one.  `hold` owns the new one.
-const at::Tensor* result(PyObject* given, Common& c, at::IntArrayRef shape, at::Tensor& hold) {
-  if (given == Py_None) {
-    hold = make(shape, c.type, c.device);
-    return &hold;
+// The result: `given`, checked by the caller, or a new tensor.
+class Result {
+ public:
+  Result(PyObject* given, const at::Tensor* t) : given_(given), address_(t ? t->data_ptr() : nullptr) {}
+  // its address; allocates a new one (without the lock)
+  void* address(const Common& c, at::IntArrayRef shape) {
+    if (given_ != Py_None) return address_;
+    fresh_ = make(shape, c.type, c.device);
+    return fresh_.data_ptr();
   }
-  const at::Tensor* t = take(given, c);
-  return t != nullptr && t->sizes() == shape ? t : nullptr;
-}
-PyObject* give(PyObject* given, const at::Tensor& hold) {
-  if (given == Py_None) return THPVariable_Wrap(hold);
-  Py_INCREF(given);
-  return given;
+  PyObject* give() {
+    if (given_ == Py_None) return THPVariable_Wrap(fresh_);
+    Py_INCREF(given_);
+    return given_;
+  }
+
+ private:
+  PyObject* given_;
+  void* address_;
+  at::Tensor fresh_;
+};
+
+// Whether `given` can be the result; `t` is the tensor behind it (null for None).
+bool result_ok(PyObject* given, Common& c, at::IntArrayRef shape, const at::Tensor** t) {
+  *t = nullptr;
+  if (given == Py_None) return true;
+  *t = take(given, c);
+  return *t != nullptr && (*t)->sizes() == shape;
 }
 
 // softmax(query, key, value, out, scale, key_layout, flags)
@@ -131,13 +156,18 @@ PyObject* py_softmax(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const double scale = PyFloat_AsDouble(a[4]);
     const long flags = PyLong_AsLong(a[6]);
     if (PyErr_Occurred() || flags < INT_MIN || flags > INT_MAX) return nullptr;
-    at::Tensor hold;
-    const at::Tensor* out = result(a[3], c, {b, M, N}, hold);
-    if (out == nullptr) return nullptr;
-    if (g_softmax(q->data_ptr(), k->data_ptr(), v->data_ptr(), out->data_ptr(), b, M, N, K, L, c.code, layout,
-                  static_cast<float>(scale), static_cast<int>(flags), nullptr, 0, g_status[c.device], stream_of(c.device)) != 0)
-      return nullptr;
-    return give(a[3], hold);
+    const int64_t shape[3] = {b, M, N};
+    const at::Tensor* given;
+    if (!result_ok(a[3], c, shape, &given)) return nullptr;
+    const void *qp = q->data_ptr(), *kp = k->data_ptr(), *vp = v->data_ptr();
+    Result out(a[3], given);
+    int rc;
+    {
+      WithoutLock unlocked;
+      rc = g_softmax(qp, kp, vp, out.address(c, shape), b, M, N, K, L, c.code, layout, static_cast<float>(scale),
+                     static_cast<int>(flags), nullptr, 0, g_status[c.device], stream_of(c.device));
+    }
+    return rc ? nullptr : out.give();
   });
 }
 
@@ -154,19 +184,25 @@ PyObject* py_mha(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int64_t b = x->size(0), M = x->size(1), k3 = x->size(2);
     if (k3 % (3 * heads) || !fits({b, M, k3})) return nullptr;
     const int64_t hidden = k3 / 3;
-    at::Tensor hold;
-    const at::Tensor* out = result(a[2], c, {b, M, hidden}, hold);
-    if (out == nullptr) return nullptr;
-    if (g_mha(x->data_ptr(), out->data_ptr(), b, M, heads, hidden / heads, c.code, static_cast<float>(scale), static_cast<int>(flags),
-              g_status[c.device], stream_of(c.device)) != 0)
-      return nullptr;
-    return give(a[2], hold);
+    const int64_t shape[3] = {b, M, hidden};
+    const at::Tensor* given;
+    if (!result_ok(a[2], c, shape, &given)) return nullptr;
+    const void* xp = x->data_ptr();
+    Result out(a[2], given);
+    int rc;
+    {
+      WithoutLock unlocked;
+      rc = g_mha(xp, out.address(c, shape), b, M, heads, hidden / heads, c.code, static_cast<float>(scale), static_cast<int>(flags),
+                 g_status[c.device], stream_of(c.device));
+    }
+    return rc ? nullptr : out.give();
   });
 }
 
 // The operands of the MLP chain and the feed-forward block: x [M, K] or [batch, M, K], weights likewise.
 struct Chain {
   const at::Tensor *x, *w1, *w2;
+  const void *xp, *w1p, *w2p;     // their addresses
   int64_t b, M, N, K, L;
   int layout;                     // 1: weights [out, in]
   bool flat;                      // x is a matrix, and so is the result
@@ -194,20 +230,26 @@ bool chain_of(PyObject* px, PyObject* pw1, PyObject* pw2, PyObject* layout, Comm
   r.K = x[2];
   r.L = r.layout ? u[1] : u[2];
   r.N = r.layout ? v[1] : v[2];
+  r.xp = r.x->data_ptr();
+  r.w1p = r.w1->data_ptr();
+  r.w2p = r.w2->data_ptr();
   return u[0] == r.b && v[0] == r.b && (r.layout ? u[2] : u[1]) == r.K && (r.layout ? v[2] : v[1]) == r.L &&
          fits({r.b, r.M, r.N, r.K, r.L});
 }
 // As the operators' Python path takes it: a given result may be a matrix or have a batch dimension of its own.
-const at::Tensor* chain_result(PyObject* given, Common& c, const Chain& r, at::Tensor& hold) {
-  if (given == Py_None) {
-    hold = r.flat ? make({r.M, r.N}, c.type, c.device) : make({r.b, r.M, r.N}, c.type, c.device);
-    return &hold;
-  }
-  const at::Tensor* t = take(given, c);
-  if (t == nullptr) return nullptr;
-  const bool ok = (t->dim() == 2 && r.b == 1 && t->size(0) == r.M && t->size(1) == r.N) || shape_is(*t, r.b, r.M, r.N);
-  return ok ? t : nullptr;
+bool chain_result_ok(PyObject* given, Common& c, const Chain& r, const at::Tensor** t) {
+  *t = nullptr;
+  if (given == Py_None) return true;
+  *t = take(given, c);
+  return *t != nullptr && (((*t)->dim() == 2 && r.b == 1 && (*t)->size(0) == r.M && (*t)->size(1) == r.N) || shape_is(**t, r.b, r.M, r.N));
 }
+// The shape of a new result.
+struct ChainShape {
+  int64_t d[3];
+  bool flat;
+  explicit ChainShape(const Chain& r) : d{r.b, r.M, r.N}, flat(r.flat) {}
+  operator at::IntArrayRef() const { return flat ? at::IntArrayRef(d + 1, 2) : at::IntArrayRef(d, 3); }
+};
 // Scratch memory of a call, in stream order from the caching allocator: its own for every stream, thread and captured graph.
 at::Tensor scratch_for(const Common& c, int64_t b, int64_t M, int64_t N, int64_t K, int64_t L, size_t* bytes) {
   *bytes = g_bytes(kOpGemmReluGemm, b, M, N, K, L, c.code);
@@ -225,15 +267,21 @@ PyObject* py_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Common c;
     Chain r;
     if (!chain_of(a[0], a[1], a[2], a[5], c, r)) return nullptr;
-    at::Tensor hold, ws;
-    const at::Tensor* out = chain_result(a[3], c, r, hold);
-    if (out == nullptr) return nullptr;
-    size_t bytes = 0;
-    if (a[6] == Py_True) ws = scratch_for(c, r.b, r.M, r.N, r.K, r.L, &bytes);
-    if (g_gemm(r.x->data_ptr(), r.w1->data_ptr(), r.w2->data_ptr(), out->data_ptr(), r.b, r.M, r.N, r.K, r.L, c.code, r.layout, act,
-               bytes ? ws.data_ptr() : nullptr, bytes, g_status[c.device], stream_of(c.device)) != 0)
-      return nullptr;
-    return give(a[3], hold);
+    const at::Tensor* given;
+    if (!chain_result_ok(a[3], c, r, &given)) return nullptr;
+    const bool scratch = a[6] == Py_True;
+    Result out(a[3], given);
+    int rc;
+    {
+      WithoutLock unlocked;
+      size_t bytes = 0;
+      at::Tensor ws;
+      void* y = out.address(c, ChainShape(r));
+      if (scratch) ws = scratch_for(c, r.b, r.M, r.N, r.K, r.L, &bytes);
+      rc = g_gemm(r.xp, r.w1p, r.w2p, y, r.b, r.M, r.N, r.K, r.L, c.code, r.layout, act, bytes ? ws.data_ptr() : nullptr, bytes,
+                  g_status[c.device], stream_of(c.device));
+    }
+    return rc ? nullptr : out.give();
   });
 }
 
@@ -256,15 +304,19 @@ PyObject* py_ffn(PyObject*, PyObject* const* a, Py_ssize_t n) {
       if (t == nullptr || t->numel() != r.b * (i == 0 ? r.L : r.N)) return nullptr;
       bias[i] = t->data_ptr();
     }
-    at::Tensor hold;
-    const at::Tensor* out = chain_result(a[5], c, r, hold);
-    if (out == nullptr) return nullptr;
-    size_t bytes = 0;
-    at::Tensor ws = scratch_for(c, r.b, r.M, r.N, r.K, r.L, &bytes);
-    if (g_ffn(r.x->data_ptr(), r.w1->data_ptr(), bias[0], r.w2->data_ptr(), bias[1], out->data_ptr(), r.b, r.M, r.N, r.K, r.L, c.code,
-              r.layout, act1, act2, bytes ? ws.data_ptr() : nullptr, bytes, g_status[c.device], stream_of(c.device)) != 0)
-      return nullptr;
-    return give(a[5], hold);
+    const at::Tensor* given;
+    if (!chain_result_ok(a[5], c, r, &given)) return nullptr;
+    Result out(a[5], given);
+    int rc;
+    {
+      WithoutLock unlocked;
+      size_t bytes = 0;
+      void* y = out.address(c, ChainShape(r));
+      at::Tensor ws = scratch_for(c, r.b, r.M, r.N, r.K, r.L, &bytes);
+      rc = g_ffn(r.xp, r.w1p, bias[0], r.w2p, bias[1], y, r.b, r.M, r.N, r.K, r.L, c.code, r.layout, act1, act2,
+                 bytes ? ws.data_ptr() : nullptr, bytes, g_status[c.device], stream_of(c.device));
+    }
+    return rc ? nullptr : out.give();
   });
 }
 
@@ -293,50 +345,52 @@ PyObject* py_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (n < 3 || !PyCapsule_IsValid(a[0], kPlanName)) return nullptr;
     const Plan& p = *static_cast<const Plan*>(PyCapsule_GetPointer(a[0], kPlanName));
     const at::Tensor* t[6];
+    void* ptr[6];
     const int count = static_cast<int>(n - 1);
     if (count > 6) return nullptr;
     Common c;
-    for (int i = 0; i < count; ++i)
+    for (int i = 0; i < count; ++i) {
       if ((t[i] = take(a[i + 1], c)) == nullptr) return nullptr;
+      ptr[i] = t[i]->data_ptr();
+    }
     if (c.code != p.code) return nullptr;
     int* status = g_status[c.device];
-    int rc = -1;
     if (p.kind <= 1) {
       if (count != 4 || !shape_is(*t[0], p.b, p.M, p.K) || !shape_is(*t[1], p.b, p.K, p.L) || !shape_is(*t[2], p.b, p.L, p.N) ||
           !shape_is(*t[3], p.b, p.M, p.N))
         return nullptr;
-      if (p.kind == 0) {
-        rc = g_softmax(t[0]->data_ptr(), t[1]->data_ptr(), t[2]->data_ptr(), t[3]->data_ptr(), p.b, p.M, p.N, p.K, p.L, p.code, 0,
-                       p.scale, 0, nullptr, 0, status, stream_of(c.device));
-      } else {
-        size_t bytes = 0;
-        at::Tensor ws = scratch_for(c, p.b, p.M, p.N, p.K, p.L, &bytes);
-        rc = g_gemm(t[0]->data_ptr(), t[1]->data_ptr(), t[2]->data_ptr(), t[3]->data_ptr(), p.b, p.M, p.N, p.K, p.L, p.code, 0, p.act1,
-                    bytes ? ws.data_ptr() : nullptr, bytes, status, stream_of(c.device));
-      }
     } else if (p.kind == 2) {
       if (count != 2 || !shape_is(*t[0], p.b, p.M, 3 * p.N) || !shape_is(*t[1], p.b, p.M, p.N)) return nullptr;
-      rc = g_mha(t[0]->data_ptr(), t[1]->data_ptr(), p.b, p.M, p.heads, p.N / p.heads, p.code, p.scale, 0, status, stream_of(c.device));
     } else {
       // x, w1 [L, K], (b1 [L]), w2 [N, L], (b2 [N]), out; x and out keep whatever leading dimensions the layer has
       if (count != 4 + p.bias1 + p.bias2) return nullptr;
-      int i = 0;
+      const int i2 = 2 + p.bias1;                      // w2
       auto matrix = [](const at::Tensor& m, int64_t r, int64_t k) { return m.dim() == 2 && m.size(0) == r && m.size(1) == k; };
       auto vector = [](const at::Tensor& v, int64_t k) { return v.dim() == 1 && v.size(0) == k; };
-      const at::Tensor* x = t[i++];
-      const at::Tensor* w1 = t[i++];
-      const at::Tensor* b1 = p.bias1 ? t[i++] : nullptr;
-      const at::Tensor* w2 = t[i++];
-      const at::Tensor* b2 = p.bias2 ? t[i++] : nullptr;
-      const at::Tensor* out = t[i];
-      if (x->numel() != p.M * p.K || out->numel() != p.M * p.N || !matrix(*w1, p.L, p.K) || !matrix(*w2, p.N, p.L) ||
-          (b1 && !vector(*b1, p.L)) || (b2 && !vector(*b2, p.N)))
+      if (t[0]->numel() != p.M * p.K || t[count - 1]->numel() != p.M * p.N || !matrix(*t[1], p.L, p.K) || !matrix(*t[i2], p.N, p.L) ||
+          (p.bias1 && !vector(*t[2], p.L)) || (p.bias2 && !vector(*t[i2 + 1], p.N)))
         return nullptr;
+    }
+    int rc = -1;
+    {
+      WithoutLock unlocked;
+      void* stream = stream_of(c.device);
       size_t bytes = 0;
-      at::Tensor ws = scratch_for(c, 1, p.M, p.N, p.K, p.L, &bytes);
-      rc = g_ffn(x->data_ptr(), w1->data_ptr(), b1 ? b1->data_ptr() : nullptr, w2->data_ptr(), b2 ? b2->data_ptr() : nullptr,
-                 out->data_ptr(), 1, p.M, p.N, p.K, p.L, p.code, 1, p.act1, p.act2, bytes ? ws.data_ptr() : nullptr, bytes, status,
-                 stream_of(c.device));
+      at::Tensor ws;
+      if (p.kind == 0) {
+        rc = g_softmax(ptr[0], ptr[1], ptr[2], ptr[3], p.b, p.M, p.N, p.K, p.L, p.code, 0, p.scale, 0, nullptr, 0, status, stream);
+      } else if (p.kind == 1) {
+        ws = scratch_for(c, p.b, p.M, p.N, p.K, p.L, &bytes);
+        rc = g_gemm(ptr[0], ptr[1], ptr[2], ptr[3], p.b, p.M, p.N, p.K, p.L, p.code, 0, p.act1, bytes ? ws.data_ptr() : nullptr, bytes,
+                    status, stream);
+      } else if (p.kind == 2) {
+        rc = g_mha(ptr[0], ptr[1], p.b, p.M, p.heads, p.N / p.heads, p.code, p.scale, 0, status, stream);
+      } else {
+        const int i2 = 2 + p.bias1;
+        ws = scratch_for(c, 1, p.M, p.N, p.K, p.L, &bytes);
+        rc = g_ffn(ptr[0], ptr[1], p.bias1 ? ptr[2] : nullptr, ptr[i2], p.bias2 ? ptr[i2 + 1] : nullptr, ptr[count - 1], 1, p.M, p.N, p.K,
+                   p.L, p.code, 1, p.act1, p.act2, bytes ? ws.data_ptr() : nullptr, bytes, status, stream);
+      }
     }
     if (rc != 0) return nullptr;
     Py_RETURN_TRUE;

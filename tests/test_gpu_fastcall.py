@@ -1,9 +1,12 @@
 """The native call path against the checked Python path: the same calls give the same bits and shapes, and what the checked
 path refuses is refused with its errors, whichever path saw the call first."""
+import ctypes
+import threading
+
 import pytest
 import torch
 
-from ditto_b200 import ops
+from ditto_b200 import _lib, ops
 
 pytestmark = pytest.mark.gpu
 
@@ -74,3 +77,55 @@ def test_native_path_answers_like_the_checked_path(cuda):
         else:
             assert native.shape == checked.shape and native.dtype == checked.dtype and torch.equal(native, checked), name
     assert ops.device_status(cuda) == 0
+
+
+def test_entry_points_run_without_the_interpreter_lock(cuda):
+    """With each C entry point replaced by PyGILState_Check -- 0, a successful call, where the calling thread does not hold the lock."""
+    q, x, w1, w2, qkv = _t(1, 16, 16), _t(16, 128), _t(128, 64), _t(64, 256), _t(1, 16, 48)
+    ops.bmm_softmax_bmm(q, q, q, key_layout="LK")
+    fast, lib = ops._fast, _lib.load()
+    address = lambda fn: ctypes.cast(fn, ctypes.c_void_p).value                       # noqa: E731
+    own = [address(getattr(lib, "ditto_b200_" + n)) for n in ("bmm_softmax_bmm", "multi_head_attention", "gemm_relu_gemm", "ffn_ws", "workspace_bytes")]
+    check = address(ctypes.pythonapi.PyGILState_Check)
+    ab, a2 = torch.empty(16, 256, device=cuda, dtype=x.dtype), torch.empty(1, 16, 16, device=cuda, dtype=x.dtype)
+    fp16 = ops._DTYPE_CODE[x.dtype]
+    plans = [(fast.plan(0, 1, 16, 16, 16, 16, fp16, 1, 1.0, 0, 0, 0, 0), (q, q, q, a2)),
+             (fast.plan(1, 1, 16, 16, 16, 16, fp16, 1, 1.0, 1, 0, 0, 0), (q, q, q, a2)),
+             (fast.plan(2, 1, 16, 16, 16, 16, fp16, 1, 1.0, 0, 0, 0, 0), (qkv, a2)),
+             (fast.plan(3, 1, 16, 256, 128, 64, fp16, 1, 1.0, 1, 0, 0, 0), (x, w1.T.contiguous(), w2.T.contiguous(), ab))]
+    fast.bind(check, check, check, check, own[4])
+    try:
+        got = [fast.softmax(q, q, q, None, 1.0, "LK", 0), fast.mha(qkv, 1, None, 1.0, 0),
+               fast.gemm(x, w1, w2, None, "relu", "IO", True), fast.ffn(x, w1, None, w2, None, None, "relu", "relu", "IO")]
+        called = [fast.call(plan, *tensors) for plan, tensors in plans]
+    finally:
+        fast.bind(*own)
+    assert all(isinstance(t, torch.Tensor) for t in got)
+    assert called == [True] * 4
+
+
+def test_two_threads(cuda):
+    """Calls from two threads, each on a stream of its own, give the bits of calls in turn."""
+    torch.manual_seed(4)
+    work = []
+    for M in (144, 272):
+        q, x, w1, w2 = _t(6, M, 64), _t(M, 256), _t(256, 1024) / 16, _t(1024, 256) / 32
+        calls = (lambda q=q: ops.bmm_softmax_bmm(q, q, q, scale=0.125, key_layout="LK"),
+                 lambda x=x, u=w1, v=w2: ops.gemm_relu_gemm(x, u, v), lambda x=x, u=w1, v=w2: ops.ffn(x, u, None, v, None, weight_layout="IO"))
+        work.append([(c, c()) for c in calls])
+    torch.cuda.synchronize()
+    wrong = []
+
+    def run(items):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(50):
+                got = [c() for c, _ in items]
+            torch.cuda.current_stream().synchronize()
+            wrong.extend(i for i, (g, (_, want)) in enumerate(zip(got, items)) if not torch.equal(g, want))
+
+    threads = [threading.Thread(target=run, args=(items,)) for items in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong and ops.device_status(cuda) == 0
