@@ -14,7 +14,6 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libditto_b200.so")
-FASTCALL_PATH = os.path.join(LIB_DIR, "_fastcall.so")     # the operators' call path (csrc/fastcall.cpp)
 SOURCES = ["api.cu", "host_util.cu", "attention_sm100.cu", "attention_persistent_sm100.cu", "attention_narrow_sm100.cu", "mlp_sm100.cu", "mlp_wide_sm100.cu", "mlp_pair_sm100.cu", "mlp_flow_sm100.cu", "mlp_tiles_sm100.cu", "selftest_sm100.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -29,10 +28,17 @@ def _nvcc():
     return exe
 
 
+def fastcall_path():
+    """The operators' call path (csrc/fastcall.cpp).  torch's C++ interface is only good for the version that brings it, so
+    the file's name says what it was compiled against: for another torch or Python there is no such file yet."""
+    import torch
+    return os.path.join(LIB_DIR, f"_fastcall-{torch.__version__}-cp{sys.version_info[0]}{sys.version_info[1]}.so")
+
+
 def _stale():
-    if not os.path.exists(LIB_PATH) or not os.path.exists(FASTCALL_PATH):
+    if not os.path.exists(LIB_PATH) or not os.path.exists(fastcall_path()):
         return True
-    t = min(os.path.getmtime(LIB_PATH), os.path.getmtime(FASTCALL_PATH))
+    t = min(os.path.getmtime(LIB_PATH), os.path.getmtime(fastcall_path()))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
     deps.append(os.path.join(HERE, "..", "include", "ditto_b200.h"))
     return any(os.path.getmtime(d) > t for d in deps if os.path.isfile(d))
@@ -46,7 +52,7 @@ def _fastcall_command():
     inc = [f"-I{p}" for p in cpp_extension.include_paths()]
     inc += [f"-I{sysconfig.get_paths()['include']}", f"-I{os.path.join(os.path.dirname(os.path.dirname(_nvcc())), 'include')}"]
     return ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-            *inc, os.path.join(CSRC, "fastcall.cpp"), "-o", FASTCALL_PATH, f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
+            *inc, os.path.join(CSRC, "fastcall.cpp"), "-o", fastcall_path(), f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
             "-ltorch_cuda", "-ltorch_python"]
 
 

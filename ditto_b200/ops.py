@@ -7,10 +7,11 @@ import ctypes
 import importlib.machinery
 import importlib.util
 import os
+import warnings
 
 import torch
 
-from . import _lib
+from . import _lib, build_lib
 
 _DTYPE_CODE = {torch.float16: _lib.DTYPE_FP16, torch.bfloat16: _lib.DTYPE_BF16}
 
@@ -57,19 +58,37 @@ def _status_ptr(device):
 
 # The call path in native code (csrc/fastcall.cpp), set up by the first checked call on a device: it handles the
 # straight case -- everything valid, on the current device -- and answers None for all others, which then take the
-# checked path below and its error messages.
+# checked path below and its error messages.  Where it was not built for the torch that runs, that path serves
+# every call, some 9 us slower each.
 _fast = None
+_fast_refused = False
+
+
+def _load_fast():
+    """The native call path's module, or None (said once)."""
+    global _fast_refused
+    if _fast_refused:
+        return None
+    path = build_lib.fastcall_path()
+    try:
+        if not os.path.exists(path):
+            raise ImportError(f"{path} not found")
+        loader = importlib.machinery.ExtensionFileLoader("_fastcall", path)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastcall", path, loader=loader))
+        loader.exec_module(mod)
+        return mod
+    except ImportError as e:
+        _fast_refused = True
+        warnings.warn(f"ditto_b200: calls take the slower Python path ({e}); `python -m ditto_b200.build_lib` builds the native one")
+        return None
 
 
 def _enable_fast(device):
     global _fast
     if _fast is None:
-        path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "_fastcall.so")
-        if not os.path.exists(path):
-            raise ImportError(f"{path} not found: build it with `python -m ditto_b200.build_lib`")
-        loader = importlib.machinery.ExtensionFileLoader("_fastcall", path)
-        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastcall", path, loader=loader))
-        loader.exec_module(mod)
+        mod = _load_fast()
+        if mod is None:
+            return
         lib = _lib.load()
         mod.bind(*(ctypes.cast(fn, ctypes.c_void_p).value for fn in (
             lib.ditto_b200_bmm_softmax_bmm, lib.ditto_b200_multi_head_attention, lib.ditto_b200_gemm_relu_gemm,

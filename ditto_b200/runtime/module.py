@@ -103,7 +103,7 @@ class ChainModule:
                 ops.bmm_softmax_bmm(a, b, c, out=f, scale=s.scale, key_layout="KL")
             else:
                 ops.gemm_relu_gemm(a, b, c, out=f, activation="relu" if s.kind == "relu" else "identity")
-        if self._plan is None:
+        if self._plan is None and ops._fast is not None:
             act1 = 1 if s.kind == "relu" else ops._ACT_CODE[s.act1]
             self._plan = ops._fast.plan({"softmax": 0, "mha": 2, "ffn": 3}.get(s.kind, 1), s.batch, s.M, s.N, s.K, s.L,
                                         ops._DTYPE_CODE[_TORCH_DTYPE[s.dtype]], s.heads, float(s.scale), act1,

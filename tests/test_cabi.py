@@ -75,3 +75,21 @@ def test_ops_refuse_cpu_tensors():
         ops.bmm_softmax_bmm(q, q, q)
     with pytest.raises(TypeError):
         ops.gemm_relu_gemm(q, q, q)
+
+
+def test_native_call_path_may_be_missing_or_foreign(monkeypatch, tmp_path):
+    """Without _fastcall for the torch that runs -- or with a file that is none -- the Python path serves the calls, with a warning."""
+    from ditto_b200 import build_lib, ops
+    import torch
+    assert torch.__version__ in build_lib.fastcall_path()
+    (tmp_path / "broken.so").write_bytes(b"not a library")
+    for name in ("nope.so", "broken.so"):
+        monkeypatch.setattr(build_lib, "fastcall_path", lambda name=name: str(tmp_path / name))
+        monkeypatch.setattr(ops, "_fast_refused", False)
+        with pytest.warns(UserWarning, match="Python path"):
+            assert ops._load_fast() is None
+        monkeypatch.setattr(ops, "_fast", None)
+        ops._enable_fast(torch.device("cuda:0"))                # said once, and no error
+        assert ops._fast is None
+    monkeypatch.setattr(build_lib, "fastcall_path", lambda: str(tmp_path / "nope.so"))
+    assert build_lib._stale()
