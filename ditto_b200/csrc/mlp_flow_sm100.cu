@@ -373,6 +373,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           good = wait_count(count + r, min(per_round, p.tn1 - r * per_round) * kEpiWarps, abort_word, 0x30);
         ok = __all_sync(0xffffffffu, good);
         if (!ok) break;
+        __syncwarp();                                      // (a vote orders no memory: the lane that polled is not the one that loads)
         fence_proxy_async_global();
       }
       // 64-column unit k of the hidden dimension in summation order: unit e of round i is quarter e / cr of chunk
@@ -576,6 +577,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         if (lane == 0) ok = wait_count(what, target, abort_word, 0x310);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
+        __syncwarp();                                      // (as above: one lane polled, all of them load or store)
         if (first) fence_proxy_async_global();
         else __threadfence();
       }
