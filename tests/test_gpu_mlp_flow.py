@@ -79,3 +79,23 @@ def test_flow_kernel_needs_its_scratch_memory(cuda):
     need = _lib.load().ditto_b200_workspace_bytes(_lib.OP_GEMM_RELU_GEMM, 1, 256, 256, 128, 2048, _lib.DTYPE_BF16)
     dirty = torch.full((need,), 0xA5, dtype=torch.uint8, device=cuda)
     assert torch.equal(ops.gemm_relu_gemm(x, w1, w2, workspace=dirty), ops.gemm_relu_gemm(x, w1, w2))
+
+
+def test_search_for_a_plan_is_short_and_kept(cuda):
+    """The host's share of a large call: the search for a shape that is new, batches of thousands of entries included, and
+    the look-up of one that a few hundred other shapes were called after.  (48 us and under 1 us; the limits leave room for a busy host.)"""
+    import time
+    lib = _lib.load()
+    shapes = [(b, M, N, N, 4 * N) for b, M in ((1, 16384), (1, 8208), (24, 384), (512, 256), (2048, 160), (1, 131072)) for N in (512, 1024)]
+    shapes += [(1, 16384 + 16 * i, 1024, 1024, 4096) for i in range(60)]
+    call = lambda b, M, N, K, L: lib.ditto_b200_workspace_bytes(_lib.OP_GEMM_RELU_GEMM | _lib.EPILOGUE_FLOW_MMA, b, M, N, K, L, 1)     # noqa: E731
+    call(1, 4096, 512, 512, 2048)                          # (the kernel's attributes are set here)
+    times = []
+    for _ in range(2):
+        times.append([])
+        for s in shapes:
+            t = time.perf_counter()
+            assert call(*s) > 0
+            times[-1].append(time.perf_counter() - t)
+    assert sorted(times[0])[-3] < 1e-3, sorted(times[0])[-5:]
+    assert sorted(times[1])[len(shapes) // 2] < 20e-6, times[1]
