@@ -713,12 +713,40 @@ static int resolve_variant(int variant, int N, int K, int L, int w_layout) {
   return kMlpQuad;
 }
 
+// The form of a call that is given scratch memory.
+//
+// The flow kernel multiplies 256-row blocks and the tile and cluster kernels 128-row ones, batch entry by batch entry:
+// it is the fastest form of large calls (1.15 PFLOP/s of whatever it multiplies) unless entries of few rows make it multiply
+// zeros.  The cluster kernel, at its best with results of 768 and 1024 columns, does 0.97 PFLOP/s of whole rounds of
+// clusters.  Measured, us, cluster / flow / tile kernel, 1024 -> 4096 -> 1024: 64 entries of 128 rows 185 / 253 / 211; 256 of 16
+// 655 / 905 / 684; 33 of 336 217 / 232 / 235; 40 of 128 169 / 165 / 142; 24 of 384 239 / 183 / 157; 100 of 400 895 / 697 / 918;
+// 768 -> 3072 -> 768: 64 of 128 120 / 154 / 132, 100 of 128 219 / 231 / 246.
+// Other widths: the cluster kernel does 0.3 to 0.6 PFLOP/s and the tile kernel is the better form of 128-row blocks
+// (256 -> 1024 -> 256, 1024 of 128: 430 / 425 / 307; 1280 -> 5120 -> 1280, 64 of 128: 481 / 376 / 361) up to hidden layers that
+// are no longer read out of L2 (512 -> 2048 -> 512, hidden layers of 105, 134 and 268 MB: 200 of 128 219 / 231 / 214, 512 of 64
+// 484 / 551 / 437, 512 of 128 490 / 570 / 541).
+enum MlpForm { kFormCluster, kFormTiles, kFormFlow };
+static MlpForm form_with_scratch(int batch, int M, int N, int K, int L, bool bf16) {
+  if (!mlp_flow_supported(N, K, L)) return kFormCluster;
+  if (mlp_tiles_faster(batch, M, N, K, L)) return kFormTiles;
+  const double row = 2.0 * L * (static_cast<double>(K) + N);
+  const long long blocks = static_cast<long long>(batch) * ((M + 127) / 128), pairs = static_cast<long long>(batch) * ((M + 255) / 256);
+  int slots = 0;
+  if (mlp_wide_supported(N, K, L) && batch <= 65535 && (N == 768 || N == 1024) && mlp_wide_cluster_slots(bf16, &slots) == DITTO_OK) {
+    const double cluster = (blocks + slots - 1) / slots * slots * 128 * row / 0.97e15, flow = pairs * 256 * row / 1.15e15;
+    if (flow > 1.03 * cluster) return kFormCluster;
+  }
+  if (M > 128) return kFormFlow;
+  return batch <= 65535 && N <= 1024 && N >= 512 && mlp_tiles_workspace_bytes(batch, M, L) > (static_cast<size_t>(192) << 20) ? kFormCluster : kFormTiles;
+}
+
 size_t mlp_workspace_bytes(int batch, int M, int N, int K, int L, bool bf16, int w_layout, int variant) {
   int slots = 0;
-  if (variant == kMlpAuto && mlp_flow_supported(N, K, L) && mlp_tiles_faster(batch, M, N, K, L)) return mlp_tiles_workspace_bytes(batch, M, L);
-  if ((variant == kMlpAuto || variant == kMlpFlow) && mlp_flow_supported(N, K, L))
-    return mlp_flow_pair_slots(bf16, &slots) == DITTO_OK ? mlp_flow_workspace_bytes(batch, M, N, L, mlp_flow_plan(batch, M, N, K, L, slots)) : 0;
-  if (variant == kMlpFlow) return 0;
+  const MlpForm form = variant == kMlpAuto ? form_with_scratch(batch, M, N, K, L, bf16) : variant == kMlpFlow ? kFormFlow : kFormCluster;
+  if (form == kFormTiles) return mlp_tiles_workspace_bytes(batch, M, L);
+  if (form == kFormFlow)
+    return mlp_flow_supported(N, K, L) && mlp_flow_pair_slots(bf16, &slots) == DITTO_OK
+               ? mlp_flow_workspace_bytes(batch, M, N, L, mlp_flow_plan(batch, M, N, K, L, slots)) : 0;
   switch (resolve_variant(variant, N, K, L, w_layout)) {
     case kMlpWide:
       if (!mlp_wide_supported(N, K, L) || mlp_wide_cluster_slots(bf16, &slots) != DITTO_OK) return 0;
@@ -739,11 +767,14 @@ int launch_mlp_chain(const void* x, const void* w1, const void* w2, void* y, int
   // shared by several clusters, if the caller provided the scratch memory that form needs.
   int slots = 0, rc = 0;
   // With scratch memory for the hidden layer small calls run as two launches over tiles, with scratch memory for a ring of
-  // hidden tiles large ones run as one flow of 2-SM tiles: measured faster than the cluster kernels at every size.
+  // hidden tiles large ones run as one flow of 2-SM tiles, where that is the faster form (form_with_scratch).
   // Without it (or with too little) the hidden layer stays inside a cluster.
-  if ((variant == kMlpAuto || variant == kMlpFlow) && workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && mlp_flow_supported(N, K, L)) {
-    if (variant == kMlpAuto && mlp_tiles_faster(batch, M, N, K, L) && ws_bytes >= mlp_tiles_workspace_bytes(batch, M, L))
-      return launch_mlp_tiles(x, w1, w2, y, batch, M, N, K, L, bf16, w_layout, act1, act2, b1, b2, mlp_tiles_plan(batch, M, N, K, L), workspace, status, stream);
+  const MlpForm form = workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 15) != 0 ? kFormCluster
+                       : variant == kMlpAuto ? form_with_scratch(batch, M, N, K, L, bf16)
+                       : variant == kMlpFlow && mlp_flow_supported(N, K, L) ? kFormFlow : kFormCluster;
+  if (form == kFormTiles && ws_bytes >= mlp_tiles_workspace_bytes(batch, M, L))
+    return launch_mlp_tiles(x, w1, w2, y, batch, M, N, K, L, bf16, w_layout, act1, act2, b1, b2, mlp_tiles_plan(batch, M, N, K, L), workspace, status, stream);
+  if (form != kFormCluster) {
     if ((rc = mlp_flow_pair_slots(bf16, &slots)) != DITTO_OK) return rc;
     const FlowPlan plan = mlp_flow_plan(batch, M, N, K, L, slots);
     if (ws_bytes >= mlp_flow_workspace_bytes(batch, M, N, L, plan))

@@ -88,3 +88,26 @@ def test_tile_kernel_streams_and_changed_weights(cuda):
     assert ops.device_status(cuda) == 0
     for g, w in got:
         assert torch.equal(g, w)
+
+
+@pytest.mark.parametrize("shape,form", [
+    ((64, 128, 1024, 512, 4096), _lib.EPILOGUE_WIDE_MMA),     # entries of one 128-row block, whole rounds of clusters
+    ((33, 336, 1024, 256, 4096), _lib.EPILOGUE_WIDE_MMA),     # three of them
+    ((40, 128, 1024, 1024, 4096), "tiles"),                   # a second round of seven clusters only
+    ((60, 112, 1280, 256, 5120), "tiles"),                    # a width the cluster kernel computes in two groups
+    ((520, 128, 256, 64, 1024), "tiles"),                     # a hidden layer larger than L2
+    ((400, 128, 512, 64, 2048), _lib.EPILOGUE_WIDE_MMA),      # ... and wide enough for the cluster kernel
+    ((24, 384, 768, 768, 3072), _lib.EPILOGUE_FLOW_MMA),      # a quarter of the flow kernel's rows are zero
+    ((16, 512, 1024, 1024, 4096), _lib.EPILOGUE_FLOW_MMA),
+])
+def test_form_of_batched_calls(cuda, shape, form):
+    """Rules on sizes for weights of every entry's own (seen by the scratch memory asked for), and the form's result."""
+    batch, M, N, K, L = shape
+    need = _lib.load().ditto_b200_workspace_bytes
+    want = batch * M * L * 2 if form == "tiles" else need(_lib.OP_GEMM_RELU_GEMM | form, *shape, 1)
+    assert need(_lib.OP_GEMM_RELU_GEMM, *shape, 1) == want
+    _, x, w1, w2 = _operands(cuda, batch, M, N, K, L, torch.bfloat16, 45)
+    out = ops.gemm_relu_gemm(x, w1, w2)
+    for i in (0, batch // 2, batch - 1):
+        ref = torch.relu(x[i].float() @ w1[i].float()).bfloat16().float() @ w2[i].float()
+        _assert_close(out[i], ref, torch.bfloat16, shape, cuda)
