@@ -251,9 +251,16 @@ struct ChainShape {
   operator at::IntArrayRef() const { return flat ? at::IntArrayRef(d + 1, 2) : at::IntArrayRef(d, 3); }
 };
 // Scratch memory of a call, in stream order from the caching allocator: its own for every stream, thread and captured graph.
+// None where there is no memory left for it: the call then takes the form that needs none.
 at::Tensor scratch_for(const Common& c, int64_t b, int64_t M, int64_t N, int64_t K, int64_t L, size_t* bytes) {
   *bytes = g_bytes(kOpGemmReluGemm, b, M, N, K, L, c.code);
-  return *bytes ? make({static_cast<int64_t>(*bytes)}, at::kByte, c.device) : at::Tensor();
+  if (*bytes == 0) return at::Tensor();
+  try {
+    return make({static_cast<int64_t>(*bytes)}, at::kByte, c.device);
+  } catch (const c10::OutOfMemoryError&) {
+    *bytes = 0;
+    return at::Tensor();
+  }
 }
 
 // gemm(x, w1, w2, out, activation, weight_layout, scratch)

@@ -214,11 +214,15 @@ _VARIANT_BITS = {"auto": 0, "pair": 0x200, "quad": 0x400, "wide": 0x800, "flow":
 def _scratch(lib, op, batch, M, N, K, L, dtype, device):
     """(tensor, pointer, bytes) of the scratch memory a call runs fastest with (the C ABI itself allocates nothing).
     Taken from the caching allocator per call: in stream order, so calls on several streams and threads and
-    captured graphs each have their own."""
+    captured graphs each have their own.  Where there is no memory left for it the call goes without: the kernels
+    that keep the hidden layer inside a cluster need none."""
     need = lib.ditto_b200_workspace_bytes(op, batch, M, N, K, L, _DTYPE_CODE[dtype])
     if not need:
         return None, None, 0
-    buf = torch.empty(need, dtype=torch.uint8, device=device)
+    try:
+        buf = torch.empty(need, dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        return None, None, 0
     return buf, buf.data_ptr(), need
 
 

@@ -215,3 +215,37 @@ def test_model_level_flow_attention_then_feed_forward(cuda, oracle, factory):
                  scale=float(np.abs(want).max()))
     cost = engine.get_function("timeit")(20).value
     assert 0 < cost < 5
+
+
+def test_mlp_calls_do_without_scratch_memory_when_there_is_none_left(cuda):
+    """With no 20 MiB left to the allocator and 50 MB of scratch memory asked for, on the native and on the checked path: the
+    result of the kernels that need none."""
+    g = torch.Generator(device=cuda).manual_seed(51)
+    M, N, K, L = 24592, 256, 16, 1024
+    x = torch.randn(M, K, device=cuda, generator=g).half()
+    w1, w2 = torch.randn(K, L, device=cuda, generator=g).half() / 4, torch.randn(L, N, device=cuda, generator=g).half() / 32
+    b1 = torch.randn(L, device=cuda, generator=g).half()
+    want = ops.gemm_relu_gemm(x, w1, w2, workspace=None)
+    outs = [torch.zeros_like(want) for _ in range(4)]
+    assert _lib.load().ditto_b200_workspace_bytes(_lib.OP_GEMM_RELU_GEMM, 1, M, N, K, L, 0) > 40 << 20
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    fast, total, rest = ops._fast, torch.cuda.get_device_properties(cuda).total_memory, []
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (48 << 20)) / total)
+        with pytest.raises(torch.OutOfMemoryError):
+            while True:
+                rest.append(torch.empty(20 << 20, dtype=torch.uint8, device=cuda))
+        for path, (chain, block) in zip((fast, None), (outs[:2], outs[2:])):
+            ops._fast = path
+            ops.gemm_relu_gemm(x, w1, w2, out=chain)
+            ops.ffn(x, w1, b1, w2, None, out=block, act1="relu", act2="identity", weight_layout="IO")
+    finally:
+        ops._fast = fast
+        torch.cuda.set_per_process_memory_fraction(1.0)
+        rest.clear()
+    assert ops.device_status(cuda) == 0
+    ref = torch.relu(x.float() @ w1.float() + b1.float()).half().float() @ w2.float()
+    for chain, block in (outs[:2], outs[2:]):
+        assert torch.equal(chain, want)
+        assert ((block.float() - ref).abs() <= 2e-2 * ref.abs() + 2e-3 * ref.abs().max()).all()
