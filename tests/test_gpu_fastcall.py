@@ -66,16 +66,81 @@ def _calls():
     yield "short bias", lambda: ops.ffn(x, w1, _t(319), w2, None, weight_layout="IO")
 
 
+class _Recorder:
+    """The native module, noting what its functions answered."""
+
+    def __init__(self, module):
+        self.module, self.answers = module, []
+
+    def __getattr__(self, name):
+        def call(*args):
+            self.answers.append(getattr(self.module, name)(*args))
+            return self.answers[-1]
+        return call
+
+
 def test_native_path_answers_like_the_checked_path(cuda):
+    """... and answers itself where the call is valid, and not at all where it is refused."""
     ops.bmm_softmax_bmm(_t(1, 16, 16), _t(1, 16, 16), _t(1, 16, 16), key_layout="LK")     # sets the native path up
     assert ops._fast is not None
     torch.manual_seed(3)
+    fast = ops._fast
     for name, call in _calls():
-        native, checked = _both(call)
+        ops._fast = recorder = _Recorder(fast)
+        try:
+            native, checked = _both(call)
+        finally:
+            ops._fast = fast
+        assert len(recorder.answers) == 1, name
         if isinstance(checked, tuple):
-            assert native == checked, name
+            assert native == checked and recorder.answers == [None], name
         else:
+            assert recorder.answers[0] is native, name
             assert native.shape == checked.shape and native.dtype == checked.dtype and torch.equal(native, checked), name
+    assert ops.device_status(cuda) == 0
+
+
+def _modules():
+    """Built modules of every kind with valid arguments, results last."""
+    from ditto_b200.auto_tensorize import ChainSchedule
+    from ditto_b200.runtime.module import ChainModule
+
+    def module(kind, batch, M, N, K, L, **more):
+        return ChainModule(ChainSchedule(layer=None, kind=kind, batch=batch, M=M, N=N, K=K, L=L, dtype="float16", device=None,
+                                         param=None, **{"scale": 1.0, **more}))
+
+    b, M, N, K, L = 2, 48, 64, 32, 80
+    chain = (_t(b, M, K), _t(b, K, L), _t(b, L, N), _t(b, M, N))
+    for kind in ("softmax", "relu", "identity"):
+        yield module(kind, b, M, N, K, L), chain
+    yield module("mha", 2, 48, 64, 32, 48, heads=2, scale=0.5), (_t(2, 48, 192), _t(2, 48, 64))
+    M, N, K, L = 48, 256, 128, 320
+    x, w1, b1, w2, b2, y = _t(M, K), _t(L, K), _t(L), _t(N, L), _t(N), _t(M, N)
+    for bias1, bias2 in ((0, 0), (1, 0), (0, 1), (1, 1)):
+        args = (x, w1, *((b1,) if bias1 else ()), w2, *((b2,) if bias2 else ()), y)
+        yield module("ffn", 1, M, N, K, L, bias1=bool(bias1), bias2=bool(bias2), act1="gelu", act2="relu"), args
+
+
+def test_modules_answer_in_native_code(cuda):
+    """Every kind of module: the second call is the native one, with the bits of the first; wrong arguments are refused by it and
+    reported by the checked path."""
+    torch.manual_seed(6)
+    for module, args in _modules():
+        what = (module.schedule.kind, len(args))
+        module(*args)                                       # the checked path
+        want = args[-1].clone()
+        args[-1].zero_()
+        assert ops._fast.call(module._plan, *args) is True, what
+        assert torch.equal(args[-1], want), what
+        for i in range(len(args)):
+            for bad in (args[i][..., :-16].contiguous(), args[i].bfloat16(), args[i].cpu()):
+                wrong = args[:i] + (bad,) + args[i + 1:]
+                assert ops._fast.call(module._plan, *wrong) is None, (what, i)
+                with pytest.raises((TypeError, ValueError)):
+                    module(*wrong)
+        assert ops._fast.call(module._plan, *args[:-1]) is None, what
+        with pytest.raises(TypeError):
+            module(*args[:-1])
     assert ops.device_status(cuda) == 0
 
 

@@ -1,11 +1,10 @@
-"""The MLP chain's two forms with scratch memory at the sizes where each can go wrong, against float32 products (bounds as
-in the random-shape sweeps): the tile kernel, which small calls take, in all its tile widths, reduction splits and
-epilogues, and the flow kernel, asked for by name at the shapes that small calls no longer bring to it."""
+"""The tile kernel, which small calls of the MLP chain with scratch memory take, at the sizes where it can go wrong, against
+float32 products (bounds as in the random-shape sweeps): all its tile widths, reduction splits and epilogues; and the rules
+on sizes that choose between it, the flow kernel and the cluster kernels."""
 import pytest
 import torch
 
 from ditto_b200 import _lib, ops
-from tests.test_gpu_mlp_flow import SHAPES
 from tests.test_gpu_random_shapes import _act, _assert_close
 
 pytestmark = pytest.mark.gpu
@@ -21,26 +20,16 @@ def _operands(cuda, batch, M, N, K, L, dtype, seed):
 
 @pytest.mark.parametrize("layout", ["IO", "OI"])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-def test_flow_kernel_by_name(cuda, dtype, layout):
-    # the last two are large enough for "auto" to take it
-    for batch, M, N, K, L in SHAPES + ((1, 3344, 1280, 1280, 5120), (1, 16400, 512, 512, 2048)):
+def test_large_calls(cuda, dtype, layout):
+    # large enough for the flow kernel
+    for batch, M, N, K, L in ((1, 3344, 1280, 1280, 5120), (1, 16400, 512, 512, 2048)):
         _, x, w1, w2 = _operands(cuda, batch, M, N, K, L, dtype, 41)
         a1, a2 = (w1, w2) if layout == "IO" else (w1.transpose(1, 2).contiguous(), w2.transpose(1, 2).contiguous())
         for act in ("relu", "identity"):
-            out = ops.gemm_relu_gemm(x, a1, a2, activation=act, weight_layout=layout, variant="flow")
+            out = ops.gemm_relu_gemm(x, a1, a2, activation=act, weight_layout=layout)
+            assert torch.equal(out, ops.gemm_relu_gemm(x, a1, a2, activation=act, weight_layout=layout, variant="flow"))
             ref = _act(x.float() @ w1.float(), act).to(dtype).float() @ w2.float()
             _assert_close(out, ref, dtype, (act, batch, M, N, K, L, str(dtype), layout), cuda)
-
-
-@pytest.mark.parametrize("acts", [("gelu", "identity"), ("relu", "relu"), ("relu", "identity"), ("gelu", "relu")])
-def test_flow_kernel_epilogues(cuda, acts):
-    batch, M, N, K, L = 1, 3344, 1280, 1280, 5120
-    g, x, w1, w2 = _operands(cuda, batch, M, N, K, L, torch.bfloat16, 42)
-    b1 = (torch.randn(1, L, device=cuda, generator=g) * 0.5).bfloat16()
-    b2 = (torch.randn(1, N, device=cuda, generator=g) * 0.5).bfloat16()
-    out = ops.ffn(x, w1, b1, w2, b2, act1=acts[0], act2=acts[1], weight_layout="IO")
-    h = _act(x.float() @ w1.float() + b1.float()[:, None], acts[0]).bfloat16().float()
-    _assert_close(out, _act(h @ w2.float() + b2.float()[:, None], acts[1]), torch.bfloat16, acts, cuda)
 
 
 # one k-step in either GEMM; clusters of four and eight; a last tile wider than what is left of the result (256, 192 and
