@@ -209,7 +209,7 @@ class DeviceRun:
             self.flush.zero_()
         torch.cuda.synchronize(self.device)
         barrier()
-        launches0 = self.ops.launch_count
+        launches0 = self.ops.kernel_launches()
         starts = [torch.cuda.Event(enable_timing=True) for _ in range(steps)]
         stops = [torch.cuda.Event(enable_timing=True) for _ in range(steps)]
         for i in range(steps):
@@ -219,7 +219,7 @@ class DeviceRun:
             self.flush.zero_()
         torch.cuda.synchronize(self.device)
         barrier()
-        return sum(s.elapsed_time(e) for s, e in zip(starts, stops)), self.ops.launch_count - launches0
+        return sum(s.elapsed_time(e) for s, e in zip(starts, stops)), self.ops.kernel_launches() - launches0
 
     def time_back_to_back(self, steps, warmup, barrier):
         """Device time of `steps` launches back to back inside one pair of events, ms (the way a serving loop
@@ -229,7 +229,7 @@ class DeviceRun:
             self.launch()
         torch.cuda.synchronize(self.device)
         barrier()
-        launches0 = self.ops.launch_count
+        launches0 = self.ops.kernel_launches()
         start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         start.record()
         for _ in range(steps):
@@ -237,7 +237,7 @@ class DeviceRun:
         stop.record()
         torch.cuda.synchronize(self.device)
         barrier()
-        return start.elapsed_time(stop), self.ops.launch_count - launches0
+        return start.elapsed_time(stop), self.ops.kernel_launches() - launches0
 
     def time_sustained(self, seconds, ms_per_launch, barrier):
         """At least `seconds` of back-to-back launches: (ms per launch, launches).  Long enough for the clocks

@@ -45,6 +45,7 @@ EXPORTS = (
     "ditto_b200_check_status",
     "ditto_b200_strerror",
     "ditto_b200_last_cuda_error",
+    "ditto_b200_kernel_launches",
     "ditto_b200_version",
 )
 
@@ -107,6 +108,8 @@ def load():
     lib.ditto_b200_strerror.restype = ctypes.c_char_p
     lib.ditto_b200_last_cuda_error.argtypes = []
     lib.ditto_b200_last_cuda_error.restype = ctypes.c_char_p
+    lib.ditto_b200_kernel_launches.argtypes = []
+    lib.ditto_b200_kernel_launches.restype = ctypes.c_ulonglong
     lib.ditto_b200_version.argtypes = []
     lib.ditto_b200_version.restype = i
     _lib = lib

@@ -414,6 +414,8 @@ const char* ditto_b200_strerror(int code) {
 
 const char* ditto_b200_last_cuda_error(void) { return ditto_b200::last_error_text(); }
 
+unsigned long long ditto_b200_kernel_launches(void) { return ditto_b200::g_kernel_launches.load(std::memory_order_relaxed); }
+
 int ditto_b200_version(void) { return 100; }
 
 }  // extern "C"

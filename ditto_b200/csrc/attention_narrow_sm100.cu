@@ -17,6 +17,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "host_util.cuh"
 #include "mlp_common.cuh"
 #include "sm100_ptx.cuh"
 #include "softmax_step.cuh"
@@ -26,7 +27,6 @@ namespace ditto_b200 {
 namespace {
 
 constexpr int kBM = 128, kBN = 64, kD = 64;
-constexpr int kMaxDevices = 64;
 constexpr int kTileQ = kBM * kD * 2;      // 16 KB
 constexpr int kTileKV = kBN * kD * 2;     // 8 KB
 constexpr int kOffQ = 0;
@@ -321,7 +321,7 @@ static cudaError_t launch_n(const AttnParams& p, long long items, cudaStream_t s
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, p);
+  return launch_kernel(cfg, kern, p);
 }
 
 cudaError_t launch_attention_narrow(const AttnParams& p, int batch, bool bf16, int mode, cudaStream_t stream) {

@@ -19,6 +19,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "host_util.cuh"
 #include "sm100_ptx.cuh"
 #include "softmax_step.cuh"
 
@@ -46,7 +47,6 @@ namespace ditto_b200 {
 namespace {
 
 constexpr int kBM = 128, kBN = 128, kD = 64;
-constexpr int kMaxDevices = 64;
 constexpr int kStages = 2;
 constexpr int kTileQ = kBM * kD * 2;     // 16 KB
 constexpr int kTileKV = kBN * kD * 2;    // 16 KB
@@ -481,7 +481,7 @@ static cudaError_t launch_p(const AttnParams& p, long long total_items, cudaStre
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, p, static_cast<int>(total_items));
+  return launch_kernel(cfg, kern, p, static_cast<int>(total_items));
 }
 
 cudaError_t launch_attention_persistent(const AttnParams& p, int batch, bool bf16, int mode, cudaStream_t stream) {

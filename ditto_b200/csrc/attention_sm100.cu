@@ -42,6 +42,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "host_util.cuh"
 #include "sm100_ptx.cuh"
 #include "softmax_step.cuh"
 
@@ -834,7 +835,7 @@ static cudaError_t launch_one(const AttnParams& p, int batch, int parts, cudaStr
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = SPLIT ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kern, q);
+  return launch_kernel(cfg, kern, q);
 }
 
 cudaError_t launch_attention(const AttnParams& p, int batch, int d, bool bf16, int nt, bool psmem, int mode,

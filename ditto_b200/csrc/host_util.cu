@@ -9,6 +9,8 @@
 
 namespace ditto_b200 {
 
+std::atomic<unsigned long long> g_kernel_launches{0};
+
 namespace {
 
 thread_local char g_last_error[256] = "";

@@ -62,4 +62,13 @@ inline void mark_device_configured(std::atomic<unsigned long long>& done, int de
   done.fetch_or(1ull << dev, std::memory_order_release);
 }
 
+// Every kernel of the operators is launched through this: counts the launches of the process (ditto_b200_kernel_launches).
+extern std::atomic<unsigned long long> g_kernel_launches;
+template <class Kernel, class... Args>
+cudaError_t launch_kernel(const cudaLaunchConfig_t& cfg, Kernel kernel, Args&&... args) {
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Args&&>(args)...);
+  if (e == cudaSuccess) g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+  return e;
+}
+
 }  // namespace ditto_b200

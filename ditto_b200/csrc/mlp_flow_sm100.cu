@@ -4,8 +4,8 @@
 // The cluster kernels (mlp_wide_sm100.cu and its relatives) keep the hidden layer inside a cluster of four SMs.
 // That costs them the operand reuse of a plain GEMM -- every CTA brings 48 KB per 128 x 256 x 64 step, the hidden
 // tiles travel through distributed shared memory, and a result wider than 1024 columns recomputes GEMM1 -- and
-// they end at 0.6 of the tensor peak.  Here the hidden layer passes through a small ring of scratch memory that
-// stays in L2 (a few row blocks; the ring is rewritten long before its lines are evicted), and both GEMMs run on
+// they end at 0.6 of the tensor peak.  Here the hidden layer passes through a ring of scratch memory, as long as the
+// row blocks that are on their way at a time (50 MB of the 134 MB hidden layer for 16384 x 4096), and both GEMMs run on
 // tiles of 256 x 256 (or 256 x 128) by CTA pairs: 2-SM MMAs with 32 KB of operands per CTA and 512 clocks of
 // tensor work, against the 87 B/clk per SM that TMA loads from L2 were measured to deliver on all SMs at once.
 //
@@ -829,7 +829,9 @@ FlowPlan mlp_flow_plan(int batch, int M, int N, int K, int L, int pair_slots) {
   FlowPlan best = {};
   double best_t = 0.0;
   // Panels are the unit of the hand-out order: small ones keep few hidden tiles alive, large ones make GEMM2 wait less.
-  // The ring has to stay in L2 beside the weights: half of it at most, or what panels of four blocks need.
+  // The ring should stay in L2 beside the weights: half of it at most, or what panels of four blocks need.  Those are not cut:
+  // with 64 MB at most GEMM1 would wait for GEMM2 tiles that take longer than the ring (measured, as it is -> cut, us:
+  // 16384 x 128 -> 8192 -> 256 167 -> 341, 16384 x 256 -> 16384 -> 256 358 -> 1261, 4096 x 2048 -> 65536 -> 2048 1510 -> 1714).
   constexpr size_t kRingBytes = static_cast<size_t>(64) << 20;
   const long long wide_tiles = static_cast<long long>(blocks) * ((L + 255) / 256 + N / 256);
   // A range of a split tile is at least eight 64-column units, and a hidden size of 1024 or less is not split.
@@ -942,7 +944,7 @@ int launch_mlp_flow(const void* x, const void* w1, const void* w2, void* y, int 
   const int counters = static_cast<int>(z.counters);
   cfg.gridDim = dim3(static_cast<unsigned>(std::min(32, (counters + 1023) / 1024)), 1, 1);
   cfg.blockDim = dim3(256, 1, 1);
-  cudaError_t e = cudaLaunchKernelEx(&cfg, mlp_flow_reset_kernel, p.ticket, counters);
+  cudaError_t e = launch_kernel(cfg, mlp_flow_reset_kernel, p.ticket, counters);
   if (e != cudaSuccess) return cuda_fail("mlp flow reset launch", e);
   const long long items = static_cast<long long>(z.blocks) * (z.tn1 + static_cast<long long>(z.tn2) * plan.split);
   cfg.gridDim = dim3(static_cast<unsigned>(2 * std::min<long long>(items, slots)), 1, 1);
@@ -954,14 +956,14 @@ int launch_mlp_flow(const void* x, const void* w1, const void* w2, void* y, int 
   const int epi = none && act2 == 0 && act1 == 1 ? 1 : none && act2 == 0 && act1 == 0 ? 4
                   : both && act1 == 1 && act2 == 1 ? 2 : both && act1 == 2 && act2 == 0 ? 3 : both && act1 == 1 && act2 == 0 ? 5 : 0;
 #define DITTO_FLOW_LAUNCH(E) \
-  case E: e = bf16 ? cudaLaunchKernelEx(&cfg, mlp_flow_kernel<true, E>, p) : cudaLaunchKernelEx(&cfg, mlp_flow_kernel<false, E>, p); break;
+  case E: e = bf16 ? launch_kernel(cfg, mlp_flow_kernel<true, E>, p) : launch_kernel(cfg, mlp_flow_kernel<false, E>, p); break;
   switch (epi) {
     DITTO_FLOW_LAUNCH(1)
     DITTO_FLOW_LAUNCH(2)
     DITTO_FLOW_LAUNCH(3)
     DITTO_FLOW_LAUNCH(4)
     DITTO_FLOW_LAUNCH(5)
-    default: e = bf16 ? cudaLaunchKernelEx(&cfg, mlp_flow_kernel<true, 0>, p) : cudaLaunchKernelEx(&cfg, mlp_flow_kernel<false, 0>, p);
+    default: e = bf16 ? launch_kernel(cfg, mlp_flow_kernel<true, 0>, p) : launch_kernel(cfg, mlp_flow_kernel<false, 0>, p);
   }
 #undef DITTO_FLOW_LAUNCH
   return e == cudaSuccess ? DITTO_OK : cuda_fail("mlp flow kernel launch", e);

@@ -758,7 +758,7 @@ int launch_mlp_pair(const void* x, const void* w1, const void* w2, void* y, int 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = split ? 0 : 1;           // a launch with shared row blocks follows its own counter reset: plain stream order
-  cudaError_t e = bf16 ? cudaLaunchKernelEx(&cfg, mlp_pair_kernel<true>, p) : cudaLaunchKernelEx(&cfg, mlp_pair_kernel<false>, p);
+  cudaError_t e = bf16 ? launch_kernel(cfg, mlp_pair_kernel<true>, p) : launch_kernel(cfg, mlp_pair_kernel<false>, p);
   return e == cudaSuccess ? DITTO_OK : cuda_fail("mlp pair kernel launch", e);
 }
 

@@ -547,7 +547,7 @@ cudaError_t quad_launch(const cudaLaunchConfig_t& cfg, const MlpParams& p) {
     if (e != cudaSuccess) return e;
     mark_device_configured(configured, dev);
   }
-  return cudaLaunchKernelEx(&cfg, mlp_chain_kernel<BF16>, p);
+  return launch_kernel(cfg, mlp_chain_kernel<BF16>, p);
 }
 
 bool quad_supported(int N, int K, int L) {

@@ -330,7 +330,7 @@ cudaError_t launch_one(const TilesParams& p, int ctas, cudaStream_t stream) {
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = p.parts > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kern, p);
+  return launch_kernel(cfg, kern, p);
 }
 
 // D [batch, M, N] = act(A [batch, M, K] * B + bias)

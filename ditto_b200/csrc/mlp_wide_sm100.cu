@@ -984,16 +984,16 @@ int launch_wide_group(const void* x, const void* w1, const void* w2, void* y, in
                   : (act1 == 0 && act2 == 0 && none) ? 4 : 0;
   cudaError_t e = cudaErrorInvalidValue;
   switch (epi * 2 + (bf16 ? 1 : 0)) {
-    case 0: e = cudaLaunchKernelEx(&cfg, mlp_wide_kernel<false, 0>, p); break;
-    case 1: e = cudaLaunchKernelEx(&cfg, mlp_wide_kernel<true, 0>, p); break;
-    case 2: e = cudaLaunchKernelEx(&cfg, mlp_wide_kernel<false, 1>, p); break;
-    case 3: e = cudaLaunchKernelEx(&cfg, mlp_wide_kernel<true, 1>, p); break;
-    case 4: e = cudaLaunchKernelEx(&cfg, mlp_wide_kernel<false, 2>, p); break;
-    case 5: e = cudaLaunchKernelEx(&cfg, mlp_wide_kernel<true, 2>, p); break;
-    case 6: e = cudaLaunchKernelEx(&cfg, mlp_wide_kernel<false, 3>, p); break;
-    case 7: e = cudaLaunchKernelEx(&cfg, mlp_wide_kernel<true, 3>, p); break;
-    case 8: e = cudaLaunchKernelEx(&cfg, mlp_wide_kernel<false, 4>, p); break;
-    default: e = cudaLaunchKernelEx(&cfg, mlp_wide_kernel<true, 4>, p); break;
+    case 0: e = launch_kernel(cfg, mlp_wide_kernel<false, 0>, p); break;
+    case 1: e = launch_kernel(cfg, mlp_wide_kernel<true, 0>, p); break;
+    case 2: e = launch_kernel(cfg, mlp_wide_kernel<false, 1>, p); break;
+    case 3: e = launch_kernel(cfg, mlp_wide_kernel<true, 1>, p); break;
+    case 4: e = launch_kernel(cfg, mlp_wide_kernel<false, 2>, p); break;
+    case 5: e = launch_kernel(cfg, mlp_wide_kernel<true, 2>, p); break;
+    case 6: e = launch_kernel(cfg, mlp_wide_kernel<false, 3>, p); break;
+    case 7: e = launch_kernel(cfg, mlp_wide_kernel<true, 3>, p); break;
+    case 8: e = launch_kernel(cfg, mlp_wide_kernel<false, 4>, p); break;
+    default: e = launch_kernel(cfg, mlp_wide_kernel<true, 4>, p); break;
   }
   return e == cudaSuccess ? DITTO_OK : cuda_fail("mlp wide kernel launch", e);
 }

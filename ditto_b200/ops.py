@@ -34,8 +34,13 @@ def _on_device(device):
     return torch.cuda.device(device)
 _status_words = {}
 
-# number of kernel launches issued through this module (benchmarks report it)
+# operator calls made through this module; a call is one kernel launch, or two and more for the MLP chain (kernel_launches)
 launch_count = 0
+
+
+def kernel_launches():
+    """Launches of this package's kernels by this process so far (a replayed graph's are those of its capture)."""
+    return _lib.load().ditto_b200_kernel_launches()
 
 
 _status_ptrs = {}

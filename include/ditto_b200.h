@@ -77,7 +77,7 @@ int ditto_b200_bmm_softmax_bmm(const void* q, const void* k, const void* v, void
 int ditto_b200_multi_head_attention(const void* qkv, void* out, int batch, int M, int heads, int head_dim, int dtype,
                                     float scale, int flags, int* status_word, void* stream);
 
-/* Fused MLP chain  y = act(X W1) W2 in one kernel, replacing the
+/* Fused MLP chain  y = act(X W1) W2 in one call, replacing the
  * module built from BatchGemmReluGemm (python_test/auto_tensorize/test_hyper_fusion_cpu.py:24-96,
  * evaluation/cpu/bmm_relu_bmm.py:56-125) and, with epilogue 0, BatchGemmGemm
  * (benchmark/chimera/cuda/bmm_bmm_cuda.py:69-150).
@@ -86,10 +86,14 @@ int ditto_b200_multi_head_attention(const void* qkv, void* out, int batch, int M
  *   epilogue 0: identity between the GEMMs; 1: ReLU; | DITTO_EPILOGUE_PAIR_MMA / _QUAD_MMA / _WIDE_MMA / _FLOW_MMA
  *   forces one of the kernels (same results up to fp32 summation order; default: by shape)
  *   workspace / ws_bytes: optional scratch memory (ditto_b200_workspace_bytes; contents irrelevant on entry,
- *   undefined on return).  With it the hidden activations pass through a ring of a few row blocks (at most about
- *   64 MB, rewritten while it is in L2) between the tiles of the two GEMMs, the fastest form at every size; a
- *   forced cluster kernel uses it to share row blocks between clusters when there are few.  NULL or too small:
- *   the hidden activations stay inside a cluster, one cluster per row block.
+ *   undefined on return).  With it calls up to about 48 GFLOP, and batch entries of up to 128 rows, keep the whole
+ *   hidden layer there between two launches; larger calls pass it through a ring of row blocks between the tiles
+ *   of the two GEMMs, behind a launch that clears the ring's counters.  The ring holds the row blocks that are on
+ *   their way: at most 64 MB up to a hidden size of about 5000, more where a row block is longer or the other widths are
+ *   small (96 MB for 1024 -> 8192 -> 1024, 512 MB for 2048 -> 65536 -> 2048), never more than the hidden layer.  Where
+ *   batch entries of few rows make another form the faster one, and when a cluster kernel is forced, it is used to
+ *   share row blocks between clusters.  NULL or too small: the hidden activations stay inside a cluster, one cluster
+ *   per row block, in one launch for up to 1024 result columns: 1.2 to 3 times the time, more for wider results.
  * Shapes: N <= 128 and K <= 128 (any multiples of 16, either weight layout): the reference's own shape family;
  * otherwise L % 128 == 0, K % 64 == 0, N in {256, 512, 768, 1024}, or -- on the default kernel -- L % 64 == 0,
  * K % 16 == 0 and N any multiple of 256 up to 16384 (results wider than 1024 columns are computed in column
@@ -135,8 +139,8 @@ int ditto_b200_ffn(const void* x, const void* w1, const void* b1, const void* w2
                    void* stream);
 
 /* ditto_b200_ffn with scratch memory (ditto_b200_workspace_bytes with DITTO_OP_GEMM_RELU_GEMM; contents irrelevant on
- * entry, undefined on return): the hidden layer, or a ring of its tiles, then stays in L2 there, which is the
- * faster form at every size.  NULL or too small: as ditto_b200_ffn. */
+ * entry, undefined on return): the hidden layer, or a ring of its tiles, is kept there, as for the chain above.
+ * NULL or too small: as ditto_b200_ffn. */
 int ditto_b200_ffn_ws(const void* x, const void* w1, const void* b1, const void* w2, const void* b2, void* y, int batch,
                       int M, int N, int K, int L, int dtype, int w_layout, int act1, int act2, void* workspace,
                       size_t ws_bytes, int* status_word, void* stream);
@@ -183,6 +187,10 @@ int ditto_b200_check_status(int* status_word, void* stream, int* code_out);
 const char* ditto_b200_strerror(int code);
 /* Text of the last CUDA / driver error seen by the calling thread ("" if none). */
 const char* ditto_b200_last_cuda_error(void);
+/* Kernels the operators of this process have launched so far (a self test's are not counted, a replayed graph's once,
+ * when it was captured).  A call of an attention entry point is one launch, of an MLP entry point one or more. */
+unsigned long long ditto_b200_kernel_launches(void);
+
 int ditto_b200_version(void);
 
 #ifdef __cplusplus

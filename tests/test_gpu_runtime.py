@@ -249,3 +249,14 @@ def test_mlp_calls_do_without_scratch_memory_when_there_is_none_left(cuda):
     for chain, block in (outs[:2], outs[2:]):
         assert torch.equal(chain, want)
         assert ((block.float() - ref).abs() <= 2e-2 * ref.abs() + 2e-3 * ref.abs().max()).all()
+
+
+def test_kernel_launches_are_counted(cuda):
+    """One launch of an attention call, two of a small MLP call with scratch memory, one without, two of a large one."""
+    q = torch.zeros(1, 128, 64, device=cuda, dtype=torch.float16)
+    x, w1, w2 = (torch.zeros(*s, device=cuda, dtype=torch.float16) for s in ((24592, 16), (16, 1024), (1024, 256)))
+    for call, want in ((lambda: ops.bmm_softmax_bmm(q, q, q, key_layout="LK"), 1), (lambda: ops.gemm_relu_gemm(x[:128], w1, w2), 2),
+                       (lambda: ops.gemm_relu_gemm(x[:128], w1, w2, workspace=None), 1), (lambda: ops.gemm_relu_gemm(x, w1, w2), 2)):
+        before = ops.kernel_launches()
+        call()
+        assert ops.kernel_launches() - before == want
