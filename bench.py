@@ -530,7 +530,7 @@ def mlp_cluster_slots():
 def unfused_context(run, w, barrier):
     """Context only, never on the product path: the same shape as two library GEMMs with the hidden layer
     written to and read back from HBM (torch.matmul -> relu -> torch.matmul), cold launches like the fused
-    number beside it.  What the fused form pays or gains for keeping the hidden layer on chip."""
+    number beside it.  What the fused form gains for not passing the whole hidden layer through memory between two calls."""
     torch = run.torch
     x, (w1, w2) = run.inputs[0], run.resident
     def step():

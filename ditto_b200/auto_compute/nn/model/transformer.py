@@ -6,7 +6,7 @@ from ..module import Linear, Module, MultiHeadAttentionMMA, ReLU
 class PositionwiseFeedForward(Module):
     """activation(w_2(activation(w_1(x)))) with biased [out, in] linears and ReLU, as in the reference
     (transformer.py:21-34).  Built as four layers (linear, relu, linear, relu); `chimera.graph_fusion`
-    turns them into one feed-forward layer that runs as a single kernel with the hidden layer on chip."""
+    turns them into one feed-forward layer that runs as one fused call."""
 
     def __init__(self, d_model, d_ff, dtype="float32", out_dtype="float32"):
         super().__init__()

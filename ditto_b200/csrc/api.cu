@@ -303,8 +303,8 @@ int ditto_b200_ffn(const void* x, const void* w1, const void* b1, const void* w2
 }
 
 size_t ditto_b200_workspace_bytes(int op, int batch, int M, int N, int K, int L, int dtype) {
-  // The attention chain keeps everything on chip.  The MLP chain runs fastest with its hidden layer, or a ring of
-  // hidden tiles, in scratch memory that stays in L2; without it the hidden layer stays inside a cluster.
+  // The attention chain keeps everything on chip.  The MLP chain mostly runs fastest with its hidden layer, or a ring of
+  // hidden tiles, in scratch memory; without it the hidden layer stays inside a cluster.
   if ((op & 0xff) != DITTO_OP_GEMM_RELU_GEMM || batch <= 0 || M <= 0 || N <= 0 || K <= 0 || L <= 0) return 0;
   if (N <= 128 && K <= 128) return 0;
   // `op` may carry a kernel's DITTO_EPILOGUE_* bit like the call's `epilogue` argument

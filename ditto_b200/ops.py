@@ -232,7 +232,7 @@ def _scratch(lib, op, batch, M, N, K, L, dtype, device):
 
 
 def gemm_relu_gemm(x, w1, w2, out=None, activation="relu", weight_layout="IO", variant="auto", workspace="auto"):
-    """out = act(x @ w1) @ w2, fused: the hidden activations stay in L2 (scratch memory) or inside a cluster.
+    """out = act(x @ w1) @ w2, fused: the hidden activations pass through scratch memory or stay inside a cluster.
 
     x [batch, M, K] or [M, K]; w1 [batch, K, L] / [K, L]; w2 [batch, L, N] / [L, N] when
     weight_layout == "IO" ([in, out]); "OI" takes the transposed [out, in] weights of
