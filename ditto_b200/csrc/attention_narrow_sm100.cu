@@ -43,7 +43,8 @@ constexpr uint32_t kColO = 64;
 // second block (with the first, the other kernels' first block), within 5 later (8 there).  Error against float64, other
 // kernels / this one with 8 throughout / this one: 2.88e-4 / 2.90e-4 / 2.88e-4 for fp16 rows of 512 keys at
 // scale d^-0.5, 2.19e-4 / 2.28e-4 / 2.15e-4 unscaled; 144 keys at 0.35, simulated, 2.33e-4 / 2.60e-4 / 2.29e-4.
-// The price is about one rescale an item, 56.4 -> 58.2 us for 2048 items of 512 keys.
+// The price is about one rescale an item, 56.4 -> 58.2 us for 2048 items of 512 keys, 7.5 -> 8.0 for one wave of 304; all
+// of O in one piece, or the rescale behind P, spill or delay every item (65.6 and 59.0 us).
 constexpr float kRescaleThreshold = 5.0f, kSecondBlockThreshold = 1.0f;
 constexpr int kModeSoftmax = 0, kModeRelu = 1;
 
