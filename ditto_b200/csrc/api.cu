@@ -43,21 +43,36 @@ int make_map_3d(CUtensorMap* map, bool bf16, const void* base, uint64_t cols, ui
   return ditto_b200::make_tensor_map(map, bf16, base, 3, dims, strides, box);
 }
 
-// CTAs that share an item's keys: as the caller's flags say, else by shape unless they name another tiling.
-int parts_for(int flags, bool any, long long batch, int M, int L, int d, int mode = 0) {
-  const int asked = (flags & DITTO_FLAG_SPLIT_MASK) / DITTO_FLAG_SPLIT_UNIT, blocks = (L + 127) / 128;
-  if (!any || (asked == 0 && batch > 4096)) return 1;
-  if (asked == 0) return ditto_b200::attention_parts(static_cast<int>(batch), M, L, d, mode);
-  int parts = 1 << (asked - 1);
-  while (parts > blocks) parts /= 2;
-  return parts;
-}
-
 // The kernel with 64-key blocks (head dimensions up to 64): where the caller asks for it, or by shape.
 bool narrow_for(int flags, bool any, long long batch, int M, int L, int d, int mode = 0) {
   if (!any || d != 64) return false;
   if (flags & DITTO_FLAG_NARROW) return true;
-  return !(flags & DITTO_FLAG_SPLIT_MASK) && ditto_b200::attention_narrow_pays(static_cast<int>(batch), M, L, mode);
+  return !(flags & DITTO_FLAG_SPLIT_MASK) && ditto_b200::attention_narrow_pays(static_cast<int>(batch), M, L, mode) &&
+         !ditto_b200::attention_few(static_cast<int>(batch), M, L, d, mode).here;
+}
+
+// The form of an attention-shaped call: as the caller's flags say, else by shape.  The 64-key kernel is settled before (`narrow`: its
+// tensor maps have boxes of their own), `any` says that the flags name no tiling.
+cudaError_t launch_attention_form(const ditto_b200::AttnParams& p, int slices, int d, bool bf16, int nt, bool psmem, int mode,
+                                  int flags, bool any, bool narrow, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (narrow) return ditto_b200::launch_attention_narrow(p, slices, bf16, mode, st);
+  if (any) {
+    const int asked = (flags & DITTO_FLAG_SPLIT_MASK) / DITTO_FLAG_SPLIT_UNIT, blocks = (p.L + 127) / 128;
+    ditto_b200::AttnFew few = {1, false};
+    if (asked == 0) {
+      few = ditto_b200::attention_few(slices, p.M, p.L, d, mode);
+    } else {
+      few.parts = 1 << (asked - 1);
+      while (few.parts > blocks) few.parts /= 2;
+      few.here = few.parts > 1;
+    }
+    if (few.here) return ditto_b200::launch_attention_short(p, slices, d, bf16, mode, few.parts, st);
+    if (few.parts > 1) return ditto_b200::launch_attention_split(p, slices, bf16, mode, few.parts, st);
+    // few key blocks per item: the persistent kernel hides the per-item start-up, which long sequences amortise anyway
+    if (d == 64 && p.L <= kPersistentMaxKeys) return ditto_b200::launch_attention_persistent(p, slices, bf16, mode, st);
+  }
+  return ditto_b200::launch_attention(p, slices, d, bf16, nt, psmem, mode, st);
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -122,15 +137,7 @@ int ditto_b200_bmm_softmax_bmm(const void* q, const void* k, const void* v, void
 #ifdef DITTO_TRACE
   p.trace = ws_bytes >= 1280 * sizeof(long long) ? static_cast<long long*>(workspace) : nullptr;
 #endif
-  // head dimensions up to 64 with few key blocks per item take the persistent kernel (it hides the
-  // per-item start-up, which long sequences amortise anyway) unless a flag asks for a specific tiling
-  const bool persistent = any && d == 64 && L <= kPersistentMaxKeys;
-  const int parts = parts_for(flags, any, batch, M, L, d);
-  cudaError_t e = narrow      ? ditto_b200::launch_attention_narrow(p, batch, bf16, 0, static_cast<cudaStream_t>(stream))
-                  : parts > 1 ? ditto_b200::launch_attention_split(p, batch, d, bf16, 0, parts, static_cast<cudaStream_t>(stream))
-                  : persistent
-                      ? ditto_b200::launch_attention_persistent(p, batch, bf16, 0, static_cast<cudaStream_t>(stream))
-                      : ditto_b200::launch_attention(p, batch, d, bf16, nt, psmem, 0, static_cast<cudaStream_t>(stream));
+  const cudaError_t e = launch_attention_form(p, batch, d, bf16, nt, psmem, 0, flags, any, narrow, stream);
   if (e != cudaSuccess) return cuda_fail("bmm_softmax_bmm launch", e);
   return DITTO_OK;
 }
@@ -172,15 +179,7 @@ int ditto_b200_multi_head_attention(const void* qkv, void* out, int batch, int M
   p.out_ld = hidden;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = status_word;
-  const bool persistent = any && d == 64 && M <= kPersistentMaxKeys;
-  const int parts = parts_for(flags, any, batch * heads, M, M, d);
-  cudaError_t e = narrow      ? ditto_b200::launch_attention_narrow(p, batch * heads, bf16, 0, static_cast<cudaStream_t>(stream))
-                  : parts > 1 ? ditto_b200::launch_attention_split(p, batch * heads, d, bf16, 0, parts,
-                                                                 static_cast<cudaStream_t>(stream))
-                  : persistent ? ditto_b200::launch_attention_persistent(p, batch * heads, bf16, 0,
-                                                                       static_cast<cudaStream_t>(stream))
-                             : ditto_b200::launch_attention(p, batch * heads, d, bf16, nt, false, 0,
-                                                            static_cast<cudaStream_t>(stream));
+  const cudaError_t e = launch_attention_form(p, batch * heads, d, bf16, nt, false, 0, flags, any, narrow, stream);
   if (e != cudaSuccess) return cuda_fail("multi_head_attention launch", e);
   return DITTO_OK;
 }
@@ -239,12 +238,7 @@ int ditto_b200_gemm_relu_gemm(const void* x, const void* w1, const void* w2, voi
     p.scale_log2 = 1.0f;
     p.status = status_word;
     const int nt = (dk == 64 || M <= 128) ? 1 : 2;
-    const int parts = parts_for(0, true, batch, M, L, dk, mode);
-    cudaError_t e = narrow      ? ditto_b200::launch_attention_narrow(p, batch, bf16, mode, static_cast<cudaStream_t>(stream))
-                    : parts > 1 ? ditto_b200::launch_attention_split(p, batch, dk, bf16, mode, parts, static_cast<cudaStream_t>(stream))
-                    : (dk == 64 && L <= kPersistentMaxKeys) ? ditto_b200::launch_attention_persistent(p, batch, bf16, mode, static_cast<cudaStream_t>(stream))
-                             : ditto_b200::launch_attention(p, batch, dk, bf16, nt, false, mode,
-                                                            static_cast<cudaStream_t>(stream));
+    const cudaError_t e = launch_attention_form(p, batch, dk, bf16, nt, false, mode, 0, true, narrow, stream);
     if (e != cudaSuccess) return cuda_fail("gemm_relu_gemm launch", e);
     return DITTO_OK;
   }

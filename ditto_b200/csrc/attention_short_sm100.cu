@@ -1,0 +1,610 @@
+// Fused bmm -> softmax -> bmm for calls of few items: one 128-row tile per CTA, or per cluster of CTAs that divide its keys
+// between them, and two softmax warps on every quarter of the rows.
+//
+// Such a call lasts as long as one CTA: set-up, first loads, its blocks of 128 keys one after another, write-out.  Little else
+// runs on the SM meanwhile, so a block should take as little time as the chain
+//   scores in tensor memory -> registers -> row maximum -> exponentials -> P in tensor memory -> P*V
+// allows.  With one thread a row (the other kernels) each of the four warps has its sub-partition's units to itself and
+// leaves them idle whenever it waits; here two warps share a row's 128 scores -- 32-key groups 0 and 2, and 1 and 3 -- and
+// tell each other their maxima through shared memory.  S, O and P have tensor-memory columns of their own, so the next
+// block's scores are ready by then, and a last block ends with its keys.
+//
+// Roles: warps 0-7 softmax and write-out (warps w and w + 4: rows 32 w .. 32 w + 31, TMEM lanes alike), 8 loads, 9 MMAs.
+// With `parts` CTAs in the cluster each takes a contiguous part of the tile's blocks; they combine (max, sum, O) through
+// distributed shared memory at the end.
+//
+// Two CTAs fit an SM at head dimension 64 (83 KB, 256 tensor-memory columns, 95 registers): the next call's are set up under this
+// one's.  What it measured stands at attention_few.
+#include "attention_sm100.cuh"
+
+#include <algorithm>
+#include <atomic>
+
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include "host_util.cuh"
+#include "mlp_common.cuh"
+#include "sm100_ptx.cuh"
+#include "softmax_step.cuh"
+
+namespace ditto_b200 {
+
+namespace {
+
+constexpr int kBM = 128, kBN = 128;
+constexpr int kStages = 2;
+constexpr int kSoftmaxWarps = 8, kWarpLoad = 8, kWarpMma = 9;
+constexpr int kThreads = 10 * 32;
+constexpr int kFirstKeys = 64;            // of a block, in the first part of P (groups 0 and 1); the rest follows by itself
+// As in the kernel with 64-key blocks, some of whose calls come here: the closer a row's reference follows its maximum, the
+// smaller the rounding error of its largest weights.
+constexpr float kRescaleThreshold = 5.0f, kSecondBlockThreshold = 1.0f;
+constexpr int kModeSoftmax = 0, kModeRelu = 1;
+
+template <int D>
+struct Layout {
+  static constexpr int kTileQ = kBM * D * 2;
+  static constexpr int kTileKV = kBN * D * 2;
+  static constexpr int kOffQ = 0;
+  static constexpr int kOffK = kOffQ + kTileQ;
+  static constexpr int kOffV = kOffK + kStages * kTileKV;
+  static constexpr int kOffPair = kOffV + kStages * kTileKV;      // float [2][2][128]: maxima, by parity of the block and half
+  static constexpr int kOffRows = kOffPair + 2 * 2 * kBM * 4;     // float2 [128]: (max, sum) for the cluster
+  static constexpr int kOffBar = kOffRows + kBM * 8;
+  static constexpr int kBytes = kOffBar + 256 + 1024;
+  static constexpr uint32_t kColS = 0, kColO = 128, kColP = 128 + D;
+  static constexpr uint32_t kTmemCols = D == 64 ? 256 : 512;
+};
+
+struct SBars {
+  uint64_t q_full, k_full[kStages], k_empty[kStages], v_full[kStages], v_empty[kStages];
+  uint64_t s_full, s_taken, p_part[2], o_done;
+  uint64_t pair[4];                       // the two warps of a quarter have written what the other one reads
+  uint32_t tmem_base;
+  uint32_t abort_word;
+};
+static_assert(sizeof(SBars) <= 256, "barrier block too large");
+
+// The largest of 32 scores and m.
+__device__ __forceinline__ float max_with(float m, const uint32_t* s) {
+  auto v = [&](int i) { return __uint_as_float(s[i]); };
+  float a[4] = {m, v(0), v(1), v(2)};
+  // 29 scores left, two at a time on four chains
+#pragma unroll
+  for (int i = 3; i < 27; i += 8) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) a[u] = max3(a[u], v(i + 2 * u), v(i + 2 * u + 1));
+  }
+  a[0] = max3(a[0], v(27), v(28));
+  a[1] = max3(a[1], v(29), v(30));
+  a[2] = max3(a[2], a[3], v(31));
+  return max3(a[0], a[1], a[2]);
+}
+
+// 32 scores of a row -> their weights 2^(s c - mc), rounded to the operand type and packed; the sums take them before rounding.
+template <bool BF16>
+__device__ __forceinline__ void softmax_weights(const uint32_t* s, float c, float mc, float& sum0, float& sum1, uint32_t (&w)[16]) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const float a = ex2_approx(fmaf(__uint_as_float(s[2 * i]), c, -mc)), b = ex2_approx(fmaf(__uint_as_float(s[2 * i + 1]), c, -mc));
+    sum0 += a;
+    sum1 += b;
+    w[i] = pack2<BF16>(a, b);
+  }
+}
+
+// The same place of the chains without a softmax.
+template <bool BF16, bool RELU>
+__device__ __forceinline__ void pass_on(const uint32_t* s, uint32_t (&w)[16]) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    float a = __uint_as_float(s[2 * i]), b = __uint_as_float(s[2 * i + 1]);
+    if constexpr (RELU) {                              // if_then_else(D > 0, D, 0) as in the reference
+      a = a > 0.f ? a : 0.f;
+      b = b > 0.f ? b : 0.f;
+    }
+    w[i] = pack2<BF16>(a, b);
+  }
+}
+
+}  // namespace
+
+template <bool BF16, int D, int MODE>
+__global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __grid_constant__ AttnParams p) {
+  using SM = Layout<D>;
+  constexpr int kAtoms = D / 64;
+  extern __shared__ uint8_t smem_raw[];
+  // the CTAs of a cluster round up by the same amount: offsets match across the cluster
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  SBars* bar = reinterpret_cast<SBars*>(smem + SM::kOffBar);
+  volatile uint32_t* abort_word = &bar->abort_word;
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int tiles = (p.M + kBM - 1) / kBM;
+  // the CTAs of a cluster are consecutive: rank r of `parts` takes K/V blocks [r * n / parts, (r + 1) * n / parts)
+  const int parts = p.parts, part = static_cast<int>(cluster_ctarank());
+  const int id = static_cast<int>(blockIdx.x) / parts;
+  const int slice = id / tiles, seq = slice / p.heads;
+  const int head_col = (slice - seq * p.heads) * p.d;
+  const int m0 = (id - slice * tiles) * kBM;
+  const int blocks = (p.L + kBN - 1) / kBN;
+  const int j0 = part * blocks / parts, nkv = (part + 1) * blocks / parts - j0;
+  // keys of this CTA's last block, a multiple of 16
+  const int last_keys = part == parts - 1 ? p.L - (blocks - 1) * kBN : kBN;
+
+  if (threadIdx.x == 0) {
+    mbar_init(&bar->q_full, 1);
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&bar->k_full[s], 1);
+      mbar_init(&bar->k_empty[s], 1);
+      mbar_init(&bar->v_full[s], 1);
+      mbar_init(&bar->v_empty[s], 1);
+    }
+    mbar_init(&bar->s_full, 1);
+    mbar_init(&bar->s_taken, kSoftmaxWarps);
+    mbar_init(&bar->p_part[0], kSoftmaxWarps);
+    mbar_init(&bar->p_part[1], kSoftmaxWarps);
+    mbar_init(&bar->o_done, 1);
+    for (int q = 0; q < 4; ++q) mbar_init(&bar->pair[q], 2);
+    bar->abort_word = 0;
+    fence_mbar_init();
+  }
+  if (warp == 0) {
+    tmem_alloc(&bar->tmem_base, SM::kTmemCols);
+    tmem_relinquish();
+  }
+  if (warp == kWarpLoad && lane == 0) {
+    tma_prefetch_desc(&p.map_q);
+    tma_prefetch_desc(&p.map_k);
+    tma_prefetch_desc(&p.map_v);
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = bar->tmem_base;
+  // Programmatic dependent launch: nothing above touches global memory.
+  grid_dependency_wait();
+  grid_launch_dependents();
+
+  bool ok = true;
+  float row_m = 0.f, row_l = 0.f;          // this CTA's maximum and sum of the thread's row
+  const int quarter = warp & 3, half = (warp >> 2) & 1;
+  const int row = quarter * 32 + lane;
+  const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+
+  if (warp == kWarpLoad) {
+    // ------------------------------------------------------------ TMA producer (one thread)
+    if (lane == 0) {
+      mbar_arrive_expect_tx(&bar->q_full, SM::kTileQ);
+      for (int a = 0; a < kAtoms; ++a)
+        tma_load_3d(smem + SM::kOffQ + a * (kBM * 128), &p.map_q, &bar->q_full, p.q_col0 + head_col + a * 64, m0, seq);
+      for (int j = 0; j < nkv; ++j) {
+        const int s = j % kStages;
+        const uint32_t ph = (j / kStages) & 1;
+        ok = mbar_wait(&bar->k_empty[s], ph ^ 1, abort_word, 0x100 + j);
+        if (!ok) break;
+        uint8_t* k = smem + SM::kOffK + s * SM::kTileKV;
+        mbar_arrive_expect_tx(&bar->k_full[s], SM::kTileKV);
+        if (p.k_transposed) {
+          for (int a = 0; a < kBN / 64; ++a)
+            tma_load_3d(k + a * (D * 128), &p.map_k, &bar->k_full[s], (j0 + j) * kBN + a * 64, 0, slice);
+        } else {
+          for (int a = 0; a < kAtoms; ++a)
+            tma_load_3d(k + a * (kBN * 128), &p.map_k, &bar->k_full[s], p.k_col0 + head_col + a * 64, (j0 + j) * kBN, seq);
+        }
+        ok = mbar_wait(&bar->v_empty[s], ph ^ 1, abort_word, 0x200 + j);
+        if (!ok) break;
+        uint8_t* v = smem + SM::kOffV + s * SM::kTileKV;
+        mbar_arrive_expect_tx(&bar->v_full[s], SM::kTileKV);
+        if (p.v_transposed) {
+          for (int a = 0; a < kBN / 64; ++a)
+            tma_load_3d(v + a * (D * 128), &p.map_v, &bar->v_full[s], (j0 + j) * kBN + a * 64, 0, slice);
+        } else {
+          for (int a = 0; a < kAtoms; ++a)
+            tma_load_3d(v + a * (kBN * 128), &p.map_v, &bar->v_full[s], p.v_col0 + head_col + a * 64, (j0 + j) * kBN, seq);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == kWarpMma) {
+    // ------------------------------------------------------------ MMA issuer (converged warp, elected lane issues)
+    const uint32_t issuer = elect_one();
+    const bool kt = p.k_transposed != 0, vt = p.v_transposed != 0;
+    const int ksteps_d = p.d / 16;
+    const uint32_t idesc_s = umma_idesc_f16(BF16, kBM, kBN, false, kt);
+    const uint32_t idesc_o = umma_idesc_f16(BF16, kBM, p.dv, false, !vt);   // (columns past dv are not stored)
+    const uint64_t dq = umma_desc_sw128(smem_u32(smem + SM::kOffQ), 16, 1024);
+    const uint64_t dk0 = kt ? umma_desc_sw128(smem_u32(smem + SM::kOffK), D * 128, 1024) : umma_desc_sw128(smem_u32(smem + SM::kOffK), 16, 1024);
+    const uint64_t dv0 = vt ? umma_desc_sw128(smem_u32(smem + SM::kOffV), 16, 1024) : umma_desc_sw128(smem_u32(smem + SM::kOffV), kBN * 128, 1024);
+    auto wait = [&](uint64_t* b, uint32_t parity, uint32_t code) {
+      bool r = mbar_wait(b, parity, abort_word, code);
+      r = __all_sync(0xffffffffu, r);
+      tc_fence_after_sync();
+      return r;
+    };
+    auto issue_s = [&](int stage) {
+      const uint64_t db = dk0 + ((stage * SM::kTileKV) >> 4);
+#pragma unroll
+      for (int i = 0; i < D / 16; ++i) {
+        const uint32_t off = ((i / 4) * (kBM * 128) + (i % 4) * 32) >> 4;
+        if (i < ksteps_d)
+          umma_ss_elected(tmem_base + SM::kColS, dq + off, db + (kt ? static_cast<uint32_t>((i * 2048) >> 4) : off), idesc_s,
+                          i > 0 ? 1u : 0u, issuer);
+      }
+      umma_commit_elected(&bar->s_full, issuer);
+      umma_commit_elected(&bar->k_empty[stage], issuer);
+    };
+    auto issue_pv = [&](int stage, int from, int to, bool first) {
+      const uint64_t db = dv0 + ((stage * SM::kTileKV) >> 4);
+#pragma unroll
+      for (int i = 0; i < kFirstKeys / 16; ++i) {
+        const int step = from / 16 + i;
+        if (step * 16 < to) {
+          const uint32_t off = vt ? static_cast<uint32_t>(((step / 4) * (D * 128) + (step % 4) * 32) >> 4) : static_cast<uint32_t>((step * 2048) >> 4);
+          umma_ts_elected(tmem_base + SM::kColO, tmem_base + SM::kColP + step * 8, db + off, idesc_o, first && i == 0 ? 0u : 1u, issuer);
+        }
+      }
+    };
+    ok = wait(&bar->k_full[0], 0, 0x300) && wait(&bar->q_full, 0, 0x301);
+    if (ok) issue_s(0);
+    for (int j = 0; j < nkv && ok; ++j) {
+      const int st = j % kStages, sn = (j + 1) % kStages;
+      const bool more = j + 1 < nkv;
+      const int keys = more ? kBN : last_keys;
+      if (more) {
+        // the softmax warps must have taken S(j) out of tensor memory before S(j + 1) lands there
+        ok = wait(&bar->k_full[sn], ((j + 1) / kStages) & 1, 0x310) && wait(&bar->s_taken, j & 1, 0x320);
+        if (!ok) break;
+        issue_s(sn);
+      }
+      ok = wait(&bar->v_full[st], (j / kStages) & 1, 0x330) && wait(&bar->p_part[0], j & 1, 0x340);
+      if (!ok) break;
+      issue_pv(st, 0, min(keys, kFirstKeys), j == 0);
+      ok = wait(&bar->p_part[1], j & 1, 0x350);
+      if (!ok) break;
+      issue_pv(st, kFirstKeys, keys, false);
+      umma_commit_elected(&bar->v_empty[st], issuer);     // also tells the softmax warps that P*V(j) is done
+      if (!more) umma_commit_elected(&bar->o_done, issuer);
+    }
+  } else {
+    // ------------------------------------------------------------ softmax (warps 0-7)
+    const uint32_t s_col = lane_base + SM::kColS, o_col = lane_base + SM::kColO + half * (D / 2), p_col = lane_base + SM::kColP;
+    const float c = p.scale_log2;
+    float* told = reinterpret_cast<float*>(smem + SM::kOffPair) + row;     // [parity][half][row]
+    RowReference ref(c);
+    float l = 0.f;
+    for (int j = 0; j < nkv; ++j) {
+      const uint32_t par = j & 1;
+      ok = mbar_wait(&bar->s_full, par, abort_word, 0x800);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after_sync();
+      uint32_t sv[64];                                     // groups `half` and 2 + `half` of 32 keys
+      tmem_ld_2x32_wait(s_col + 32 * half, s_col + 64 + 32 * half, sv);
+      tc_fence_before_sync();
+      mbar_arrive_warp(&bar->s_taken, lane);
+      const int keys = j == nkv - 1 ? last_keys : kBN;
+      if constexpr (MODE == kModeSoftmax) {
+        if (keys != kBN) {
+          // a partial last block brings zero-filled rows, whose scores must not count
+#pragma unroll
+          for (int i = 0; i < 64; ++i)
+            if (64 * (i / 32) + 32 * half + i % 32 >= keys) sv[i] = __float_as_uint(-INFINITY);
+        }
+        float m_new = max_with(max_with(ref.m, sv), sv + 32);
+        told[(par * 2 + half) * kBM] = m_new;
+        mbar_arrive_warp(&bar->pair[quarter], lane);
+        ok = mbar_wait(&bar->pair[quarter], par, abort_word, 0x880);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        m_new = fmaxf(m_new, told[(par * 2 + (half ^ 1)) * kBM]);
+        if (j > 0) {
+          // P*V(j-1) must have finished before P is overwritten or O is rescaled (S(j) was issued ahead of it)
+          ok = mbar_wait(&bar->v_empty[(j - 1) % kStages], ((j - 1) / kStages) & 1, abort_word, 0x900);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after_sync();
+        }
+        // lazy rescale, as in attention_sm100.cu; both warps of a quarter see the same maxima and decide alike
+        if (__any_sync(0xffffffffu, ref.asks(m_new, c, j == 1 ? kSecondBlockThreshold : kRescaleThreshold))) {
+          const float f = ref.move(m_new, c);
+          if (j > 0) {
+#pragma unroll 1
+            for (int h = 0; h < D / 2; h += 16) {
+              uint32_t o[16];
+              tmem_ld_x16_wait(o_col + h, o);
+#pragma unroll
+              for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
+              tmem_st_x16(o_col + h, o);
+            }
+            tmem_wait_st();
+          }
+          l *= f;
+          ref.subtract(sv);
+        }
+      } else if (j > 0) {
+        ok = mbar_wait(&bar->v_empty[(j - 1) % kStages], ((j - 1) / kStages) & 1, abort_word, 0x900);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after_sync();
+      }
+      const float mc = ref.offset(c);
+      float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        if (64 * g + 32 * half < keys) {                   // (P*V reads no others)
+          uint32_t w[16];
+          if constexpr (MODE == kModeSoftmax) softmax_weights<BF16>(sv + 32 * g, c, mc, sum0, sum1, w);
+          else pass_on<BF16, MODE == kModeRelu>(sv + 32 * g, w);
+          tmem_st_x16(p_col + 32 * g + 16 * half, w);
+        }
+        tmem_wait_st();
+        tc_fence_before_sync();
+        mbar_arrive_warp(&bar->p_part[g], lane);
+      }
+      l += sum0 + sum1;
+    }
+    if (ok && MODE == kModeSoftmax) {
+      // the row's sum, in the same order in both warps
+      told[((nkv & 1) * 2 + half) * kBM] = l;
+      mbar_arrive_warp(&bar->pair[quarter], lane);
+      ok = mbar_wait(&bar->pair[quarter], nkv & 1, abort_word, 0x890);
+      ok = __all_sync(0xffffffffu, ok);
+      if (ok) l = told[(nkv & 1) * 2 * kBM] + told[((nkv & 1) * 2 + 1) * kBM];
+    }
+    if (ok) {
+      ok = mbar_wait(&bar->o_done, 0, abort_word, 0xA00);
+      ok = __all_sync(0xffffffffu, ok);
+      tc_fence_after_sync();
+    }
+    row_m = ref.m;
+    row_l = l;
+    if (ok && parts == 1) {
+      const float inv = MODE == kModeSoftmax ? 1.0f / l : 1.0f;
+      // Turned around in 2 or 4 KB of the K ring per warp (every MMA has retired), 16-byte pieces swizzled by row, so that a
+      // store instruction writes rows of 64 or 128 contiguous bytes.
+      constexpr int kPieces = D / 16;                      // 16-byte pieces of a row's half
+      uint8_t* stage = smem + SM::kOffK + warp * (kPieces * 512);
+      uint32_t o[D / 2];
+      if constexpr (D == 128) tmem_ld_x64_wait(o_col, o); else tmem_ld_x32_wait(o_col, o);
+#pragma unroll
+      for (int i = 0; i < kPieces; ++i) {
+        uint32_t w[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          w[u] = pack2<BF16>(__uint_as_float(o[8 * i + 2 * u]) * inv, __uint_as_float(o[8 * i + 2 * u + 1]) * inv);
+        const int at = D == 128 ? i ^ (lane & 7) : i ^ ((lane >> 1) & 3);
+        *reinterpret_cast<uint4*>(stage + lane * (kPieces * 16) + at * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+      __syncwarp();
+      const size_t out_row0 = static_cast<size_t>(seq) * p.M + m0 + quarter * 32;
+      constexpr int kRowsAtOnce = 32 / kPieces;
+#pragma unroll
+      for (int i = 0; i < kPieces; ++i) {
+        const int rr = kRowsAtOnce * i + lane / kPieces, piece = lane % kPieces;
+        const int at = D == 128 ? piece ^ (rr & 7) : piece ^ ((rr >> 1) & 3);
+        const uint4 v = *reinterpret_cast<const uint4*>(stage + rr * (kPieces * 16) + at * 16);
+        const int col = half * (D / 2) + piece * 8;        // widths are multiples of 16: whole 16-byte pieces
+        if (m0 + quarter * 32 + rr < p.M && col < p.dv)
+          *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) + ((out_row0 + rr) * p.out_ld + head_col + col) * 2) = v;
+      }
+    }
+  }
+
+  if (parts > 1) {
+    // Combine the parts.  Every CTA publishes its rows' (max, sum), scales its O by
+    // 2^(max - overall max) / overall sum and hands D / parts columns of it to each CTA of the cluster, which adds
+    // what it was given and writes those columns of the result: a reduce-scatter, so the exchange (D * 512 bytes in
+    // and out of every CTA) and the write-out are spread over the cluster.  Parts are added in rank order.
+    // The incoming pieces go to the K ring, idle since the last P*V of this CTA (first cluster barrier); laid out
+    // [source][16-byte piece][row], a warp's store or load covers 512 contiguous bytes.  Both barriers are reached
+    // by every thread whether its waits expired or not.
+    float2* ml = reinterpret_cast<float2*>(smem + SM::kOffRows) + row;
+    if (warp < 4 && MODE == kModeSoftmax) *ml = make_float2(row_m, row_l);
+    __syncwarp();
+    cluster_sync_all();
+    const int cols = D / parts;                        // columns of the result that one CTA adds up: 8 to 64
+    const int cols_log2 = 31 - __clz(cols);
+    if (warp < kSoftmaxWarps) {
+      float f = 1.f;
+      if constexpr (MODE == kModeSoftmax) {
+        const uint32_t at = smem_u32(ml);
+        float mv[8], lv[8], top = -INFINITY;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          if (r < parts) {
+            ld_cluster_v2(map_to_cta(at, r), mv[r], lv[r]);
+            top = fmaxf(top, mv[r]);
+          }
+        }
+        float total = 0.f;
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+          if (r < parts) total = fmaf(lv[r], ex2_approx((mv[r] - top) * p.scale_log2), total);
+        f = ex2_approx((row_m - top) * p.scale_log2) / total;
+      }
+      const uint32_t in0 = smem_u32(smem + SM::kOffK) + (part * (cols / 4) * kBM + row) * 16;
+#pragma unroll 1
+      for (int h = half * 32; h < D; h += 64) {
+        uint32_t o[32];
+        tmem_ld_x32_wait(lane_base + SM::kColO + h, o);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int col = h + 4 * q;
+          st_cluster_v4(map_to_cta(in0 + (col & (cols - 1)) * (kBM * 4), col >> cols_log2), __uint_as_float(o[4 * q]) * f,
+                        __uint_as_float(o[4 * q + 1]) * f, __uint_as_float(o[4 * q + 2]) * f,
+                        __uint_as_float(o[4 * q + 3]) * f);
+        }
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();
+    if (warp < kSoftmaxWarps && m0 + row < p.M) {
+      const float4* in = reinterpret_cast<const float4*>(smem + SM::kOffK) + row;
+      uint8_t* dst = reinterpret_cast<uint8_t*>(p.out) + ((static_cast<size_t>(seq) * p.M + m0 + row) * p.out_ld + head_col) * 2;
+#pragma unroll 1
+      for (int c8 = half; c8 < cols / 8; c8 += 2) {
+        const int col = part * cols + 8 * c8;        // widths are multiples of 16: whole 16-byte pieces
+        if (col >= p.dv) break;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+#pragma unroll 2
+        for (int r = 0; r < parts; ++r) {
+          const float4 u = in[(r * (cols / 4) + 2 * c8) * kBM], v = in[(r * (cols / 4) + 2 * c8 + 1) * kBM];
+          a.x += u.x; a.y += u.y; a.z += u.z; a.w += u.w;
+          b.x += v.x; b.y += v.y; b.z += v.z; b.w += v.w;
+        }
+        *reinterpret_cast<uint4*>(dst + col * 2) =
+            make_uint4(pack2<BF16>(a.x, a.y), pack2<BF16>(a.z, a.w), pack2<BF16>(b.x, b.y), pack2<BF16>(b.z, b.w));
+      }
+    }
+  }
+
+  // After a wait has given up, TMA loads this CTA has armed may still be in flight; they complete within microseconds.
+  if (*abort_word != 0u) {
+    for (int t = 0; t < 64; ++t) __nanosleep(1000);
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    tmem_dealloc(tmem_base, SM::kTmemCols);
+    if (lane == 0 && bar->abort_word != 0 && p.status != nullptr) atomicCAS(p.status, 0, static_cast<int>(bar->abort_word));
+  }
+}
+
+// ------------------------------------------------------------------ launcher
+template <bool BF16, int D, int MODE>
+static cudaError_t launch_s(const AttnParams& p, int ctas, cudaStream_t stream) {
+  using SM = Layout<D>;
+  auto kern = attention_short_kernel<BF16, D, MODE>;
+  static std::atomic<unsigned long long> configured{0};
+  int dev = 0;
+  cudaError_t e = current_device_checked(&dev);
+  if (e != cudaSuccess) return e;
+  if (!device_configured(configured, dev)) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::kBytes);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+    mark_device_configured(configured, dev);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(ctas), 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = SM::kBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see grid_dependency_wait in the kernel
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(p.parts);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.parts > 1 ? 2 : 1;
+  return launch_kernel(cfg, kern, p);
+}
+
+cudaError_t launch_attention_short(const AttnParams& params, int batch, int d, bool bf16, int mode, int parts, cudaStream_t stream) {
+  const int blocks = (params.L + kBN - 1) / kBN;
+  const long long ctas = static_cast<long long>((params.M + kBM - 1) / kBM) * batch * parts;
+  if ((parts != 1 && parts != 2 && parts != 4 && parts != 8) || parts > blocks || ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
+  AttnParams p = params;
+  p.parts = parts;
+  const int n = static_cast<int>(ctas);
+#define DITTO_DISPATCH(BF, DD) \
+  if (bf16 == BF && d == DD)   \
+    return mode == 0 ? launch_s<BF, DD, 0>(p, n, stream) : mode == 1 ? launch_s<BF, DD, 1>(p, n, stream) : launch_s<BF, DD, 2>(p, n, stream);
+  DITTO_DISPATCH(false, 64)
+  DITTO_DISPATCH(false, 128)
+  DITTO_DISPATCH(true, 64)
+  DITTO_DISPATCH(true, 128)
+#undef DITTO_DISPATCH
+  return cudaErrorInvalidValue;
+}
+
+// Clusters of `parts` CTAs the device holds at once.
+template <int D>
+static int cluster_places(int lg) {
+  static std::atomic<int> places[kMaxDevices][4];       // 0: not looked up yet; else clusters + 1
+  int dev = 0;
+  if (current_device_checked(&dev) != cudaSuccess) return 0;
+  int n = places[dev][lg].load(std::memory_order_relaxed);
+  if (n == 0) {
+    using SM = Layout<D>;
+    auto kern = attention_short_kernel<false, D, kModeSoftmax>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1024, 1, 1);
+    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.dynamicSmemBytes = SM::kBytes;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1u << lg;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int count = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::kBytes) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&count, kern, &cfg) != cudaSuccess)
+      return 0;
+    n = std::max(0, count) + 1;
+    places[dev][lg].store(n, std::memory_order_relaxed);
+  }
+  return n - 1;
+}
+
+// Times of a launch of this kernel (us, one call after another): fixed + per 128-key block of a CTA, fitted to 396 shapes of 1 to
+// 296 items and 1 to 64 blocks, fp16, with and without a softmax (rms 4 to 7 %).  With more CTAs than SMs two share one at
+// head dimension 64 (kShared); at 128 shared memory holds one.  More clusters than the device holds at once would be a
+// second wave, which costs more than a split saves.
+namespace {
+struct Times { double one, one_block, one_full, split, part, split_block, split_full; };      // *_full: over 100 CTAs
+constexpr Times kAlone[2][2] = {{{3.3, 1.28, 0.7, 4.3, 0.12, 1.30, 1.4}, {3.0, 0.89, 0.4, 3.7, 0.09, 0.92, 0.6}},      // [head dimension][no softmax]
+                                {{3.6, 1.39, 1.2, 5.7, 0.13, 1.37, 1.3}, {3.0, 1.14, 1.0, 4.5, 0.16, 1.16, 1.2}}};
+struct Shared { double split, part, block, full; };
+constexpr Shared kShared[2] = {{5.4, 0.30, 1.93, 0.8}, {4.2, 0.13, 1.38, 1.0}};
+}  // namespace
+
+// Where the lines lie, other kernels -> this one (us), items x blocks.  Softmax at head dimension 64: 24 x 1 5.4 -> 5.0, 24 x 2 6.6 -> 5.7, 24 x 4
+// 7.5 -> 6.5 (4 parts), 24 x 16 11.2 -> 10.6 (4), 48 x 16 15.6 -> 13.9 (4), 100 x 32 43.8 -> 37.1 (2); at 128: 24 x 1 5.7 -> 5.1, 24 x 2 7.3 ->
+// 6.3, 24 x 4 9.7 -> 8.5 (4), 24 x 16 14.9 -> 12.8 (4), 48 x 16 21.9 -> 18.9 (2), 100 x 32 64.6 -> 55.4.  Split over few CTAs with long parts
+// the kernel with a thread a row costs less per block at head dimension 64 (1.16 against 1.30: no word from another warp before the
+// exponentials): 74 x 32 27.4 -> 27.7, 74 x 64 46.4 -> 48.7; without a softmax from four blocks on (48 x 8 7.4 -> 7.8, 12 x 64 10.7 ->
+// 12.0), and 148 x 1 4.4 -> 4.7.  Unsplit and two CTAs an SM it pays for up to four blocks (200 x 2 8.1 -> 7.6, 256 x 4 12.3 -> 11.9;
+// 296 x 8 22.3 -> 22.5).  One tile a sequence at head dimension 128 has no second tile to work beside: there it pays in any number
+// from six blocks on (200 x 8 36.8 -> 33.2, 256 x 16 69.0 -> 58.1).
+AttnFew attention_few(int batch, int M, int L, int d, int mode) {
+  constexpr int kSms = 148;
+  const long long items = static_cast<long long>((M + kBM - 1) / kBM) * batch;
+  const int blocks = (L + kBN - 1) / kBN;
+  const bool soft = mode == kModeSoftmax;
+  const Times& t = kAlone[d == 64 ? 0 : 1][soft ? 0 : 1];
+  const Shared& two = kShared[soft ? 0 : 1];
+  AttnFew best = {1, false};
+  if (items > 2 * kSms || (items > kSms && d == 128)) {
+    best.here = d == 128 && M <= kBM && blocks >= 6;
+    return best;
+  }
+  double best_t = items <= kSms ? t.one + t.one_block * blocks + (items > 100 ? t.one_full : 0.0) : 1e30;
+  for (int lg = 1; lg <= 3 && (1 << lg) <= blocks; ++lg) {
+    const int parts = 1 << lg, own = (blocks + parts - 1) / parts;
+    const long long ctas = items * parts;
+    if (ctas > (d == 64 ? 2 * kSms : kSms) || items > (d == 64 ? cluster_places<64>(lg) : cluster_places<128>(lg))) break;
+    const double time = ctas <= kSms ? t.split + t.part * parts + t.split_block * own + (ctas > 100 ? t.split_full : 0.0)
+                                     : two.split + two.part * parts + two.block * own + two.full * static_cast<double>(ctas - kSms) / kSms;
+    if (time < best_t) {
+      best.parts = parts;
+      best_t = time;
+    }
+  }
+  const int own = (blocks + best.parts - 1) / best.parts;
+  if (d == 128) best.here = true;
+  else if (best.parts > 1) best.here = items * best.parts > kSms || own <= (soft ? 16 : 3);
+  else if (items > kSms) best.here = soft ? blocks <= 4 : blocks == 2 || blocks == 3;
+  else best.here = soft ? blocks <= 8 : blocks <= 6 && (blocks > 1 || items <= 74);
+  return best;
+}
+
+}  // namespace ditto_b200

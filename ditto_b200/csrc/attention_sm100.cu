@@ -861,85 +861,20 @@ cudaError_t launch_attention(const AttnParams& p, int batch, int d, bool bf16, i
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_attention_split(const AttnParams& p, int batch, int d, bool bf16, int mode, int parts, cudaStream_t stream) {
+cudaError_t launch_attention_split(const AttnParams& p, int batch, bool bf16, int mode, int parts, cudaStream_t stream) {
   const int blocks = (p.L + kBN - 1) / kBN;
   const long long ctas = static_cast<long long>((p.M + kBM - 1) / kBM) * batch * parts;
   if ((parts != 2 && parts != 4 && parts != 8) || parts > blocks || ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
-#define DITTO_DISPATCH(BF, DD, MO)              \
-  if (bf16 == BF && d == DD && mode == MO) \
-    return launch_one<BF, DD, 1, false, MO, true>(p, batch, parts, stream);
-#define DITTO_DISPATCH_SHAPES(MO)  \
-  DITTO_DISPATCH(false, 64, MO)  \
-  DITTO_DISPATCH(false, 128, MO) \
-  DITTO_DISPATCH(true, 64, MO)   \
-  DITTO_DISPATCH(true, 128, MO)
-  DITTO_DISPATCH_SHAPES(kModeSoftmax)
-  DITTO_DISPATCH_SHAPES(kModeRelu)
-  DITTO_DISPATCH_SHAPES(kModeIdentity)
-#undef DITTO_DISPATCH_SHAPES
+#define DITTO_DISPATCH(BF, MO) \
+  if (bf16 == BF && mode == MO) return launch_one<BF, 64, 1, false, MO, true>(p, batch, parts, stream);
+  DITTO_DISPATCH(false, kModeSoftmax)
+  DITTO_DISPATCH(false, kModeRelu)
+  DITTO_DISPATCH(false, kModeIdentity)
+  DITTO_DISPATCH(true, kModeSoftmax)
+  DITTO_DISPATCH(true, kModeRelu)
+  DITTO_DISPATCH(true, kModeIdentity)
 #undef DITTO_DISPATCH
   return cudaErrorInvalidValue;
-}
-
-// Clusters of `parts` CTAs the device holds at once.
-template <int D>
-static int split_places(int lg) {
-  static std::atomic<int> places[64][4];                // 0: not looked up yet; else clusters + 1
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  int n = places[dev][lg].load(std::memory_order_relaxed);
-  if (n == 0) {
-    using SM = Smem<D, 1, false>;
-    auto kern = attention_kernel<false, D, 1, false, kModeSoftmax, true>;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1024, 1, 1);
-    cfg.blockDim = dim3(threads_for(1), 1, 1);
-    cfg.dynamicSmemBytes = SM::kBytes;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1u << lg;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int count = 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::kBytes) != cudaSuccess ||
-        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&count, kern, &cfg) != cudaSuccess)
-      return 0;
-    n = std::max(0, count) + 1;
-    places[dev][lg].store(n, std::memory_order_relaxed);
-  }
-  return n - 1;
-}
-
-// The split pays when a launch is one wave of few, long items: a launch lasts as long as its longest CTA.  With more
-// clusters than the device holds at once a second wave costs more than the split saves, so those are left alone.
-// Times of one launch (us, back to back in a graph) as fixed + per 128-key block, fitted to 62 shapes of 1 to 384
-// items and 2 to 64 blocks, fp16; a chain without a softmax takes about 0.6 of the time per block.  Measured, whole ->
-// chosen parts: head dimension 64: 1 x 16 rows, 8192 keys 78 -> 14.7; 8 tiles, 1024 keys 13.7 -> 7.5; 64 tiles, 8192 keys
-// 80 -> 34; 48 tiles, 512 keys 9.0 -> 8.6; 128: 16 tiles, 2048 keys 32.7 -> 13.2; 48 tiles, 512 keys 12.9 -> 9.7.
-int attention_parts(int batch, int M, int L, int d, int mode) {
-  constexpr int kSms = 148;
-  const long long items = static_cast<long long>((M + kBM - 1) / kBM) * batch;
-  const int blocks = (L + kBN - 1) / kBN;
-  if (items > kSms || blocks < 2) return 1;
-  const double f = mode == kModeSoftmax ? 1.0 : 0.6;
-  const double whole = d == 64 ? 4.2 + 1.16 * f * blocks : M <= kBM ? 4.1 + 1.5 * f * blocks : 5.8 + 1.7 * f * blocks;
-  int best = 1;
-  double best_t = 0.96 * whole;                         // a gain that is sure
-  for (int lg = 1; lg <= 3 && (1 << lg) <= blocks; ++lg) {
-    const int parts = 1 << lg, own = (blocks + parts - 1) / parts;
-    if (items * parts > 2 * kSms || items > (d == 64 ? split_places<64>(lg) : split_places<128>(lg))) break;
-    const bool crowded = items * parts > kSms;          // two CTAs on some SMs
-    const double t = d == 128 ? 6.6 + 1.6 * f * own
-                     : crowded ? 7.7 + 1.6 * f * own : 5.8 + (items * parts > 100 ? 0.6 : 0.0) + 1.16 * f * own;
-    if (t < best_t) {
-      best = parts;
-      best_t = t;
-    }
-  }
-  return best;
 }
 
 }  // namespace ditto_b200

@@ -33,18 +33,23 @@ struct AttnParams {
 cudaError_t launch_attention(const AttnParams& p, int batch, int d, bool bf16, int nt, bool psmem, int mode,
                              cudaStream_t stream);
 
-// One 128-row tile per cluster of `parts` (2, 4 or 8, at most the number of 128-key blocks) CTAs that divide the keys
-// between them and combine on chip.
-cudaError_t launch_attention_split(const AttnParams& p, int batch, int d, bool bf16, int mode, int parts, cudaStream_t stream);
+// One 128-row tile per CTA or per cluster of `parts` (1, 2, 4 or 8, at most the number of 128-key blocks) CTAs that divide the
+// keys between them and combine on chip, for few items (attention_short_sm100.cu).
+cudaError_t launch_attention_short(const AttnParams& p, int batch, int d, bool bf16, int mode, int parts, cudaStream_t stream);
+// The same with a thread a row, head dimensions up to 64, parts above 1: the faster one where every CTA has many blocks.
+cudaError_t launch_attention_split(const AttnParams& p, int batch, bool bf16, int mode, int parts, cudaStream_t stream);
+// The number of parts that is expected to be fastest for a shape (1: no split), and whether it is the kernel for few items'.
+struct AttnFew {
+  int parts;
+  bool here;
+};
+AttnFew attention_few(int batch, int M, int L, int d, int mode);
 
 // Head dimensions up to 64 and many items (attention_narrow_sm100.cu): a small CTA an item, 64-key blocks (map_k / map_v
 // boxes of 64 rows).  mode as above.
 cudaError_t launch_attention_narrow(const AttnParams& p, int batch, bool bf16, int mode, cudaStream_t stream);
 // Whether it is expected to be the fastest form for a shape.
 bool attention_narrow_pays(int batch, int M, int L, int mode);
-
-// The number of parts that is expected to be fastest for a shape (1: no split).
-int attention_parts(int batch, int M, int L, int d, int mode);
 
 // Persistent variant for head dimensions up to 64 (attention_persistent_sm100.cu): two CTAs per SM walk the
 // (slice, tile) work items.  mode as above.

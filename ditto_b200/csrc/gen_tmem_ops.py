@@ -22,6 +22,19 @@ def emit_ld(n):
 }}
 """)
 
+def emit_ld_2x32():
+    outs = ", ".join(f'"=r"(r[{i}])' for i in range(64))
+    print(f"""// two runs of 32 columns
+__device__ __forceinline__ void tmem_ld_2x32_wait(uint32_t first, uint32_t second, uint32_t (&r)[64]) {{
+  asm volatile(
+    "tcgen05.ld.sync.aligned.32x32b.x32.b32 {{{regs(32, 0)}}}, [%64];\\n\\t"
+    "tcgen05.ld.sync.aligned.32x32b.x32.b32 {{{regs(32, 32)}}}, [%65];\\n\\t"
+    "tcgen05.wait::ld.sync.aligned;\\n"
+    : {outs}
+    : "r"(first), "r"(second) : "memory");
+}}
+""")
+
 def emit_st(n):
     ins = ", ".join(f'"r"(r[{i}])' for i in range(n))
     print(f"""__device__ __forceinline__ void tmem_st_x{n}(uint32_t taddr, const uint32_t (&r)[{n}]) {{
@@ -37,6 +50,7 @@ print("#include <stdint.h>")
 print("namespace ditto_b200 {")
 for n in (8, 16, 32, 64, 128):
     emit_ld(n)
+emit_ld_2x32()
 for n in (8, 16, 32, 64):
     emit_st(n)
 print("}  // namespace ditto_b200")

@@ -1,0 +1,133 @@
+"""Attention and small chains of few items, which take the kernel with two softmax warps per quarter of the rows by themselves, against
+float64 products of the same 16-bit operands: every length of a last block, one and several blocks, row tails, widths below
+the kernel's, both layouts and types; and, for every form of the attention kernel, single weights and scores that are not finite."""
+import pytest
+import torch
+
+from ditto_b200 import _lib, ops
+from tests.test_gpu_attention_masked_rows import FORMS
+from tests.test_gpu_attention_split import _close, _reference
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("N,K", [(64, 64), (16, 48), (128, 128), (80, 80), (112, 16)])
+@pytest.mark.parametrize("b,M,L", [(2, 128, 128), (1, 16, 16), (1, 144, 32), (2, 208, 48), (1, 128, 64), (1, 32, 80), (3, 128, 96), (1, 272, 112),
+                                   (2, 64, 208), (1, 128, 192), (1, 128, 368)])
+def test_shapes(dtype, N, K, b, M, L):
+    g = torch.Generator(device="cuda").manual_seed(b * M + L)
+    q = torch.randn(b, M, K, generator=g, device="cuda").to(dtype)
+    k = torch.randn(b, L, K, generator=g, device="cuda").to(dtype)
+    v = torch.randn(b, L, N, generator=g, device="cuda").to(dtype)
+    for layout in ("LK", "KL"):
+        keys = k if layout == "LK" else k.transpose(1, 2).contiguous()
+        out = ops.bmm_softmax_bmm(q, keys, v, scale=2 * K ** -0.5, key_layout=layout)
+        assert ops.device_status() == 0
+        _close(out, _reference(q, k, v, 2 * K ** -0.5), dtype)
+        assert torch.equal(out, ops.bmm_softmax_bmm(q, keys, v, scale=2 * K ** -0.5, key_layout=layout))
+
+
+@pytest.mark.parametrize("act", ["identity", "relu"])
+@pytest.mark.parametrize("layout", ["IO", "OI"])
+@pytest.mark.parametrize("b,M,N,K,L", [(1, 144, 64, 64, 80), (2, 16, 128, 96, 208), (3, 128, 16, 64, 512), (74, 128, 64, 64, 1024)])
+def test_chains(act, layout, b, M, N, K, L):
+    g = torch.Generator(device="cuda").manual_seed(M + L)
+    x = torch.randn(b, M, K, generator=g, device="cuda").half()
+    w1 = (torch.randn(b, K, L, generator=g, device="cuda") * K ** -0.5).half()
+    w2 = (torch.randn(b, L, N, generator=g, device="cuda") * L ** -0.5).half()
+    h = x.double() @ w1.double()
+    want = (h.relu() if act == "relu" else h).half().double() @ w2.double()
+    ws = (w1, w2) if layout == "IO" else (w1.transpose(1, 2).contiguous(), w2.transpose(1, 2).contiguous())
+    out = ops.gemm_relu_gemm(x, *ws, activation=act, weight_layout=layout)
+    assert ops.device_status() == 0
+    _close(out, want, torch.float16)
+
+
+@pytest.mark.parametrize("b,M,L", [(74, 128, 4352), (37, 256, 4240)])
+def test_long_parts(b, M, L):
+    """Many blocks a part: the split kernel with a thread a row."""
+    g = torch.Generator(device="cuda").manual_seed(b)
+    q = torch.randn(b, M, 64, generator=g, device="cuda").half()
+    k = torch.randn(b, L, 64, generator=g, device="cuda").half()
+    v = torch.randn(b, L, 64, generator=g, device="cuda").half()
+    out = ops.bmm_softmax_bmm(q, k, v, scale=0.125, key_layout="LK")
+    assert ops.device_status() == 0
+    for i in range(0, b, 9):
+        _close(out[i:i + 1], _reference(q[i:i + 1], k[i:i + 1], v[i:i + 1], 0.125), torch.float16)
+
+
+@pytest.mark.parametrize("b,M,L", [(70, 16, 208), (200, 128, 512), (250, 128, 784), (296, 64, 144), (149, 128, 128)])
+@pytest.mark.parametrize("d", [64, 128])
+def test_more_items_than_sms(b, M, L, d):
+    g = torch.Generator(device="cuda").manual_seed(b)
+    q = torch.randn(b, M, d, generator=g, device="cuda").half()
+    k = torch.randn(b, L, d, generator=g, device="cuda").half()
+    v = torch.randn(b, L, d, generator=g, device="cuda").half()
+    out = ops.bmm_softmax_bmm(q, k, v, scale=d ** -0.5, key_layout="LK")
+    assert ops.device_status() == 0
+    for i in range(0, b, 11):
+        _close(out[i:i + 1], _reference(q[i:i + 1], k[i:i + 1], v[i:i + 1], d ** -0.5), torch.float16)
+
+
+ALL_FORMS = {**FORMS, "few items": 0}
+
+
+@pytest.mark.parametrize("form,d", [(f, d) for f in ALL_FORMS for d in (64, 128) if d == 64 or f != "narrow"])
+def test_every_weight(form, d):
+    """V is the identity, d keys at a time: the result is the weights themselves.  They differ from float64's by the rounding of
+    the 16-bit weight (2^-11, or 2^-25 where it is subnormal: the row's largest is 1 before the division) and of the result."""
+    g = torch.Generator(device="cuda").manual_seed(d)
+    L = 2 * d + 16
+    q = torch.randn(1, 128, d, generator=g, device="cuda").half()
+    k = torch.randn(1, L, d, generator=g, device="cuda").half()
+    p = torch.softmax(q.double() @ k.double().transpose(1, 2) * 0.5, -1)
+    for first in range(0, L, d):
+        v = torch.zeros(1, L, d, device="cuda", dtype=torch.float16)
+        n = min(d, L - first)
+        v[0, first:first + n, :n] = torch.eye(n, device="cuda", dtype=torch.float16)
+        out = ops.bmm_softmax_bmm(q, k, v, scale=0.5, key_layout="LK", flags=ALL_FORMS[form])
+        want = p[:, :, first:first + n]
+        # (a reference up to 2^8 below the maximum makes weights larger and subnormals rarer; the sum's own error is some 2^-13)
+        assert ((out[:, :, :n].double() - want).abs() <= 2.0 ** -10 * 1.2 * want + 2.0 ** -24).all()
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("form,d", [(f, d) for f in ALL_FORMS for d in (64, 128) if d == 64 or f != "narrow"])
+def test_rows_with_scores_that_are_not_numbers(form, d, bad):
+    """A score of NaN, or of +inf, makes its row NaN as in torch.softmax, wherever the key lies; the other rows are what they were."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q = torch.randn(1, 128, d, generator=g, device="cuda").bfloat16()
+    k = torch.randn(1, 400, d, generator=g, device="cuda").bfloat16()
+    v = torch.randn(1, 400, d, generator=g, device="cuda").bfloat16()
+    q[:, :, 5] = q[:, :, 20] = 0.0
+    q[:, 40, 5] = 1e30                                # the product overflows float32 in that row alone
+    for key in (0, 7, 100, 127, 128, 250, 391, 399):
+        kk = k.clone()
+        kk[:, :, 5] = 0.0
+        kk[:, key, 5] = 1e30
+        qq = q.clone()
+        if bad != bad:
+            qq[:, 40, 20], kk[:, key, 20] = 1e30, -1e30   # inf - inf
+        out = ops.bmm_softmax_bmm(qq, kk, v, scale=0.125, key_layout="LK", flags=ALL_FORMS[form])
+        assert out[:, 40].isnan().all()
+        keep = [i for i in range(128) if i != 40]
+        _close(out[:, keep], _reference(qq[:, keep], kk, v, 0.125), torch.bfloat16)
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("b,L", [(24, 208), (128, 512), (32, 512)])
+def test_no_less_precise_than_the_other_kernels(b, L, dtype):
+    """The norm of the error against float64 beside those of the 64-key kernel and of the one with a thread a row.  The error is the
+    rounding of some 10^5 results and more, so that two kernels of the same precision differ by about 1 %."""
+    g = torch.Generator(device="cuda").manual_seed(L)
+    q = torch.randn(b, 256, 64, generator=g, device="cuda").to(dtype)
+    k = torch.randn(b, L, 64, generator=g, device="cuda").to(dtype)
+    v = torch.randn(b, L, 64, generator=g, device="cuda").to(dtype)
+    for scale in (0.125, 0.35, 1.0):
+        want = _reference(q, k, v, scale)
+        few, narrow, whole = ((ops.bmm_softmax_bmm(q, k, v, scale=scale, key_layout="LK", flags=f).double() - want).norm().item()
+                              for f in (0, _lib.FLAG_NARROW, _lib.FLAG_SPLIT_UNIT))
+        assert few <= 1.01 * max(narrow, whole), (scale, few, narrow, whole)
