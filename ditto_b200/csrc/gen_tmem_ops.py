@@ -23,8 +23,9 @@ def emit_ld(n):
 """)
 
 def emit_ld_2x32():
-    outs = ", ".join(f'"=r"(r[{i}])' for i in range(64))
-    print(f"""// two runs of 32 columns
+    # early-clobber: the first load writes its registers before the second one reads its address
+    outs = ", ".join(f'"=&r"(r[{i}])' for i in range(64))
+    print(f"""// two runs of 32 columns (early-clobber outputs: the second address is read after the first load has begun to write)
 __device__ __forceinline__ void tmem_ld_2x32_wait(uint32_t first, uint32_t second, uint32_t (&r)[64]) {{
   asm volatile(
     "tcgen05.ld.sync.aligned.32x32b.x32.b32 {{{regs(32, 0)}}}, [%64];\\n\\t"
