@@ -24,6 +24,7 @@ FLAG_P_VIA_SMEM = 1
 FLAG_ONE_TILE = 2
 FLAG_TWO_TILES = 4
 FLAG_NARROW = 8
+FLAG_FEW = 16             # two threads a row, a CTA per tile or as many as the split says
 FLAG_SPLIT_UNIT = 256     # 1, 2, 3, 4 of these: 1, 2, 4, 8 CTAs share a tile's keys
 EPILOGUE_PAIR_MMA = 0x200
 EPILOGUE_QUAD_MMA = 0x400

@@ -47,7 +47,7 @@ int make_map_3d(CUtensorMap* map, bool bf16, const void* base, uint64_t cols, ui
 bool narrow_for(int flags, bool any, long long batch, int M, int L, int d, int mode = 0) {
   if (!any || d != 64) return false;
   if (flags & DITTO_FLAG_NARROW) return true;
-  return !(flags & DITTO_FLAG_SPLIT_MASK) && ditto_b200::attention_narrow_pays(static_cast<int>(batch), M, L, mode) &&
+  return !(flags & (DITTO_FLAG_FEW | DITTO_FLAG_SPLIT_MASK)) && ditto_b200::attention_narrow_pays(static_cast<int>(batch), M, L, mode) &&
          !ditto_b200::attention_few(static_cast<int>(batch), M, L, d, mode).here;
 }
 
@@ -60,12 +60,12 @@ cudaError_t launch_attention_form(const ditto_b200::AttnParams& p, int slices, i
   if (any) {
     const int asked = (flags & DITTO_FLAG_SPLIT_MASK) / DITTO_FLAG_SPLIT_UNIT, blocks = (p.L + 127) / 128;
     ditto_b200::AttnFew few = {1, false};
-    if (asked == 0) {
+    if (asked == 0 && !(flags & DITTO_FLAG_FEW)) {
       few = ditto_b200::attention_few(slices, p.M, p.L, d, mode);
     } else {
-      few.parts = 1 << (asked - 1);
+      if (asked > 1) few.parts = 1 << (asked - 1);
       while (few.parts > blocks) few.parts /= 2;
-      few.here = few.parts > 1;
+      few.here = (flags & DITTO_FLAG_FEW) || (few.parts > 1 && d == 128);   // (the kernel with a thread a row has a split form up to 64)
     }
     if (few.here) return ditto_b200::launch_attention_short(p, slices, d, bf16, mode, few.parts, st);
     if (few.parts > 1) return ditto_b200::launch_attention_split(p, slices, bf16, mode, few.parts, st);

@@ -51,8 +51,10 @@ extern "C" {
 #define DITTO_FLAG_ONE_TILE 2     /* one 128-row query tile per CTA, one CTA per tile (no persistent work loop) */
 #define DITTO_FLAG_TWO_TILES 4    /* two query tiles per CTA even where one is the default (N = K = 64) */
 #define DITTO_FLAG_NARROW 8       /* 64-key blocks, a small CTA per tile (N, K <= 64; ignored beside the flags above) */
-#define DITTO_FLAG_SPLIT_UNIT 256  /* 1, 2, 3, 4 of these: 1, 2, 4, 8 CTAs share a tile's keys (at most one per 128 keys) */
-#define DITTO_FLAG_SPLIT_MASK (7 * DITTO_FLAG_SPLIT_UNIT)   /* not set: by shape.  Ignored beside the flags above */
+#define DITTO_FLAG_FEW 16         /* two threads a row, a CTA per tile or as many as the split below says (ignored beside the flags above) */
+#define DITTO_FLAG_SPLIT_UNIT 256  /* 1, 2, 3, 4 of these: 1, 2, 4, 8 CTAs share a tile's keys (at most one per 128 keys); without
+                                      DITTO_FLAG_FEW a thread a row where N, K <= 64 */
+#define DITTO_FLAG_SPLIT_MASK (7 * DITTO_FLAG_SPLIT_UNIT)   /* not set: by shape.  Ignored beside the first four flags */
 
 /* Fused attention chain  out = softmax(scale * Q K^T) V, replacing the module TVM builds from
  * BatchGemmSoftmaxGemmMMA (python/ditto/auto_compute/nn/functional/bmm_chain.py:5-104) under

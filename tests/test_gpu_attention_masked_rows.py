@@ -12,6 +12,7 @@ from tests.test_gpu_attention_split import _close, _reference
 pytestmark = pytest.mark.gpu
 
 FORMS = {"narrow": _lib.FLAG_NARROW, "split 2": 2 * _lib.FLAG_SPLIT_UNIT, "split 4": 3 * _lib.FLAG_SPLIT_UNIT,
+         "few 1": _lib.FLAG_FEW, "few 2": _lib.FLAG_FEW | 2 * _lib.FLAG_SPLIT_UNIT, "few 4": _lib.FLAG_FEW | 3 * _lib.FLAG_SPLIT_UNIT,
          "whole": _lib.FLAG_SPLIT_UNIT, "one tile": _lib.FLAG_ONE_TILE, "two tiles": _lib.FLAG_TWO_TILES,
          "P via smem": _lib.FLAG_P_VIA_SMEM}
 # masked keys of 512: less than a block, whole blocks at the start, in the middle and at the end, whole parts, all but a few

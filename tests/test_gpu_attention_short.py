@@ -44,17 +44,91 @@ def test_chains(act, layout, b, M, N, K, L):
     _close(out, want, torch.float16)
 
 
-@pytest.mark.parametrize("b,M,L", [(74, 128, 4352), (37, 256, 4240)])
-def test_long_parts(b, M, L):
-    """Many blocks a part: the split kernel with a thread a row."""
-    g = torch.Generator(device="cuda").manual_seed(b)
-    q = torch.randn(b, M, 64, generator=g, device="cuda").half()
-    k = torch.randn(b, L, 64, generator=g, device="cuda").half()
-    v = torch.randn(b, L, 64, generator=g, device="cuda").half()
-    out = ops.bmm_softmax_bmm(q, k, v, scale=0.125, key_layout="LK")
+def _attention(q, k, v, scale, layout, flags):
+    keys = k if layout == "LK" else k.transpose(1, 2).contiguous()
+    out = ops.bmm_softmax_bmm(q, keys, v, scale=scale, key_layout=layout, flags=flags)
     assert ops.device_status() == 0
+    return out
+
+
+def _operands(b, M, N, K, L, dtype, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return tuple(torch.randn(b, rows, cols, generator=g, device="cuda").to(dtype) for rows, cols in ((M, K), (L, K), (L, N)))
+
+
+@pytest.mark.parametrize("code", [0, 2, 3, 4])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("b,M,N,K,L,layout", [
+    (3, 128, 64, 64, 1024, "LK"), (2, 208, 64, 64, 1168, "KL"), (1, 16, 64, 64, 256, "LK"), (2, 144, 48, 16, 912, "LK"),
+    (3, 128, 128, 128, 1024, "LK"), (2, 272, 80, 80, 1168, "KL"), (1, 16, 16, 128, 272, "LK"), (300, 384, 64, 64, 384, "LK")])
+def test_parts(code, dtype, b, M, N, K, L, layout):
+    """The kernel by its name, with every number of parts (the last shape: several rounds of CTAs)."""
+    q, k, v = _operands(b, M, N, K, L, dtype, b * M + L + code)
+    flags = _lib.FLAG_FEW | code * _lib.FLAG_SPLIT_UNIT
+    out = _attention(q, k, v, 2 * K ** -0.5, layout, flags)
+    _close(out, _reference(q, k, v, 2 * K ** -0.5), dtype)
+    assert torch.equal(out, _attention(q, k, v, 2 * K ** -0.5, layout, flags))
+
+
+@pytest.mark.parametrize("code", [2, 3, 4])
+def test_a_named_split_is_the_kernel_with_a_thread_a_row(code):
+    """Up to head dimension 64 the names lead to different kernels: their references follow a row's maximum within 2^8 and within 2^5,
+    so that somewhere among 10^5 results the weights are rounded at different scales."""
+    q, k, v = _operands(4, 384, 64, 64, 8192, torch.float16, 9)
+    k *= 1.0 + torch.arange(8192, device="cuda").view(1, -1, 1).half() / 2048          # maxima that go on rising
+    by_row, few = (_attention(q, k, v, 0.125, "LK", f | code * _lib.FLAG_SPLIT_UNIT) for f in (0, _lib.FLAG_FEW))
+    assert not torch.equal(by_row, few)
+
+
+@pytest.mark.parametrize("code", [2, 3])
+@pytest.mark.parametrize("b,M,N,K,L,dtype,layout", [(74, 128, 64, 64, 4352, torch.float16, "LK"), (19, 400, 64, 64, 4240, torch.bfloat16, "KL"),
+                                                    (37, 256, 48, 32, 4240, torch.float16, "KL"), (9, 144, 64, 64, 8208, torch.bfloat16, "LK")])
+def test_long_parts(b, M, N, K, L, dtype, layout, code):
+    """Many blocks a part: the split kernel with a thread a row, by its name."""
+    q, k, v = _operands(b, M, N, K, L, dtype, b)
+    out = _attention(q, k, v, K ** -0.5, layout, code * _lib.FLAG_SPLIT_UNIT)
     for i in range(0, b, 9):
-        _close(out[i:i + 1], _reference(q[i:i + 1], k[i:i + 1], v[i:i + 1], 0.125), torch.float16)
+        _close(out[i:i + 1], _reference(q[i:i + 1], k[i:i + 1], v[i:i + 1], K ** -0.5), dtype)
+
+
+@pytest.mark.parametrize("act", ["identity", "relu"])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("layout", ["IO", "OI"])
+@pytest.mark.parametrize("b,M,N,K,L", [(1, 144, 64, 48, 8192), (3, 16, 16, 64, 4176)])
+def test_long_chains(b, M, N, K, L, layout, dtype, act):
+    """Chains of a few tiles and more than three blocks a part even in eight parts: the split kernel with a thread a row."""
+    g = torch.Generator(device="cuda").manual_seed(L)
+    x = torch.randn(b, M, K, generator=g, device="cuda").to(dtype)
+    w1 = (torch.randn(b, K, L, generator=g, device="cuda") * K ** -0.5).to(dtype)
+    w2 = (torch.randn(b, L, N, generator=g, device="cuda") * L ** -0.5).to(dtype)
+    h = x.double() @ w1.double()
+    want = (h.relu() if act == "relu" else h).to(dtype).double() @ w2.double()
+    ws = (w1, w2) if layout == "IO" else (w1.transpose(1, 2).contiguous(), w2.transpose(1, 2).contiguous())
+    out = ops.gemm_relu_gemm(x, *ws, activation=act, weight_layout=layout)
+    assert ops.device_status() == 0
+    _close(out, want, dtype)
+
+
+@pytest.mark.parametrize("code", [0, 2, 3, 4])
+@pytest.mark.parametrize("d", [64, 128])
+def test_whole_parts_of_minus_infinity(code, d):
+    q, k, v = _operands(1, 128, d, d, 1024, torch.bfloat16, 5)
+    q = q.abs() + 0.5
+    k[:, 128:] = float("-inf")                       # q is positive: these scores are -inf
+    out = _attention(q, k, v, 0.25, "LK", _lib.FLAG_FEW | code * _lib.FLAG_SPLIT_UNIT)
+    _close(out, _reference(q, k[:, :128], v[:, :128], 0.25), torch.bfloat16)
+
+
+@pytest.mark.parametrize("heads,d,M", [(4, 64, 1040), (2, 128, 528)])
+def test_packed_heads(heads, d, M):
+    g = torch.Generator(device="cuda").manual_seed(M)
+    qkv = torch.randn(2, M, 3 * heads * d, generator=g, device="cuda").half()
+    q, k, v = (t.reshape(2, M, heads, d).transpose(1, 2).reshape(2 * heads, M, d) for t in qkv.chunk(3, dim=-1))
+    want = _reference(q, k, v, d ** -0.5).reshape(2, heads, M, d).transpose(1, 2).reshape(2, M, heads * d)
+    for code in (0, 2, 3, 4):
+        out = ops.multi_head_attention(qkv, heads, scale=d ** -0.5, flags=_lib.FLAG_FEW | code * _lib.FLAG_SPLIT_UNIT)
+        assert ops.device_status() == 0
+        _close(out, want, torch.float16)
 
 
 @pytest.mark.parametrize("b,M,L", [(70, 16, 208), (200, 128, 512), (250, 128, 784), (296, 64, 144), (149, 128, 128)])
