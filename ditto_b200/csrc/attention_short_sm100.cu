@@ -569,10 +569,11 @@ constexpr Shared kShared[2] = {{5.4, 0.30, 1.93, 0.8}, {4.2, 0.13, 1.38, 1.0}};
 
 // Where the lines lie, other kernels -> this one (us), items x blocks.  Softmax at head dimension 64: 24 x 1 5.4 -> 5.0, 24 x 2 6.6 -> 5.7, 24 x 4
 // 7.5 -> 6.5 (4 parts), 24 x 16 11.2 -> 10.6 (4), 48 x 16 15.6 -> 13.9 (4), 100 x 32 43.8 -> 37.1 (2); at 128: 24 x 1 5.7 -> 5.1, 24 x 2 7.3 ->
-// 6.3, 24 x 4 9.7 -> 8.5 (4), 24 x 16 14.9 -> 12.8 (4), 48 x 16 21.9 -> 18.9 (2), 100 x 32 64.6 -> 55.4.  Split over few CTAs with long parts
-// the kernel with a thread a row costs less per block at head dimension 64 (1.16 against 1.30: no word from another warp before the
-// exponentials): 74 x 32 27.4 -> 27.7, 74 x 64 46.4 -> 48.7; without a softmax from four blocks on (48 x 8 7.4 -> 7.8, 12 x 64 10.7 ->
-// 12.0), and 148 x 1 4.4 -> 4.7.  Unsplit and two CTAs an SM it pays for up to four blocks (200 x 2 8.1 -> 7.6, 256 x 4 12.3 -> 11.9;
+// 6.3, 24 x 4 9.7 -> 8.5 (4), 24 x 16 14.9 -> 12.8 (4), 48 x 16 21.9 -> 18.9 (2), 100 x 32 64.6 -> 55.4.  At head
+// dimension 64 the kernel with a thread a row costs less per block (1.18 against 1.35: no word from another warp before the exponentials).
+// This kernel's time over that one's, split alike, by blocks a part: one 0.88, two 0.95, four 0.98, six 1.01, eight 1.03, sixteen
+// 1.07 (24 x 64, 4 parts: 27.4 against 25.9), so parts of more than four blocks take that one; without a softmax of more than
+// three (48 x 8 7.4 -> 7.8, 12 x 64 10.7 -> 12.0), and 148 x 1 4.4 -> 4.7.  Unsplit and two CTAs an SM it pays for up to four blocks (200 x 2 8.1 -> 7.6, 256 x 4 12.3 -> 11.9;
 // 296 x 8 22.3 -> 22.5).  One tile a sequence at head dimension 128 has no second tile to work beside: there it pays in any number
 // from six blocks on (200 x 8 36.8 -> 33.2, 256 x 16 69.0 -> 58.1).
 AttnFew attention_few(int batch, int M, int L, int d, int mode) {
@@ -601,7 +602,7 @@ AttnFew attention_few(int batch, int M, int L, int d, int mode) {
   }
   const int own = (blocks + best.parts - 1) / best.parts;
   if (d == 128) best.here = true;
-  else if (best.parts > 1) best.here = items * best.parts > kSms || own <= (soft ? 16 : 3);
+  else if (best.parts > 1) best.here = own <= (soft ? 4 : 3);
   else if (items > kSms) best.here = soft ? blocks <= 4 : blocks == 2 || blocks == 3;
   else best.here = soft ? blocks <= 8 : blocks <= 6 && (blocks > 1 || items <= 74);
   return best;

@@ -80,6 +80,23 @@ def test_a_named_split_is_the_kernel_with_a_thread_a_row(code):
     assert not torch.equal(by_row, few)
 
 
+FEW, UNIT = _lib.FLAG_FEW, _lib.FLAG_SPLIT_UNIT
+BY_ROW, BY_TWO = tuple(c * UNIT for c in (2, 3, 4)), tuple(FEW | c * UNIT for c in (0, 2, 3, 4))
+
+
+@pytest.mark.parametrize("tiles,blocks,d,forms,others", [
+    (24, 64, 64, BY_ROW, BY_TWO), (1, 64, 64, BY_ROW, BY_TWO),     # many blocks even in eight parts
+    (24, 16, 64, BY_TWO, BY_ROW), (24, 4, 64, BY_TWO, BY_ROW),     # four a part, and one
+])
+def test_form_by_shape(tiles, blocks, d, forms, others):
+    """Which kernel the rule takes, seen by the bits: scores that go on rising make the forms round their weights at different scales."""
+    q, k, v = _operands(tiles, 128, d, d, 128 * blocks, torch.float16, 7)
+    k *= 1.0 + torch.arange(128 * blocks, device="cuda").view(1, -1, 1).half() / (32 * blocks)
+    got = _attention(q, k, v, d ** -0.5, "LK", 0)
+    assert any(torch.equal(got, _attention(q, k, v, d ** -0.5, "LK", f)) for f in forms)
+    assert not any(torch.equal(got, _attention(q, k, v, d ** -0.5, "LK", f)) for f in others)
+
+
 @pytest.mark.parametrize("code", [2, 3])
 @pytest.mark.parametrize("b,M,N,K,L,dtype,layout", [(74, 128, 64, 64, 4352, torch.float16, "LK"), (19, 400, 64, 64, 4240, torch.bfloat16, "KL"),
                                                     (37, 256, 48, 32, 4240, torch.float16, "KL"), (9, 144, 64, 64, 8208, torch.bfloat16, "LK")])
