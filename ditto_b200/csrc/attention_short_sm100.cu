@@ -523,16 +523,18 @@ cudaError_t launch_attention_short(const AttnParams& params, int batch, int d, b
   return cudaErrorInvalidValue;
 }
 
-// Clusters of `parts` CTAs the device holds at once.
-template <int D>
+// Clusters of 1 << lg CTAs the device holds at once with a CTA an SM, asked for an instance at head dimension 128, whose shared memory
+// allows no second one.  Instances at 64 and the kernel with a thread a row run two an SM.  The query does not see that: it rounds
+// their ten or six warps up to a multiple of four and finds registers for one CTA, but 148 items of 64 blocks in two parts take
+// 68 to 76 us (59 to 66 with a thread a row) where two waves of those parts would take 90.
 static int cluster_places(int lg) {
   static std::atomic<int> places[kMaxDevices][4];       // 0: not looked up yet; else clusters + 1
   int dev = 0;
   if (current_device_checked(&dev) != cudaSuccess) return 0;
   int n = places[dev][lg].load(std::memory_order_relaxed);
   if (n == 0) {
-    using SM = Layout<D>;
-    auto kern = attention_short_kernel<false, D, kModeSoftmax>;
+    using SM = Layout<128>;
+    auto kern = attention_short_kernel<false, 128, kModeSoftmax>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(1024, 1, 1);
     cfg.blockDim = dim3(kThreads, 1, 1);
@@ -555,46 +557,53 @@ static int cluster_places(int lg) {
   return n - 1;
 }
 
-// Times of a launch of this kernel (us, one call after another): fixed + per 128-key block of a CTA, fitted to 396 shapes of 1 to
-// 296 items and 1 to 64 blocks, fp16, with and without a softmax (rms 4 to 7 %).  With more CTAs than SMs two share one at
-// head dimension 64 (kShared); at 128 shared memory holds one.  More clusters than the device holds at once would be a
-// second wave, which costs more than a split saves.
+// Times of a launch (us, one call after another) by parts and 128-key blocks of a CTA, fp16, fitted to shapes of 1 to 296 items and 1 to 64 blocks
+// (rms 3 to 8 %).  At head dimension 64 clusters share SMs once there are more than places at a CTA an SM (*Shared); more than the
+// device holds at once would be a second wave, which costs more than a split saves (36 x 16 in eight parts 18.7 us, in four
+// 14.8).  What the rule picks took on average 0.6 % longer than the best form timed (softmax, 363 shapes of up to 148 items) and 0.3 %
+// (chains, 299), at head dimension 128 0.1 % (softmax, 234); asking 4 % for a split made that worse.
 namespace {
-struct Times { double one, one_block, one_full, split, part, split_block, split_full; };      // *_full: over 100 CTAs
-constexpr Times kAlone[2][2] = {{{3.3, 1.28, 0.7, 4.3, 0.12, 1.30, 1.4}, {3.0, 0.89, 0.4, 3.7, 0.09, 0.92, 0.6}},      // [head dimension][no softmax]
-                                {{3.6, 1.39, 1.2, 5.7, 0.13, 1.37, 1.3}, {3.0, 1.14, 1.0, 4.5, 0.16, 1.16, 1.2}}};
-struct Shared { double split, part, block, full; };
-constexpr Shared kShared[2] = {{5.4, 0.30, 1.93, 0.8}, {4.2, 0.13, 1.38, 1.0}};
+struct Whole { double fixed, block, full; };                    // full: over 100 CTAs
+struct Split { double fixed, part, block, full; };              // full: over 100 CTAs; shared: times the share of SMs with two
+constexpr Whole kWhole[2][2] = {{{3.3, 1.28, 0.7}, {3.0, 0.89, 0.4}}, {{3.6, 1.39, 1.2}, {3.0, 1.14, 1.0}}};      // [head dimension][no softmax]
+constexpr Split kAlone[2][2] = {{{4.3, 0.12, 1.30, 1.4}, {3.7, 0.09, 0.92, 0.6}}, {{5.7, 0.13, 1.37, 1.3}, {4.5, 0.16, 1.16, 1.2}}};
+constexpr Split kShared[2] = {{5.4, 0.30, 1.93, 0.8}, {4.8, 0.10, 1.30, 1.1}};
+// the kernel with a thread a row
+constexpr Split kRowAlone[2] = {{5.5, 0.06, 1.18, 0.8}, {4.0, 0.09, 0.75, 1.0}}, kRowShared[2] = {{6.6, 0.05, 1.70, 1.0}, {5.3, 0.05, 1.18, 1.1}};
+constexpr int kRowFrom[2] = {5, 4};                             // blocks a part from which that one is the faster at head dimension 64
 }  // namespace
 
-// Where the lines lie, other kernels -> this one (us), items x blocks.  Softmax at head dimension 64: 24 x 1 5.4 -> 5.0, 24 x 2 6.6 -> 5.7, 24 x 4
-// 7.5 -> 6.5 (4 parts), 24 x 16 11.2 -> 10.6 (4), 48 x 16 15.6 -> 13.9 (4), 100 x 32 43.8 -> 37.1 (2); at 128: 24 x 1 5.7 -> 5.1, 24 x 2 7.3 ->
-// 6.3, 24 x 4 9.7 -> 8.5 (4), 24 x 16 14.9 -> 12.8 (4), 48 x 16 21.9 -> 18.9 (2), 100 x 32 64.6 -> 55.4.  At head
-// dimension 64 the kernel with a thread a row costs less per block (1.18 against 1.35: no word from another warp before the exponentials).
-// This kernel's time over that one's, split alike, by blocks a part: one 0.88, two 0.95, four 0.98, six 1.01, eight 1.03, sixteen
-// 1.07 (24 x 64, 4 parts: 27.4 against 25.9), so parts of more than four blocks take that one; without a softmax of more than
-// three (48 x 8 7.4 -> 7.8, 12 x 64 10.7 -> 12.0), and 148 x 1 4.4 -> 4.7.  Unsplit and two CTAs an SM it pays for up to four blocks (200 x 2 8.1 -> 7.6, 256 x 4 12.3 -> 11.9;
-// 296 x 8 22.3 -> 22.5).  One tile a sequence at head dimension 128 has no second tile to work beside: there it pays in any number
-// from six blocks on (200 x 8 36.8 -> 33.2, 256 x 16 69.0 -> 58.1).
+// Where the lines lie, the forms without this kernel and with two CTAs an SM left out of count -> the choice now (us), items x blocks of
+// sequences of 512 rows.  Softmax at head dimension 64: 24 x 1 5.3 -> 4.6, 24 x 2 6.5 -> 6.1, 24 x 4 7.3 -> 6.5 (4 parts), 24 x 16 11.0 -> 10.8 (4),
+// 48 x 16 15.6 -> 14.4 (4), 100 x 2 6.9 -> 6.3, 148 x 4 10.2 -> 9.7, with a thread a row 24 x 64 25.3 -> 21.5 (8), 100 x 32 43.1 -> 33.7 (2),
+// 148 x 64 83.1 -> 59.7 (2); at 128: 24 x 1 7.2 -> 5.2, 24 x 2 7.9 -> 6.7, 24 x 4 9.0 -> 8.3 (4), 24 x 16 14.3 -> 13.2 (4), 48 x 16 20.3 -> 18.9 (2),
+// 100 x 32 64.4 -> 51.6; without a softmax 48 x 16 17.6 -> 14.5, 100 x 32 57.2 -> 39.5.
+// At head dimension 64 the kernel with a thread a row costs less per block (1.18 against 1.35: no word from another warp before the
+// exponentials).  This kernel's time over that one's, split alike, by blocks a part: one 0.88, two 0.95, four 0.98, six 1.01, eight
+// 1.03, sixteen 1.07 (24 x 64 in four parts 27.0 against 25.3), so parts of more than four blocks take that one; without a softmax
+// of more than three (48 x 8 7.4 -> 7.8, 12 x 64 10.7 -> 12.0), and 148 x 1 4.4 -> 4.7.
+// Unsplit and two CTAs an SM it pays for up to four blocks (200 x 2 8.1 -> 7.6, 256 x 4 12.3 -> 11.9; 296 x 8 22.3 -> 22.5).  One tile
+// a sequence at head dimension 128 has no second tile to work beside: there it pays in any number from six blocks on (200 x 8 36.8
+// -> 33.2, 256 x 16 69.0 -> 58.1).
 AttnFew attention_few(int batch, int M, int L, int d, int mode) {
   constexpr int kSms = 148;
   const long long items = static_cast<long long>((M + kBM - 1) / kBM) * batch;
   const int blocks = (L + kBN - 1) / kBN;
-  const bool soft = mode == kModeSoftmax;
-  const Times& t = kAlone[d == 64 ? 0 : 1][soft ? 0 : 1];
-  const Shared& two = kShared[soft ? 0 : 1];
+  const int m = mode == kModeSoftmax ? 0 : 1, wide = d == 64 ? 0 : 1;
   AttnFew best = {1, false};
   if (items > 2 * kSms || (items > kSms && d == 128)) {
     best.here = d == 128 && M <= kBM && blocks >= 6;
     return best;
   }
-  double best_t = items <= kSms ? t.one + t.one_block * blocks + (items > 100 ? t.one_full : 0.0) : 1e30;
+  const Whole& w = kWhole[wide][m];
+  double best_t = items <= kSms ? w.fixed + w.block * blocks + (items > 100 ? w.full : 0.0) : 1e30;
   for (int lg = 1; lg <= 3 && (1 << lg) <= blocks; ++lg) {
-    const int parts = 1 << lg, own = (blocks + parts - 1) / parts;
-    const long long ctas = items * parts;
-    if (ctas > (d == 64 ? 2 * kSms : kSms) || items > (d == 64 ? cluster_places<64>(lg) : cluster_places<128>(lg))) break;
-    const double time = ctas <= kSms ? t.split + t.part * parts + t.split_block * own + (ctas > 100 ? t.split_full : 0.0)
-                                     : two.split + two.part * parts + two.block * own + two.full * static_cast<double>(ctas - kSms) / kSms;
+    const int parts = 1 << lg, own = (blocks + parts - 1) / parts, places = cluster_places(lg);
+    if (items > (wide ? places : 2 * places)) break;
+    const bool by_row = !wide && own >= kRowFrom[m], shared = items > places;
+    const Split& s = by_row ? (shared ? kRowShared[m] : kRowAlone[m]) : shared ? kShared[m] : kAlone[wide][m];
+    const double time = s.fixed + s.part * parts + s.block * own +
+                        s.full * (shared ? static_cast<double>(items - places) / places : items * parts > 100 ? 1.0 : 0.0);
     if (time < best_t) {
       best.parts = parts;
       best_t = time;
@@ -602,9 +611,9 @@ AttnFew attention_few(int batch, int M, int L, int d, int mode) {
   }
   const int own = (blocks + best.parts - 1) / best.parts;
   if (d == 128) best.here = true;
-  else if (best.parts > 1) best.here = own <= (soft ? 4 : 3);
-  else if (items > kSms) best.here = soft ? blocks <= 4 : blocks == 2 || blocks == 3;
-  else best.here = soft ? blocks <= 8 : blocks <= 6 && (blocks > 1 || items <= 74);
+  else if (best.parts > 1) best.here = own < kRowFrom[m];
+  else if (items > kSms) best.here = m == 0 ? blocks <= 4 : blocks == 2 || blocks == 3;
+  else best.here = m == 0 ? blocks <= 8 : blocks <= 6 && (blocks > 1 || items <= 74);
   return best;
 }
 

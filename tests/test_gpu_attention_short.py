@@ -86,6 +86,9 @@ BY_ROW, BY_TWO = tuple(c * UNIT for c in (2, 3, 4)), tuple(FEW | c * UNIT for c 
 
 @pytest.mark.parametrize("tiles,blocks,d,forms,others", [
     (24, 64, 64, BY_ROW, BY_TWO), (1, 64, 64, BY_ROW, BY_TWO),     # many blocks even in eight parts
+    (148, 16, 64, BY_ROW[:1], BY_TWO + (UNIT,)),                   # two CTAs an SM, as many clusters of two as SMs
+    (60, 16, 64, BY_TWO[2:3], BY_ROW + (UNIT,)),                   # ... clusters of four where a CTA an SM leaves no room for them
+    (16, 64, 64, BY_ROW[2:], BY_TWO + (UNIT,)),
     (24, 16, 64, BY_TWO, BY_ROW), (24, 4, 64, BY_TWO, BY_ROW),     # four a part, and one
 ])
 def test_form_by_shape(tiles, blocks, d, forms, others):
