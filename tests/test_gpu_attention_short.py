@@ -30,7 +30,8 @@ def test_shapes(dtype, N, K, b, M, L):
 
 @pytest.mark.parametrize("act", ["identity", "relu"])
 @pytest.mark.parametrize("layout", ["IO", "OI"])
-@pytest.mark.parametrize("b,M,N,K,L", [(1, 144, 64, 64, 80), (2, 16, 128, 96, 208), (3, 128, 16, 64, 512), (74, 128, 64, 64, 1024)])
+@pytest.mark.parametrize("b,M,N,K,L", [(1, 144, 64, 64, 80), (2, 16, 128, 96, 208), (3, 128, 16, 64, 512), (74, 128, 64, 64, 1024),
+                                       (100, 128, 64, 64, 128), (296, 16, 48, 64, 80)])
 def test_chains(act, layout, b, M, N, K, L):
     g = torch.Generator(device="cuda").manual_seed(M + L)
     x = torch.randn(b, M, K, generator=g, device="cuda").half()
