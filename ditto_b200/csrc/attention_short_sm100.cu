@@ -587,10 +587,8 @@ constexpr int kRowFrom[2] = {5, 4};                             // blocks a part
 // with a softmax have the kernel with 64-key blocks up to four blocks (that one -> this one, rows 128 / 512 / 208: 296 x 2 9.6 -> 10.6 /
 // 8.3 -> 8.7 / 8.8 -> 9.4, 200 x 3 11.0 -> 11.3 / 9.7 -> 10.2 / 10.1 -> 10.9, 180 x 2 8.7 -> 8.6 / 7.8 -> 7.6 / 8.0 -> 8.2; 256 x 4 14.1 -> 13.9 /
 // 12.5 -> 13.1 / 13.1 -> 13.5).  One tile
-// a sequence at head dimension 128 has no second tile to work beside: there it pays in any number of items, without a softmax from
-// six blocks on (200 x 8 35.0 -> 29.7, 1000 x 8 118 -> 109, 4000 x 6 382 -> 365), with one from more blocks the more items the other
-// kernel's work loop has to hide start and write-out in (200 x 6 29.1 -> 27.7, 400 x 6 45.6 -> 45.7, 592 x 6 62.2 -> 65.7, 1480 x 6 150 -> 163;
-// 592 x 8 76.8 -> 76.8, 1480 x 8 195 -> 201; 1000 x 9 0.97 of the time, 1000 x 16 254 -> 232).
+// a sequence at head dimension 128 has no second tile to work beside: there it pays in any number from six blocks on (200 x 8 36.8
+// -> 33.2, 256 x 16 69.0 -> 58.1).
 AttnFew attention_few(int batch, int M, int L, int d, int mode) {
   constexpr int kSms = 148;
   const long long items = static_cast<long long>((M + kBM - 1) / kBM) * batch;
@@ -598,7 +596,7 @@ AttnFew attention_few(int batch, int M, int L, int d, int mode) {
   const int m = mode == kModeSoftmax ? 0 : 1, wide = d == 64 ? 0 : 1;
   AttnFew best = {1, false};
   if (items > 2 * kSms || (items > kSms && d == 128)) {
-    best.here = d == 128 && M <= kBM && blocks >= (m == 1 || items <= 400 ? 6 : items <= 740 ? 8 : 9);
+    best.here = d == 128 && M <= kBM && blocks >= 6;
     return best;
   }
   const Whole& w = kWhole[wide][m];

@@ -92,8 +92,6 @@ BY_ROW, BY_TWO = tuple(c * UNIT for c in (2, 3, 4)), tuple(FEW | c * UNIT for c 
     (16, 64, 64, BY_ROW[2:], BY_TWO + (UNIT,)),
     (296, 2, 64, (_lib.FLAG_NARROW,), BY_TWO[:1] + (UNIT,)),       # the kernel with 64-key blocks
     (200, 3, 64, (_lib.FLAG_NARROW,), BY_TWO[:1] + (UNIT,)), (256, 4, 64, (_lib.FLAG_NARROW,), BY_TWO[:1] + (UNIT,)),
-    (592, 6, 128, (UNIT,), BY_TWO[:1]), (592, 10, 128, BY_TWO[:1], (UNIT,)), (300, 6, 128, BY_TWO[:1], (UNIT,)),    # one tile a sequence
-    (1000, 8, 128, (UNIT,), BY_TWO[:1]),
     (24, 16, 64, BY_TWO, BY_ROW), (24, 4, 64, BY_TWO, BY_ROW),     # four a part, and one
 ])
 def test_form_by_shape(tiles, blocks, d, forms, others):
