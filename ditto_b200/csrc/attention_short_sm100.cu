@@ -582,11 +582,8 @@ constexpr int kRowFrom[2] = {5, 4};                             // blocks a part
 // exponentials).  This kernel's time over that one's, split alike, by blocks a part: one 0.88, two 0.95, four 0.98, six 1.01, eight
 // 1.03, sixteen 1.07 (24 x 64 in four parts 27.0 against 25.3), so parts of more than four blocks take that one; without a softmax
 // of more than three (48 x 8 7.4 -> 7.8, 12 x 64 10.7 -> 12.0).
-// Unsplit and two CTAs an SM it pays for one block (200 x 1 5.8 -> 5.5), without a softmax for up to three (148 x 1 4.4 -> 3.7, 200 x 1 4.7 -> 4.3,
-// 200 x 2 5.9 -> 5.4); longer items
-// with a softmax have the kernel with 64-key blocks up to four blocks (that one -> this one, rows 128 / 512 / 208: 296 x 2 9.6 -> 10.6 /
-// 8.3 -> 8.7 / 8.8 -> 9.4, 200 x 3 11.0 -> 11.3 / 9.7 -> 10.2 / 10.1 -> 10.9, 180 x 2 8.7 -> 8.6 / 7.8 -> 7.6 / 8.0 -> 8.2; 256 x 4 14.1 -> 13.9 /
-// 12.5 -> 13.1 / 13.1 -> 13.5).  One tile
+// Unsplit and two CTAs an SM it pays for up to four blocks (200 x 2 8.1 -> 7.6, 256 x 4 12.3 -> 11.9; 296 x 8 22.3 -> 22.5), without a softmax
+// for up to three (148 x 1 4.4 -> 3.7, 200 x 1 4.7 -> 4.3, 200 x 2 5.9 -> 5.4).  One tile
 // a sequence at head dimension 128 has no second tile to work beside: there it pays in any number from six blocks on (200 x 8 36.8
 // -> 33.2, 256 x 16 69.0 -> 58.1).
 AttnFew attention_few(int batch, int M, int L, int d, int mode) {
@@ -616,7 +613,7 @@ AttnFew attention_few(int batch, int M, int L, int d, int mode) {
   const int own = (blocks + best.parts - 1) / best.parts;
   if (d == 128) best.here = true;
   else if (best.parts > 1) best.here = own < kRowFrom[m];
-  else if (items > kSms) best.here = blocks <= (m == 0 ? 1 : 3);
+  else if (items > kSms) best.here = blocks <= (m == 0 ? 4 : 3);
   else best.here = blocks <= (m == 0 ? 8 : 6);
   return best;
 }
