@@ -37,15 +37,11 @@ constexpr int kSmemBytes = kOffBar + 128 + 1024;
 constexpr int kThreads = 160;
 constexpr uint32_t kTmemCols = 128;
 constexpr uint32_t kColO = 64;
-// How far (log2 units) a row's maximum may run ahead of its reference.  The largest weights decide a row's rounding error: one that
-// the reference was taken from is exactly 1, one above a stale reference is rounded like any other.  With blocks half as
-// long as in the other kernels the reference is stale more often, so it has to follow more closely: nearly always at the
-// second block (with the first, the other kernels' first block), within 5 later (8 there).  Error against float64, other
-// kernels / this one with 8 throughout / this one: 2.88e-4 / 2.90e-4 / 2.88e-4 for fp16 rows of 512 keys at
-// scale d^-0.5, 2.19e-4 / 2.28e-4 / 2.15e-4 unscaled; 144 keys at 0.35, simulated, 2.33e-4 / 2.60e-4 / 2.29e-4.
+// What the close references (softmax_step.cuh) do here: with blocks half as long as in the other kernels a reference is stale more
+// often.  Error against float64, other kernels / this one with 8 throughout / this one: 2.88e-4 / 2.90e-4 / 2.88e-4 for fp16 rows of
+// 512 keys at scale d^-0.5, 2.19e-4 / 2.28e-4 / 2.15e-4 unscaled; 144 keys at 0.35, simulated, 2.33e-4 / 2.60e-4 / 2.29e-4.
 // The price is about one rescale an item, 56.4 -> 58.2 us for 2048 items of 512 keys, 7.5 -> 8.0 for one wave of 304; all
 // of O in one piece, or the rescale behind P, spill or delay every item (65.6 and 59.0 us).
-constexpr float kRescaleThreshold = 5.0f, kSecondBlockThreshold = 1.0f;
 constexpr int kModeSoftmax = 0, kModeRelu = 1;
 
 struct NBars {
@@ -209,7 +205,7 @@ __global__ void __launch_bounds__(kThreads, 4) attention_narrow_kernel(const __g
         for (int u = 0; u < 4; ++u) mx[u] = fmaxf(mx[u], mx[u + 4]);
         const float m_new = fmaxf(fmaxf(ref.m, mx[0]), fmaxf(fmaxf(mx[1], mx[2]), mx[3]));
         // lazy rescale, as in attention_sm100.cu; s_full(g) implies that P*V(g - 1) is done, so O is quiescent
-        if (__any_sync(0xffffffffu, ref.asks(m_new, c, g == 1 ? kSecondBlockThreshold : kRescaleThreshold))) {
+        if (__any_sync(0xffffffffu, ref.asks(m_new, c, g == 1 ? kCloseSecondBlock : kCloseRescale))) {
           const float f = ref.move(m_new, c);
           if (g > 0) {
 #pragma unroll 1

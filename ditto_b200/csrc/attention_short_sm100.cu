@@ -37,9 +37,6 @@ constexpr int kStages = 2;
 constexpr int kSoftmaxWarps = 8, kWarpLoad = 8, kWarpMma = 9;
 constexpr int kThreads = 10 * 32;
 constexpr int kFirstKeys = 64;            // of a block, in the first part of P (groups 0 and 1); the rest follows by itself
-// As in the kernel with 64-key blocks, some of whose calls come here: the closer a row's reference follows its maximum, the
-// smaller the rounding error of its largest weights.
-constexpr float kRescaleThreshold = 5.0f, kSecondBlockThreshold = 1.0f;
 constexpr int kModeSoftmax = 0, kModeRelu = 1;
 
 template <int D>
@@ -307,7 +304,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __gr
           tc_fence_after_sync();
         }
         // lazy rescale, as in attention_sm100.cu; both warps of a quarter see the same maxima and decide alike
-        if (__any_sync(0xffffffffu, ref.asks(m_new, c, j == 1 ? kSecondBlockThreshold : kRescaleThreshold))) {
+        if (__any_sync(0xffffffffu, ref.asks(m_new, c, j == 1 ? kCloseSecondBlock : kCloseRescale))) {
           const float f = ref.move(m_new, c);
           if (j > 0) {
 #pragma unroll 1
@@ -575,17 +572,22 @@ constexpr int kRowFrom[2] = {5, 4};                             // blocks a part
 
 // Where the lines lie, the forms without this kernel and with two CTAs an SM left out of count -> the choice now (us), items x blocks of
 // sequences of 512 rows.  Softmax at head dimension 64: 24 x 1 5.3 -> 4.6, 24 x 2 6.5 -> 6.1, 24 x 4 7.3 -> 6.5 (4 parts), 24 x 16 11.0 -> 10.8 (4),
-// 48 x 16 15.6 -> 14.4 (4), 100 x 2 6.9 -> 6.3, 148 x 4 10.2 -> 9.7, with a thread a row 24 x 64 25.3 -> 21.5 (8), 100 x 32 43.1 -> 33.7 (2),
-// 148 x 64 83.1 -> 59.7 (2); at 128: 24 x 1 7.2 -> 5.2, 24 x 2 7.9 -> 6.7, 24 x 4 9.0 -> 8.3 (4), 24 x 16 14.3 -> 13.2 (4), 48 x 16 20.3 -> 18.9 (2),
+// 48 x 16 15.6 -> 14.4 (4), 100 x 2 6.9 -> 6.3, 148 x 4 10.2 -> 9.7, with a thread a row 24 x 64 25.3 -> 21.2 (8), 100 x 32 43.1 -> 33.6 (2),
+// 148 x 64 83.1 -> 61.7 (2); at 128: 24 x 1 7.2 -> 5.2, 24 x 2 7.9 -> 6.7, 24 x 4 9.0 -> 8.3 (4), 24 x 16 14.3 -> 13.2 (4), 48 x 16 20.3 -> 18.9 (2),
 // 100 x 32 64.4 -> 51.6; without a softmax 48 x 16 17.6 -> 14.5, 100 x 32 57.2 -> 39.5.
 // At head dimension 64 the kernel with a thread a row costs less per block (1.18 against 1.35: no word from another warp before the
-// exponentials).  This kernel's time over that one's, split alike, by blocks a part: one 0.88, two 0.95, four 0.98, six 1.01, eight
-// 1.03, sixteen 1.07 (24 x 64 in four parts 27.0 against 25.3), so parts of more than four blocks take that one; without a softmax
-// of more than three (48 x 8 7.4 -> 7.8, 12 x 64 10.7 -> 12.0).
-// Unsplit and two CTAs an SM it pays for up to four blocks (200 x 2 8.1 -> 7.6, 256 x 4 12.3 -> 11.9; 296 x 8 22.3 -> 22.5), without a softmax
-// for up to three (148 x 1 4.4 -> 3.7, 200 x 1 4.7 -> 4.3, 200 x 2 5.9 -> 5.4).  One tile
-// a sequence at head dimension 128 has no second tile to work beside: there it pays in any number from six blocks on (200 x 8 36.8
-// -> 33.2, 256 x 16 69.0 -> 58.1).
+// exponentials).  This kernel's time over that one's, split alike, by blocks a part, a CTA an SM / two: one 0.90 / 0.99, two 0.93 / 0.99, four
+// 0.97 / 1.01, six 1.00 / 1.05, eight 1.02 / 1.06, sixteen 1.06 / 1.11, so parts of more than four blocks take that one; without a
+// softmax of more than three (48 x 8 7.4 -> 7.8, 12 x 64 10.7 -> 12.0).
+// Unsplit and two CTAs an SM it serves one to four blocks: one block is faster here (200 x 1 5.8 -> 5.5), two to four are about as fast as
+// in the kernel with 64-key blocks, whose references are those of shorter blocks (200 x 2 7.8 -> 7.7, 200 x 3 9.7 -> 10.2, 256 x 4
+// 12.5 -> 13.1, at worst, of one tile a sequence, 296 x 3 11.8 -> 12.8; its error against float64 is 1 to 3 % larger at scale
+// d^-0.5 and up to 10 % on uniform operands at scale 1); longer ones have no gain (296 x 8 20.8 -> 20.9 and the same error).  Without a
+// softmax it pays for up to three (148 x 1 4.4 -> 3.7, 200 x 1 4.7 -> 4.3, 200 x 2 5.9 -> 5.4).
+// One tile a sequence at head dimension 128 has no second tile to work beside: there it pays in any number of items from six blocks on,
+// without a softmax (200 x 8 35.0 -> 29.7, 1000 x 8 118 -> 109, 4000 x 6 382 -> 365) and with one (200 x 8 36.4 -> 33.5, 256 x 16 74 -> 65, 1000 x 16
+// 254 -> 232); many items of six to eight are no faster (592 x 6 62.2 -> 65.7, 1480 x 6 150 -> 163, 1480 x 8 195 -> 201), but 1 % closer to
+// float64 at scale d^-0.5 and 10 % where the scores spread further: the other kernel keeps its references within 2^8 only.
 AttnFew attention_few(int batch, int M, int L, int d, int mode) {
   constexpr int kSms = 148;
   const long long items = static_cast<long long>((M + kBM - 1) / kBM) * batch;

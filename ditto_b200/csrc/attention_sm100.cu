@@ -554,8 +554,10 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
         }
       }
       // Lazy rescale: keep the stale maximum while the true one is within
-      // 2^kRescaleThreshold of it; the final division by l cancels the difference.
-      const bool need = MODE == kModeSoftmax && ref.asks(m_new, c, kRescaleThreshold);
+      // 2^kRescaleThreshold of it; the final division by l cancels the difference.  (Split items, which the kernel for few items
+      // shares with this one, keep closer.)
+      const float threshold = !SPLIT ? kRescaleThreshold : j == 1 ? kCloseSecondBlock : kCloseRescale;
+      const bool need = MODE == kModeSoftmax && ref.asks(m_new, c, threshold);
       if (MODE == kModeSoftmax && __any_sync(0xffffffffu, need)) {
         const float f = ref.move(m_new, c);
         if (j > 0) {

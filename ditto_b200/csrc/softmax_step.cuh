@@ -10,6 +10,11 @@ namespace ditto_b200 {
 // exponents by at most 2^-13, which is below the rounding of the 16-bit probabilities.
 constexpr float kFusedReference = 4096.0f;
 
+// How far (log2 units) a row's maximum may run ahead of its reference in the kernels for few items, split or not, and in the one with
+// 64-key blocks, at the second block and later (8 throughout in the others).  The largest weights decide a row's rounding error: one that the
+// reference was taken from is exactly 1, one above a stale reference is rounded like any other.
+constexpr float kCloseSecondBlock = 1.0f, kCloseRescale = 5.0f;
+
 // m is the (possibly stale) maximum that a row's exponentials refer to, c = scale * log2(e): a score's weight is
 // ex2(fmaf(s, c, -mc)), at most 2^(rescale threshold).
 //
