@@ -47,8 +47,7 @@ int make_map_3d(CUtensorMap* map, bool bf16, const void* base, uint64_t cols, ui
 bool narrow_for(int flags, bool any, long long batch, int M, int L, int d, int mode = 0) {
   if (!any || d != 64) return false;
   if (flags & DITTO_FLAG_NARROW) return true;
-  return !(flags & (DITTO_FLAG_FEW | DITTO_FLAG_SPLIT_MASK)) && ditto_b200::attention_narrow_pays(static_cast<int>(batch), M, L, mode) &&
-         !ditto_b200::attention_few(static_cast<int>(batch), M, L, d, mode).here;
+  return !(flags & (DITTO_FLAG_FEW | DITTO_FLAG_SPLIT_MASK)) && ditto_b200::attention_narrow_pays(static_cast<int>(batch), M, L, mode);
 }
 
 // The form of an attention-shaped call: as the caller's flags say, else by shape.  The 64-key kernel is settled before (`narrow`: its

@@ -329,20 +329,20 @@ cudaError_t launch_attention_narrow(const AttnParams& p, int batch, bool bf16, i
   return bf16 ? launch_n<true, 2>(p, items, stream) : launch_n<false, 2>(p, items, stream);
 }
 
-// Where the lines lie: up to three 128-key blocks an item this is the faster form as soon as most SMs have one, with four as
-// soon as some SMs have two, up to eight with more items than the other kernels hold at once (296) and a half-full wave of
-// them; for longer items the other kernels' 128-key blocks cost less (1.6 us for two a SM against 2 x 1.0), and it pays again
-// once a launch is three waves of those or more.  Measured, us, others -> this kernel: 2048 items of 512 keys 74.8 -> 63.2; 1200
-// of 208 30.0 -> 25.0; 1000 of 128 17.5 -> 14.4; 640 of 64 13.9 -> 8.8; 384 of 512 20.7 -> 18.4; 180 of 512 12.0 -> 12.0; 110 of 208
-// 7.5 -> 7.1; 400 of 1024 36.2 -> 32.2; 1024 of 8192 393 -> 368; and left alone: 48 of 512 9.0 -> 9.8, 144 of 512 10.4 -> 10.6,
-// 320 of 1024 30.2 -> 31.8, 128 of 2048 23.8 -> 30.4, 384 of 2048 51.7 -> 56.8, 320 of 8192 179 -> 209.  A chain without a softmax
-// has less between the hand-overs: it gains with one or two blocks and many items only (600 x 208 rows and keys 19.4 -> 18.0,
-// 640 of 64 9.4 -> 7.4; 640 of 1024 would go 40 -> 43, 144 of 512 7.4 -> 8.6).
+// Where the lines lie: calls of up to 296 items have other forms (attention_few: of up to four 128-key blocks, and of any number up to 148 items;
+// those between are not long enough for this one, 200 x 5 blocks 14.3 -> 14.0, 200 x 8 19.9 -> 20.6).  Above, it is the faster form up to four
+// 128-key blocks an item, up to eight with a half-full wave more than the other kernels hold at once; for longer items the other
+// kernels' 128-key blocks cost less (1.6 us for two a SM against 2 x 1.0), and it pays again once a launch is three waves of those
+// or more.  Measured, us, others -> this kernel: 2048 items of 512 keys 74.8 -> 63.2; 1200 of 208 30.0 -> 25.0; 1000 of 128
+// 17.5 -> 14.4; 640 of 64 13.9 -> 8.8; 384 of 512 20.7 -> 18.4; 400 of 1024 36.2 -> 32.2; 1024 of 8192 393 -> 368; and left alone: 320 of
+// 1024 30.2 -> 31.8, 384 of 2048 51.7 -> 56.8, 320 of 8192 179 -> 209.  A chain without a softmax has less between the hand-overs:
+// it gains with one or two blocks and many items only (600 x 208 rows and keys 19.4 -> 18.0, 640 of 64 9.4 -> 7.4; 640 of 1024
+// would go 40 -> 43).
 bool attention_narrow_pays(int batch, int M, int L, int mode) {
   const long long items = static_cast<long long>((M + kBM - 1) / kBM) * batch;
   const int blocks = (L + 127) / 128;
   if (mode != kModeSoftmax) return blocks <= 2 && items > 296;
-  return items > (blocks <= 3 ? 100 : blocks == 4 ? 148 : blocks <= 8 ? 349 : 887);
+  return items > (blocks <= 4 ? 296 : blocks <= 8 ? 349 : 887);
 }
 
 }  // namespace ditto_b200

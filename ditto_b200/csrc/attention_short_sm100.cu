@@ -13,7 +13,7 @@
 // With `parts` CTAs in the cluster each takes a contiguous part of the tile's blocks; they combine (max, sum, O) through
 // distributed shared memory at the end.
 //
-// Two CTAs fit an SM at head dimension 64 (83 KB, 256 tensor-memory columns, 95 registers): the next call's are set up under this
+// Two CTAs fit an SM at head dimension 64 (84 KB, 256 tensor-memory columns, 94 registers): the next call's are set up under this
 // one's.  What it measured stands at attention_few.
 #include "attention_sm100.cuh"
 
@@ -582,7 +582,7 @@ constexpr int kRowFrom[2] = {5, 4};                             // blocks a part
 // Unsplit and two CTAs an SM it serves one to four blocks: one block is faster here (200 x 1 5.8 -> 5.5), two to four are about as fast as
 // in the kernel with 64-key blocks, whose references are those of shorter blocks (200 x 2 7.8 -> 7.7, 200 x 3 9.7 -> 10.2, 256 x 4
 // 12.5 -> 13.1, at worst, of one tile a sequence, 296 x 3 11.8 -> 12.8; its error against float64 is 1 to 3 % larger at scale
-// d^-0.5 and up to 10 % on uniform operands at scale 1); longer ones have no gain (296 x 8 20.8 -> 20.9 and the same error).  Without a
+// d^-0.5 and up to 10 % on uniform operands at scale 1); longer ones have no gain (296 x 8 20.2 -> 21.2).  Without a
 // softmax it pays for up to three (148 x 1 4.4 -> 3.7, 200 x 1 4.7 -> 4.3, 200 x 2 5.9 -> 5.4).
 // One tile a sequence at head dimension 128 has no second tile to work beside: there it pays in any number of items from six blocks on,
 // without a softmax (200 x 8 35.0 -> 29.7, 1000 x 8 118 -> 109, 4000 x 6 382 -> 365) and with one (200 x 8 36.4 -> 33.5, 256 x 16 74 -> 65, 1000 x 16

@@ -89,8 +89,8 @@ template <int D, int NT, bool PSMEM>
 constexpr bool kSeparateP = (NT == 1 && D == 64 && !PSMEM);
 
 // Instances whose CTAs walk several work items (the others are launched with one CTA per item).
-template <int D, int NT, bool PSMEM, bool SPLIT>
-constexpr bool kLoopItems = (D == 128 && !kSeparateP<D, NT, PSMEM> && !SPLIT);
+template <int D>
+constexpr bool kLoopItems = D == 128;             // (separate P and split items are forms of head dimension 64)
 
 template <int D, int NT, bool PSMEM>
 struct Smem {
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
   const int tiles = (p.M + NT * kBM - 1) / (NT * kBM);
   // The loop is a compile-time property of the instance (head dimension 128; see the launcher): with one item
   // per CTA known at compile time the other instances keep the code -- and the registers -- of a single pass.
-  constexpr bool kLoop = kLoopItems<D, NT, PSMEM, SPLIT>;
+  constexpr bool kLoop = kLoopItems<D>;
   // the CTAs of a cluster are consecutive: rank r of `parts` takes K/V blocks [r * n / parts, (r + 1) * n / parts)
   const int part = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
   const int parts = SPLIT ? p.parts : 1;
@@ -822,7 +822,7 @@ static cudaError_t launch_one(const AttnParams& p, int batch, int parts, cudaStr
   // The work loop pays where an item is long enough for its fixed cost to show and short enough for it to
   // matter: measured at head dimension 128 (S = 512: -5 %, 2048: -1 % per item); at 64, where the exponentials
   // set the pace, one CTA per item was faster (S = 2048: 109 against 119 us), so those launches keep it.
-  constexpr bool loop = kLoopItems<D, NT, PSMEM, SPLIT>;
+  constexpr bool loop = kLoopItems<D>;
   const int grid = loop ? std::min(q.items, places[dev].load(std::memory_order_relaxed)) : q.items * parts;
   cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
   cfg.blockDim = dim3(threads_for(NT), 1, 1);
