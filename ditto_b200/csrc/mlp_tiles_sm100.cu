@@ -37,8 +37,8 @@ constexpr int kATile = 16 * 1024;                // 128 rows x 64
 constexpr int kMaxStages = 8;
 // Two epilogue warps per quarter of the rows, which take a tile's columns in turn: the read-out of the accumulator (act, bias,
 // turn around, store) is a chain of 32-column pieces at the end of either launch, and half as long for it.  Four warps -> eight,
-// us: 512 x 768 -> 3072 -> 768 with biases and GELU 18.1 -> 16.8, 2048 x 768 32.9 -> 31.5, 4096 x 768 54.3 -> 52.3; 2048 x 1024
-// with ReLU alone, whose pieces are short, 41.4 -> 41.1.
+// us: 512 x 768 -> 3072 -> 768 with biases and GELU 18.1 -> 16.8, 2048 x 768 32.9 -> 31.5, 4096 x 768 54.3 -> 52.3; with
+// ReLU alone, whose pieces are short, no difference (2048 x 1024 41.7).
 constexpr int kEpiWarps = 8;
 constexpr int kWarpA = kEpiWarps, kWarpB = kEpiWarps + 1, kWarpMma = kEpiWarps + 2;
 constexpr int kThreads = (kEpiWarps + 3) * 32;
@@ -399,7 +399,9 @@ namespace {
 // Modelled time (us, without a launch's fixed part) of D [M, N] over `steps` k-steps.  Waves of tiles: a step on an SM
 // with a full set of CTAs, and one of a lone CTA, which is longer where too few bytes are in flight (bn = 64; a 96 KB
 // ring).  The constants are fitted to 390 timings (13 shapes of 16 to 16384 rows, each with 10 to 20 ways to cut either
-// GEMM); the cut it picks is on average 1.3 % slower than the best one timed.
+// GEMM) of the kernel with four epilogue warps.  With eight, whose ends are shorter, the cut it picks is on average 3 % slower than
+// the best one timed (17 shapes, ReLU and GELU with biases), at worst 12 %: 16384 x 256, first GEMM 128 wide 30.2 us, 256 wide 26.6;
+// 512 x 1024, second GEMM in eight parts of 128 columns 22.4 us, four of 64 20.0.
 double tiles_time(long long blocks, int N, int steps, const TilesGemm& g) {
   const double shared = 0.109 + 0.00059 * g.bn;
   const double lone = std::max(g.per_sm == 1 ? 0.382 - 0.00333 * g.bn : -0.066 + 0.00242 * g.bn, shared);
@@ -436,9 +438,10 @@ TilesGemm best_gemm(long long blocks, int N, int steps, double* time) {
 }  // namespace
 
 // Where two launches are the faster form.  The flow kernel's waits cost it about 10 us a call, and it is 20 % faster
-// per operation once its pairs are busy: measured, flow -> tiles, 16 x 1024 -> 4096 -> 1024 24.3 -> 12.9 us, 512 x 768 24.4 ->
-// 16.6, 2048 x 1024 (34 GFLOP) 40.8 -> 33.0, 4096 x 768 (39) 52.3 -> 45.9; 1024 x 2048 (69) 67.0 -> 67.6, 16384 x 512 (69)
-// 67 -> 74, 3328 x 1280 (87) 75 -> 82.  The hidden layer has to stay in L2 beside the operands.
+// per operation once its pairs are busy: measured, flow -> tiles, 16 x 1024 -> 4096 -> 1024 25.9 -> 16.2 us, 512 x 768 23.7 ->
+// 15.2, 2048 x 1024 (34 GFLOP) 42.0 -> 37.0, 4096 x 768 (39) 46.6 -> 43.3, 2560 x 1024 (43) 50.5 -> 51.5; on the other side either is
+// the faster one: 6144 x 768 (58) 53.4 -> 49.0, 4096 x 1024 (69) 60.1 -> 58.5, 1024 x 2048 (69) 64.2 -> 65.7, 16384 x 512 (69) 66.9 ->
+// 73.7, 3328 x 1280 (87) 70.2 -> 71.3.  The hidden layer has to stay in L2 beside the operands.
 bool mlp_tiles_faster(int batch, int M, int N, int K, int L) {
   return 2.0 * batch * M * static_cast<double>(L) * (static_cast<double>(K) + N) <= 4.8e10 &&
          mlp_tiles_workspace_bytes(batch, M, L) <= (static_cast<size_t>(48) << 20);
