@@ -42,6 +42,12 @@ constexpr uint32_t kColO = 64;
 // 512 keys at scale d^-0.5, 2.19e-4 / 2.28e-4 / 2.15e-4 unscaled; 144 keys at 0.35, simulated, 2.33e-4 / 2.60e-4 / 2.29e-4.
 // The price is about one rescale an item, 56.4 -> 58.2 us for 2048 items of 512 keys, 7.5 -> 8.0 for one wave of 304; all
 // of O in one piece, or the rescale behind P, spill or delay every item (65.6 and 59.0 us).
+// Of every eight pairs of weights, how many the multiply-add pipe computes (ex2_fma_f32x2).  Four softmax warps on a scheduler keep
+// the special-function unit 63 % busy over a long launch and issue in half of the slots; an eighth of the exponentials elsewhere is
+// what pays (0 / 1 / 2 / 3 of eight, us: 1024 items of 8192 keys 370 / 347 / 358 / 377, 2048 of 512 59.4 / 57.0 / 59.1 / 60.5, 600 of 208
+// 15.7 / 15.4 / 15.6 / 15.8; without the packed arithmetic 362, 58.4 and 15.5): beyond that the longer instruction stream, and the clock under
+// the power it takes, cost more.
+constexpr int kFmaPairs = 1;
 constexpr int kModeSoftmax = 0, kModeRelu = 1;
 
 struct NBars {
@@ -223,7 +229,8 @@ __global__ void __launch_bounds__(kThreads, 4) attention_narrow_kernel(const __g
         }
       }
       const float mc = ref.offset(c);
-      float sum0 = 0.f, sum1 = 0.f;
+      const uint64_t c2 = pack_f32x2(c, c), nmc2 = pack_f32x2(-mc, -mc);
+      uint64_t sum[2] = {0, 0};
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         uint32_t pk[16];
@@ -231,10 +238,9 @@ __global__ void __launch_bounds__(kThreads, 4) attention_narrow_kernel(const __g
         for (int i = 0; i < 16; ++i) {
           float p0 = __uint_as_float(sv[32 * h + 2 * i]), p1 = __uint_as_float(sv[32 * h + 2 * i + 1]);
           if constexpr (MODE == kModeSoftmax) {
-            p0 = ex2_approx(fmaf(p0, c, -mc));
-            p1 = ex2_approx(fmaf(p1, c, -mc));
-            sum0 += p0;
-            sum1 += p1;
+            const uint64_t w = softmax_weights(sv[32 * h + 2 * i], sv[32 * h + 2 * i + 1], c2, nmc2, i % 8 >= 8 - kFmaPairs);
+            sum[i & 1] = add_f32x2(sum[i & 1], w);
+            unpack_f32x2(w, p0, p1);
           } else if constexpr (MODE == kModeRelu) {
             p0 = p0 > 0.f ? p0 : 0.f;
             p1 = p1 > 0.f ? p1 : 0.f;
@@ -243,6 +249,8 @@ __global__ void __launch_bounds__(kThreads, 4) attention_narrow_kernel(const __g
         }
         tmem_st_x16(s_col + 16 * h, pk);           // (every lane's scores are in registers: the load is warp-collective)
       }
+      float sum0, sum1;
+      unpack_f32x2(add_f32x2(sum[0], sum[1]), sum0, sum1);
       l += sum0 + sum1;
       tmem_wait_st();
       tc_fence_before_sync();

@@ -334,6 +334,13 @@ __host__ __device__ constexpr uint32_t umma_idesc_f16(bool bf16, uint32_t m, uin
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// ---------------------------------------------------------------- registers
+// A warp group gives registers back to the CTA, or takes them (waits until they are there): all four warps execute it.
+template <int N>
+__device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // ---------------------------------------------------------------- math
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
@@ -344,6 +351,58 @@ __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// Two float32 values in a 64-bit register: one instruction of the multiply-add pipe for both.
+__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// The larger of two values, NaN if either is.
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
+
+// 2^x of a pair on the multiply-add pipe, for softmax exponents: x <= 127; -inf and what lies below -127 give 0, NaN stays NaN.
+// x = n + f with n the nearest integer: adding 1.5 * 2^23 + 127 leaves n + 127 in the low bits of the sum, which shifted up
+// are 2^n.  2^f = 1 + f q(f) on [-1/2, 1/2] with q of degree 4, least maximum relative error (iteratively reweighted least
+// squares): 9.2e-8, less than ex2.approx's own 2^-22.
+__device__ __forceinline__ uint64_t ex2_fma_f32x2(uint64_t x_in) {
+  float x0, x1, t0, t1;
+  unpack_f32x2(x_in, x0, x1);
+  const uint64_t x = pack_f32x2(max_nan(x0, -127.0f), max_nan(x1, -127.0f));
+  constexpr float kShift = 12582912.0f + 127.0f;
+  const uint64_t t = add_f32x2(x, pack_f32x2(kShift, kShift));
+  const uint64_t n = add_f32x2(t, pack_f32x2(-kShift, -kShift));
+  const uint64_t f = fma_f32x2(n, pack_f32x2(-1.0f, -1.0f), x);
+  unpack_f32x2(t, t0, t1);
+  const uint64_t s = pack_f32x2(__uint_as_float(__float_as_uint(t0) << 23), __uint_as_float(__float_as_uint(t1) << 23));
+  uint64_t q = fma_f32x2(f, pack_f32x2(0x1.5bba14p-10f, 0x1.5bba14p-10f), pack_f32x2(0x1.3cea88p-7f, 0x1.3cea88p-7f));
+  q = fma_f32x2(q, f, pack_f32x2(0x1.c6b752p-5f, 0x1.c6b752p-5f));
+  q = fma_f32x2(q, f, pack_f32x2(0x1.ebf9bcp-3f, 0x1.ebf9bcp-3f));
+  q = fma_f32x2(q, f, pack_f32x2(0x1.62e42ap-1f, 0x1.62e42ap-1f));
+  return fma_f32x2(q, mul_f32x2(f, s), s);
 }
 
 // Two exponentials per special-function instruction: 2^x0, 2^x1 evaluated on the packed 16-bit pair and

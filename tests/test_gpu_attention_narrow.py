@@ -106,3 +106,29 @@ def test_no_less_precise_than_longer_blocks(L, dtype):
         narrow, whole = ((ops.bmm_softmax_bmm(q, k, v, scale=scale, key_layout="LK", flags=f).double() - want).norm().item()
                          for f in (NARROW, _lib.FLAG_SPLIT_UNIT))
         assert narrow <= 1.01 * whole, (scale, narrow / want.norm().item(), whole / want.norm().item())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_weights_far_apart_and_scores_that_are_not_numbers(dtype):
+    """Weights come from two pipes, by a key's place in the block: both give 2^x down to where it is nothing, 0 for -inf and NaN for
+    NaN.  A row's tolerance is _close's (rounding of the weights and of the result); exponents differ by up to 2^-13 (kFusedReference)."""
+    g = torch.Generator(device="cuda").manual_seed(9)
+    b, M, d, L = 1, 128, 64, 128
+    q = torch.ones(b, M, d, device="cuda", dtype=dtype)
+    v = torch.randn(b, L, d, generator=g, device="cuda").to(dtype)
+    # scores d * x with x from 0 to -3.5: weights 1 to 2^-320, in an order that gives every place in a block all sizes
+    for turn in range(4):
+        x = torch.linspace(0, -3.5, L, device="cuda").roll(17 * turn)[torch.randperm(L, generator=g, device="cuda")]
+        k = x[None, :, None].expand(b, L, d).to(dtype).contiguous()
+        _close(ops.bmm_softmax_bmm(q, k, v, key_layout="LK", flags=NARROW), _reference(q, k, v, 1.0), dtype)
+    k = torch.randn(b, L, d, generator=g, device="cuda").to(dtype)
+    for key in list(range(16)) + [63, 64, 127]:
+        for bad, place in ((float("nan"), k), (float("inf"), k)):
+            broken = place.clone()
+            broken[0, key] = bad
+            assert torch.isnan(ops.bmm_softmax_bmm(q, broken, v, scale=0.125, key_layout="LK", flags=NARROW)).all(), (key, bad)
+        gone = k.clone()
+        gone[0, key] = float("-inf")
+        rest = [i for i in range(L) if i != key]
+        _close(ops.bmm_softmax_bmm(q, gone, v, scale=0.125, key_layout="LK", flags=NARROW), _reference(q, k[:, rest], v[:, rest], 0.125), dtype)
+    assert ops.device_status() == 0
