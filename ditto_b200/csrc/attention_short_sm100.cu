@@ -79,14 +79,21 @@ __device__ __forceinline__ float max_with(float m, const uint32_t* s) {
   return max3(a[0], a[1], a[2]);
 }
 
+// Of every eight pairs of weights, how many the multiply-add pipe computes: a block is a chain of one warp's steps here, and the
+// exponentials its longest.  None (and scalar arithmetic) / 1 / 2 / 3, us: head dimension 64, 12 slices of 512 rows and keys 7.86 / 7.77 /
+// 7.78 / 7.87, 40 of them 11.97 / 11.58 / 11.74 / 12.24; 128, 140 tiles of 1024 keys 16.5 / 16.0 / 15.8 / 16.3.
+constexpr int kFmaPairs = 1;
+
 // 32 scores of a row -> their weights 2^(s c - mc), rounded to the operand type and packed; the sums take them before rounding.
 template <bool BF16>
-__device__ __forceinline__ void softmax_weights(const uint32_t* s, float c, float mc, float& sum0, float& sum1, uint32_t (&w)[16]) {
+__device__ __forceinline__ void row_weights(const uint32_t* s, float c, float mc, uint64_t& sum, uint32_t (&w)[16]) {
+  const uint64_t c2 = pack_f32x2(c, c), nmc2 = pack_f32x2(-mc, -mc);
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
-    const float a = ex2_approx(fmaf(__uint_as_float(s[2 * i]), c, -mc)), b = ex2_approx(fmaf(__uint_as_float(s[2 * i + 1]), c, -mc));
-    sum0 += a;
-    sum1 += b;
+    const uint64_t p = softmax_weights(s[2 * i], s[2 * i + 1], c2, nmc2, i % 8 >= 8 - kFmaPairs);
+    sum = add_f32x2(sum, p);
+    float a, b;
+    unpack_f32x2(p, a, b);
     w[i] = pack2<BF16>(a, b);
   }
 }
@@ -327,12 +334,12 @@ __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __gr
         tc_fence_after_sync();
       }
       const float mc = ref.offset(c);
-      float sum0 = 0.f, sum1 = 0.f;
+      uint64_t sum = 0;
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
         if (64 * g + 32 * half < keys) {                   // (P*V reads no others)
           uint32_t w[16];
-          if constexpr (MODE == kModeSoftmax) softmax_weights<BF16>(sv + 32 * g, c, mc, sum0, sum1, w);
+          if constexpr (MODE == kModeSoftmax) row_weights<BF16>(sv + 32 * g, c, mc, sum, w);
           else pass_on<BF16, MODE == kModeRelu>(sv + 32 * g, w);
           tmem_st_x16(p_col + 32 * g + 16 * half, w);
         }
@@ -340,6 +347,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __gr
         tc_fence_before_sync();
         mbar_arrive_warp(&bar->p_part[g], lane);
       }
+      float sum0, sum1;
+      unpack_f32x2(sum, sum0, sum1);
       l += sum0 + sum1;
     }
     if (ok && MODE == kModeSoftmax) {
