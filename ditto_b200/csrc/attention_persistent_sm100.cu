@@ -60,6 +60,8 @@ constexpr uint32_t kTmemCols = 256;
 constexpr uint32_t kColS = 0, kColO = 128, kColP = 192;
 constexpr int kSplit = 96;               // K/V rows in the first part of P
 constexpr float kRescaleThreshold = 8.0f;
+// Weights are computed two at a time (softmax_weights); scalar -> packed, us: 200 slices of 128 rows x 1024 keys 20.5 -> 19.5, 50 of
+// 512 x 640 15.0 -> 14.1, 260 of 128 x 768 16.8 -> 15.8.
 constexpr int kModeSoftmax = 0, kModeRelu = 1;
 
 struct PBars {
@@ -337,7 +339,9 @@ __global__ void __launch_bounds__(kThreads, 2) attention_persistent_kernel(const
           l *= f;
         }
         const float mc = ref.offset(c);
-        float sum0 = 0.f, sum1 = 0.f;
+        const uint64_t c2 = pack_f32x2(c, c), nmc2 = pack_f32x2(-mc, -mc);
+        uint64_t sum2[2] = {0, 0};
+        [[maybe_unused]] float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
         for (int part = 0; part < 2; ++part) {
           constexpr int kFirst = kSplit / 2;
@@ -356,14 +360,15 @@ __global__ void __launch_bounds__(kThreads, 2) attention_persistent_kernel(const
                 sum1 += pf.y;
                 continue;
               } else if constexpr (MODE == kModeSoftmax) {
-                p0 = ex2_approx(fmaf(p0, c, -mc));
-                p1 = ex2_approx(fmaf(p1, c, -mc));
+                const uint64_t w = softmax_weights(sv[2 * (w0 + i)], sv[2 * (w0 + i) + 1], c2, nmc2, false);
+                sum2[i & 1] = add_f32x2(sum2[i & 1], w);
+                unpack_f32x2(w, p0, p1);
+                pk[i] = pack2<BF16>(p0, p1);
+                continue;
               } else if constexpr (MODE == kModeRelu) {
                 p0 = p0 > 0.f ? p0 : 0.f;
                 p1 = p1 > 0.f ? p1 : 0.f;
               }
-              sum0 += p0;
-              sum1 += p1;
               pk[i] = pack2<BF16>(p0, p1);
             }
           }
@@ -386,6 +391,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_persistent_kernel(const
           mbar_arrive(&bar->p_part[part]);
           DITTO_STAMP(1024 + it * 16 + 4 + j * 2 + part);
         }
+        if constexpr (DITTO_PACKED_EX2 == 0) unpack_f32x2(add_f32x2(sum2[0], sum2[1]), sum0, sum1);
         l += sum0 + sum1;
         DITTO_STAMP(it * 16 + j * 2 + 1);
       }

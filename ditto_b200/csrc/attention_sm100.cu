@@ -107,6 +107,16 @@ struct Smem {
   static constexpr int kBytes = kOffStage + NT * 4 * 4096 + 1024;  // ... + slack for 1024-byte alignment
 };
 
+// Of every eight pairs of weights, how many the multiply-add pipe computes (ex2_fma_f32x2).  One tile at head dimension 128 is a
+// chain of one softmax warp a scheduler, whose exponentials are its longest step: none / 1 / 2 / 3, us: 1000 slices of 128 rows x 512
+// keys 69.4 / 69.1 / 70.7 / 73.9, 600 x 2048 156.6 / 154.7 / 155.4 / 160.0.  With two softmax warps a scheduler the longer instruction
+// stream costs more: two tiles of 8192 keys 1688 / 1697 / 1856 clocks a block, head dimension 64 1503 / 1525.
+// The packed arithmetic alone, scalar -> packed, us: two tiles, 148 slices of 512 x 8192 272 -> 260, 512 of 512 x 512 85.6 -> 82.4, 256 of
+// 208 x 208 at d = 80 19.1 -> 18.1; head dimension 64, 16 slices of 8192 x 8192 383 -> 375, 100 of 512 x 2048 53.1 -> 50.8.  (1024 slices
+// of 2048 x 2048 stay at 2.05 ms: 1716 -> 1667 clocks a block, but 1480 -> 1440 MHz under the power cap.)
+template <int D, int NT>
+constexpr int kFmaPairs = D == 128 && NT == 1 ? 1 : 0;
+
 struct Barriers {
   uint64_t q_full[2], q_empty[2];   // per query tile: Q has landed / the item's last S MMA has read it
   uint64_t k_full[4], k_empty[4], v_full[4], v_empty[4];
@@ -579,7 +589,9 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
 
       if ((warp & 3) == 0) DITTO_STAMP(t * 256, k * nkv + j, 2);
       const float mc = ref.offset(c);
-      float sum0 = 0.f, sum1 = 0.f;
+      const uint64_t c2 = pack_f32x2(c, c), nmc2 = pack_f32x2(-mc, -mc);
+      uint64_t sum2[2] = {0, 0};
+      [[maybe_unused]] float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
       for (int part = 0; part < 2; ++part) {
         constexpr int kFirst = kSplit / 2;               // packed 32-bit words in part 0
@@ -598,14 +610,15 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
               sum1 += pf.y;
               continue;
             } else if constexpr (MODE == kModeSoftmax) {
-              p0 = ex2_approx(fmaf(p0, c, -mc));
-              p1 = ex2_approx(fmaf(p1, c, -mc));
+              const uint64_t w = softmax_weights(sv[2 * (w0 + i)], sv[2 * (w0 + i) + 1], c2, nmc2, i % 8 >= 8 - kFmaPairs<D, NT>);
+              sum2[i & 1] = add_f32x2(sum2[i & 1], w);
+              unpack_f32x2(w, p0, p1);
+              pk[i] = pack2<BF16>(p0, p1);
+              continue;
             } else if constexpr (MODE == kModeRelu) {
               p0 = p0 > 0.f ? p0 : 0.f;                  // if_then_else(D > 0, D, 0) as in the reference
               p1 = p1 > 0.f ? p1 : 0.f;
             }
-            sum0 += p0;
-            sum1 += p1;
             pk[i] = pack2<BF16>(p0, p1);
           }
         }
@@ -643,6 +656,7 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
         mbar_arrive(&bar->p_part[t][part]);
         if (part == 0 && (warp & 3) == 0) DITTO_STAMP(t * 256, k * nkv + j, 4);
       }
+      if constexpr (DITTO_PACKED_EX2 == 0) unpack_f32x2(add_f32x2(sum2[0], sum2[1]), sum0, sum1);
       l += sum0 + sum1;
       if ((warp & 3) == 0) DITTO_STAMP(t * 256, k * nkv + j, 5); else DITTO_STAMP(t * 256, k * nkv + j, 5 + (warp & 3));
     }
