@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(kThreads, 2) mlp_tiles_kernel(const __grid_con
     // thread reaches both barriers whether its waits expired or not.
     __syncwarp();
     cluster_sync_all();
-    const int cols = p.bn / p.parts;                     // 16, 32 or 64
+    const int cols = p.bn / p.parts;                     // 16, 32, 64 or 128
     const int row = (warp & 3) * 32 + lane;
     if (warp < kEpiWarps) {
       const int cols_log2 = 31 - __clz(cols);
@@ -416,12 +416,17 @@ double tiles_time(long long blocks, int N, int steps, const TilesGemm& g) {
 }
 
 // (A reduction over 1024 or less is not split, as in the flow kernel: the result has the bits of the cluster kernels.)
+// 256 columns in two parts, alone on their SMs (an incoming share is 128 KB), keep as many SMs busy as 128 columns unsplit do, but a
+// k-step of them brings 48 KB for 512 clocks of tensor work and not 32 KB for 256: 64 of those took 376 clocks each out of L2, 32 of
+// these take 565.  In a graph, us, without -> with: 2048 x 1024 -> 4096 -> 1024 34.9 -> 32.9, 1120 x 560 -> 6144 -> 1536 38.0 -> 33.1,
+// 1152 x 1280 -> 5120 -> 1280 39.2 -> 35.6, 2544 x 768 -> 3072 -> 768 29.3 -> 28.6; least of fourteen shapes that take it, 2784 x 352 -> 3072 ->
+// 768 25.2 -> 25.3.  (Four or eight parts of 256 columns are no faster than those of 128: 256 x 1536 22.4 -> 24.9.)
 TilesGemm best_gemm(long long blocks, int N, int steps, double* time) {
   TilesGemm best = {128, 1, 2};
   *time = tiles_time(blocks, N, steps, best);
   for (int bn = 64; bn <= 256; bn += 64)
-    for (int parts = 1; parts <= (bn == 128 ? 8 : bn == 64 ? 4 : 1) && (parts == 1 || steps > 16); parts *= 2)
-      for (int per_sm = 1; per_sm <= 2; ++per_sm) {
+    for (int parts = 1; parts <= (bn == 128 ? 8 : bn == 64 ? 4 : bn == 256 ? 2 : 1) && (parts == 1 || steps > 16); parts *= 2)
+      for (int per_sm = 1; per_sm <= (bn == 256 && parts > 1 ? 1 : 2); ++per_sm) {
         const long long ctas = blocks * ((N + bn - 1) / bn) * parts;
         // all clusters at once; alone on their SMs, large ones leave part of a GPC unused
         if (parts > 1 && ctas > (per_sm == 2 ? 296 : parts == 2 ? 148 : 112)) continue;

@@ -9,7 +9,7 @@ namespace ditto_b200 {
 // How one GEMM is cut: tiles of 128 x bn by clusters of `parts` CTAs that divide the reduction between them.
 struct TilesGemm {
   int bn;              // 64, 128, 192 or 256
-  int parts;           // 1, 2, 4 or 8; above 1: bn is 128 (64: at most 4), so that an incoming share fits the operand ring
+  int parts;           // 1, 2, 4 or 8; above 1: bn is 128 (64: at most 4; 256: 2, one CTA an SM), so that an incoming share fits the operand ring
   int per_sm;          // CTAs an SM holds: 1 (a ring of 192 KB) or 2 (96 KB)
 };
 struct TilesPlan {

@@ -33,10 +33,12 @@ def test_large_calls(cuda, dtype, layout):
 
 
 # one k-step in either GEMM; clusters of four and eight; a last tile wider than what is left of the result (256, 192 and
-# 128 columns); two CTAs per SM over several waves; a K tail; batches with partial row blocks
+# 128 columns); two CTAs per SM over several waves; a K tail; batches with partial row blocks; 256 columns in two parts, with an
+# odd number of chunks to divide, and of entries with partial row blocks
 @pytest.mark.parametrize("shape", [(1, 16, 256, 16, 64), (1, 16, 1024, 1024, 4096), (1, 144, 256, 4096, 128),
                                    (1, 512, 768, 768, 3072), (1, 2064, 1024, 1024, 4096), (1, 8208, 256, 272, 1088),
-                                   (1, 4096, 768, 768, 3072), (5, 80, 512, 144, 576), (1, 1040, 2048, 512, 2112)])
+                                   (1, 4096, 768, 768, 3072), (5, 80, 512, 144, 576), (1, 1040, 2048, 512, 2112),
+                                   (1, 2352, 768, 256, 3136), (2, 608, 1280, 128, 5120)])
 @pytest.mark.parametrize("layout", ["IO", "OI"])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_tile_kernel(cuda, shape, layout, dtype):
