@@ -41,6 +41,24 @@ __device__ __forceinline__ float act_apply(float v) {
   }
 }
 
+// The same for two neighbouring values: GELU with its products and sums two at a time (the same operations in the same order).
+template <int ACT>
+__device__ __forceinline__ void act_apply_pair(float& v0, float& v1) {
+  if constexpr (ACT == 2) {
+    const uint64_t v = pack_f32x2(v0, v1), one = pack_f32x2(1.0f, 1.0f);
+    const uint64_t x = mul_f32x2(mul_f32x2(v, pack_f32x2(0.7978845608f, 0.7978845608f)),
+                                 fma_f32x2(mul_f32x2(v, pack_f32x2(0.044715f, 0.044715f)), v, one));
+    float t0, t1;
+    unpack_f32x2(x, t0, t1);
+    asm("tanh.approx.f32 %0, %0;" : "+f"(t0));
+    asm("tanh.approx.f32 %0, %0;" : "+f"(t1));
+    unpack_f32x2(mul_f32x2(mul_f32x2(v, pack_f32x2(0.5f, 0.5f)), add_f32x2(pack_f32x2(t0, t1), one)), v0, v1);
+  } else {
+    v0 = act_apply<ACT>(v0);
+    v1 = act_apply<ACT>(v1);
+  }
+}
+
 // N fp32 accumulator values of one row (+ a 16-bit bias vector, the same address in every lane: broadcast
 // loads) -> activation -> N / 2 packed 16-bit pairs.  The activation and the presence of a bias are
 // compile-time here: a run-time test per element costs a branch per element, which made this loop the
@@ -70,7 +88,8 @@ __device__ __forceinline__ void act_pack_fixed(const uint32_t (&acc)[N], const u
       v0 += bb.x;
       v1 += bb.y;
     }
-    out[j] = pack2<BF16>(act_apply<ACT>(v0), act_apply<ACT>(v1));
+    act_apply_pair<ACT>(v0, v1);
+    out[j] = pack2<BF16>(v0, v1);
   }
 }
 // The same with the bias values already in registers (two 16-bit values per word).
@@ -79,7 +98,9 @@ __device__ __forceinline__ void act_pack_words(const uint32_t (&acc)[N], const u
 #pragma unroll
   for (int j = 0; j < N / 2; ++j) {
     const float2 bb = unpack2<BF16>(bw[j]);
-    out[j] = pack2<BF16>(act_apply<ACT>(__uint_as_float(acc[2 * j]) + bb.x), act_apply<ACT>(__uint_as_float(acc[2 * j + 1]) + bb.y));
+    float v0 = __uint_as_float(acc[2 * j]) + bb.x, v1 = __uint_as_float(acc[2 * j + 1]) + bb.y;
+    act_apply_pair<ACT>(v0, v1);
+    out[j] = pack2<BF16>(v0, v1);
   }
 }
 // One warp-uniform dispatch per call instead of one per element.
