@@ -391,8 +391,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_persistent_kernel(const
           mbar_arrive(&bar->p_part[part]);
           DITTO_STAMP(1024 + it * 16 + 4 + j * 2 + part);
         }
-        if constexpr (DITTO_PACKED_EX2 == 0) unpack_f32x2(add_f32x2(sum2[0], sum2[1]), sum0, sum1);
-        l += sum0 + sum1;
+        if constexpr (MODE == kModeSoftmax && DITTO_PACKED_EX2 == 0) unpack_f32x2(add_f32x2(sum2[0], sum2[1]), sum0, sum1);
+        if constexpr (MODE == kModeSoftmax) l += sum0 + sum1;
         DITTO_STAMP(it * 16 + j * 2 + 1);
       }
       if (!ok) break;

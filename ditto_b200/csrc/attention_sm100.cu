@@ -656,8 +656,8 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
         mbar_arrive(&bar->p_part[t][part]);
         if (part == 0 && (warp & 3) == 0) DITTO_STAMP(t * 256, k * nkv + j, 4);
       }
-      if constexpr (DITTO_PACKED_EX2 == 0) unpack_f32x2(add_f32x2(sum2[0], sum2[1]), sum0, sum1);
-      l += sum0 + sum1;
+      if constexpr (MODE == kModeSoftmax && DITTO_PACKED_EX2 == 0) unpack_f32x2(add_f32x2(sum2[0], sum2[1]), sum0, sum1);
+      if constexpr (MODE == kModeSoftmax) l += sum0 + sum1;
       if ((warp & 3) == 0) DITTO_STAMP(t * 256, k * nkv + j, 5); else DITTO_STAMP(t * 256, k * nkv + j, 5 + (warp & 3));
     }
 

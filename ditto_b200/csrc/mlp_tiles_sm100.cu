@@ -462,6 +462,9 @@ TilesGemm best_gemm(long long blocks, int N, int steps, double* time) {
 // 15.2, 2048 x 1024 (34 GFLOP) 42.0 -> 37.0, 4096 x 768 (39) 46.6 -> 43.3, 2560 x 1024 (43) 50.5 -> 51.5; on the other side either is
 // the faster one: 6144 x 768 (58) 53.4 -> 49.0, 4096 x 1024 (69) 60.1 -> 58.5, 1024 x 2048 (69) 64.2 -> 65.7, 16384 x 512 (69) 66.9 ->
 // 73.7, 3328 x 1280 (87) 70.2 -> 71.3.  The hidden layer has to stay in L2 beside the operands.
+// With GEMM2 in two parts of 256 columns the tiles win between 48 and 90 GFLOP while their operands stay in L2 (a graph of the same
+// call, 3072 x 1024 (52) 53.4 -> 45.9, 1024 x 2048 (69) 65.2 -> 60.8), and lose or draw with new operands call after call, under the power cap (55.8 ->
+// 58.7, 71.4 -> 71.7, 2048 x 1536 (77) 78.2 -> 83.0): the line stays.
 bool mlp_tiles_faster(int batch, int M, int N, int K, int L) {
   return 2.0 * batch * M * static_cast<double>(L) * (static_cast<double>(K) + N) <= 4.8e10 &&
          mlp_tiles_workspace_bytes(batch, M, L) <= (static_cast<size_t>(48) << 20);
