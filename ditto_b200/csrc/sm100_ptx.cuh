@@ -334,13 +334,6 @@ __host__ __device__ constexpr uint32_t umma_idesc_f16(bool bf16, uint32_t m, uin
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// ---------------------------------------------------------------- registers
-// A warp group gives registers back to the CTA, or takes them (waits until they are there): all four warps execute it.
-template <int N>
-__device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N>
-__device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-
 // ---------------------------------------------------------------- math
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
