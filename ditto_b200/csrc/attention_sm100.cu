@@ -107,15 +107,12 @@ struct Smem {
   static constexpr int kBytes = kOffStage + NT * 4 * 4096 + 1024;  // ... + slack for 1024-byte alignment
 };
 
-// Of every eight pairs of weights, how many the multiply-add pipe computes (ex2_fma_f32x2).  One tile at head dimension 128 is a
-// chain of one softmax warp a scheduler, whose exponentials are its longest step: none / 1 / 2 / 3, us: 1000 slices of 128 rows x 512
-// keys 69.4 / 69.1 / 70.7 / 73.9, 600 x 2048 156.6 / 154.7 / 155.4 / 160.0.  With two softmax warps a scheduler the longer instruction
-// stream costs more: two tiles of 8192 keys 1688 / 1697 / 1856 clocks a block, head dimension 64 1503 / 1525.
-// The packed arithmetic alone, scalar -> packed, us: two tiles, 148 slices of 512 x 8192 272 -> 260, 512 of 512 x 512 85.6 -> 82.4, 256 of
-// 208 x 208 at d = 80 19.1 -> 18.1; head dimension 64, 16 slices of 8192 x 8192 383 -> 375, 100 of 512 x 2048 53.1 -> 50.8.  (1024 slices
-// of 2048 x 2048 stay at 2.05 ms: 1716 -> 1667 clocks a block, but 1480 -> 1440 MHz under the power cap.)
-template <int D, int NT>
-constexpr int kFmaPairs = D == 128 && NT == 1 ? 1 : 0;
+// Weights are computed two at a time (softmax_weights), all of them on the special-function unit.  Scalar -> packed, us: two tiles, 148
+// slices of 512 x 8192 272 -> 260, 512 of 512 x 512 85.6 -> 82.4, 256 of 208 x 208 at d = 80 19.1 -> 18.1; head dimension 64, 16 slices
+// of 8192 x 8192 383 -> 375, 100 of 512 x 2048 53.1 -> 50.8.  (1024 slices of 2048 x 2048 stay at 2.05 ms: 1716 -> 1667 clocks a block,
+// but 1480 -> 1440 MHz under the power cap.)  ex2_fma_f32x2 is not for these kernels: PlainReference lets exponents pass 127 from
+// |m c| = 2^31 on, and one pair of eight of it was worth 1 % where it paid (one tile at head dimension 128, 600 slices of 128 x 2048 156.6
+// -> 154.7 us; two tiles of 8192 keys 1688 -> 1697 clocks a block, head dimension 64 with two CTAs an SM 1503 -> 1525).
 
 struct Barriers {
   uint64_t q_full[2], q_empty[2];   // per query tile: Q has landed / the item's last S MMA has read it
@@ -610,7 +607,7 @@ __global__ void __launch_bounds__(threads_for(NT), kSeparateP<D, NT, PSMEM> ? 2 
               sum1 += pf.y;
               continue;
             } else if constexpr (MODE == kModeSoftmax) {
-              const uint64_t w = softmax_weights(sv[2 * (w0 + i)], sv[2 * (w0 + i) + 1], c2, nmc2, i % 8 >= 8 - kFmaPairs<D, NT>);
+              const uint64_t w = softmax_weights(sv[2 * (w0 + i)], sv[2 * (w0 + i) + 1], c2, nmc2, false);
               sum2[i & 1] = add_f32x2(sum2[i & 1], w);
               unpack_f32x2(w, p0, p1);
               pk[i] = pack2<BF16>(p0, p1);

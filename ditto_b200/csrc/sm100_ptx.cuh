@@ -377,7 +377,8 @@ __device__ __forceinline__ float max_nan(float a, float b) {
   return d;
 }
 
-// 2^x of a pair on the multiply-add pipe, for softmax exponents: x <= 127; -inf and what lies below -127 give 0, NaN stays NaN.
+// 2^x of a pair on the multiply-add pipe, for softmax exponents that a RowReference bounds: x <= 127 (above, the exponent's bits run
+// over into the sign, where ex2.approx gives infinity); -inf and what lies below -127 give 0, NaN stays NaN.
 // x = n + f with n the nearest integer: adding 1.5 * 2^23 + 127 leaves n + 127 in the low bits of the sum, which shifted up
 // are 2^n.  2^f = 1 + f q(f) on [-1/2, 1/2] with q of degree 4, least maximum relative error (iteratively reweighted least
 // squares): 9.2e-8, less than ex2.approx's own 2^-22.

@@ -74,7 +74,8 @@ struct PlainReference {
 };
 
 // Weights 2^(s c - mc) of two scores (c2 and nmc2 hold c and -mc twice), with the scale-and-subtract of both in one instruction.
-// on_fma: on the multiply-add pipe instead of the special-function unit.
+// on_fma: on the multiply-add pipe instead of the special-function unit, for rows with a RowReference: exponents there stay below
+// the few units of its rescale threshold.  Behind a PlainReference the rounding of m * c alone can pass what ex2_fma_f32x2 takes.
 __device__ __forceinline__ uint64_t softmax_weights(uint32_t s0, uint32_t s1, uint64_t c2, uint64_t nmc2, bool on_fma) {
   const uint64_t x = fma_f32x2(pack_f32x2(__uint_as_float(s0), __uint_as_float(s1)), c2, nmc2);
   if (on_fma) return ex2_fma_f32x2(x);

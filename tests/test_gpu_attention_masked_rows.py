@@ -60,3 +60,33 @@ def test_row_without_a_finite_score(form, d):
     assert out[:, 40].isnan().all()
     keep = [i for i in range(128) if i != 40]
     _close(out[:, keep], _reference(q[:, keep], k, v, 0.125), torch.bfloat16)
+
+
+@pytest.mark.parametrize("form,d", [(f, d) for f in FORMS for d in (64, 128) if d == 64 or f != "narrow"])
+def test_references_that_rounding_moves(form, d):
+    """Scores of about 2^31 one unit in the last place apart, at scales that make an exponent of 2 of them about 2^32: rounding the
+    reference's alone moves a row's exponents by up to 256, above what float32 holds.  A row may be NaN then, or what its largest
+    score says (the next one weighs 2^-257 of it); weights that have run over into the sign or into small numbers it may not show."""
+    g = torch.Generator(device="cuda").manual_seed(13)
+    M, L = 128, 128
+    q = torch.zeros(1, M, d, device="cuda")
+    q[:, :, :2] = 1.0
+    v = torch.randn(1, L, d, generator=g, device="cuda").bfloat16()
+    for first in list(range(16)) + [47, 127]:
+        k = torch.zeros(1, L, d, device="cuda")
+        k[:, [first, 20], 0] = 255.0 * 2 ** 23                 # (with the second column 24 bits: exact in float32)
+        k[:, first, 1], k[:, 20, 1] = 256.0, 128.0
+        for step in range(24):
+            scale = 1.4 * (1 + step / 2000)
+            c = torch.tensor(scale, dtype=torch.float32) * torch.tensor(1.4426950408889634, dtype=torch.float32)
+            score = torch.tensor(255.0 * 2 ** 23 + 256.0)
+            moved = (score.double() * c.double() - (score * c).double()).item()
+            assert (score * c).item() > 2 ** 32 and abs(moved) <= 256
+            if 125 < moved < 128.1:                            # 1 / sum is below the smallest normal number
+                continue
+            out = ops.bmm_softmax_bmm(q.bfloat16(), k.bfloat16(), v, scale=scale, key_layout="LK", flags=FORMS[form])
+            want = v[:, first:first + 1].expand(1, M, d)
+            rows = out.isnan().all(dim=-1)
+            assert not out.isnan().any() or rows.all(), (first, scale, moved)
+            assert rows.all() or (out.double() - want.double()).abs().max() <= 2 ** -7 * want.abs().max(), (first, scale, moved)
+    assert ops.device_status() == 0
