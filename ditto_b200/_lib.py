@@ -40,6 +40,7 @@ EXPORTS = (
     "ditto_b200_ffn_ws",
     "ditto_b200_workspace_bytes",
     "ditto_b200_mlp_cluster_slots",
+    "ditto_b200_mlp_tiles_cut",
     "ditto_b200_selftest_umma",
     "ditto_b200_selftest_umma_pair",
     "ditto_b200_selftest_wait_limit",
@@ -97,6 +98,8 @@ def load():
     lib.ditto_b200_workspace_bytes.restype = sz
     lib.ditto_b200_mlp_cluster_slots.argtypes = [i, i]
     lib.ditto_b200_mlp_cluster_slots.restype = i
+    lib.ditto_b200_mlp_tiles_cut.argtypes = [i, i, i, i, i, i, ctypes.POINTER(i)]
+    lib.ditto_b200_mlp_tiles_cut.restype = i
     lib.ditto_b200_selftest_umma.argtypes = [vp, vp, vp, i, i, i, i, i, vp, vp]
     lib.ditto_b200_selftest_umma.restype = i
     lib.ditto_b200_selftest_umma_pair.argtypes = [vp, vp, vp, i, i, i, i, vp, vp]

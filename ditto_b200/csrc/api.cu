@@ -13,7 +13,9 @@
 
 #include "attention_sm100.cuh"
 #include "host_util.cuh"
+#include "mlp_flow_sm100.cuh"
 #include "mlp_sm100.cuh"
+#include "mlp_tiles_sm100.cuh"
 #include "selftest_sm100.cuh"
 
 namespace {
@@ -319,6 +321,18 @@ int ditto_b200_mlp_cluster_slots(int dtype, int variant) {
            : variant == DITTO_EPILOGUE_WIDE_MMA ? ditto_b200::mlp_wide_cluster_slots(dtype == DITTO_DTYPE_BF16, &slots)
                                                 : DITTO_ERR_INVALID_ARG;
   return rc ? rc : slots;
+}
+
+int ditto_b200_mlp_tiles_cut(int gemm, int batch, int M, int N, int K, int L, int* cut) {
+  if ((gemm != 1 && gemm != 2) || cut == nullptr) return DITTO_ERR_INVALID_ARG;
+  if (batch <= 0 || M <= 0 || N <= 0 || K <= 0 || L <= 0 || M % 16) return DITTO_ERR_INVALID_ARG;
+  if (!ditto_b200::mlp_flow_supported(N, K, L)) return DITTO_ERR_UNSUPPORTED;      // (the tile kernel's widths are the flow kernel's)
+  const ditto_b200::TilesPlan plan = ditto_b200::mlp_tiles_plan(batch, M, N, K, L);
+  const ditto_b200::TilesGemm& g = gemm == 1 ? plan.g1 : plan.g2;
+  cut[0] = g.bn;
+  cut[1] = g.parts;
+  cut[2] = g.per_sm;
+  return DITTO_OK;
 }
 
 int ditto_b200_selftest_umma(const void* a, const void* b, float* c, int N, int K, int dtype, int b_mn, int a_tmem,

@@ -161,6 +161,12 @@ size_t ditto_b200_workspace_bytes(int op, int batch, int M, int N, int K, int L,
  * sized by the hardware table of python/ditto/hardware/__init__.py:43-54). */
 int ditto_b200_mlp_cluster_slots(int dtype, int variant);
 
+/* How a call of the MLP chain with scratch memory that runs as two launches over tiles cuts its GEMM 1 or 2 (`gemm`): tiles
+ * of 128 rows x cut[0] columns, each by a cluster of cut[1] CTAs that divide the reduction, cut[2] CTAs an SM.  Sums of
+ * a reduction that is not divided (cut[1] == 1) have the bits that the call has without scratch memory.
+ * Needs no GPU.  No counterpart in the reference. */
+int ditto_b200_mlp_tiles_cut(int gemm, int batch, int M, int N, int K, int L, int* cut);
+
 /* Single-CTA check of one tcgen05 MMA chain: c[128, N] (fp32) = a[128, K] * b.
  *   b_mn 0: b is [N, K]; 1: b is [K, N].  a_tmem 1: the A operand is read from tensor memory.
  * N, K multiples of 64, at most 256.  Exists so the descriptor encodings the fused kernels depend

@@ -93,3 +93,20 @@ def test_native_call_path_may_be_missing_or_foreign(monkeypatch, tmp_path):
         assert ops._fast is None
     monkeypatch.setattr(build_lib, "fastcall_path", lambda: str(tmp_path / "nope.so"))
     assert build_lib._stale()
+
+
+def test_tile_kernel_cuts_and_the_shapes_that_are_tested():
+    """Every way to cut either GEMM that a rule on sizes can pick is one that the tile kernel's tests run."""
+    from tests.test_gpu_mlp_tiles import SHAPES
+    lib = _lib.load()
+    cut = (ctypes.c_int * 3)()
+    seen = {1: set(), 2: set()}
+    for shape in SHAPES:
+        for gemm in seen:
+            assert lib.ditto_b200_mlp_tiles_cut(gemm, *shape, cut) == _lib.OK
+            seen[gemm].add((cut[0], cut[1]))
+    every = {(64, 1), (64, 2), (64, 4), (128, 1), (128, 2), (128, 4), (128, 8), (192, 1), (256, 1), (256, 2)}
+    assert seen[1] == seen[2] == every, (every - seen[1], every - seen[2])
+    assert lib.ditto_b200_mlp_tiles_cut(3, 1, 16, 256, 16, 64, cut) == _lib.ERR_INVALID_ARG
+    assert lib.ditto_b200_mlp_tiles_cut(1, 1, 16, 256, 16, 64, None) == _lib.ERR_INVALID_ARG
+    assert lib.ditto_b200_mlp_tiles_cut(1, 1, 16, 64, 64, 64, cut) == _lib.ERR_UNSUPPORTED

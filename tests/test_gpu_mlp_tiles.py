@@ -32,13 +32,17 @@ def test_large_calls(cuda, dtype, layout):
             _assert_close(out, ref, dtype, (act, batch, M, N, K, L, str(dtype), layout), cuda)
 
 
-# one k-step in either GEMM; clusters of four and eight; a last tile wider than what is left of the result (256, 192 and
-# 128 columns); two CTAs per SM over several waves; a K tail; batches with partial row blocks; 256 columns in two parts, with an
-# odd number of chunks to divide, and of entries with partial row blocks
-@pytest.mark.parametrize("shape", [(1, 16, 256, 16, 64), (1, 16, 1024, 1024, 4096), (1, 144, 256, 4096, 128),
-                                   (1, 512, 768, 768, 3072), (1, 2064, 1024, 1024, 4096), (1, 8208, 256, 272, 1088),
-                                   (1, 4096, 768, 768, 3072), (5, 80, 512, 144, 576), (1, 1040, 2048, 512, 2112),
-                                   (1, 2352, 768, 256, 3136), (2, 608, 1280, 128, 5120)])
+# one k-step in either GEMM; a last tile wider than what is left of the result (256, 192 and 128 columns); two CTAs per SM over
+# several waves; a K tail; batches with partial row blocks; 256 columns in two parts, with an odd number of chunks to divide, and
+# of entries with partial row blocks; clusters of two, four and eight for either GEMM (test_cabi.py sees that all cuts are here)
+SHAPES = ((1, 16, 256, 16, 64), (1, 16, 1024, 1024, 4096), (1, 144, 256, 4096, 128), (1, 512, 768, 768, 3072),
+          (1, 2064, 1024, 1024, 4096), (1, 8208, 256, 272, 1088), (1, 4096, 768, 768, 3072), (5, 80, 512, 144, 576),
+          (1, 1040, 2048, 512, 2112), (1, 2352, 768, 256, 3136), (2, 608, 1280, 128, 5120), (1, 512, 1024, 1024, 4096),
+          (1, 16, 256, 2624, 6272), (2, 16, 2048, 16, 1536), (1, 16, 512, 1216, 3456), (1, 544, 1280, 48, 1856),
+          (1, 32, 256, 5488, 64), (1, 16, 256, 2112, 3328), (1, 1376, 512, 8000, 1472), (3, 1168, 1024, 16, 320))
+
+
+@pytest.mark.parametrize("shape", SHAPES)
 @pytest.mark.parametrize("layout", ["IO", "OI"])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_tile_kernel(cuda, shape, layout, dtype):
