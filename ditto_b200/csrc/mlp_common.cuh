@@ -64,8 +64,8 @@ __device__ __forceinline__ void act_apply_pair(float& v0, float& v1) {
 // compile-time here: a run-time test per element costs a branch per element, which made this loop the
 // longest step of the hidden-chunk hand-over.
 // VEC: the bias pointer is 16-byte aligned and is read eight values at a time (a load per pair of columns is
-// 64 load instructions per thread and hidden chunk).
-template <bool BF16, int ACT, bool BIAS, int N, bool VEC = false>
+// 64 load instructions per thread and hidden chunk).  PAIRS: GELU two values at a time.
+template <bool BF16, int ACT, bool BIAS, int N, bool VEC = false, bool PAIRS = true>
 __device__ __forceinline__ void act_pack_fixed(const uint32_t (&acc)[N], const uint32_t* bias, uint32_t (&out)[N / 2]) {
   uint32_t bw[BIAS ? N / 2 : 1];
   if constexpr (BIAS) {
@@ -88,7 +88,12 @@ __device__ __forceinline__ void act_pack_fixed(const uint32_t (&acc)[N], const u
       v0 += bb.x;
       v1 += bb.y;
     }
-    act_apply_pair<ACT>(v0, v1);
+    if constexpr (PAIRS) {
+      act_apply_pair<ACT>(v0, v1);
+    } else {
+      v0 = act_apply<ACT>(v0);
+      v1 = act_apply<ACT>(v1);
+    }
     out[j] = pack2<BF16>(v0, v1);
   }
 }
@@ -104,16 +109,16 @@ __device__ __forceinline__ void act_pack_words(const uint32_t (&acc)[N], const u
   }
 }
 // One warp-uniform dispatch per call instead of one per element.
-template <bool BF16, int N>
+template <bool BF16, bool PAIRS = true, int N>
 __device__ __forceinline__ void act_pack(const uint32_t (&acc)[N], const uint32_t* bias, int act, uint32_t (&out)[N / 2]) {
   if (bias == nullptr) {
-    if (act == 1) act_pack_fixed<BF16, 1, false, N>(acc, bias, out);
-    else if (act == 2) act_pack_fixed<BF16, 2, false, N>(acc, bias, out);
-    else act_pack_fixed<BF16, 0, false, N>(acc, bias, out);
+    if (act == 1) act_pack_fixed<BF16, 1, false, N, false, PAIRS>(acc, bias, out);
+    else if (act == 2) act_pack_fixed<BF16, 2, false, N, false, PAIRS>(acc, bias, out);
+    else act_pack_fixed<BF16, 0, false, N, false, PAIRS>(acc, bias, out);
   } else {
-    if (act == 1) act_pack_fixed<BF16, 1, true, N>(acc, bias, out);
-    else if (act == 2) act_pack_fixed<BF16, 2, true, N>(acc, bias, out);
-    else act_pack_fixed<BF16, 0, true, N>(acc, bias, out);
+    if (act == 1) act_pack_fixed<BF16, 1, true, N, false, PAIRS>(acc, bias, out);
+    else if (act == 2) act_pack_fixed<BF16, 2, true, N, false, PAIRS>(acc, bias, out);
+    else act_pack_fixed<BF16, 0, true, N, false, PAIRS>(acc, bias, out);
   }
 }
 __device__ __forceinline__ float act_apply_rt(float v, int act) {
