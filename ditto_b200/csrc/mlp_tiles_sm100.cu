@@ -434,9 +434,14 @@ double tiles_time(long long blocks, int N, int steps, const TilesGemm& g) {
 // 256 columns in two parts, alone on their SMs (an incoming share is 128 KB), keep as many SMs busy as 128 columns unsplit do, but a
 // k-step of them brings 48 KB for 512 clocks of tensor work and not 32 KB for 256: 64 of those took 376 clocks each out of L2, 32 of
 // these take 565.  In a graph, us, without -> with: 2048 x 1024 -> 4096 -> 1024 34.9 -> 32.9, 1120 x 560 -> 6144 -> 1536 38.0 -> 33.1,
-// 1152 x 1280 -> 5120 -> 1280 39.2 -> 35.6, 2544 x 768 -> 3072 -> 768 29.3 -> 28.6; least of fourteen shapes that take it, 2784 x 352 -> 3072 ->
-// 768 25.2 -> 25.3.  (Four or eight parts of 256 columns are no faster than those of 128: 256 x 1536 22.4 -> 24.9.)
-TilesGemm best_gemm(long long blocks, int N, int steps, double* time) {
+// 1152 x 1280 -> 5120 -> 1280 39.2 -> 35.6, 2544 x 768 -> 3072 -> 768 29.3 -> 28.6; least of those that take it for GEMM2, 3072 x 768 -> 3072
+// -> 768 29.4 -> 29.8.  (Four or eight parts of 256 columns are no faster than those of 128: 256 x 1536 22.4 -> 24.9.)
+// GEMM1, whose operands come from memory and whose end the second launch waits for, takes them in place of 128 columns unsplit from 96
+// k-steps on only.  Operands new call after call, us, without -> with: 50 k-steps, 864 x 3200 -> 2176 -> 2048 28.8 -> 30.2, 51, 2016 x 3216 ->
+// 832 -> 1024 23.0 -> 24.5, 56, 2080 x 3536 -> 768 -> 256 23.3 -> 24.8, 62, 1952 x 3936 -> 960 -> 512 25.4 -> 26.2, 88, 3248 x 5584 -> 448 ->
+// 512 29.3 -> 30.0; 116, 2224 x 7424 -> 768 -> 1280 37.9 -> 36.2, 125, 1376 x 8000 -> 1472 -> 512 42.7 -> 40.1.  In place of a cut that is split
+// already they win with any number: 49, 736 x 3088 -> 1920 -> 1280 27.5 -> 26.0, 83, 2224 x 5264 -> 576 -> 768 32.4 -> 29.9.
+TilesGemm best_gemm(long long blocks, int N, int steps, bool first, double* time) {
   TilesGemm best = {128, 1, 2};
   *time = tiles_time(blocks, N, steps, best);
   for (int bn = 64; bn <= 256; bn += 64)
@@ -445,6 +450,7 @@ TilesGemm best_gemm(long long blocks, int N, int steps, double* time) {
         const long long ctas = blocks * ((N + bn - 1) / bn) * parts;
         // all clusters at once; alone on their SMs, large ones leave part of a GPC unused
         if (parts > 1 && ctas > (per_sm == 2 ? 296 : parts == 2 ? 148 : 112)) continue;
+        if (first && bn == 256 && parts > 1 && best.parts == 1 && steps < 96) continue;
         const TilesGemm g = {bn, parts, per_sm};
         const double t = tiles_time(blocks, N, steps, g);
         if (t < *time) {
@@ -474,8 +480,8 @@ TilesPlan mlp_tiles_plan(int batch, int M, int N, int K, int L) {
   const long long blocks = static_cast<long long>(batch) * ((M + kRows - 1) / kRows);
   TilesPlan plan;
   double t1, t2;
-  plan.g1 = best_gemm(blocks, L, (K + 63) / 64, &t1);
-  plan.g2 = best_gemm(blocks, N, 4 * ((L + 255) / 256), &t2);
+  plan.g1 = best_gemm(blocks, L, (K + 63) / 64, true, &t1);
+  plan.g2 = best_gemm(blocks, N, 4 * ((L + 255) / 256), false, &t2);
   return plan;
 }
 

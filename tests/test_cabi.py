@@ -107,6 +107,9 @@ def test_tile_kernel_cuts_and_the_shapes_that_are_tested():
             seen[gemm].add((cut[0], cut[1]))
     every = {(64, 1), (64, 2), (64, 4), (128, 1), (128, 2), (128, 4), (128, 8), (192, 1), (256, 1), (256, 2)}
     assert seen[1] == seen[2] == every, (every - seen[1], every - seen[2])
+    # 256 columns in two parts for the first GEMM: over 96 k-steps and more, or where the cut is split anyway
+    for shape, parts in (((2016, 1024, 3216, 832), 1), ((3248, 512, 5584, 448), 1), ((2224, 1280, 7424, 768), 2), ((736, 1280, 3088, 1920), 2)):
+        assert lib.ditto_b200_mlp_tiles_cut(1, 1, *shape, cut) == _lib.OK and cut[1] == parts, (shape, *cut)
     assert lib.ditto_b200_mlp_tiles_cut(3, 1, 16, 256, 16, 64, cut) == _lib.ERR_INVALID_ARG
     assert lib.ditto_b200_mlp_tiles_cut(1, 1, 16, 256, 16, 64, None) == _lib.ERR_INVALID_ARG
     assert lib.ditto_b200_mlp_tiles_cut(1, 1, 16, 64, 64, 64, cut) == _lib.ERR_UNSUPPORTED
