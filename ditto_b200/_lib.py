@@ -43,6 +43,7 @@ EXPORTS = (
     "ditto_b200_mlp_tiles_cut",
     "ditto_b200_selftest_umma",
     "ditto_b200_selftest_umma_pair",
+    "ditto_b200_selftest_ex2",
     "ditto_b200_selftest_wait_limit",
     "ditto_b200_check_status",
     "ditto_b200_strerror",
@@ -104,6 +105,8 @@ def load():
     lib.ditto_b200_selftest_umma.restype = i
     lib.ditto_b200_selftest_umma_pair.argtypes = [vp, vp, vp, i, i, i, i, vp, vp]
     lib.ditto_b200_selftest_umma_pair.restype = i
+    lib.ditto_b200_selftest_ex2.argtypes = [vp, vp, i, i, vp]
+    lib.ditto_b200_selftest_ex2.restype = i
     lib.ditto_b200_selftest_wait_limit.argtypes = [i, vp, vp]
     lib.ditto_b200_selftest_wait_limit.restype = i
     lib.ditto_b200_check_status.argtypes = [vp, vp, ctypes.POINTER(ctypes.c_int)]

@@ -384,6 +384,13 @@ int ditto_b200_selftest_umma_pair(const void* a, const void* b, float* c, int N,
   return DITTO_OK;
 }
 
+int ditto_b200_selftest_ex2(const float* x, float* y, int n, int on_fma, void* stream) {
+  if (!x || !y || n <= 0 || n % 2) return DITTO_ERR_INVALID_ARG;
+  cudaError_t e = ditto_b200::launch_ex2_selftest(x, y, n, on_fma != 0, static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return cuda_fail("ex2 selftest launch", e);
+  return DITTO_OK;
+}
+
 int ditto_b200_selftest_wait_limit(int code, int* status_word, void* stream) {
   if (code <= 0 || status_word == nullptr) return DITTO_ERR_INVALID_ARG;
   cudaError_t e = ditto_b200::launch_wait_limit_selftest(code, status_word, static_cast<cudaStream_t>(stream));

@@ -224,6 +224,30 @@ cudaError_t launch_umma_pair_selftest(const SelftestParams& p, cudaStream_t stre
 
 }  // namespace ditto_b200
 
+// ------------------------------------------------------------------ exponentials
+namespace ditto_b200 {
+
+__global__ void ex2_selftest_kernel(const float* x, float* y, int pairs, bool on_fma) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < pairs; i += gridDim.x * blockDim.x) {
+    float a = x[2 * i], b = x[2 * i + 1];
+    if (on_fma) {
+      unpack_f32x2(ex2_fma_f32x2(pack_f32x2(a, b)), a, b);
+    } else {
+      a = ex2_approx(a);
+      b = ex2_approx(b);
+    }
+    y[2 * i] = a;
+    y[2 * i + 1] = b;
+  }
+}
+
+cudaError_t launch_ex2_selftest(const float* x, float* y, int n, bool on_fma, cudaStream_t stream) {
+  ex2_selftest_kernel<<<256, 256, 0, stream>>>(x, y, n / 2, on_fma);
+  return cudaGetLastError();
+}
+
+}  // namespace ditto_b200
+
 // ------------------------------------------------------------------ bounded-wait self test
 // The failure path every kernel of the library relies on, run on purpose and harmlessly: a barrier
 // that is never signalled, the shared bounded wait, the abort word, the host-visible status word.

@@ -19,6 +19,9 @@ cudaError_t launch_umma_selftest(const SelftestParams& p, cudaStream_t stream);
 // CTA-pair variant: A has 256 rows (box 64 x 128 per CTA), B boxes cover half of N.
 cudaError_t launch_umma_pair_selftest(const SelftestParams& p, cudaStream_t stream);
 
+// The softmax's exponentials by themselves: y = 2^x for n values (n even).
+cudaError_t launch_ex2_selftest(const float* x, float* y, int n, bool on_fma, cudaStream_t stream);
+
 // One CTA runs the library's bounded wait on a barrier nobody signals and reports `code` through `status`.
 cudaError_t launch_wait_limit_selftest(int code, int* status, cudaStream_t stream);
 

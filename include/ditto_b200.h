@@ -179,6 +179,10 @@ int ditto_b200_selftest_umma(const void* a, const void* b, float* c, int N, int 
 int ditto_b200_selftest_umma_pair(const void* a, const void* b, float* c, int N, int K, int dtype, int b_mn,
                                   int* status_word, void* stream);
 
+/* y[i] = 2^x[i] for n values (float32, n even), as the attention kernels compute their weights: on the special-function unit (on_fma 0) or
+ * on the multiply-add pipe (1; x <= 127).  No counterpart in the reference. */
+int ditto_b200_selftest_ex2(const float* x, float* y, int n, int on_fma, void* stream);
+
 /* Exercises the failure path of the device-side waits without faulting anything: one CTA waits, with the
  * same bounded wait every kernel here uses, on a barrier that nothing ever signals; when the limit is
  * reached the wait gives up, the kernel writes `code` to *status_word and ends normally, and the context

@@ -132,3 +132,25 @@ def test_weights_far_apart_and_scores_that_are_not_numbers(dtype):
         rest = [i for i in range(L) if i != key]
         _close(ops.bmm_softmax_bmm(q, gone, v, scale=0.125, key_layout="LK", flags=NARROW), _reference(q, k[:, rest], v[:, rest], 0.125), dtype)
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("on_fma", [0, 1])
+def test_exponentials_by_themselves(on_fma):
+    """Both pipes against float64: 2^-22 of the value, which is ex2.approx's bound and 1.4 times what the polynomial in float32 is
+    off by; 0 from -127 on (below -126 values are no normal numbers and a pipe may give 0) and for -inf, NaN for NaN."""
+    lib = _lib.load()
+
+    def ex2(x):
+        y = torch.full_like(x, float("nan"))
+        assert lib.ditto_b200_selftest_ex2(x.data_ptr(), y.data_ptr(), x.numel(), on_fma, torch.cuda.current_stream().cuda_stream) == 0
+        return y
+    for lo, hi in ((-126, 127), (-30, 9), (-1, 1), (-2 ** -10, 2 ** -10)):
+        x = torch.linspace(lo, hi, 1 << 22, device="cuda", dtype=torch.float64).float()
+        assert ((ex2(x).double() / torch.exp2(x.double()) - 1).abs().max()) <= 2 ** -22, (lo, hi)
+    x = torch.arange(-126, 128, device="cuda").float()
+    assert torch.equal(ex2(x).double(), torch.exp2(x.double()))
+    x = torch.linspace(-127, -126, 4096, device="cuda")
+    assert (ex2(x).double() - torch.exp2(x.double())).abs().max() <= 2 ** -126
+    low = torch.tensor([-127.0, -127.5, -128.0, -150.0, -1e4, -3e38, -1e30, float("-inf")], device="cuda")
+    assert torch.equal(ex2(low), torch.zeros_like(low))
+    assert ex2(torch.full((2,), float("nan"), device="cuda")).isnan().all()
