@@ -42,11 +42,13 @@ constexpr uint32_t kColO = 64;
 // 512 keys at scale d^-0.5, 2.19e-4 / 2.28e-4 / 2.15e-4 unscaled; 144 keys at 0.35, simulated, 2.33e-4 / 2.60e-4 / 2.29e-4.
 // The price is about one rescale an item, 56.4 -> 58.2 us for 2048 items of 512 keys, 7.5 -> 8.0 for one wave of 304; all
 // of O in one piece, or the rescale behind P, spill or delay every item (65.6 and 59.0 us).
+
 // Of every eight pairs of weights, how many the multiply-add pipe computes (ex2_fma_f32x2).  Four softmax warps on a scheduler keep
 // the special-function unit 63 % busy over a long launch and issue in half of the slots; an eighth of the exponentials elsewhere is
-// what pays (0 / 1 / 2 / 3 of eight, us: 1024 items of 8192 keys 370 / 347 / 358 / 377, 2048 of 512 59.4 / 57.0 / 59.1 / 60.5, 600 of 208
-// 15.7 / 15.4 / 15.6 / 15.8; without the packed arithmetic 362, 58.4 and 15.5): beyond that the longer instruction stream, and the clock under
-// the power it takes, cost more.
+// what pays (0 / 1 / 2 / 3 of eight, us, with a polynomial one degree lower: 1024 items of 8192 keys 370 / 347 / 358 / 377, 2048 of 512 59.4 /
+// 57.0 / 59.1 / 60.5, 600 of 208 15.7 / 15.4 / 15.6 / 15.8; without the packed arithmetic 362, 58.4 and 15.5): beyond that the longer
+// instruction stream, and the clock under the power it takes, cost more.  In long runs at the power cap, without packed arithmetic / so / with
+// the polynomial in use: 401.5 / 382.6 / 385.4, 72.7 / 71.3 / 71.7 and 16.4 / 16.2 / 16.4.
 constexpr int kFmaPairs = 1;
 constexpr int kModeSoftmax = 0, kModeRelu = 1;
 

@@ -80,8 +80,9 @@ __device__ __forceinline__ float max_with(float m, const uint32_t* s) {
 }
 
 // Of every eight pairs of weights, how many the multiply-add pipe computes: a block is a chain of one warp's steps here, and the
-// exponentials its longest.  None (and scalar arithmetic) / 1 / 2 / 3, us: head dimension 64, 12 slices of 512 rows and keys 7.86 / 7.77 /
-// 7.78 / 7.87, 40 of them 11.97 / 11.58 / 11.74 / 12.24; 128, 140 tiles of 1024 keys 16.5 / 16.0 / 15.8 / 16.3.
+// exponentials its longest.  None (and scalar arithmetic) / 1 / 2 / 3, us, with a polynomial one degree lower (the one in use adds at most
+// 1 %): head dimension 64, 12 slices of 512 rows and keys 7.86 / 7.77 / 7.78 / 7.87, 40 of them 11.97 / 11.58 / 11.74 / 12.24; 128, 140 tiles of
+// 1024 keys 16.5 / 16.0 / 15.8 / 16.3.  (Two softmax warps share a scheduler; at head dimension 64 two CTAs' may.)
 constexpr int kFmaPairs = 1;
 
 // 32 scores of a row -> their weights 2^(s c - mc), rounded to the operand type and packed; the sums take them before rounding.
