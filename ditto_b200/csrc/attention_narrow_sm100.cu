@@ -43,13 +43,11 @@ constexpr uint32_t kColO = 64;
 // The price is about one rescale an item, 56.4 -> 58.2 us for 2048 items of 512 keys, 7.5 -> 8.0 for one wave of 304; all
 // of O in one piece, or the rescale behind P, spill or delay every item (65.6 and 59.0 us).
 
-// Of every eight pairs of weights, how many the multiply-add pipe computes (ex2_fma_f32x2).  Four softmax warps on a scheduler keep
-// the special-function unit 63 % busy over a long launch and issue in half of the slots; an eighth of the exponentials elsewhere is
-// what pays (0 / 1 / 2 / 3 of eight, us, with a polynomial one degree lower: 1024 items of 8192 keys 370 / 347 / 358 / 377, 2048 of 512 59.4 /
-// 57.0 / 59.1 / 60.5, 600 of 208 15.7 / 15.4 / 15.6 / 15.8; without the packed arithmetic 362, 58.4 and 15.5): beyond that the longer
-// instruction stream, and the clock under the power it takes, cost more.  In long runs at the power cap, without packed arithmetic / so / with
-// the polynomial in use: 401.5 / 382.6 / 385.4, 72.7 / 71.3 / 71.7 and 16.4 / 16.2 / 16.4.
-constexpr int kFmaPairs = 1;
+// Some weights are computed on the multiply-add pipe (weights_on_fma).  Four softmax warps on a scheduler keep the special-function unit
+// 63 % busy over a long launch and issue in half of the slots; a tenth of the exponentials elsewhere is what pays, beyond that the
+// longer instruction stream, and the clock under the power it takes, cost more.  Scalar arithmetic / packed with 1 / 2 / 3 / 4 of 32
+// pairs there, us, at the power cap: 16 slices of 8192 x 8192 405 / 391.6 / 389.5 / 388.9 / 389.7, 64 of 2048 x 2048 107.0 / 104.4 / 103.6 /
+// 103.4 / 103.4, 512 of 512 x 512 66.4 / 64.5 / 64.5 / 65.1 / 65.5, 1024 of 208 x 208 41.6 / 40.3 / 40.3 / 40.8 / 41.0.
 constexpr int kModeSoftmax = 0, kModeRelu = 1;
 
 struct NBars {
@@ -240,7 +238,7 @@ __global__ void __launch_bounds__(kThreads, 4) attention_narrow_kernel(const __g
         for (int i = 0; i < 16; ++i) {
           float p0 = __uint_as_float(sv[32 * h + 2 * i]), p1 = __uint_as_float(sv[32 * h + 2 * i + 1]);
           if constexpr (MODE == kModeSoftmax) {
-            const uint64_t w = softmax_weights(sv[32 * h + 2 * i], sv[32 * h + 2 * i + 1], c2, nmc2, i % 8 >= 8 - kFmaPairs);
+            const uint64_t w = softmax_weights(sv[32 * h + 2 * i], sv[32 * h + 2 * i + 1], c2, nmc2, weights_on_fma(16 * h + i));
             sum[i & 1] = add_f32x2(sum[i & 1], w);
             unpack_f32x2(w, p0, p1);
           } else if constexpr (MODE == kModeRelu) {

@@ -79,19 +79,17 @@ __device__ __forceinline__ float max_with(float m, const uint32_t* s) {
   return max3(a[0], a[1], a[2]);
 }
 
-// Of every eight pairs of weights, how many the multiply-add pipe computes: a block is a chain of one warp's steps here, and the
-// exponentials its longest.  None (and scalar arithmetic) / 1 / 2 / 3, us, with a polynomial one degree lower (the one in use adds at most
-// 1 %): head dimension 64, 12 slices of 512 rows and keys 7.86 / 7.77 / 7.78 / 7.87, 40 of them 11.97 / 11.58 / 11.74 / 12.24; 128, 140 tiles of
-// 1024 keys 16.5 / 16.0 / 15.8 / 16.3.  (Two softmax warps share a scheduler; at head dimension 64 two CTAs' may.)
-constexpr int kFmaPairs = 1;
-
-// 32 scores of a row -> their weights 2^(s c - mc), rounded to the operand type and packed; the sums take them before rounding.
+// The 32 scores of a row's group g -> their weights 2^(s c - mc), rounded to the operand type and packed; the sums take them before rounding.
+// A block is a chain of one warp's steps here, and the exponentials its longest: some are computed on the multiply-add pipe
+// (weights_on_fma).  Scalar arithmetic / packed with 2 / 3 / 4 of 32 pairs there, us: head dimension 64, 12 slices of 512 rows and keys 7.66 /
+// 7.58 / 7.58 / 7.62, 40 of them 11.67 / 11.67 / 11.55 / 11.47, 16 of 1024 14.50 / 14.30 / 14.21 / 14.42; 128, 140 tiles of 1024 keys 16.71 / 16.34 /
+// 16.34 / 16.30, 4 slices of 1024 x 4096 18.96 / 18.39 / 18.47 / 18.60.
 template <bool BF16>
-__device__ __forceinline__ void row_weights(const uint32_t* s, float c, float mc, uint64_t& sum, uint32_t (&w)[16]) {
+__device__ __forceinline__ void row_weights(int g, const uint32_t* s, float c, float mc, uint64_t& sum, uint32_t (&w)[16]) {
   const uint64_t c2 = pack_f32x2(c, c), nmc2 = pack_f32x2(-mc, -mc);
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
-    const uint64_t p = softmax_weights(s[2 * i], s[2 * i + 1], c2, nmc2, i % 8 >= 8 - kFmaPairs);
+    const uint64_t p = softmax_weights(s[2 * i], s[2 * i + 1], c2, nmc2, weights_on_fma(16 * g + i));
     sum = add_f32x2(sum, p);
     float a, b;
     unpack_f32x2(p, a, b);
@@ -340,7 +338,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __gr
       for (int g = 0; g < 2; ++g) {
         if (64 * g + 32 * half < keys) {                   // (P*V reads no others)
           uint32_t w[16];
-          if constexpr (MODE == kModeSoftmax) row_weights<BF16>(sv + 32 * g, c, mc, sum, w);
+          if constexpr (MODE == kModeSoftmax) row_weights<BF16>(g, sv + 32 * g, c, mc, sum, w);
           else pass_on<BF16, MODE == kModeRelu>(sv + 32 * g, w);
           tmem_st_x16(p_col + 32 * g + 16 * half, w);
         }

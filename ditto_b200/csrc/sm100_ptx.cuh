@@ -382,7 +382,7 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 // x = n + f with n the nearest integer: adding 1.5 * 2^23 + 127 leaves n + 127 in the low bits of the sum, which shifted up
 // are 2^n.  2^f = 1 + f q(f) on [-1/2, 1/2] with q of degree 5, least maximum relative error (iteratively reweighted least squares, one
 // coefficient after the other fixed at its float32 value): 3.0e-9.  As evaluated, against float64, largest / root mean square: 6.6e-8 / 2.6e-8;
-// ex2.approx measured the same way 1.45e-7 / 5.3e-8.  (Degree 4, at most 0.9 % faster in a kernel: 1.7e-7 / 6.6e-8, more than it stands in for.)
+// ex2.approx measured the same way 1.45e-7 / 5.3e-8.  (Degree 4: 1.7e-7 / 6.6e-8, more than it stands in for.)
 __device__ __forceinline__ uint64_t ex2_fma_f32x2(uint64_t x_in) {
   float x0, x1, t0, t1;
   unpack_f32x2(x_in, x0, x1);

@@ -84,4 +84,7 @@ __device__ __forceinline__ uint64_t softmax_weights(uint32_t s0, uint32_t s1, ui
   return pack_f32x2(ex2_approx(x0), ex2_approx(x1));
 }
 
+// Which of a row's pairs of weights the multiply-add pipe computes in the kernels whose exponentials are shared out: three of every 32.
+__device__ __forceinline__ constexpr bool weights_on_fma(int pair) { return pair % 32 == 7 || pair % 32 == 15 || pair % 32 == 31; }
+
 }  // namespace ditto_b200
