@@ -338,12 +338,12 @@ cudaError_t launch_attention_narrow(const AttnParams& p, int batch, bool bf16, i
 }
 
 // Where the lines lie: calls of up to 296 items have other forms (attention_few: of up to four 128-key blocks, and of any number up to 148 items;
-// those between are not long enough for this one, 200 x 5 blocks 14.3 -> 14.0, 200 x 8 19.9 -> 20.6).  Above, it is the faster form up to four
+// those between are not long enough for this one, 200 x 5 blocks 13.8 -> 14.0, 200 x 8 18.6 -> 19.9).  Above, it is the faster form up to four
 // 128-key blocks an item, up to eight with a half-full wave more than the other kernels hold at once; for longer items the other
 // kernels' 128-key blocks cost less (1.6 us for two a SM against 2 x 1.0), and it pays again once a launch is three waves of those
-// or more.  Measured, us, others -> this kernel: 2048 items of 512 keys 74.8 -> 63.2; 1200 of 208 30.0 -> 25.0; 1000 of 128
-// 17.5 -> 14.4; 640 of 64 13.9 -> 8.8; 384 of 512 20.7 -> 18.4; 400 of 1024 36.2 -> 32.2; 1024 of 8192 393 -> 368; and left alone: 320 of
-// 1024 30.2 -> 31.8, 384 of 2048 51.7 -> 56.8, 320 of 8192 179 -> 209.  A chain without a softmax has less between the hand-overs:
+// or more.  Measured, us, others -> this kernel: 2048 items of 512 keys 83.8 -> 69.2; 1200 of 208 30.6 -> 27.0; 1000 of 128
+// 16.6 -> 13.8; 640 of 64 13.0 -> 8.2; 384 of 512 19.5 -> 17.4; 400 of 1024 35.9 -> 31.4; 1024 of 8192 398 -> 384; 900 of 768 53.5 -> 48.1; and left
+// alone: 320 of 1024 28.6 -> 31.3, 384 of 2048 55.7 -> 61.2, 320 of 8192 185 -> 219.  A chain without a softmax has less between the hand-overs:
 // it gains with one or two blocks and many items only (600 x 208 rows and keys 19.4 -> 18.0, 640 of 64 9.4 -> 7.4; 640 of 1024
 // would go 40 -> 43).
 bool attention_narrow_pays(int batch, int M, int L, int mode) {

@@ -566,7 +566,9 @@ static int cluster_places(int lg) {
 // (rms 3 to 8 %).  At head dimension 64 clusters share SMs once there are more than places at a CTA an SM (*Shared); more than the
 // device holds at once would be a second wave, which costs more than a split saves (36 x 16 in eight parts 18.7 us, in four
 // 14.8).  What the rule picks took on average 0.6 % longer than the best form timed (softmax, 363 shapes of up to 148 items) and 0.3 %
-// (chains, 299), at head dimension 128 0.1 % (softmax, 234); asking 4 % for a split made that worse.
+// (chains, 299), at head dimension 128 0.1 % (softmax, 234); asking 4 % for a split made that worse.  The fits are of the scalar arithmetic
+// before softmax_weights; with it, 70 shapes of up to 148 items and 48 blocks each, 0.7 % at head dimension 64 (at worst 7 %: 13 x 8 blocks 7.6
+// us, in eight parts 7.1) and nothing at 128 (1.4 %).
 namespace {
 struct Whole { double fixed, block, full; };                    // full: over 100 CTAs
 struct Split { double fixed, part, block, full; };              // full: over 100 CTAs; shared: times the share of SMs with two

@@ -415,7 +415,7 @@ namespace {
 // with a full set of CTAs, and one of a lone CTA, which is longer where too few bytes are in flight (bn = 64; a 96 KB
 // ring).  The constants are fitted to 390 timings (13 shapes of 16 to 16384 rows, each with 10 to 20 ways to cut either
 // GEMM) of the kernel with four epilogue warps.  With eight, whose ends are shorter, the cut it picks is on average 3 % slower than
-// the best one timed (17 shapes, ReLU and GELU with biases), at worst 12 %: 16384 x 256, first GEMM 128 wide 30.2 us, 256 wide 26.6;
+// the best one timed (17 shapes, ReLU and GELU with biases, before 256 columns in two parts were among the cuts), at worst 12 %: 16384 x 256, first GEMM 128 wide 30.2 us, 256 wide 26.6;
 // 512 x 1024, second GEMM in eight parts of 128 columns 22.4 us, four of 64 20.0.
 double tiles_time(long long blocks, int N, int steps, const TilesGemm& g) {
   const double shared = 0.109 + 0.00059 * g.bn;
