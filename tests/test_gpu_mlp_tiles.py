@@ -64,6 +64,22 @@ def test_tile_kernel(cuda, shape, layout, dtype):
         _assert_close(out, _act(y, "relu"), dtype, ("ffn",) + shape, cuda)
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_cuts_differ_by_the_order_of_sums_alone(cuda, dtype):
+    """Operands whose sums are whole numbers below 2^24: any order gives the same bits, those of the call without scratch memory and
+    of float64 products, however a reduction is divided."""
+    for batch, M, N, K, L in SHAPES + ((1, 2048, 1024, 1024, 4096),):
+        g = torch.Generator(device=cuda).manual_seed(46)
+        x, w1, w2 = (torch.randint(-a, a + 1, size, device=cuda, generator=g).to(dtype)
+                     for a, size in ((2, (batch, M, K)), (1, (batch, K, L)), (2, (batch, L, N))))
+        h = torch.relu(x.double() @ w1.double()).to(dtype)
+        sums = h.double() @ w2.double()
+        assert 2 * h.double().sum(dim=-1).max() < 2 ** 24 and 2 * x.abs().double().sum(dim=-1).max() < 2 ** 24
+        want = sums.float().to(dtype)
+        assert torch.equal(ops.gemm_relu_gemm(x, w1, w2), want), (batch, M, N, K, L)
+        assert torch.equal(ops.gemm_relu_gemm(x, w1, w2, workspace=None), want), (batch, M, N, K, L)
+
+
 def test_tile_kernel_streams_and_changed_weights(cuda):
     """The second launch reads its weights ahead of the first one's end: a weight written by the work just ahead in the
     stream is the one that is used, and calls on two streams have hidden layers of their own."""
