@@ -36,6 +36,20 @@ __device__ __forceinline__ void tmem_ld_2x32_wait(uint32_t first, uint32_t secon
 }}
 """)
 
+def emit_ld_split(n):
+    outs = ", ".join(f'"=r"(r[{i}])' for i in range(n))
+    inouts = ", ".join(f'"+r"(r[{i}])' for i in range(n))
+    print(f"""// a load without its wait, and the wait for it: the registers may not be touched in between
+__device__ __forceinline__ void tmem_ld_x{n}(uint32_t taddr, uint32_t (&r)[{n}]) {{
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x{n}.b32 {{{regs(n, 0)}}}, [%{n}];"
+    : {outs}
+    : "r"(taddr) : "memory");
+}}
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[{n}]) {{
+  asm volatile("tcgen05.wait::ld.sync.aligned;" : {inouts} :: "memory");
+}}
+""")
+
 def emit_st(n):
     ins = ", ".join(f'"r"(r[{i}])' for i in range(n))
     print(f"""__device__ __forceinline__ void tmem_st_x{n}(uint32_t taddr, const uint32_t (&r)[{n}]) {{
@@ -52,6 +66,7 @@ print("namespace ditto_b200 {")
 for n in (8, 16, 32, 64, 128):
     emit_ld(n)
 emit_ld_2x32()
+emit_ld_split(32)
 for n in (8, 16, 32, 64):
     emit_st(n)
 print("}  // namespace ditto_b200")

@@ -43,6 +43,7 @@
 #include "mlp_common.cuh"
 #include "mlp_flow_sm100.cuh"
 #include "mlp_tiles_sm100.cuh"
+#include "mlp_waves_sm100.cuh"
 #include "sm100_ptx.cuh"
 
 // Optional timeline capture for tuning (compiled in only with -DDITTO_TRACE): the first CTA stores
@@ -740,10 +741,32 @@ static MlpForm form_with_scratch(int batch, int M, int N, int K, int L, bool bf1
   return batch <= 65535 && N <= 1024 && N >= 512 && mlp_tiles_workspace_bytes(batch, M, L) > (static_cast<size_t>(192) << 20) ? kFormCluster : kFormTiles;
 }
 
+// Whether the wave kernel takes a call that would else go to the tile or the flow kernel.
+//
+// In place of the flow kernel, always; measured, us, operands new call after call under the power cap, flow -> waves: 16384 x 1024 -> 4096 -> 1024 235 -> 214,
+// 3328 x 1280 -> 5120 -> 1280 with GELU 86.3 -> 75.7, 4096 x 2048 -> 8192 -> 2048 224 -> 217, 16384 x 256 -> 8192 -> 256 191 -> 155, 65536 x 1024 928 -> 830; 16
+// entries of 512 x 1024 -> 4096 -> 1024 135 -> 120, 24 of 384 x 768 135 -> 97; the other way 4656 x 256 -> 8192 -> 2048 with GELU, whose GEMM1 is all
+// epilogue, 183 -> 190.  Not with a hidden layer of 512 MB or more (4096 x 2048 -> 65536 -> 2048 1570 -> 1640), of which the flow kernel
+// only holds a ring, and not with fewer than two k-steps in GEMM1: those calls keep the flow kernel, whose epilogues with biases nothing else reaches.
+// In place of the tile kernel where the modelled times say so, that one's scaled to what it measures (138 shapes).  Near a draw the tile kernel is
+// the faster one by 3 to 10 % (1024 x 1024 -> 4096 -> 1024 23.7 against 27.1), hence the factor.  Tiles -> waves: 2048 x 1024 37.1 -> 33.5, 4096 x 768 -> 3072 -> 768 with
+// GELU 47.1 -> 42.5, 1632 x 768 30.1 -> 24.4, 8192 x 512 -> 2048 -> 512 40.3 -> 35.1.
+static bool waves_faster(int batch, int M, int N, int K, int L, MlpForm form) {
+  if (K < 128 || mlp_tiles_workspace_bytes(batch, M, L) >= (static_cast<size_t>(512) << 20)) return false;
+  if (form == kFormFlow) return true;
+  double waves, tiles;
+  mlp_waves_plan(batch, M, N, K, L, &waves);
+  mlp_tiles_plan(batch, M, N, K, L, &tiles);
+  return waves < 0.93 * (1.6 * tiles - 1.7);
+}
+
 size_t mlp_workspace_bytes(int batch, int M, int N, int K, int L, bool bf16, int w_layout, int variant) {
   int slots = 0;
   const MlpForm form = variant == kMlpAuto ? form_with_scratch(batch, M, N, K, L, bf16) : variant == kMlpFlow ? kFormFlow : kFormCluster;
   if (form == kFormTiles) return mlp_tiles_workspace_bytes(batch, M, L);
+  if (form == kFormFlow && variant == kMlpAuto && waves_faster(batch, M, N, K, L, form))
+    // (enough for the flow kernel as well, which takes results that are not aligned to 32 bytes)
+    return std::max(mlp_tiles_workspace_bytes(batch, M, L), mlp_workspace_bytes(batch, M, N, K, L, bf16, w_layout, kMlpFlow));
   if (form == kFormFlow)
     return mlp_flow_supported(N, K, L) && mlp_flow_pair_slots(bf16, &slots) == DITTO_OK
                ? mlp_flow_workspace_bytes(batch, M, N, L, mlp_flow_plan(batch, M, N, K, L, slots)) : 0;
@@ -766,12 +789,17 @@ int launch_mlp_chain(const void* x, const void* w1, const void* w2, void* y, int
   // With few row blocks -- or a last wave that would leave most of the device idle -- some row blocks are
   // shared by several clusters, if the caller provided the scratch memory that form needs.
   int slots = 0, rc = 0;
-  // With scratch memory for the hidden layer small calls run as two launches over tiles, with scratch memory for a ring of
-  // hidden tiles large ones run as one flow of 2-SM tiles, where that is the faster form (form_with_scratch).
+  // With scratch memory for the hidden layer calls run as two launches over tiles, of one SM or (waves_faster) of two, or with scratch
+  // memory for a ring of hidden tiles as one flow of 2-SM tiles, where that is the faster form (form_with_scratch).
   // Without it (or with too little) the hidden layer stays inside a cluster.
   const MlpForm form = workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 15) != 0 ? kFormCluster
                        : variant == kMlpAuto ? form_with_scratch(batch, M, N, K, L, bf16)
                        : variant == kMlpFlow && mlp_flow_supported(N, K, L) ? kFormFlow : kFormCluster;
+  if (variant == kMlpAuto && form != kFormCluster && ws_bytes >= mlp_tiles_workspace_bytes(batch, M, L) && mlp_waves_aligned(y) &&
+      mlp_waves_aligned(workspace) && waves_faster(batch, M, N, K, L, form)) {
+    double time;
+    return launch_mlp_waves(x, w1, w2, y, batch, M, N, K, L, bf16, w_layout, act1, act2, b1, b2, mlp_waves_plan(batch, M, N, K, L, &time), workspace, status, stream);
+  }
   if (form == kFormTiles && ws_bytes >= mlp_tiles_workspace_bytes(batch, M, L))
     return launch_mlp_tiles(x, w1, w2, y, batch, M, N, K, L, bf16, w_layout, act1, act2, b1, b2, mlp_tiles_plan(batch, M, N, K, L), workspace, status, stream);
   if (form != kFormCluster) {

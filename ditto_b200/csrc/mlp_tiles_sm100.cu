@@ -476,12 +476,13 @@ bool mlp_tiles_faster(int batch, int M, int N, int K, int L) {
          mlp_tiles_workspace_bytes(batch, M, L) <= (static_cast<size_t>(48) << 20);
 }
 
-TilesPlan mlp_tiles_plan(int batch, int M, int N, int K, int L) {
+TilesPlan mlp_tiles_plan(int batch, int M, int N, int K, int L, double* time) {
   const long long blocks = static_cast<long long>(batch) * ((M + kRows - 1) / kRows);
   TilesPlan plan;
   double t1, t2;
   plan.g1 = best_gemm(blocks, L, (K + 63) / 64, true, &t1);
   plan.g2 = best_gemm(blocks, N, 4 * ((L + 255) / 256), false, &t2);
+  if (time != nullptr) *time = t1 + t2;
   return plan;
 }
 

@@ -16,9 +16,10 @@ struct TilesPlan {
   TilesGemm g1, g2;
 };
 
-// Whether this form is expected to be faster than the flow kernel, and its plan: pure functions of the shape.
+// Whether this form is expected to be faster than the flow kernel, and its plan (with its modelled time in us, without the launches'
+// fixed parts): pure functions of the shape.
 bool mlp_tiles_faster(int batch, int M, int N, int K, int L);
-TilesPlan mlp_tiles_plan(int batch, int M, int N, int K, int L);
+TilesPlan mlp_tiles_plan(int batch, int M, int N, int K, int L, double* time = nullptr);
 // The hidden activations [batch, M, L].
 size_t mlp_tiles_workspace_bytes(int batch, int M, int L);
 int launch_mlp_tiles(const void* x, const void* w1, const void* w2, void* y, int batch, int M, int N, int K, int L,
