@@ -15,7 +15,14 @@
 //
 // What bounds it: operand bytes out of L2 -- 16 KB + bn * 128 B a k-step against the 87 B/clk per SM that TMA loads
 // deliver on all SMs at once: 376 clocks at bn = 128 (256 of tensor work), 565 at 256 (512) -- and, in short calls,
-// two chains of launch, first load, epilogue.
+// two chains of launch, first load, k-steps, epilogue.
+//
+// Tile width and layout of B are template parameters: what an issuing warp works out per k-step is then known at compile time, and a launch
+// fetches the code of its own width alone (all widths behind a switch in one kernel: 1 to 3 us slower than run-time values).  A k-step of a lone
+// CTA at bn = 128 took 480 clocks with run-time values.  In a graph, operands new call after call, us, before -> after: 24 shapes of 16 to 8192 rows 18.6 ->
+// 17.6 (geometric mean), 512 x 768 -> 3072 -> 768 with GELU 15.5 -> 14.3, 128 x 1024 -> 4096 -> 1024 14.0 -> 12.6, 1024 x 1024 23.8 -> 22.1, 432 x 1024 -> 1856 13.9 -> 12.3.
+// Two k-steps a stage, as in the wave kernel: 1 % faster with operands in L2, 1 to 8 % slower with operands from memory.  Partial sums by bulk copies
+// instead of stores to the peers: 14.2 -> 16.0.  Results written from registers in 32-byte sectors: 17.6 -> 18.0 (spills at 80 registers).
 #include <cuda.h>
 
 #include <algorithm>
@@ -50,11 +57,10 @@ struct TilesParams {
   void* out;                // [batch, M, N]
   const void* bias;         // [batch, N] or null
   int M, N;
-  int bn, blocks_per_batch, blocks;     // 128-row blocks
+  int blocks_per_batch, blocks;         // 128-row blocks
   int steps;                // k-steps of 64
   int chunks;               // GEMM2: 256-column chunks of the hidden layer, taken in the order below (0: in order)
-  int parts, stages, stage_bytes;
-  int oi;
+  int parts, stages;
   int early_b;              // B is not written by the kernel ahead: its loads need not wait for that
   int* status;
 };
@@ -103,12 +109,13 @@ __device__ __forceinline__ void finish(const uint32_t (&v)[N], const uint32_t* b
 
 }  // namespace
 
-template <bool BF16, int ACT, bool BIAS>
+template <bool BF16, int ACT, bool BIAS, int BN, bool OI>
 __global__ void __launch_bounds__(kThreads, 2) mlp_tiles_kernel(const __grid_constant__ TilesParams p) {
+  constexpr int kStage = kATile + BN * 128;
   extern __shared__ uint8_t smem_raw[];
   // the CTAs of a cluster round up by the same amount: offsets match across the cluster
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  TilesBars* bar = reinterpret_cast<TilesBars*>(smem + p.stages * p.stage_bytes);
+  TilesBars* bar = reinterpret_cast<TilesBars*>(smem + p.stages * kStage);
   uint32_t* bias_s = reinterpret_cast<uint32_t*>(bar + 1);
   volatile uint32_t* abort_word = &bar->abort_word;
   const int warp = threadIdx.x >> 5;
@@ -119,7 +126,7 @@ __global__ void __launch_bounds__(kThreads, 2) mlp_tiles_kernel(const __grid_con
   const int n = tile / p.blocks, rb = tile - n * p.blocks;
   const int b = rb / p.blocks_per_batch;
   const int row0 = (rb - b * p.blocks_per_batch) * kRows;
-  const int col0 = n * p.bn;
+  const int col0 = n * BN;
   const int k0 = p.steps * part / p.parts, k1 = p.steps * (part + 1) / p.parts;   // parts <= steps: never empty
 
   if (threadIdx.x == 0) {
@@ -148,18 +155,20 @@ __global__ void __launch_bounds__(kThreads, 2) mlp_tiles_kernel(const __grid_con
   if (warp == kWarpB) {
     // ------------------------------------------------------------ B operand (weights)
     if (p.early_b == 0) grid_dependency_wait();
-    if (lane == 0) {
-      int st = 0;
-      uint32_t ph = 1;
-      for (int k = k0; k < k1; ++k) {
-        ok = mbar_wait(&bar->empty[st], ph, abort_word, 0x110);
-        if (!ok) break;
-        uint8_t* dst = smem + st * p.stage_bytes + kATile;
-        const int kc = step_col(k, p.chunks);
-        if (p.oi) tma_load_3d(dst, &p.map_b, &bar->full[st], kc, col0, b);
+    const uint32_t issuer = elect_one();
+    int st = 0;
+    uint32_t ph = 1;
+    for (int k = k0; k < k1; ++k) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&bar->empty[st], ph, abort_word, 0x110));
+      if (!ok) break;
+      uint8_t* dst = smem + st * kStage + kATile;
+      const int kc = step_col(k, p.chunks);
+      if (issuer) {
+        if constexpr (OI) tma_load_3d(dst, &p.map_b, &bar->full[st], kc, col0, b);
         else tma_load_4d(dst, &p.map_b, &bar->full[st], 0, kc, col0 >> 6, b);
-        if (++st == p.stages) { st = 0; ph ^= 1; }
       }
+      __syncwarp();
+      if (++st == p.stages) { st = 0; ph ^= 1; }
     }
     __syncwarp();
     if (p.early_b != 0) grid_dependency_wait();
@@ -169,35 +178,36 @@ __global__ void __launch_bounds__(kThreads, 2) mlp_tiles_kernel(const __grid_con
     grid_launch_dependents();
     if (warp == kWarpA) {
       // ---------------------------------------------------------- A operand; arms the stage for both
-      if (lane == 0) {
-        asm volatile("fence.proxy.async.global;" ::: "memory");   // A may be the kernel ahead's ordinary stores
-        int st = 0;
-        uint32_t ph = 1;
-        for (int k = k0; k < k1; ++k) {
-          ok = mbar_wait(&bar->empty[st], ph, abort_word, 0x100);
-          if (!ok) break;
-          mbar_arrive_expect_tx(&bar->full[st], static_cast<uint32_t>(p.stage_bytes));
-          tma_load_3d(smem + st * p.stage_bytes, &p.map_a, &bar->full[st], step_col(k, p.chunks), row0, b);
-          if (++st == p.stages) { st = 0; ph ^= 1; }
+      asm volatile("fence.proxy.async.global;" ::: "memory");   // A may be the kernel ahead's ordinary stores
+      const uint32_t issuer = elect_one();
+      int st = 0;
+      uint32_t ph = 1;
+      for (int k = k0; k < k1; ++k) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&bar->empty[st], ph, abort_word, 0x100));
+        if (!ok) break;
+        const int kc = step_col(k, p.chunks);
+        if (issuer) {
+          mbar_arrive_expect_tx(&bar->full[st], kStage);
+          tma_load_3d(smem + st * kStage, &p.map_a, &bar->full[st], kc, row0, b);
         }
+        __syncwarp();
+        if (++st == p.stages) { st = 0; ph ^= 1; }
       }
-      __syncwarp();
     } else if (warp == kWarpMma) {
       // ---------------------------------------------------------- MMA issuer (converged warp)
       const uint32_t issuer = elect_one();
       const uint32_t ring = smem_u32(smem);
-      const uint32_t idesc = umma_idesc_f16(BF16, kRows, p.bn, false, p.oi == 0);
+      constexpr uint32_t idesc = umma_idesc_f16(BF16, kRows, BN, false, !OI);
+      constexpr uint32_t step_b = (OI ? 32 : 2048) >> 4;
       int st = 0;
       uint32_t ph = 0;
       for (int k = k0; k < k1; ++k) {
-        ok = mbar_wait(&bar->full[st], ph, abort_word, 0x200);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = __all_sync(0xffffffffu, mbar_wait(&bar->full[st], ph, abort_word, 0x200));
         if (!ok) break;
         tc_fence_after_sync();
-        const uint32_t sa = ring + st * p.stage_bytes, sb = sa + kATile;
+        const uint32_t sa = ring + st * kStage, sb = sa + kATile;
         const uint64_t da = umma_desc_sw128(sa, 16, 1024);
-        const uint64_t db = p.oi ? umma_desc_sw128(sb, 16, 1024) : umma_desc_sw128(sb, 8192, 1024);
-        const uint32_t step_b = p.oi ? 32u >> 4 : 2048u >> 4;
+        const uint64_t db = OI ? umma_desc_sw128(sb, 16, 1024) : umma_desc_sw128(sb, 8192, 1024);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
           umma_ss_elected(tmem_base, da + ((i * 32) >> 4), db + i * step_b, idesc, (k > k0 || i > 0) ? 1u : 0u, issuer);
@@ -212,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, 2) mlp_tiles_kernel(const __grid_con
       // -> 768 16.5 -> 15.7, 2048 x 1024 -> 4096 -> 1024 37.5 -> 35.4, 4096 x 768 43.7 -> 41.6, 256 x 1536 -> 6144 -> 1536 22.7 -> 21.7.
       if constexpr (BIAS) {
         const int i = static_cast<int>(threadIdx.x);
-        if (2 * i < p.bn)
+        if (2 * i < BN)
           bias_s[i] = col0 + 2 * i < p.N ? __ldg(reinterpret_cast<const uint32_t*>(p.bias) + (static_cast<size_t>(b) * p.N + col0) / 2 + i) : 0u;
         asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
       }
@@ -226,7 +236,7 @@ __global__ void __launch_bounds__(kThreads, 2) mlp_tiles_kernel(const __grid_con
         uint8_t* stage = smem + warp * 2048;
         const int row = row0 + (warp & 3) * 32;
         uint8_t* to = static_cast<uint8_t*>(p.out) + (static_cast<size_t>(b) * p.M + row + (lane >> 2)) * p.N * 2 + (lane & 3) * 16;
-        const int cols = min(p.bn, p.N - col0);          // N is a multiple of 64
+        const int cols = min(BN, p.N - col0);          // N is a multiple of 64
 #pragma unroll 1
         for (int c = (warp >> 2) * 32; c < cols; c += 64) {
           uint32_t v[32], w[16];
@@ -256,14 +266,14 @@ __global__ void __launch_bounds__(kThreads, 2) mlp_tiles_kernel(const __grid_con
     // thread reaches both barriers whether its waits expired or not.
     __syncwarp();
     cluster_sync_all();
-    const int cols = p.bn / p.parts;                     // 16, 32, 64 or 128
+    const int cols = BN / p.parts;                     // 16, 32, 64 or 128
     const int row = (warp & 3) * 32 + lane;
     if (warp < kEpiWarps) {
       const int cols_log2 = 31 - __clz(cols);
       const uint32_t in0 = smem_u32(smem) + (part * (cols / 4) * kRows + row) * 16;
       const uint32_t acc = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
 #pragma unroll 1
-      for (int h = (warp >> 2) * 32; h < p.bn; h += 64) {
+      for (int h = (warp >> 2) * 32; h < BN; h += 64) {
         uint32_t v[32];
         tmem_ld_x32_wait(acc + h, v);
 #pragma unroll
@@ -322,9 +332,9 @@ namespace {
 constexpr int kBarBytes = sizeof(TilesBars) + 512, kSlack = 1024;    // (barriers, and the biases of 256 columns)
 constexpr int kRingLone = 192 * 1024, kRingShared = 96 * 1024;
 
-template <bool BF16, int ACT, bool BIAS>
+template <bool BF16, int ACT, bool BIAS, int BN, bool OI>
 cudaError_t launch_one(const TilesParams& p, int ctas, cudaStream_t stream) {
-  auto kern = mlp_tiles_kernel<BF16, ACT, BIAS>;
+  auto kern = mlp_tiles_kernel<BF16, ACT, BIAS, BN, OI>;
   static std::atomic<unsigned long long> configured{0};
   int dev = 0;
   cudaError_t e = current_device_checked(&dev);
@@ -339,7 +349,7 @@ cudaError_t launch_one(const TilesParams& p, int ctas, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(ctas), 1, 1);
   cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.dynamicSmemBytes = static_cast<size_t>(p.stages) * p.stage_bytes + kBarBytes + kSlack;
+  cfg.dynamicSmemBytes = static_cast<size_t>(p.stages) * (kATile + BN * 128) + kBarBytes + kSlack;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -351,6 +361,16 @@ cudaError_t launch_one(const TilesParams& p, int ctas, cudaStream_t stream) {
   cfg.attrs = attr;
   cfg.numAttrs = p.parts > 1 ? 2 : 1;
   return launch_kernel(cfg, kern, p);
+}
+
+template <bool BF16, int ACT, bool BIAS, bool OI>
+cudaError_t launch_width(const TilesParams& p, int bn, int ctas, cudaStream_t stream) {
+  switch (bn) {
+    case 64: return launch_one<BF16, ACT, BIAS, 64, OI>(p, ctas, stream);
+    case 128: return launch_one<BF16, ACT, BIAS, 128, OI>(p, ctas, stream);
+    case 192: return launch_one<BF16, ACT, BIAS, 192, OI>(p, ctas, stream);
+    default: return launch_one<BF16, ACT, BIAS, 256, OI>(p, ctas, stream);
+  }
 }
 
 // D [batch, M, N] = act(A [batch, M, K] * B + bias)
@@ -379,25 +399,24 @@ int launch_gemm(const void* a, const void* w, void* out, const void* bias, int b
   p.bias = bias;
   p.M = M;
   p.N = N;
-  p.bn = g.bn;
   p.blocks_per_batch = (M + kRows - 1) / kRows;
   p.blocks = batch * p.blocks_per_batch;
   p.chunks = second ? (K + 255) / 256 : 0;
   p.steps = second ? 4 * p.chunks : (K + 63) / 64;      // (units past the hidden size read as zero)
   p.parts = g.parts;
-  p.stage_bytes = kATile + g.bn * 128;
-  p.stages = std::min(kMaxStages, (g.per_sm == 2 ? kRingShared : kRingLone) / p.stage_bytes);
-  p.oi = w_layout == 1;
+  p.stages = std::min(kMaxStages, (g.per_sm == 2 ? kRingShared : kRingLone) / (kATile + g.bn * 128));
   p.early_b = second ? 1 : 0;
   p.status = status;
   const long long ctas = static_cast<long long>(p.blocks) * ((N + g.bn - 1) / g.bn) * g.parts;
   if (ctas > 0x7fffffffLL) return DITTO_ERR_UNSUPPORTED;
   cudaError_t e = cudaErrorInvalidValue;
 #define DITTO_TILES(BF, AC, BI) \
-  if (bf16 == BF && act == AC && (bias != nullptr) == BI) e = launch_one<BF, AC, BI>(p, static_cast<int>(ctas), stream);
+  if (bf16 == BF && act == AC && (bias != nullptr) == BI) e = w_layout == 1 ? launch_width<BF, AC, BI, true>(p, g.bn, static_cast<int>(ctas), stream) : launch_width<BF, AC, BI, false>(p, g.bn, static_cast<int>(ctas), stream);
 #define DITTO_TILES_ACTS(BF, BI) DITTO_TILES(BF, 0, BI) DITTO_TILES(BF, 1, BI) DITTO_TILES(BF, 2, BI)
+#ifndef TEST_ONLY
   DITTO_TILES_ACTS(false, false)
   DITTO_TILES_ACTS(false, true)
+#endif
   DITTO_TILES_ACTS(true, false)
   DITTO_TILES_ACTS(true, true)
 #undef DITTO_TILES_ACTS
