@@ -10,6 +10,7 @@
 // Roles: warps 0-3 softmax and write-out (thread r <-> query row r <-> TMEM lane r), warp 4 loads and MMAs.  One control
 // warp suffices because the order of events is fixed: S(g) complete frees K's stage and (S(g) is issued behind
 // P*V(g-1), and a commit covers all earlier MMAs) V's stage of block g - 1, so the loads need no "empty" barriers.
+#define DITTO_WAIT_OUT_OF_LINE   // see mbar_wait
 #include "attention_sm100.cuh"
 
 #include <atomic>

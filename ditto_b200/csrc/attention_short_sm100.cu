@@ -15,6 +15,7 @@
 //
 // Two CTAs fit an SM at head dimension 64 (84 KB, 256 tensor-memory columns, 94 registers): the next call's are set up under this
 // one's.  What it measured stands at attention_few.
+#define DITTO_WAIT_OUT_OF_LINE   // see mbar_wait
 #include "attention_sm100.cuh"
 
 #include <algorithm>

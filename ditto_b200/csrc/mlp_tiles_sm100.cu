@@ -23,6 +23,7 @@
 // 17.6 (geometric mean), 512 x 768 -> 3072 -> 768 with GELU 15.5 -> 14.3, 128 x 1024 -> 4096 -> 1024 14.0 -> 12.6, 1024 x 1024 23.8 -> 22.1, 432 x 1024 -> 1856 13.9 -> 12.3.
 // Two k-steps a stage, as in the wave kernel: 1 % faster with operands in L2, 1 to 8 % slower with operands from memory.  Partial sums by bulk copies
 // instead of stores to the peers: 14.2 -> 16.0.  Results written from registers in 32-byte sectors: 17.6 -> 18.0 (spills at 80 registers).
+#define DITTO_WAIT_OUT_OF_LINE   // see mbar_wait
 #include <cuda.h>
 
 #include <algorithm>

@@ -20,6 +20,7 @@
 // What bounds it: the tensor pipe under the power cap -- 490 to 550 clocks a k-step at 1.55 to 1.7 GHz -- and, in calls of few tiles, the
 // ends of the two launches (set-up 1.0, first load 1.2, write-out of the last tile 0.7 to 3.4, teardown 0.8, hand-over 1.2 us)
 // and a last wave that is not full.
+#define DITTO_WAIT_OUT_OF_LINE   // see mbar_wait
 #include <cuda.h>
 
 #include <algorithm>
