@@ -744,20 +744,21 @@ static MlpForm form_with_scratch(int batch, int M, int N, int K, int L, bool bf1
 // Whether the wave kernel takes a call that would else go to the tile or the flow kernel.
 //
 // In place of the flow kernel, always; measured, us, operands new call after call under the power cap, flow -> waves: 16384 x 1024 -> 4096 -> 1024 235 -> 214,
-// 3328 x 1280 -> 5120 -> 1280 with GELU 86.3 -> 75.7, 4096 x 2048 -> 8192 -> 2048 224 -> 217, 16384 x 256 -> 8192 -> 256 191 -> 155, 65536 x 1024 928 -> 830; 16
+// 3328 x 1280 -> 5120 -> 1280 with GELU 86.3 -> 74.0, 4096 x 2048 -> 8192 -> 2048 224 -> 217, 16384 x 256 -> 8192 -> 256 191 -> 155, 65536 x 1024 928 -> 830; 16
 // entries of 512 x 1024 -> 4096 -> 1024 135 -> 120, 24 of 384 x 768 135 -> 97; the other way 4656 x 256 -> 8192 -> 2048 with GELU, whose GEMM1 is all
 // epilogue, 183 -> 190.  Not with a hidden layer of 512 MB or more (4096 x 2048 -> 65536 -> 2048 1570 -> 1640), of which the flow kernel
 // only holds a ring, and not with fewer than two k-steps in GEMM1: those calls keep the flow kernel, whose epilogues with biases nothing else reaches.
-// In place of the tile kernel where the modelled times say so, that one's scaled to what it measures (138 shapes).  Near a draw the tile kernel is
-// the faster one by 3 to 10 % (1024 x 1024 -> 4096 -> 1024 23.7 against 27.1), hence the factor.  Tiles -> waves: 2048 x 1024 37.1 -> 33.5, 4096 x 768 -> 3072 -> 768 with
-// GELU 47.1 -> 42.5, 1632 x 768 30.1 -> 24.4, 8192 x 512 -> 2048 -> 512 40.3 -> 35.1.
+// In place of the tile kernel where its modelled time is less than 0.87 of that one's, which is scaled to what it measures (198 shapes, 1.64 t - 2.5): nearer to a
+// draw the tile kernel was the faster one by up to 25 % (1024 x 1024 -> 4096 -> 1024 21.6 against 26.7).  What the rule picks is 0.6 % (in bursts) to 1.2 % (under the power
+// cap) slower than the best form on average.  Tiles -> waves: 2048 x 1024 36.6 -> 33.5, 4096 x 768 -> 3072 -> 768 with GELU 46.3 -> 38.6, 1632 x 768 28.2 -> 23.6,
+// 8192 x 512 -> 2048 -> 512 40.3 -> 35.1.
 static bool waves_faster(int batch, int M, int N, int K, int L, MlpForm form) {
   if (K < 128 || mlp_tiles_workspace_bytes(batch, M, L) >= (static_cast<size_t>(512) << 20)) return false;
   if (form == kFormFlow) return true;
   double waves, tiles;
   mlp_waves_plan(batch, M, N, K, L, &waves);
   mlp_tiles_plan(batch, M, N, K, L, &tiles);
-  return waves < 0.93 * (1.6 * tiles - 1.7);
+  return waves < 1.425 * tiles - 2.2;
 }
 
 size_t mlp_workspace_bytes(int batch, int M, int N, int K, int L, bool bf16, int w_layout, int variant) {

@@ -1,7 +1,7 @@
 // GEMM -> activation -> GEMM for sm_100a as two launches of one persistent kernel over 2-SM tiles, D = act(A B + bias), with
 // the hidden layer in scratch memory.
 //
-// The form of calls with enough tiles to fill the device.  A pair of CTAs computes tiles of 256 x BN (BN 256 or 128), tile t of
+// The form of calls with enough tiles to fill the device.  A pair of CTAs computes tiles of 256 x BN (BN 256, 192 or 128), tile t of
 // pair q is q + t * pairs: nothing is drawn, counted or waited for inside a launch, so that the operands of a pair's next tile are on
 // their way while the last k-steps of this one are multiplied.  (The flow kernel, mlp_flow_sm100.cu, hands tiles out by a ticket and lets
 // GEMM2 tiles wait for hidden ones: for 16384 x 1024 -> 4096 -> 1024 its pairs stood still 0.8 us a GEMM1 tile of 6 us, and 5 us a GEMM2
@@ -43,9 +43,10 @@ constexpr int kEpiWarps = 8;
 constexpr int kWarpA = kEpiWarps, kWarpB = kEpiWarps + 1, kWarpMma = kEpiWarps + 2;
 constexpr int kThreads = (kEpiWarps + 4) * 32;
 constexpr int kRingBytes = 224 * 1024;
-template <int BN> struct Ring {
-  static constexpr int steps = BN == 256 ? 1 : 2;                         // k-steps a stage
-  static constexpr int b_tile = BN * 64;                                  // this CTA's half of the B tile of one k-step
+template <int BN, bool OI> struct Ring {
+  static constexpr int steps = BN == 128 ? 2 : 1;                         // k-steps a stage
+  // this CTA's half of the B tile of one k-step; 96 columns of an [in, out] layout come in two boxes of 64
+  static constexpr int b_tile = BN == 192 && !OI ? 128 * 128 : BN * 64;
   static constexpr int stage = steps * (kATile + b_tile);
   static constexpr int stages = kRingBytes / stage;
 };
@@ -54,7 +55,8 @@ constexpr int kOffBar = kRingBytes;
 
 struct WavesParams {
   CUtensorMap map_a;        // A (K, M, batch), box 64 x 128 x 1
-  CUtensorMap map_b;        // [out, in]: (K, N, batch), box 64 x BN / 2 x 1;  [in, out]: (64, K, N / 64, batch), box 64 x 64 x BN / 128 x 1
+  CUtensorMap map_b;        // [out, in]: (K, N, batch), box 64 x BN / 2 x 1;  [in, out]: (64, K, N / 64, batch), box 64 x 64 x BN / 128 x 1,
+                            // at 192 columns (N, K, batch), box 64 x 64 x 1
   void* out;                // [batch, M, N]
   const void* bias;         // [batch, N] or null
   int M, N;
@@ -169,7 +171,7 @@ __device__ __forceinline__ Tile tile_at(const WavesParams& p, int t) {
 template <bool BF16, int ACT, bool BIAS, int BN, bool OI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     mlp_waves_kernel(const __grid_constant__ WavesParams p) {
-  using R = Ring<BN>;
+  using R = Ring<BN, OI>;
   constexpr int kStageSteps = R::steps;
   extern __shared__ uint8_t smem_raw[];
   // both CTAs of a pair round up by the same amount: offsets match across the pair
@@ -230,8 +232,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           for (int j = 0; j < kStageSteps; ++j) {
             if (j == 0 || k + j < p.steps) {
               const int row = step_col(k + j, p.chunks);
-              if constexpr (OI) tma_load_3d_pair(dst + j * R::b_tile, &p.map_b, full0 + st * 8, row, col, b);
-              else tma_load_4d_pair(dst + j * R::b_tile, &p.map_b, full0 + st * 8, 0, row, col >> 6, b);
+              if constexpr (OI) {
+                tma_load_3d_pair(dst + j * R::b_tile, &p.map_b, full0 + st * 8, row, col, b);
+              } else if constexpr (BN == 192) {
+                tma_load_3d_pair(dst, &p.map_b, full0 + st * 8, col, row, b);
+                tma_load_3d_pair(dst + 64 * 128, &p.map_b, full0 + st * 8, col + 64, row, b);
+              } else {
+                tma_load_4d_pair(dst + j * R::b_tile, &p.map_b, full0 + st * 8, 0, row, col >> 6, b);
+              }
             }
           }
         }
@@ -405,6 +413,11 @@ cudaError_t launch_one(const WavesParams& p, cudaStream_t stream) {
   return launch_kernel(cfg, kern, p);
 }
 
+template <bool BF16, int ACT, bool BIAS, bool OI>
+cudaError_t launch_width(const WavesParams& p, int bn, cudaStream_t stream) {
+  return bn == 256 ? launch_one<BF16, ACT, BIAS, 256, OI>(p, stream) : bn == 192 ? launch_one<BF16, ACT, BIAS, 192, OI>(p, stream) : launch_one<BF16, ACT, BIAS, 128, OI>(p, stream);
+}
+
 // D [batch, M, N] = act(A [batch, M, K] * B + bias)
 int launch_gemm(const void* a, const void* w, void* out, const void* bias, int batch, int M, int N, int K, bool bf16,
                 int w_layout, int act, bool second, int bn, int* status, cudaStream_t stream) {
@@ -420,6 +433,10 @@ int launch_gemm(const void* a, const void* w, void* out, const void* bias, int b
   if (rc) return rc;
   if (w_layout == 1) {
     rc = map3(&p.map_b, w, uN, static_cast<uint32_t>(bn / 2));
+  } else if (bn == 192) {
+    const uint64_t dims[3] = {uN, uK, ub}, strides[2] = {uN * 2, uK * uN * 2};
+    const uint32_t box[3] = {64, 64, 1};
+    rc = make_tensor_map(&p.map_b, bf16, w, 3, dims, strides, box);
   } else {
     // [K, N] seen as (64 columns, K, N / 64, batch): one box brings the swizzle atoms of an MN-major operand tile
     const uint64_t dims[4] = {64, uK, uN / 64, ub}, strides[3] = {uN * 2, 128, uK * uN * 2};
@@ -444,8 +461,7 @@ int launch_gemm(const void* a, const void* w, void* out, const void* bias, int b
   cudaError_t e = cudaErrorInvalidValue;
 #define DITTO_WAVES(BF, AC, BI) \
   if (bf16 == BF && act == AC && (bias != nullptr) == BI) \
-    e = w_layout == 1 ? (bn == 256 ? launch_one<BF, AC, BI, 256, true>(p, stream) : launch_one<BF, AC, BI, 128, true>(p, stream)) \
-                      : (bn == 256 ? launch_one<BF, AC, BI, 256, false>(p, stream) : launch_one<BF, AC, BI, 128, false>(p, stream));
+    e = w_layout == 1 ? launch_width<BF, AC, BI, true>(p, bn, stream) : launch_width<BF, AC, BI, false>(p, bn, stream);
 #define DITTO_WAVES_ACTS(BF, BI) DITTO_WAVES(BF, 0, BI) DITTO_WAVES(BF, 1, BI) DITTO_WAVES(BF, 2, BI)
   DITTO_WAVES_ACTS(false, false)
   DITTO_WAVES_ACTS(false, true)
@@ -458,21 +474,38 @@ int launch_gemm(const void* a, const void* w, void* out, const void* bias, int b
 
 }  // namespace
 
-// Modelled time (us) of D [M, N] over `steps` k-steps in tiles of 256 x bn: whole rounds of 74 pairs.  Fitted to 138 shapes of the
-// chain (16 to 65536 rows, all four plans each; operands new call after call, under the power cap and in bursts): 8 % off (standard deviation); the
-// plan it picks is 0.2 to 0.8 % slower than the best of the four, 10 % at most.
+// Modelled time (us) of D [M, N] over `steps` k-steps in tiles of 256 x bn: whole rounds of 74 pairs.  Fitted to 198 shapes of the
+// chain (16 to 65536 rows, all nine plans each; operands new call after call, under the power cap and in bursts): 8 % off (standard deviation); the
+// plan it picks is 0.3 to 0.9 % slower than the best of the nine.
+// 192 columns are for rounds that 256 would leave half empty: GEMM2 of 4096 x 768 -> 3072 -> 768 is 64 tiles of 192 columns or 48 of 256, for 74 pairs
+// either way: 36.6 -> 32.8 us, under the power cap 40.5 -> 38.6; [in, out] weights, of which 128 columns are read for 96, 35.3 -> 31.9 and 38.4 -> 37.4.
+// (Widths as run-time values of one kernel cost 256 columns 4 %.  The last round's tiles in halves of 128 columns, 16384 x 1024 -> 4096 -> 1024: 210 -> 210.)
 static double waves_time(long long blocks, int N, int steps, int bn) {
   const long long tiles = blocks * ((N + bn - 1) / bn);
-  return static_cast<double>((tiles + 73) / 74) * (steps * (bn == 256 ? 0.300 : 0.192) + 1.5) + (bn == 256 ? 3.2 : 1.8);
+  const double step = bn == 256 ? 0.310 : bn == 192 ? 0.254 : 0.198, end = bn == 256 ? 2.3 : bn == 192 ? 1.6 : 1.1;
+  return static_cast<double>((tiles + 73) / 74) * (steps * step + 1.83) + end;
 }
 
 WavesPlan mlp_waves_plan(int batch, int M, int N, int K, int L, double* time) {
   const long long blocks = static_cast<long long>(batch) * ((M + 255) / 256);
-  const int steps1 = (K + 63) / 64, steps2 = 4 * ((L + 255) / 256);
-  const double narrow1 = waves_time(blocks, L, steps1, 128), wide1 = waves_time(blocks, L, steps1, 256);
-  const double narrow2 = waves_time(blocks, N, steps2, 128), wide2 = waves_time(blocks, N, steps2, 256);
-  *time = std::min(narrow1, wide1) + std::min(narrow2, wide2);
-  return {narrow1 < wide1 ? 128 : 256, narrow2 < wide2 ? 128 : 256};
+  auto best = [&](int columns, int steps) {
+    int width = 256;
+    double least = waves_time(blocks, columns, steps, 256);
+    for (int bn : {192, 128}) {
+      const double t = waves_time(blocks, columns, steps, bn);
+      if (t < least) {
+        least = t;
+        width = bn;
+      }
+    }
+    *time += least;
+    return width;
+  };
+  *time = 0.0;
+  WavesPlan plan;
+  plan.bn1 = best(L, (K + 63) / 64);
+  plan.bn2 = best(N, 4 * ((L + 255) / 256));
+  return plan;
 }
 
 int launch_mlp_waves(const void* x, const void* w1, const void* w2, void* y, int batch, int M, int N, int K, int L,

@@ -7,7 +7,7 @@
 
 namespace ditto_b200 {
 
-// Tile widths of the two GEMMs: 256 rows by 128 or 256 columns.
+// Tile widths of the two GEMMs: 256 rows by 128, 192 or 256 columns.
 struct WavesPlan {
   int bn1, bn2;
 };

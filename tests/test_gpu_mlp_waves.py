@@ -1,5 +1,5 @@
 """The wave kernel, which larger calls of the MLP chain with scratch memory take, at the sizes where it can go wrong, against float32
-products (bounds as in the random-shape sweeps): both tile widths for either GEMM, partial row blocks, tiles past the
+products (bounds as in the random-shape sweeps): all three tile widths for either GEMM, partial row blocks, tiles past the
 hidden layer, odd and half-filled k-steps, several rounds of tiles, batch entries; and what the rule on sizes and alignment picks."""
 import ctypes
 import re
@@ -13,11 +13,13 @@ from tests.test_gpu_random_shapes import _act, _assert_close
 
 pytestmark = pytest.mark.gpu
 
-# batch, M, N, K, L -> tile widths of the two GEMMs
-SHAPES = (((1, 8992, 256, 288, 192), (128, 128)), ((3, 2016, 256, 160, 384), (128, 128)), ((1, 5536, 256, 224, 320), (128, 128)),
-          ((1, 7712, 1280, 144, 64), (128, 256)), ((3, 2992, 1280, 272, 64), (128, 256)), ((1, 3344, 1024, 160, 512), (128, 256)),
-          ((1, 4080, 512, 224, 896), (256, 128)), ((1, 8528, 256, 592, 448), (256, 128)), ((1, 2064, 1024, 1024, 4096), (256, 128)),
-          ((1, 8096, 512, 368, 448), (256, 256)), ((3, 1312, 1024, 1136, 576), (256, 256)), ((1, 3344, 1280, 1280, 5120), (256, 256)),
+# batch, M, N, K, L -> tile widths of the two GEMMs: every pair of widths, even and odd numbers of k-steps
+SHAPES = (((1, 8992, 256, 288, 192), (128, 128)), ((1, 7984, 256, 480, 192), (128, 128)), ((1, 7712, 1280, 144, 64), (128, 192)),
+          ((1, 4816, 2048, 608, 64), (128, 192)), ((1, 6224, 2048, 144, 64), (128, 256)), ((3, 2928, 256, 208, 320), (192, 128)),
+          ((1, 8400, 256, 144, 384), (192, 128)), ((1, 5104, 512, 304, 512), (192, 192)), ((1, 8800, 512, 208, 320), (192, 256)),
+          ((1, 4080, 512, 224, 896), (256, 128)), ((1, 8528, 256, 592, 448), (256, 128)), ((3, 2016, 256, 272, 640), (256, 128)),
+          ((1, 2064, 1024, 1024, 4096), (256, 128)), ((1, 5280, 512, 416, 640), (256, 192)), ((1, 4096, 768, 768, 3072), (256, 192)),
+          ((3, 1312, 1024, 1136, 576), (192, 256)), ((1, 8096, 512, 368, 448), (256, 256)), ((1, 3344, 1280, 1280, 5120), (256, 256)),
           ((24, 384, 768, 768, 3072), (256, 256)))
 
 
