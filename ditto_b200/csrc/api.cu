@@ -60,7 +60,7 @@ cudaError_t launch_attention_form(const ditto_b200::AttnParams& p, int slices, i
   if (narrow) return ditto_b200::launch_attention_narrow(p, slices, bf16, mode, st);
   if (any) {
     const int asked = (flags & DITTO_FLAG_SPLIT_MASK) / DITTO_FLAG_SPLIT_UNIT, blocks = (p.L + 127) / 128;
-    ditto_b200::AttnFew few = {1, false};
+    ditto_b200::AttnFew few = {1, false, false};
     if (asked == 0 && !(flags & DITTO_FLAG_FEW)) {
       few = ditto_b200::attention_few(slices, p.M, p.L, d, mode);
     } else {
@@ -68,7 +68,7 @@ cudaError_t launch_attention_form(const ditto_b200::AttnParams& p, int slices, i
       while (few.parts > blocks) few.parts /= 2;
       few.here = (flags & DITTO_FLAG_FEW) || (few.parts > 1 && d == 128);   // (the kernel with a thread a row has a split form up to 64)
     }
-    if (few.here) return ditto_b200::launch_attention_short(p, slices, d, bf16, mode, few.parts, st);
+    if (few.here) return ditto_b200::launch_attention_short(p, slices, d, bf16, mode, few.parts, few.two, st);
     if (few.parts > 1) return ditto_b200::launch_attention_split(p, slices, bf16, mode, few.parts, st);
     // few key blocks per item: the persistent kernel hides the per-item start-up, which long sequences amortise anyway
     if (d == 64 && p.L <= kPersistentMaxKeys) return ditto_b200::launch_attention_persistent(p, slices, bf16, mode, st);

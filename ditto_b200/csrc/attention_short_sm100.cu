@@ -14,7 +14,9 @@
 // distributed shared memory at the end.
 //
 // Two CTAs fit an SM at head dimension 64 (84 KB, 256 tensor-memory columns, 94 registers): the next call's are set up under this
-// one's.  What it measured stands at attention_few.
+// one's.  At head dimension 128 (TWO) they do with one stage of K and of V and with P in the place of S (100 KB, 256 columns): a CTA by itself
+// is a chain then -- scores, softmax, P*V, next scores -- and two of them fill each other's gaps; for more items than SMs.  What it measured
+// stands at attention_few.
 #define DITTO_WAIT_OUT_OF_LINE   // see mbar_wait
 #include "attention_sm100.cuh"
 
@@ -34,14 +36,15 @@ namespace ditto_b200 {
 namespace {
 
 constexpr int kBM = 128, kBN = 128;
-constexpr int kStages = 2;
 constexpr int kSoftmaxWarps = 8, kWarpLoad = 8, kWarpMma = 9;
 constexpr int kThreads = 10 * 32;
 constexpr int kFirstKeys = 64;            // of a block, in the first part of P (groups 0 and 1); the rest follows by itself
 constexpr int kModeSoftmax = 0, kModeRelu = 1;
 
-template <int D>
+// TWO: the form of which two CTAs fit an SM at head dimension 128
+template <int D, bool TWO>
 struct Layout {
+  static constexpr int kStages = TWO ? 1 : 2;
   static constexpr int kTileQ = kBM * D * 2;
   static constexpr int kTileKV = kBN * D * 2;
   static constexpr int kOffQ = 0;
@@ -51,12 +54,12 @@ struct Layout {
   static constexpr int kOffRows = kOffPair + 2 * 2 * kBM * 4;     // float2 [128]: (max, sum) for the cluster
   static constexpr int kOffBar = kOffRows + kBM * 8;
   static constexpr int kBytes = kOffBar + 256 + 1024;
-  static constexpr uint32_t kColS = 0, kColO = 128, kColP = 128 + D;
-  static constexpr uint32_t kTmemCols = D == 64 ? 256 : 512;
+  static constexpr uint32_t kColS = 0, kColO = 128, kColP = TWO ? 0 : 128 + D;
+  static constexpr uint32_t kTmemCols = D == 64 || TWO ? 256 : 512;
 };
 
 struct SBars {
-  uint64_t q_full, k_full[kStages], k_empty[kStages], v_full[kStages], v_empty[kStages];
+  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2];
   uint64_t s_full, s_taken, p_part[2], o_done;
   uint64_t pair[4];                       // the two warps of a quarter have written what the other one reads
   uint32_t tmem_base;
@@ -114,10 +117,10 @@ __device__ __forceinline__ void pass_on(const uint32_t* s, uint32_t (&w)[16]) {
 
 }  // namespace
 
-template <bool BF16, int D, int MODE>
+template <bool BF16, int D, int MODE, bool TWO>
 __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __grid_constant__ AttnParams p) {
-  using SM = Layout<D>;
-  constexpr int kAtoms = D / 64;
+  using SM = Layout<D, TWO>;
+  constexpr int kAtoms = D / 64, kStages = SM::kStages;
   extern __shared__ uint8_t smem_raw[];
   // the CTAs of a cluster round up by the same amount: offsets match across the cluster
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -256,7 +259,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __gr
       const int st = j % kStages, sn = (j + 1) % kStages;
       const bool more = j + 1 < nkv;
       const int keys = more ? kBN : last_keys;
-      if (more) {
+      if (!TWO && more) {
         // the softmax warps must have taken S(j) out of tensor memory before S(j + 1) lands there
         ok = wait(&bar->k_full[sn], ((j + 1) / kStages) & 1, 0x310) && wait(&bar->s_taken, j & 1, 0x320);
         if (!ok) break;
@@ -270,6 +273,11 @@ __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __gr
       issue_pv(st, kFirstKeys, keys, false);
       umma_commit_elected(&bar->v_empty[st], issuer);     // also tells the softmax warps that P*V(j) is done
       if (!more) umma_commit_elected(&bar->o_done, issuer);
+      if (TWO && more) {
+        // P lies where S was: the next scores follow its last use in the order of issue
+        ok = wait(&bar->k_full[0], (j + 1) & 1, 0x310);
+        if (ok) issue_s(0);
+      }
     }
   } else {
     // ------------------------------------------------------------ softmax (warps 0-7)
@@ -287,7 +295,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __gr
       uint32_t sv[64];                                     // groups `half` and 2 + `half` of 32 keys
       tmem_ld_2x32_wait(s_col + 32 * half, s_col + 64 + 32 * half, sv);
       tc_fence_before_sync();
-      mbar_arrive_warp(&bar->s_taken, lane);
+      if (!TWO) mbar_arrive_warp(&bar->s_taken, lane);
       const int keys = j == nkv - 1 ? last_keys : kBN;
       if constexpr (MODE == kModeSoftmax) {
         if (keys != kBN) {
@@ -303,7 +311,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __gr
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         m_new = fmaxf(m_new, told[(par * 2 + (half ^ 1)) * kBM]);
-        if (j > 0) {
+        if (TWO) tc_fence_after_sync();                    // (the other warp has its scores too: P may take their place)
+        if (!TWO && j > 0) {
           // P*V(j-1) must have finished before P is overwritten or O is rescaled (S(j) was issued ahead of it)
           ok = mbar_wait(&bar->v_empty[(j - 1) % kStages], ((j - 1) / kStages) & 1, abort_word, 0x900);
           ok = __all_sync(0xffffffffu, ok);
@@ -327,6 +336,13 @@ __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __gr
           l *= f;
           ref.subtract(sv);
         }
+      } else if (TWO) {
+        // P takes the place of the scores once both warps of the quarter have theirs
+        mbar_arrive_warp(&bar->pair[quarter], lane);
+        ok = mbar_wait(&bar->pair[quarter], par, abort_word, 0x880);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after_sync();
       } else if (j > 0) {
         ok = mbar_wait(&bar->v_empty[(j - 1) % kStages], ((j - 1) / kStages) & 1, abort_word, 0x900);
         ok = __all_sync(0xffffffffu, ok);
@@ -479,10 +495,10 @@ __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __gr
 }
 
 // ------------------------------------------------------------------ launcher
-template <bool BF16, int D, int MODE>
+template <bool BF16, int D, int MODE, bool TWO>
 static cudaError_t launch_s(const AttnParams& p, int ctas, cudaStream_t stream) {
-  using SM = Layout<D>;
-  auto kern = attention_short_kernel<BF16, D, MODE>;
+  using SM = Layout<D, TWO>;
+  auto kern = attention_short_kernel<BF16, D, MODE, TWO>;
   static std::atomic<unsigned long long> configured{0};
   int dev = 0;
   cudaError_t e = current_device_checked(&dev);
@@ -511,20 +527,22 @@ static cudaError_t launch_s(const AttnParams& p, int ctas, cudaStream_t stream) 
   return launch_kernel(cfg, kern, p);
 }
 
-cudaError_t launch_attention_short(const AttnParams& params, int batch, int d, bool bf16, int mode, int parts, cudaStream_t stream) {
+cudaError_t launch_attention_short(const AttnParams& params, int batch, int d, bool bf16, int mode, int parts, bool two, cudaStream_t stream) {
   const int blocks = (params.L + kBN - 1) / kBN;
   const long long ctas = static_cast<long long>((params.M + kBM - 1) / kBM) * batch * parts;
-  if ((parts != 1 && parts != 2 && parts != 4 && parts != 8) || parts > blocks || ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
+  if ((parts != 1 && parts != 2 && parts != 4 && parts != 8) || parts > blocks || ctas > 0x7fffffffLL || (two && (d != 128 || parts > 1))) return cudaErrorInvalidValue;
   AttnParams p = params;
   p.parts = parts;
   const int n = static_cast<int>(ctas);
-#define DITTO_DISPATCH(BF, DD) \
-  if (bf16 == BF && d == DD)   \
-    return mode == 0 ? launch_s<BF, DD, 0>(p, n, stream) : mode == 1 ? launch_s<BF, DD, 1>(p, n, stream) : launch_s<BF, DD, 2>(p, n, stream);
-  DITTO_DISPATCH(false, 64)
-  DITTO_DISPATCH(false, 128)
-  DITTO_DISPATCH(true, 64)
-  DITTO_DISPATCH(true, 128)
+#define DITTO_DISPATCH(BF, DD, TW) \
+  if (bf16 == BF && d == DD && two == TW) \
+    return mode == 0 ? launch_s<BF, DD, 0, TW>(p, n, stream) : mode == 1 ? launch_s<BF, DD, 1, TW>(p, n, stream) : launch_s<BF, DD, 2, TW>(p, n, stream);
+  DITTO_DISPATCH(false, 64, false)
+  DITTO_DISPATCH(false, 128, false)
+  DITTO_DISPATCH(false, 128, true)
+  DITTO_DISPATCH(true, 64, false)
+  DITTO_DISPATCH(true, 128, false)
+  DITTO_DISPATCH(true, 128, true)
 #undef DITTO_DISPATCH
   return cudaErrorInvalidValue;
 }
@@ -539,8 +557,8 @@ static int cluster_places(int lg) {
   if (current_device_checked(&dev) != cudaSuccess) return 0;
   int n = places[dev][lg].load(std::memory_order_relaxed);
   if (n == 0) {
-    using SM = Layout<128>;
-    auto kern = attention_short_kernel<false, 128, kModeSoftmax>;
+    using SM = Layout<128, false>;
+    auto kern = attention_short_kernel<false, 128, kModeSoftmax, false>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(1024, 1, 1);
     cfg.blockDim = dim3(kThreads, 1, 1);
@@ -595,20 +613,28 @@ constexpr int kRowFrom[2] = {5, 4};                             // blocks a part
 // 12.5 -> 13.1, at worst, of one tile a sequence, 296 x 3 11.8 -> 12.8; its error against float64 is 1 to 3 % larger at scale
 // d^-0.5 and up to 10 % on uniform operands at scale 1); longer ones have no gain (296 x 8 20.2 -> 21.2).  Without a
 // softmax it pays for up to three (148 x 1 4.4 -> 3.7, 200 x 1 4.7 -> 4.3, 200 x 2 5.9 -> 5.4).
-// One tile a sequence at head dimension 128 has no second tile to work beside: there it pays in any number of items from six blocks on,
-// without a softmax (200 x 8 35.0 -> 29.7, 1000 x 8 118 -> 109, 4000 x 6 382 -> 365) and with one (200 x 8 36.4 -> 33.5, 256 x 16 74 -> 65, 1000 x 16
-// 254 -> 232); many items of six to eight are no faster (592 x 6 62.2 -> 65.7, 1480 x 6 150 -> 163, 1480 x 8 195 -> 201), but 1 % closer to
-// float64 at scale d^-0.5 and 10 % where the scores spread further: the other kernel keeps its references within 2^8 only.
+// More than 148 items at head dimension 128: two CTAs an SM, each with a K and a V stage and P in the place of S, work beside each other, where the kernel
+// with two tiles a CTA needs two tiles of one sequence.  One tile a sequence, us, before -> now: 150 x 4 17.7 -> 13.3, 296 x 1 9.0 -> 6.9, 450 x 8 61.3 -> 52.2, 600 x 3 38.4
+// -> 35.9, 1000 x 8 136 -> 113, 2000 x 4 144 -> 116, without a softmax 150 x 4 14.0 -> 10.2, 600 x 4 46.5 -> 39.2; many items of one or two blocks are bound by what
+// is loaded, which the other kernel asks for an item ahead (1000 x 1 28.9 -> 31.3, x 2 41.9 -> 43.7).  More tiles a sequence, up to 296 items: 296 x 1 8.0 -> 6.6, x 4 15.0 -> 14.0,
+// with a softmax only as long as there are few blocks (160 x 8 21.1 -> 22.9, 150 x 16 35.9 -> 38.4; of 208 or 256 rows, 80 wide, x 4 12.4 -> 12.9; at worst x 2 of 208
+// keys 9.15 -> 9.40), without one always (150 x 64 122 -> 111); more items without a softmax
+// where a sequence has two tiles and four blocks (512 x 16 of 208 rows 75.0 -> 69.3, 600 x 4 37.1 -> 33.6; x 2 19.3 -> 21.1; of 2048 rows 1024 x 4 37.0 -> 39.3).
+// Its error against float64 is 1 to 3 % smaller: the other kernel keeps its references within 2^8 only.
 AttnFew attention_few(int batch, int M, int L, int d, int mode) {
   constexpr int kSms = 148;
   const long long items = static_cast<long long>((M + kBM - 1) / kBM) * batch;
   const int blocks = (L + kBN - 1) / kBN;
   const int m = mode == kModeSoftmax ? 0 : 1, wide = d == 64 ? 0 : 1;
-  AttnFew best = {1, false};
-  if (items > 2 * kSms || (items > kSms && d == 128)) {
-    best.here = d == 128 && M <= kBM && blocks >= 6;
+  AttnFew best = {1, false, false};
+  if (items > kSms && d == 128) {
+    if (M <= kBM) best.two = items <= 3 * kSms || blocks >= 3;
+    else if (items <= 2 * kSms) best.two = m == 1 || blocks <= (M <= 2 * kBM ? 3 : 4);
+    else best.two = m == 1 && M <= 2 * kBM && blocks >= 4;
+    best.here = best.two;
     return best;
   }
+  if (items > 2 * kSms) return best;
   const Whole& w = kWhole[wide][m];
   double best_t = items <= kSms ? w.fixed + w.block * blocks + (items > 100 ? w.full : 0.0) : 1e30;
   for (int lg = 1; lg <= 3 && (1 << lg) <= blocks; ++lg) {

@@ -35,13 +35,14 @@ cudaError_t launch_attention(const AttnParams& p, int batch, int d, bool bf16, i
 
 // One 128-row tile per CTA or per cluster of `parts` (1, 2, 4 or 8, at most the number of 128-key blocks) CTAs that divide the
 // keys between them and combine on chip, for few items (attention_short_sm100.cu).
-cudaError_t launch_attention_short(const AttnParams& p, int batch, int d, bool bf16, int mode, int parts, cudaStream_t stream);
+cudaError_t launch_attention_short(const AttnParams& p, int batch, int d, bool bf16, int mode, int parts, bool two, cudaStream_t stream);
 // The same with a thread a row, head dimensions up to 64, parts above 1: the faster one where every CTA has many blocks.
 cudaError_t launch_attention_split(const AttnParams& p, int batch, bool bf16, int mode, int parts, cudaStream_t stream);
 // The number of parts that is expected to be fastest for a shape (1: no split), and whether it is the kernel for few items'.
 struct AttnFew {
   int parts;
   bool here;
+  bool two;            // in the form of which two CTAs fit an SM at head dimension 128
 };
 AttnFew attention_few(int batch, int M, int L, int d, int mode);
 
