@@ -51,9 +51,15 @@ struct Layout {
   static constexpr int kOffK = kOffQ + kTileQ;
   static constexpr int kOffV = kOffK + kStages * kTileKV;
   static constexpr int kOffPair = kOffV + kStages * kTileKV;      // float [2][2][128]: maxima, by parity of the block and half
-  static constexpr int kOffRows = kOffPair + 2 * 2 * kBM * 4;     // float2 [128]: (max, sum) for the cluster
+  static constexpr int kOffRows = kOffPair + 2 * 2 * kBM * 4;     // float2 [128]: (max, sum) for the cluster, eight parts
   static constexpr int kOffBar = kOffRows + kBM * 8;
-  static constexpr int kBytes = kOffBar + 256 + 1024;
+  // the other parts' (max, sum), float2 [parts - 1][128], and columns, float4 [parts - 1][D / parts / 4][128]
+  static constexpr int kOffMl = kOffBar + 256;
+  static __host__ __device__ constexpr bool own_memory(int parts) { return parts == 2 || parts == 4; }
+  static __host__ __device__ constexpr int off_in(int parts) { return kOffMl + (parts - 1) * kBM * 8; }
+  static __host__ __device__ constexpr int bytes(int parts) {
+    return (own_memory(parts) ? off_in(parts) + (parts - 1) * (D / parts) * kBM * 4 : kOffMl) + 1024;
+  }
   static constexpr uint32_t kColS = 0, kColO = 128, kColP = TWO ? 0 : 128 + D;
   static constexpr uint32_t kTmemCols = D == 64 || TWO ? 256 : 512;
 };
@@ -66,6 +72,7 @@ struct SBars {
   uint32_t abort_word;
 };
 static_assert(sizeof(SBars) <= 256, "barrier block too large");
+static_assert(2 * (Layout<64, false>::bytes(4) + 1024) <= 228 * 1024 && Layout<128, false>::bytes(4) <= 227 * 1024, "shared memory budget");
 
 // The largest of 32 scores and m.
 __device__ __forceinline__ float max_with(float m, const uint32_t* s) {
@@ -117,7 +124,8 @@ __device__ __forceinline__ void pass_on(const uint32_t* s, uint32_t (&w)[16]) {
 
 }  // namespace
 
-template <bool BF16, int D, int MODE, bool TWO>
+// PARTS: CTAs that share an item's keys
+template <bool BF16, int D, int MODE, int PARTS, bool TWO>
 __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __grid_constant__ AttnParams p) {
   using SM = Layout<D, TWO>;
   constexpr int kAtoms = D / 64, kStages = SM::kStages;
@@ -130,7 +138,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __gr
   const int lane = threadIdx.x & 31;
   const int tiles = (p.M + kBM - 1) / kBM;
   // the CTAs of a cluster are consecutive: rank r of `parts` takes K/V blocks [r * n / parts, (r + 1) * n / parts)
-  const int parts = p.parts, part = static_cast<int>(cluster_ctarank());
+  constexpr int parts = PARTS;
+  const int part = PARTS == 1 ? 0 : static_cast<int>(cluster_ctarank());
   const int id = static_cast<int>(blockIdx.x) / parts;
   const int slice = id / tiles, seq = slice / p.heads;
   const int head_col = (slice - seq * p.heads) * p.d;
@@ -169,6 +178,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __gr
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  // (a peer's shared memory may be written once the peer has started)
+  if (SM::own_memory(PARTS)) cluster_arrive();
   const uint32_t tmem_base = bar->tmem_base;
   // Programmatic dependent launch: nothing above touches global memory.
   grid_dependency_wait();
@@ -382,7 +393,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __gr
     }
     row_m = ref.m;
     row_l = l;
-    if (ok && parts == 1) {
+    if (ok && PARTS == 1) {
       const float inv = MODE == kModeSoftmax ? 1.0f / l : 1.0f;
       // Turned around in 2 or 4 KB of the K ring per warp (every MMA has retired), 16-byte pieces swizzled by row, so that a
       // store instruction writes rows of 64 or 128 contiguous bytes.
@@ -414,7 +425,106 @@ __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __gr
     }
   }
 
-  if (parts > 1) {
+  if constexpr (SM::own_memory(PARTS)) {
+    // Combine the parts.  Every CTA hands each of the others D / PARTS columns of its O and its rows' (max, sum), into memory of their own; once it has
+    // theirs it scales what it was given and its own columns, which are still in tensor memory, by 2^(max - overall max) / overall sum, adds them in
+    // rank order and writes those columns of the result: a reduce-scatter, so the exchange and the write-out are spread over the cluster.
+    // Laid out [source][16-byte piece][row], a warp's store or load covers 512 contiguous bytes.  Both barriers are reached by every thread
+    // whether its waits expired or not.
+    // One barrier between the last P*V and the result (the first one has long been passed: it says that the peers have started), the number of parts
+    // known at compile time.  Against (max, sum) read from the peers behind a barrier, columns through the K ring and a number of parts known at
+    // run time: 0.88 to 0.92 of the time of a call in two parts (one ViT-Base image 5.9 -> 5.3 us), and unsplit calls, which bring none of this code, 0.98 to 0.99.
+    __syncwarp();
+    cluster_wait();
+    constexpr int kCols = D / PARTS, kPiece = kCols >= 32 ? 16 : kCols / 2;
+    const uint32_t o_base = lane_base + SM::kColO;
+    float2* ml = reinterpret_cast<float2*>(smem + SM::kOffMl) + row;       // [PARTS - 1][row]
+    float4* in = reinterpret_cast<float4*>(smem + SM::off_in(PARTS)) + row;  // [PARTS - 1][kCols / 4][row]
+    if (warp < kSoftmaxWarps) {
+      if (MODE == kModeSoftmax && half == 0) {
+#pragma unroll
+        for (int i = 0; i < PARTS - 1; ++i) {
+          const int to = i + (i >= part);
+          st_cluster_v2(map_to_cta(smem_u32(ml + (part - (part > to)) * kBM), to), row_m, row_l);
+        }
+      }
+#pragma unroll 1
+      for (int c = half; c < (PARTS - 1) * kCols / 16; c += 2) {
+        const int i = c / (kCols / 16), sub = c - i * (kCols / 16), to = i + (i >= part);
+        uint32_t o[16];
+        tmem_ld_x16_wait(o_base + to * kCols + sub * 16, o);
+        const uint32_t at = map_to_cta(smem_u32(in + ((part - (part > to)) * (kCols / 4) + sub * 4) * kBM), to);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          st_cluster_v4(at + q * (kBM * 16), __uint_as_float(o[4 * q]), __uint_as_float(o[4 * q + 1]), __uint_as_float(o[4 * q + 2]), __uint_as_float(o[4 * q + 3]));
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();
+    if (warp < kSoftmaxWarps) {
+      float f[PARTS];                                    // factors of the parts
+      if constexpr (MODE == kModeSoftmax) {
+        float2 t[PARTS];
+        float top = -INFINITY, total = 0.f;
+#pragma unroll
+        for (int r = 0; r < PARTS; ++r) {
+          t[r] = r == part ? make_float2(row_m, row_l) : ml[(r - (r > part)) * kBM];
+          top = fmaxf(top, t[r].x);
+        }
+#pragma unroll
+        for (int r = 0; r < PARTS; ++r) {
+          f[r] = ex2_approx((t[r].x - top) * p.scale_log2);
+          total = fmaf(t[r].y, f[r], total);
+        }
+#pragma unroll
+        for (int r = 0; r < PARTS; ++r) f[r] = f[r] / total;
+      }
+      uint8_t* dst = reinterpret_cast<uint8_t*>(p.out) + ((static_cast<size_t>(seq) * p.M + m0 + row) * p.out_ld + head_col) * 2;
+#pragma unroll 1
+      for (int c = half * kPiece; c < kCols; c += 2 * kPiece) {
+        const int col = part * kCols + c;                // widths are multiples of 16
+        if (col >= p.dv) break;
+        uint32_t own[kPiece];
+        if constexpr (kPiece == 16) tmem_ld_x16_wait(o_base + col, own); else tmem_ld_x8_wait(o_base + col, own);
+        float sum[kPiece];
+        if constexpr (PARTS == 2 && MODE == kModeSoftmax) {          // (two terms: either order is the same sum)
+          const float mine = part == 0 ? f[0] : f[1], theirs = part == 0 ? f[1] : f[0];
+#pragma unroll
+          for (int q = 0; q < kPiece / 4; ++q) {
+            const float4 g = in[(c / 4 + q) * kBM];
+            sum[4 * q] = __fadd_rn(__fmul_rn(__uint_as_float(own[4 * q]), mine), __fmul_rn(g.x, theirs));
+            sum[4 * q + 1] = __fadd_rn(__fmul_rn(__uint_as_float(own[4 * q + 1]), mine), __fmul_rn(g.y, theirs));
+            sum[4 * q + 2] = __fadd_rn(__fmul_rn(__uint_as_float(own[4 * q + 2]), mine), __fmul_rn(g.z, theirs));
+            sum[4 * q + 3] = __fadd_rn(__fmul_rn(__uint_as_float(own[4 * q + 3]), mine), __fmul_rn(g.w, theirs));
+          }
+        } else {
+#pragma unroll
+          for (int r = 0; r < PARTS; ++r) {
+            const float4* from = in + ((r - (r > part)) * (kCols / 4) + c / 4) * kBM;
+#pragma unroll
+            for (int q = 0; q < kPiece / 4; ++q) {
+              float4 g = make_float4(__uint_as_float(own[4 * q]), __uint_as_float(own[4 * q + 1]), __uint_as_float(own[4 * q + 2]), __uint_as_float(own[4 * q + 3]));
+              if (r != part) g = from[q * kBM];
+              if constexpr (MODE == kModeSoftmax) g = make_float4(__fmul_rn(g.x, f[r]), __fmul_rn(g.y, f[r]), __fmul_rn(g.z, f[r]), __fmul_rn(g.w, f[r]));
+              sum[4 * q] = r == 0 ? g.x : sum[4 * q] + g.x;
+              sum[4 * q + 1] = r == 0 ? g.y : sum[4 * q + 1] + g.y;
+              sum[4 * q + 2] = r == 0 ? g.z : sum[4 * q + 2] + g.z;
+              sum[4 * q + 3] = r == 0 ? g.w : sum[4 * q + 3] + g.w;
+            }
+          }
+        }
+        if (m0 + row < p.M) {
+#pragma unroll
+          for (int q = 0; q < kPiece / 8; ++q)
+            *reinterpret_cast<uint4*>(dst + col * 2 + 16 * q) = make_uint4(pack2<BF16>(sum[8 * q], sum[8 * q + 1]), pack2<BF16>(sum[8 * q + 2], sum[8 * q + 3]),
+                                                                           pack2<BF16>(sum[8 * q + 4], sum[8 * q + 5]), pack2<BF16>(sum[8 * q + 6], sum[8 * q + 7]));
+        }
+      }
+    }
+  }
+
+  if constexpr (PARTS > 1 && !SM::own_memory(PARTS)) {
+    // (Eight parts: their columns in memory of their own leave room for one CTA an SM at head dimension 64, and take 0 to 4 % longer at 128.)
     // Combine the parts.  Every CTA publishes its rows' (max, sum), scales its O by
     // 2^(max - overall max) / overall sum and hands D / parts columns of it to each CTA of the cluster, which adds
     // what it was given and writes those columns of the result: a reduce-scatter, so the exchange (D * 512 bytes in
@@ -495,16 +605,16 @@ __global__ void __launch_bounds__(kThreads, 2) attention_short_kernel(const __gr
 }
 
 // ------------------------------------------------------------------ launcher
-template <bool BF16, int D, int MODE, bool TWO>
+template <bool BF16, int D, int MODE, int PARTS, bool TWO>
 static cudaError_t launch_s(const AttnParams& p, int ctas, cudaStream_t stream) {
   using SM = Layout<D, TWO>;
-  auto kern = attention_short_kernel<BF16, D, MODE, TWO>;
+  auto kern = attention_short_kernel<BF16, D, MODE, PARTS, TWO>;
   static std::atomic<unsigned long long> configured{0};
   int dev = 0;
   cudaError_t e = current_device_checked(&dev);
   if (e != cudaSuccess) return e;
   if (!device_configured(configured, dev)) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::kBytes);
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::bytes(PARTS));
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
@@ -513,7 +623,7 @@ static cudaError_t launch_s(const AttnParams& p, int ctas, cudaStream_t stream) 
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(ctas), 1, 1);
   cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.dynamicSmemBytes = SM::kBytes;
+  cfg.dynamicSmemBytes = SM::bytes(PARTS);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see grid_dependency_wait in the kernel
@@ -534,15 +644,18 @@ cudaError_t launch_attention_short(const AttnParams& params, int batch, int d, b
   AttnParams p = params;
   p.parts = parts;
   const int n = static_cast<int>(ctas);
-#define DITTO_DISPATCH(BF, DD, TW) \
-  if (bf16 == BF && d == DD && two == TW) \
-    return mode == 0 ? launch_s<BF, DD, 0, TW>(p, n, stream) : mode == 1 ? launch_s<BF, DD, 1, TW>(p, n, stream) : launch_s<BF, DD, 2, TW>(p, n, stream);
-  DITTO_DISPATCH(false, 64, false)
-  DITTO_DISPATCH(false, 128, false)
-  DITTO_DISPATCH(false, 128, true)
-  DITTO_DISPATCH(true, 64, false)
-  DITTO_DISPATCH(true, 128, false)
-  DITTO_DISPATCH(true, 128, true)
+#define DITTO_DISPATCH(BF, DD, PA, TW) \
+  if (bf16 == BF && d == DD && parts == PA && two == TW) \
+    return mode == 0 ? launch_s<BF, DD, 0, PA, TW>(p, n, stream) : mode == 1 ? launch_s<BF, DD, 1, PA, TW>(p, n, stream) : launch_s<BF, DD, 2, PA, TW>(p, n, stream);
+#define DITTO_DISPATCH_PARTS(BF, DD) \
+  DITTO_DISPATCH(BF, DD, 1, false) DITTO_DISPATCH(BF, DD, 2, false) DITTO_DISPATCH(BF, DD, 4, false) DITTO_DISPATCH(BF, DD, 8, false)
+  DITTO_DISPATCH_PARTS(false, 64)
+  DITTO_DISPATCH_PARTS(false, 128)
+  DITTO_DISPATCH_PARTS(true, 64)
+  DITTO_DISPATCH_PARTS(true, 128)
+  DITTO_DISPATCH(false, 128, 1, true)
+  DITTO_DISPATCH(true, 128, 1, true)
+#undef DITTO_DISPATCH_PARTS
 #undef DITTO_DISPATCH
   return cudaErrorInvalidValue;
 }
@@ -558,11 +671,11 @@ static int cluster_places(int lg) {
   int n = places[dev][lg].load(std::memory_order_relaxed);
   if (n == 0) {
     using SM = Layout<128, false>;
-    auto kern = attention_short_kernel<false, 128, kModeSoftmax, false>;
+    auto kern = attention_short_kernel<false, 128, kModeSoftmax, 8, false>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(1024, 1, 1);
     cfg.blockDim = dim3(kThreads, 1, 1);
-    cfg.dynamicSmemBytes = SM::kBytes;
+    cfg.dynamicSmemBytes = SM::bytes(8);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1u << lg;
@@ -571,7 +684,7 @@ static int cluster_places(int lg) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int count = 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::kBytes) != cudaSuccess ||
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::bytes(8)) != cudaSuccess ||
         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&count, kern, &cfg) != cudaSuccess)
       return 0;
@@ -581,22 +694,21 @@ static int cluster_places(int lg) {
   return n - 1;
 }
 
-// Times of a launch (us, one call after another) by parts and 128-key blocks of a CTA, fp16, fitted to shapes of 1 to 296 items and 1 to 64 blocks
-// (rms 3 to 8 %).  At head dimension 64 clusters share SMs once there are more than places at a CTA an SM (*Shared); more than the
+// Times of a launch (us, one call after another) by parts and 128-key blocks of a CTA, bf16, fitted to shapes of 1 to 148 items and 1 to 64 blocks
+// (rms 1 to 7 %).  At head dimension 64 clusters share SMs once there are more than places at a CTA an SM (*Shared); more than the
 // device holds at once would be a second wave, which costs more than a split saves (36 x 16 in eight parts 18.7 us, in four
-// 14.8).  What the rule picks took on average 0.6 % longer than the best form timed (softmax, 363 shapes of up to 148 items) and 0.3 %
-// (chains, 299), at head dimension 128 0.1 % (softmax, 234); asking 4 % for a split made that worse.  The fits are of the scalar arithmetic
-// before softmax_weights; with it, 70 shapes of up to 148 items and 48 blocks each, 0.7 % at head dimension 64 (at worst 7 %: 13 x 8 blocks 7.6
-// us, in eight parts 7.1) and nothing at 128 (1.4 %).
+// 14.8).  What the rule picks takes on average 0.3 % longer than the best form timed (softmax, 90 shapes), 0.5 % (chains), at head dimension 128 0.2 %; 8 % at worst.
 namespace {
 struct Whole { double fixed, block, full; };                    // full: over 100 CTAs
 struct Split { double fixed, part, block, full; };              // full: over 100 CTAs; shared: times the share of SMs with two
-constexpr Whole kWhole[2][2] = {{{3.3, 1.28, 0.7}, {3.0, 0.89, 0.4}}, {{3.6, 1.39, 1.2}, {3.0, 1.14, 1.0}}};      // [head dimension][no softmax]
-constexpr Split kAlone[2][2] = {{{4.3, 0.12, 1.30, 1.4}, {3.7, 0.09, 0.92, 0.6}}, {{5.7, 0.13, 1.37, 1.3}, {4.5, 0.16, 1.16, 1.2}}};
-constexpr Split kShared[2] = {{5.4, 0.30, 1.93, 0.8}, {4.8, 0.10, 1.30, 1.1}};
+constexpr Whole kWhole[2][2] = {{{2.89, 1.25, 0.32}, {2.39, 0.88, 0.36}}, {{3.65, 1.29, 0.70}, {2.84, 1.02, 0.69}}};      // [head dimension][no softmax]
+constexpr Split kAlone[2][2] = {{{3.24, 0.18, 1.26, 0.36}, {2.76, 0.13, 0.87, 0.39}}, {{4.43, 0.24, 1.32, 0.89}, {3.75, 0.24, 1.04, 1.02}}};
+constexpr Split kShared[2] = {{3.22, 0.44, 1.85, 0.80}, {3.40, 0.23, 1.10, 0.79}};
 // the kernel with a thread a row
-constexpr Split kRowAlone[2] = {{5.5, 0.06, 1.18, 0.8}, {4.0, 0.09, 0.75, 1.0}}, kRowShared[2] = {{6.6, 0.05, 1.70, 1.0}, {5.3, 0.05, 1.18, 1.1}};
-constexpr int kRowFrom[2] = {5, 4};                             // blocks a part from which that one is the faster at head dimension 64
+constexpr Split kRowAlone[2] = {{5.53, 0.04, 1.18, 0.65}, {4.37, 0.05, 0.69, 0.64}}, kRowShared[2] = {{6.49, 0.13, 1.65, 0.48}, {5.40, 0.13, 0.99, 0.42}};
+// Blocks a part from which that one is taken at head dimension 64: a CTA an SM, two, and in eight parts, whose columns arrive in the K ring here.
+constexpr int kRowFrom[2][2] = {{20, 8}, {12, 10}}, kRowFromEight = 8;
+bool by_row(int parts, int own, int m, bool shared) { return own >= (parts == 8 ? kRowFromEight : kRowFrom[m][shared ? 1 : 0]); }
 }  // namespace
 
 // Where the lines lie, the forms without this kernel and with two CTAs an SM left out of count -> the choice now (us), items x blocks of
@@ -604,10 +716,9 @@ constexpr int kRowFrom[2] = {5, 4};                             // blocks a part
 // 48 x 16 15.6 -> 14.4 (4), 100 x 2 6.9 -> 6.3, 148 x 4 10.2 -> 9.7, with a thread a row 24 x 64 25.3 -> 21.2 (8), 100 x 32 43.1 -> 33.6 (2),
 // 148 x 64 83.1 -> 61.7 (2); at 128: 24 x 1 7.2 -> 5.2, 24 x 2 7.9 -> 6.7, 24 x 4 9.0 -> 8.3 (4), 24 x 16 14.3 -> 13.2 (4), 48 x 16 20.3 -> 18.9 (2),
 // 100 x 32 64.4 -> 51.6; without a softmax 48 x 16 17.6 -> 14.5, 100 x 32 57.2 -> 39.5.
-// At head dimension 64 the kernel with a thread a row costs less per block (1.18 against 1.35: no word from another warp before the
-// exponentials).  This kernel's time over that one's, split alike, by blocks a part, a CTA an SM / two: one 0.90 / 0.99, two 0.93 / 0.99, four
-// 0.97 / 1.01, six 1.00 / 1.05, eight 1.02 / 1.06, sixteen 1.06 / 1.11, so parts of more than four blocks take that one; without a
-// softmax of more than three (48 x 8 7.4 -> 7.8, 12 x 64 10.7 -> 12.0).
+// At head dimension 64 the kernel with a thread a row costs less per block (1.18 against 1.26: no word from another warp before the
+// exponentials) and more to combine.  This kernel / that one, split alike: 12 x 32 blocks in two parts 23.4 / 24.1, x 16 in four 9.1 / 10.5, in eight 7.7 / 8.7, 1 x 64 in eight
+// 14.0 / 14.7; two CTAs an SM 148 x 16 in two 20.6 / 20.7, x 32 36.0 / 33.6.
 // Unsplit and two CTAs an SM it serves one to four blocks: one block is faster here (200 x 1 5.8 -> 5.5), two to four are about as fast as
 // in the kernel with 64-key blocks, whose references are those of shorter blocks (200 x 2 7.8 -> 7.7, 200 x 3 9.7 -> 10.2, 256 x 4
 // 12.5 -> 13.1, at worst, of one tile a sequence, 296 x 3 11.8 -> 12.8; its error against float64 is 1 to 3 % larger at scale
@@ -640,18 +751,18 @@ AttnFew attention_few(int batch, int M, int L, int d, int mode) {
   for (int lg = 1; lg <= 3 && (1 << lg) <= blocks; ++lg) {
     const int parts = 1 << lg, own = (blocks + parts - 1) / parts, places = cluster_places(lg);
     if (items > (wide ? places : 2 * places)) break;
-    const bool by_row = !wide && own >= kRowFrom[m], shared = items > places;
-    const Split& s = by_row ? (shared ? kRowShared[m] : kRowAlone[m]) : shared ? kShared[m] : kAlone[wide][m];
+    const bool shared = items > places, row = !wide && by_row(parts, own, m, shared);
+    const Split& s = row ? (shared ? kRowShared[m] : kRowAlone[m]) : shared ? kShared[m] : kAlone[wide][m];
     const double time = s.fixed + s.part * parts + s.block * own +
                         s.full * (shared ? static_cast<double>(items - places) / places : items * parts > 100 ? 1.0 : 0.0);
     if (time < best_t) {
       best.parts = parts;
+      best.here = !row;
       best_t = time;
     }
   }
-  const int own = (blocks + best.parts - 1) / best.parts;
   if (d == 128) best.here = true;
-  else if (best.parts > 1) best.here = own < kRowFrom[m];
+  else if (best.parts > 1) return best;
   else if (items > kSms) best.here = blocks <= (m == 0 ? 4 : 3);
   else best.here = blocks <= (m == 0 ? 8 : 6);
   return best;
