@@ -17,10 +17,12 @@
 // deliver on all SMs at once: 376 clocks at bn = 128 (256 of tensor work), 565 at 256 (512) -- and, in short calls,
 // two chains of launch, first load, k-steps, epilogue.
 //
-// Tile width and layout of B are template parameters: what an issuing warp works out per k-step is then known at compile time, and a launch
+// Tile width, layout of B and the number of parts are template parameters: what an issuing warp works out per k-step is then known at compile time, and a launch
 // fetches the code of its own width alone (all widths behind a switch in one kernel: 1 to 3 us slower than run-time values).  A k-step of a lone
 // CTA at bn = 128 took 480 clocks with run-time values.  In a graph, operands new call after call, us, before -> after: 24 shapes of 16 to 8192 rows 18.6 ->
-// 17.6 (geometric mean), 512 x 768 -> 3072 -> 768 with GELU 15.5 -> 14.3, 128 x 1024 -> 4096 -> 1024 14.0 -> 12.6, 1024 x 1024 23.8 -> 22.1, 432 x 1024 -> 1856 13.9 -> 12.3.
+// 17.6 (geometric mean), 512 x 768 -> 3072 -> 768 with GELU 15.5 -> 14.3, 128 x 1024 -> 4096 -> 1024 14.0 -> 12.6, 1024 x 1024 23.8 -> 22.1, 432 x 1024 -> 1856 13.9 -> 12.3; the
+// number of parts (and waits out of line) 17.3 -> 16.9, 512 x 768 14.3 -> 13.7.  (A CTA's own columns of a divided tile kept in tensor memory instead of going through
+// its ring: no difference.)
 // Two k-steps a stage, as in the wave kernel: 1 % faster with operands in L2, 1 to 8 % slower with operands from memory.  Partial sums by bulk copies
 // instead of stores to the peers: 14.2 -> 16.0.  Results written from registers in 32-byte sectors: 17.6 -> 18.0 (spills at 80 registers).
 #define DITTO_WAIT_OUT_OF_LINE   // see mbar_wait
@@ -61,7 +63,7 @@ struct TilesParams {
   int blocks_per_batch, blocks;         // 128-row blocks
   int steps;                // k-steps of 64
   int chunks;               // GEMM2: 256-column chunks of the hidden layer, taken in the order below (0: in order)
-  int parts, stages;
+  int stages;
   int early_b;              // B is not written by the kernel ahead: its loads need not wait for that
   int* status;
 };
@@ -110,7 +112,7 @@ __device__ __forceinline__ void finish(const uint32_t (&v)[N], const uint32_t* b
 
 }  // namespace
 
-template <bool BF16, int ACT, bool BIAS, int BN, bool OI>
+template <bool BF16, int ACT, bool BIAS, int BN, bool OI, int PARTS>
 __global__ void __launch_bounds__(kThreads, 2) mlp_tiles_kernel(const __grid_constant__ TilesParams p) {
   constexpr int kStage = kATile + BN * 128;
   extern __shared__ uint8_t smem_raw[];
@@ -122,13 +124,13 @@ __global__ void __launch_bounds__(kThreads, 2) mlp_tiles_kernel(const __grid_con
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   // clusters are consecutive CTAs; row blocks innermost, so that neighbours share weights
-  const int part = static_cast<int>(cluster_ctarank());
-  const int tile = static_cast<int>(blockIdx.x) / p.parts;
+  const int part = PARTS == 1 ? 0 : static_cast<int>(cluster_ctarank());
+  const int tile = static_cast<int>(blockIdx.x) / PARTS;
   const int n = tile / p.blocks, rb = tile - n * p.blocks;
   const int b = rb / p.blocks_per_batch;
   const int row0 = (rb - b * p.blocks_per_batch) * kRows;
   const int col0 = n * BN;
-  const int k0 = p.steps * part / p.parts, k1 = p.steps * (part + 1) / p.parts;   // parts <= steps: never empty
+  const int k0 = p.steps * part / PARTS, k1 = p.steps * (part + 1) / PARTS;   // parts <= steps: never empty
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) {
@@ -230,7 +232,7 @@ __global__ void __launch_bounds__(kThreads, 2) mlp_tiles_kernel(const __grid_con
       ok = mbar_wait(&bar->acc_full, 0, abort_word, 0x300);
       ok = __all_sync(0xffffffffu, ok);
       tc_fence_after_sync();
-      if (ok && p.parts == 1) {
+      if (ok && PARTS == 1) {
         // 32 columns at a time, turned around in 2 KB of the (now idle) ring per warp -- 64-byte rows of four 16-byte
         // pieces, swizzled: no bank conflicts -- so that a store instruction writes 64 contiguous bytes of eight rows
         const uint32_t acc = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
@@ -260,17 +262,17 @@ __global__ void __launch_bounds__(kThreads, 2) mlp_tiles_kernel(const __grid_con
     }
   }
 
-  if (p.parts > 1) {
+  if constexpr (PARTS > 1) {
     // The CTAs of the cluster hold partial sums of the same tile.  Each hands bn / parts columns of its own to every
     // CTA (into its ring, idle since the last MMA: first barrier), adds what it was given in rank order and finishes
     // those columns.  Laid out [source][four columns][row], a warp's store or load covers 512 contiguous bytes.  Every
     // thread reaches both barriers whether its waits expired or not.
     __syncwarp();
     cluster_sync_all();
-    const int cols = BN / p.parts;                     // 16, 32, 64 or 128
+    constexpr int cols = BN / PARTS;                   // 16, 32, 64 or 128
     const int row = (warp & 3) * 32 + lane;
     if (warp < kEpiWarps) {
-      const int cols_log2 = 31 - __clz(cols);
+      constexpr int cols_log2 = cols == 16 ? 4 : cols == 32 ? 5 : cols == 64 ? 6 : 7;
       const uint32_t in0 = smem_u32(smem) + (part * (cols / 4) * kRows + row) * 16;
       const uint32_t acc = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
 #pragma unroll 1
@@ -297,8 +299,8 @@ __global__ void __launch_bounds__(kThreads, 2) mlp_tiles_kernel(const __grid_con
         float sum[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) sum[j] = 0.f;
-#pragma unroll 2
-        for (int r = 0; r < p.parts; ++r) {
+#pragma unroll
+        for (int r = 0; r < PARTS; ++r) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const float4 t = in[(r * (cols / 4) + c / 4 + q) * kRows];
@@ -333,9 +335,9 @@ namespace {
 constexpr int kBarBytes = sizeof(TilesBars) + 512, kSlack = 1024;    // (barriers, and the biases of 256 columns)
 constexpr int kRingLone = 192 * 1024, kRingShared = 96 * 1024;
 
-template <bool BF16, int ACT, bool BIAS, int BN, bool OI>
+template <bool BF16, int ACT, bool BIAS, int BN, bool OI, int PARTS>
 cudaError_t launch_one(const TilesParams& p, int ctas, cudaStream_t stream) {
-  auto kern = mlp_tiles_kernel<BF16, ACT, BIAS, BN, OI>;
+  auto kern = mlp_tiles_kernel<BF16, ACT, BIAS, BN, OI, PARTS>;
   static std::atomic<unsigned long long> configured{0};
   int dev = 0;
   cudaError_t e = current_device_checked(&dev);
@@ -356,22 +358,30 @@ cudaError_t launch_one(const TilesParams& p, int ctas, cudaStream_t stream) {
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = static_cast<unsigned>(p.parts);
+  attr[1].val.clusterDim.x = PARTS;
   attr[1].val.clusterDim.y = 1;
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = p.parts > 1 ? 2 : 1;
+  cfg.numAttrs = PARTS > 1 ? 2 : 1;
   return launch_kernel(cfg, kern, p);
 }
 
 template <bool BF16, int ACT, bool BIAS, bool OI>
-cudaError_t launch_width(const TilesParams& p, int bn, int ctas, cudaStream_t stream) {
-  switch (bn) {
-    case 64: return launch_one<BF16, ACT, BIAS, 64, OI>(p, ctas, stream);
-    case 128: return launch_one<BF16, ACT, BIAS, 128, OI>(p, ctas, stream);
-    case 192: return launch_one<BF16, ACT, BIAS, 192, OI>(p, ctas, stream);
-    default: return launch_one<BF16, ACT, BIAS, 256, OI>(p, ctas, stream);
-  }
+cudaError_t launch_cut(const TilesParams& p, const TilesGemm& g, int ctas, cudaStream_t stream) {
+#define DITTO_CUT(BN, PARTS) \
+  if (g.bn == BN && g.parts == PARTS) return launch_one<BF16, ACT, BIAS, BN, OI, PARTS>(p, ctas, stream);
+  DITTO_CUT(64, 1)
+  DITTO_CUT(64, 2)
+  DITTO_CUT(64, 4)
+  DITTO_CUT(128, 1)
+  DITTO_CUT(128, 2)
+  DITTO_CUT(128, 4)
+  DITTO_CUT(128, 8)
+  DITTO_CUT(192, 1)
+  DITTO_CUT(256, 1)
+  DITTO_CUT(256, 2)
+#undef DITTO_CUT
+  return cudaErrorInvalidValue;
 }
 
 // D [batch, M, N] = act(A [batch, M, K] * B + bias)
@@ -404,7 +414,6 @@ int launch_gemm(const void* a, const void* w, void* out, const void* bias, int b
   p.blocks = batch * p.blocks_per_batch;
   p.chunks = second ? (K + 255) / 256 : 0;
   p.steps = second ? 4 * p.chunks : (K + 63) / 64;      // (units past the hidden size read as zero)
-  p.parts = g.parts;
   p.stages = std::min(kMaxStages, (g.per_sm == 2 ? kRingShared : kRingLone) / (kATile + g.bn * 128));
   p.early_b = second ? 1 : 0;
   p.status = status;
@@ -412,12 +421,10 @@ int launch_gemm(const void* a, const void* w, void* out, const void* bias, int b
   if (ctas > 0x7fffffffLL) return DITTO_ERR_UNSUPPORTED;
   cudaError_t e = cudaErrorInvalidValue;
 #define DITTO_TILES(BF, AC, BI) \
-  if (bf16 == BF && act == AC && (bias != nullptr) == BI) e = w_layout == 1 ? launch_width<BF, AC, BI, true>(p, g.bn, static_cast<int>(ctas), stream) : launch_width<BF, AC, BI, false>(p, g.bn, static_cast<int>(ctas), stream);
+  if (bf16 == BF && act == AC && (bias != nullptr) == BI) e = w_layout == 1 ? launch_cut<BF, AC, BI, true>(p, g, static_cast<int>(ctas), stream) : launch_cut<BF, AC, BI, false>(p, g, static_cast<int>(ctas), stream);
 #define DITTO_TILES_ACTS(BF, BI) DITTO_TILES(BF, 0, BI) DITTO_TILES(BF, 1, BI) DITTO_TILES(BF, 2, BI)
-#ifndef TEST_ONLY
   DITTO_TILES_ACTS(false, false)
   DITTO_TILES_ACTS(false, true)
-#endif
   DITTO_TILES_ACTS(true, false)
   DITTO_TILES_ACTS(true, true)
 #undef DITTO_TILES_ACTS
