@@ -347,11 +347,13 @@ cudaError_t launch_attention_narrow(const AttnParams& p, int batch, bool bf16, i
 // alone: 320 of 1024 28.6 -> 31.3, 384 of 2048 55.7 -> 61.2, 320 of 8192 185 -> 219.  A chain without a softmax has less between the hand-overs:
 // it gains with one or two blocks and many items only (600 x 208 rows and keys 19.4 -> 18.0, 640 of 64 9.4 -> 7.4; 640 of 1024
 // would go 40 -> 43).
+// From three items an SM on it is ahead up to 24 blocks too: 444 x 10 36.7 -> 32.4, 450 x 16 64.5 -> 59.4, 520 x 16 58.9 -> 56.0, 592 x 24 96.4 -> 92.2, 700 x 16 82.4 -> 80.2, 640 x 24
+// 111.9 -> 112.1; just below, and with more blocks, it is not (420 x 10 35.1 -> 37.6, 640 x 64 291 -> 301).
 bool attention_narrow_pays(int batch, int M, int L, int mode) {
   const long long items = static_cast<long long>((M + kBM - 1) / kBM) * batch;
   const int blocks = (L + 127) / 128;
   if (mode != kModeSoftmax) return blocks <= 2 && items > 296;
-  return items > (blocks <= 4 ? 296 : blocks <= 8 ? 349 : 887);
+  return items > (blocks <= 4 ? 296 : blocks <= 8 ? 349 : blocks <= 24 ? 443 : 887);
 }
 
 }  // namespace ditto_b200
