@@ -13,7 +13,7 @@
 // With `parts` CTAs in the cluster each takes a contiguous part of the tile's blocks; they combine (max, sum, O) through
 // distributed shared memory at the end.
 //
-// Two CTAs fit an SM at head dimension 64 (84 KB, 256 tensor-memory columns, 94 registers): the next call's are set up under this
+// Two CTAs fit an SM at head dimension 64 (84 KB, 112 with four parts; 256 tensor-memory columns, 94 registers): the next call's are set up under this
 // one's.  At head dimension 128 (TWO) they do with one stage of K and of V and with P in the place of S (100 KB, 256 columns): a CTA by itself
 // is a chain then -- scores, softmax, P*V, next scores -- and two of them fill each other's gaps; for more items than SMs.  What it measured
 // stands at attention_few.

@@ -26,8 +26,11 @@
 // next is multiplied.  Every epilogue warp turns 32 rows x 64 columns around in 4 KB of shared memory of its own, so
 // that a store instruction writes whole 128-byte rows.
 //
+// Two launches over tiles (mlp_tiles_sm100.cu, mlp_waves_sm100.cu) are the faster form wherever they are possible; this one serves hidden layers
+// of 512 MB and more, first GEMMs of one k-step, results that are not aligned to 32 bytes, and callers who ask for it.
+//
 // What bounds it: the tensor pipe under the power cap for large inputs; the chain first load -> GEMM1 tile -> hidden
-// tile announced -> GEMM2 tile (about 13 us) and tile quantisation for short ones.  Measured, cluster kernel -> this one:
+// tile announced -> GEMM2 tile (about 13 us) and tile quantisation for short ones.  Measured, cluster kernel -> this one (two launches: 214 and 203, 33, 13 and 72):
 //   16384 x 1024 -> 4096 -> 1024        290 -> 238 us sustained (260 -> 204 us for twenty launches)
 //   2048 x 1024 -> 4096 -> 1024         59.7 -> 43 us      512 x 768 -> 3072 -> 768   53.5 -> 28 us (host-bound)
 //   3328 x 1280 -> 5120 -> 1280         216 -> 87 us (no GEMM1 recomputed for a second column group)

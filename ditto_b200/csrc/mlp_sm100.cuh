@@ -16,8 +16,8 @@ namespace ditto_b200 {
 //               N in {512, 1024} ([in, out] weights) or {256, 512, 768, 1024} ([out, in])
 //   kMlpWide    four-CTA clusters, single-SM MMAs, 256-wide hidden chunks (mlp_wide_sm100.cu): L % 256 == 0,
 //               K % 16 == 0, N in {256, 512, 768, 1024}
-//   kMlpFlow    both GEMMs in one launch over 2-SM tiles (mlp_flow_sm100.cu); kMlpAuto takes it, or two launches of
-//               mlp_tiles_sm100.cu, where the caller gives scratch memory
+//   kMlpFlow    both GEMMs in one launch over 2-SM tiles (mlp_flow_sm100.cu); kMlpAuto takes two launches of mlp_tiles_sm100.cu or
+//               mlp_waves_sm100.cu, or where neither fits this one, if the caller gives scratch memory
 enum MlpVariant { kMlpAuto = 0, kMlpQuad = 1, kMlpPair = 2, kMlpWide = 3, kMlpFlow = 4 };
 
 // Returns a DITTO_* status code (0 on success).  act1 / act2: activation after the first / second GEMM

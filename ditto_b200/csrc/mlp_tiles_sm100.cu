@@ -490,7 +490,7 @@ TilesGemm best_gemm(long long blocks, int N, int steps, bool first, double* time
 
 }  // namespace
 
-// Where two launches are the faster form.  The flow kernel's waits cost it about 10 us a call, and it is 20 % faster
+// Where two launches over these tiles are a faster form than the flow kernel (which of them then go to the wave kernel, waves_faster says).  The flow kernel's waits cost it about 10 us a call, and it is 20 % faster
 // per operation once its pairs are busy: measured, flow -> tiles, 16 x 1024 -> 4096 -> 1024 25.9 -> 16.2 us, 512 x 768 23.7 ->
 // 15.2, 2048 x 1024 (34 GFLOP) 42.0 -> 37.0, 4096 x 768 (39) 46.6 -> 43.3, 2560 x 1024 (43) 50.5 -> 51.5; on the other side either is
 // the faster one: 6144 x 768 (58) 53.4 -> 49.0, 4096 x 1024 (69) 60.1 -> 58.5, 1024 x 2048 (69) 64.2 -> 65.7, 16384 x 512 (69) 66.9 ->

@@ -88,13 +88,13 @@ int ditto_b200_multi_head_attention(const void* qkv, void* out, int batch, int M
  *   epilogue 0: identity between the GEMMs; 1: ReLU; | DITTO_EPILOGUE_PAIR_MMA / _QUAD_MMA / _WIDE_MMA / _FLOW_MMA
  *   forces one of the kernels (same results up to fp32 summation order; default: by shape)
  *   workspace / ws_bytes: optional scratch memory (ditto_b200_workspace_bytes; contents irrelevant on entry,
- *   undefined on return).  With it calls up to about 48 GFLOP, and batch entries of up to 128 rows, keep the whole
- *   hidden layer there between two launches; larger calls pass it through a ring of row blocks between the tiles
- *   of the two GEMMs, behind a launch that clears the ring's counters.  The ring holds the row blocks that are on
- *   their way: at most 64 MB up to a hidden size of about 5000, more where a row block is longer or the other widths are
- *   small (96 MB for 1024 -> 8192 -> 1024, 512 MB for 2048 -> 65536 -> 2048), never more than the hidden layer.  Where
- *   batch entries of few rows make another form the faster one, and when a cluster kernel is forced, it is used to
- *   share row blocks between clusters.  NULL or too small: the hidden activations stay inside a cluster, one cluster
+ *   undefined on return).  With it calls keep the whole hidden layer there between two launches, up to 512 MB of it; larger
+ *   hidden layers, and with K < 128 or a `y` or workspace that is not aligned to 32 bytes calls of more than about 48 GFLOP, pass through a
+ *   ring of row blocks between the tiles of the two GEMMs, behind a launch that clears the ring's counters.  The ring holds the row
+ *   blocks that are on their way: at most 64 MB up to a hidden size of about 5000, more where a row block is longer or the other
+ *   widths are small (512 MB for 2048 -> 65536 -> 2048), never more than the hidden layer.  Where batch entries of few rows make
+ *   another form the faster one, and when a cluster kernel is forced, it is used to share row blocks between clusters.  Enough for the
+ *   ring alone: the ring.  NULL or too small: the hidden activations stay inside a cluster, one cluster
  *   per row block, in one launch for up to 1024 result columns: 1.2 to 3 times the time, more for wider results.
  * Shapes: N <= 128 and K <= 128 (any multiples of 16, either weight layout): the reference's own shape family;
  * otherwise L % 128 == 0, K % 64 == 0, N in {256, 512, 768, 1024}, or -- on the default kernel -- L % 64 == 0,
@@ -161,9 +161,10 @@ size_t ditto_b200_workspace_bytes(int op, int batch, int M, int N, int K, int L,
  * sized by the hardware table of python/ditto/hardware/__init__.py:43-54). */
 int ditto_b200_mlp_cluster_slots(int dtype, int variant);
 
-/* How a call of the MLP chain with scratch memory that runs as two launches over tiles cuts its GEMM 1 or 2 (`gemm`): tiles
+/* How a call of the MLP chain with scratch memory that runs as two launches over tiles of one SM cuts its GEMM 1 or 2 (`gemm`): tiles
  * of 128 rows x cut[0] columns, each by a cluster of cut[1] CTAs that divide the reduction, cut[2] CTAs an SM.  Sums of
- * a reduction that is not divided (cut[1] == 1) have the bits that the call has without scratch memory.
+ * a reduction that is not divided (cut[1] == 1) have the bits that the call has without scratch memory.  (Larger calls take tiles of two SMs, which
+ * divide no reduction; what is written here then holds for a `y` that is not aligned to 32 bytes.)
  * Needs no GPU.  No counterpart in the reference. */
 int ditto_b200_mlp_tiles_cut(int gemm, int batch, int M, int N, int K, int L, int* cut);
 

@@ -90,6 +90,23 @@ def test_results_aligned_to_16_bytes_alone(cuda, shape, form):
     assert form in _widths(lambda: ops.gemm_relu_gemm(x, w1, w2, out=out))
 
 
+# cuts of the tile kernel that only calls have which else take the wave kernel: 256 columns for GEMM1, whole and in two parts, 192 of few tiles for GEMM2
+@pytest.mark.parametrize("shape", [(1, 2064, 1024, 1024, 4096), (1, 2352, 768, 256, 3136), (1, 1376, 512, 8000, 1472), (1, 4096, 768, 768, 3072)])
+@pytest.mark.parametrize("layout", ["IO", "OI"])
+def test_tile_kernel_for_results_aligned_to_16_bytes_alone(cuda, shape, layout):
+    batch, M, N, K, L = shape
+    g, x, w1, w2, given = _operands(cuda, *shape, torch.bfloat16, layout, 54)
+    out = torch.full((batch * M * N + 16,), float("nan"), dtype=torch.bfloat16, device=cuda)[8:8 + batch * M * N].view(batch, M, N)
+    ops.gemm_relu_gemm(x, *given, out=out, weight_layout=layout)
+    ref = torch.relu(x.float() @ w1.float()).to(torch.bfloat16).float() @ w2.float()
+    _assert_close(out, ref, torch.bfloat16, shape, cuda)
+    assert set(_widths(lambda: ops.gemm_relu_gemm(x, *given, out=out, weight_layout=layout))) == {"mlp_tiles_kernel"}
+    b1, b2 = (torch.randn(batch, n, device=cuda, generator=g).to(torch.bfloat16) for n in (L, N))
+    ops.ffn(x, given[0], b1, given[1], b2, out=out, act1="gelu", act2="identity", weight_layout=layout)
+    h = _act(x.float() @ w1.float() + b1.float().view(batch, 1, L), "gelu").to(torch.bfloat16)
+    _assert_close(out, h.float() @ w2.float() + b2.float().view(batch, 1, N), torch.bfloat16, ("ffn",) + shape, cuda)
+
+
 def test_wave_kernel_streams_and_changed_weights(cuda):
     """The second launch reads its weights ahead of the first one's end: a weight written by the work just ahead in the
     stream is the one that is used, and calls on two streams have hidden layers of their own."""
