@@ -35,6 +35,8 @@ constexpr int kOffK = kOffQ + kTileQ;     // two stages each
 constexpr int kOffV = kOffK + 2 * kTileKV;
 constexpr int kOffBar = kOffV + 2 * kTileKV;
 constexpr int kSmemBytes = kOffBar + 128 + 1024;
+// For as many items as three CTAs an SM take (an SM's 228 KB hold one KB more a CTA), see launch_n.
+constexpr int kSmemBytesThree = 75 * 1024;
 constexpr int kThreads = 160;
 constexpr uint32_t kTmemCols = 128;
 constexpr uint32_t kColO = 64;
@@ -311,7 +313,7 @@ static cudaError_t launch_n(const AttnParams& p, long long items, cudaStream_t s
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
   if (!((configured.load(std::memory_order_acquire) >> dev) & 1ull)) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytesThree);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
@@ -320,7 +322,11 @@ static cudaError_t launch_n(const AttnParams& p, long long items, cudaStream_t s
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(items), 1, 1);
   cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.dynamicSmemBytes = kSmemBytes;
+  // Up to three items an SM: no place for a fourth.  The CTAs of a call go to the places that the call before it leaves free, while that one still runs (the
+  // launch is programmatic): with four an SM they end up four on some SMs and two on others, and the call lasts as long as one of 592
+  // items.  us, four places -> three, calls one after another: 300 items of 128 / 512 / 1024 keys 7.0 -> 6.3, 16.6 -> 14.3, 29.1 -> 25.1, 384 of 512 17.5 -> 14.4,
+  // 444 of 512 17.0 -> 14.7; behind another kernel the placing is even and nothing changes (17.1 -> 17.0).
+  cfg.dynamicSmemBytes = items > 296 && items <= 444 ? kSmemBytesThree : kSmemBytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see grid_dependency_wait in the kernel
@@ -339,21 +345,20 @@ cudaError_t launch_attention_narrow(const AttnParams& p, int batch, bool bf16, i
 }
 
 // Where the lines lie: calls of up to 296 items have other forms (attention_few: of up to four 128-key blocks, and of any number up to 148 items;
-// those between are not long enough for this one, 200 x 5 blocks 13.8 -> 14.0, 200 x 8 18.6 -> 19.9).  Above, it is the faster form up to four
-// 128-key blocks an item, up to eight with a half-full wave more than the other kernels hold at once; for longer items the other
-// kernels' 128-key blocks cost less (1.6 us for two a SM against 2 x 1.0), and it pays again once a launch is three waves of those
-// or more.  Measured, us, others -> this kernel: 2048 items of 512 keys 83.8 -> 69.2; 1200 of 208 30.6 -> 27.0; 1000 of 128
-// 16.6 -> 13.8; 640 of 64 13.0 -> 8.2; 384 of 512 19.5 -> 17.4; 400 of 1024 35.9 -> 31.4; 1024 of 8192 398 -> 384; 900 of 768 53.5 -> 48.1; and left
-// alone: 320 of 1024 28.6 -> 31.3, 384 of 2048 55.7 -> 61.2, 320 of 8192 185 -> 219.  A chain without a softmax has less between the hand-overs:
-// it gains with one or two blocks and many items only (600 x 208 rows and keys 19.4 -> 18.0, 640 of 64 9.4 -> 7.4; 640 of 1024
-// would go 40 -> 43).
-// From three items an SM on it is ahead up to 24 blocks too: 444 x 10 36.7 -> 32.4, 450 x 16 64.5 -> 59.4, 520 x 16 58.9 -> 56.0, 592 x 24 96.4 -> 92.2, 700 x 16 82.4 -> 80.2, 640 x 24
-// 111.9 -> 112.1; just below, and with more blocks, it is not (420 x 10 35.1 -> 37.6, 640 x 64 291 -> 301).
+// those between are not long enough for this one, 200 x 5 blocks 13.8 -> 14.0, 200 x 8 18.6 -> 19.9).  With three items an SM and no place for a fourth this is the
+// faster form for all numbers of blocks, with a softmax and without; us, others -> this kernel: softmax, 300 items of 5, 8, 16, 64 blocks 19.0 -> 17.2, 27.5 -> 25.5, 49.1 -> 46.7,
+// 173.7 -> 171.1, 384 22.8 -> 17.6, 31.9 -> 26.3, 50.4 -> 46.9, 175.5 -> 170.8, 444 25.1 -> 18.8, 34.7 -> 26.2, 51.3 -> 46.8, 200 -> 194; chains, 300 items of 1, 4, 8, 32 blocks
+// 6.4 -> 5.0, 12.2 -> 10.3, 20.1 -> 17.8, 62.0 -> 60.4, 444 7.5 -> 5.6, 14.0 -> 11.2, 23.5 -> 18.9, 71.1 -> 66.9.  (With a fourth place, 300 x 16 53.8 and 384 x 32 106.7 against
+// 91.4 of the others.)  Above, it is ahead up to 24 blocks: 450 x 16 64.5 -> 59.4, 520 x 16 58.9 -> 56.0, 592 x 24 96.4 -> 92.2, 700 x 16 82.4 -> 80.2, 640 x 24
+// 111.9 -> 112.1, 2048 x 4 83.8 -> 69.2, 1200 of 208 keys 30.6 -> 27.0, 640 of 64 13.0 -> 8.2; for longer items the other
+// kernels' 128-key blocks cost less (1.6 us for two a SM against 2 x 1.0; 640 x 64 291 -> 301), and it pays again once a launch is three waves of those
+// or more: 1024 x 64 398 -> 384.  A chain without a softmax has less between the hand-overs: there
+// it gains with one or two blocks only (600 x 208 rows and keys 19.4 -> 18.0, 640 of 64 9.4 -> 7.4; 640 of 1024 would go 40 -> 43).
 bool attention_narrow_pays(int batch, int M, int L, int mode) {
   const long long items = static_cast<long long>((M + kBM - 1) / kBM) * batch;
   const int blocks = (L + 127) / 128;
-  if (mode != kModeSoftmax) return blocks <= 2 && items > 296;
-  return items > (blocks <= 4 ? 296 : blocks <= 8 ? 349 : blocks <= 24 ? 443 : 887);
+  if (items <= 444) return items > 296;
+  return mode != kModeSoftmax ? blocks <= 2 : blocks <= 24 || items > 887;
 }
 
 }  // namespace ditto_b200
