@@ -15,6 +15,8 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libditto_b200.so")
 SOURCES = ["api.cu", "host_util.cu", "attention_sm100.cu", "attention_persistent_sm100.cu", "attention_narrow_sm100.cu", "attention_short_sm100.cu", "mlp_sm100.cu", "mlp_wide_sm100.cu", "mlp_pair_sm100.cu", "mlp_flow_sm100.cu", "mlp_tiles_sm100.cu", "mlp_waves_sm100.cu", "selftest_sm100.cu"]
+# sources that are compiled in parts, an object and a GPU module each: (file, macro, number of parts)
+IN_PARTS = [("mlp_tiles_kernel_sm100.cu", "DITTO_TILES_PART", 8)]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "--use_fast_math",
@@ -63,9 +65,11 @@ def build(force=False, verbose=False):
     os.makedirs(LIB_DIR, exist_ok=True)
     objs = []
     procs = []
-    for src in SOURCES:
-        obj = os.path.join(LIB_DIR, src.replace(".cu", ".o"))
-        cmd = [_nvcc(), *NVCC_FLAGS, "-c", os.path.join(CSRC, src), "-o", obj]
+    units = [(src, src.replace(".cu", ".o"), []) for src in SOURCES]
+    units += [(src, src.replace(".cu", f"_{i}.o"), [f"-D{macro}={i}"]) for src, macro, n in IN_PARTS for i in range(n)]
+    for src, name, defines in units:
+        obj = os.path.join(LIB_DIR, name)
+        cmd = [_nvcc(), *NVCC_FLAGS, *defines, "-c", os.path.join(CSRC, src), "-o", obj]
         if verbose:
             cmd.insert(1, "-Xptxas=-v")
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
