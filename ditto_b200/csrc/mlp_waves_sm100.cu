@@ -156,7 +156,7 @@ constexpr int kGroup = 8;
 struct Tile { int rb, n, b, row; };      // row block, column of tiles, batch entry, first row in it
 __device__ __forceinline__ Tile tile_at(const WavesParams& p, int t) {
   const int per = p.per_group, g = t / per, r = t - g * per;
-  const int gs = min(kGroup, p.blocks - g * kGroup);
+  const int gs = max(1, min(kGroup, p.blocks - g * kGroup));    // (the loops work out one tile past the end, in a group that may be empty)
   Tile x;
   x.n = r / gs;
   x.rb = g * kGroup + r - x.n * gs;
