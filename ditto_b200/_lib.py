@@ -20,6 +20,7 @@ DTYPE_FP16 = 0
 DTYPE_BF16 = 1
 OP_BMM_SOFTMAX_BMM = 0
 OP_GEMM_RELU_GEMM = 1
+OP_LESS_SCRATCH = 0x2000
 FLAG_P_VIA_SMEM = 1
 FLAG_ONE_TILE = 2
 FLAG_TWO_TILES = 4

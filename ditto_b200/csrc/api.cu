@@ -308,6 +308,8 @@ size_t ditto_b200_workspace_bytes(int op, int batch, int M, int N, int K, int L,
                       : (op & DITTO_EPILOGUE_WIDE_MMA) ? ditto_b200::kMlpWide
                       : (op & DITTO_EPILOGUE_FLOW_MMA) ? ditto_b200::kMlpFlow
                                                        : ditto_b200::kMlpAuto;
+  if (op & DITTO_OP_LESS_SCRATCH)
+    return variant == ditto_b200::kMlpAuto ? ditto_b200::mlp_less_workspace_bytes(batch, M, N, K, L, dtype == DITTO_DTYPE_BF16) : 0;
   size_t a = ditto_b200::mlp_workspace_bytes(batch, M, N, K, L, dtype == DITTO_DTYPE_BF16, 0, variant);
   size_t b = ditto_b200::mlp_workspace_bytes(batch, M, N, K, L, dtype == DITTO_DTYPE_BF16, 1, variant);
   return a > b ? a : b;

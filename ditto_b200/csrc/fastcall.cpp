@@ -40,7 +40,7 @@ BytesFn g_bytes = nullptr;
 constexpr int kDevices = 64;
 int* g_status[kDevices] = {};       // device status words, registered by ops.py
 
-constexpr int kOpGemmReluGemm = 1;
+constexpr int kOpGemmReluGemm = 1, kOpLessScratch = 0x2000;
 
 // What all tensors of a call have in common.
 struct Common {
@@ -251,16 +251,19 @@ struct ChainShape {
   operator at::IntArrayRef() const { return flat ? at::IntArrayRef(d + 1, 2) : at::IntArrayRef(d, 3); }
 };
 // Scratch memory of a call, in stream order from the caching allocator: its own for every stream, thread and captured graph.
-// None where there is no memory left for it: the call then takes the form that needs none.
+// Where there is no memory left for the whole hidden layer of a large call, the ring of the next best form; none where there is
+// none for that: the call then takes the form that needs none.
 at::Tensor scratch_for(const Common& c, int64_t b, int64_t M, int64_t N, int64_t K, int64_t L, size_t* bytes) {
-  *bytes = g_bytes(kOpGemmReluGemm, b, M, N, K, L, c.code);
-  if (*bytes == 0) return at::Tensor();
-  try {
-    return make({static_cast<int64_t>(*bytes)}, at::kByte, c.device);
-  } catch (const c10::OutOfMemoryError&) {
-    *bytes = 0;
-    return at::Tensor();
+  for (const int op : {kOpGemmReluGemm, kOpGemmReluGemm | kOpLessScratch}) {
+    *bytes = g_bytes(op, b, M, N, K, L, c.code);
+    if (*bytes == 0) break;
+    try {
+      return make({static_cast<int64_t>(*bytes)}, at::kByte, c.device);
+    } catch (const c10::OutOfMemoryError&) {
+      *bytes = 0;
+    }
   }
+  return at::Tensor();
 }
 
 // gemm(x, w1, w2, out, activation, weight_layout, scratch)

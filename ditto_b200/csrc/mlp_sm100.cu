@@ -784,6 +784,12 @@ size_t mlp_workspace_bytes(int batch, int M, int N, int K, int L, bool bf16, int
   }
 }
 
+size_t mlp_less_workspace_bytes(int batch, int M, int N, int K, int L, bool bf16) {
+  if (form_with_scratch(batch, M, N, K, L, bf16) != kFormFlow || !waves_faster(batch, M, N, K, L, kFormFlow)) return 0;
+  const size_t ring = mlp_workspace_bytes(batch, M, N, K, L, bf16, 0, kMlpFlow);
+  return ring < mlp_tiles_workspace_bytes(batch, M, L) ? ring : 0;
+}
+
 int launch_mlp_chain(const void* x, const void* w1, const void* w2, void* y, int batch, int M, int N, int K, int L,
                      bool bf16, int w_layout, int act1, int act2, const void* b1, const void* b2, int variant,
                      void* workspace, size_t ws_bytes, int* status, cudaStream_t stream, long long* trace) {

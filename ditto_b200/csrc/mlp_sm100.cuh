@@ -30,6 +30,8 @@ int launch_mlp_chain(const void* x, const void* w1, const void* w2, void* y, int
 
 // Scratch bytes with which the chain runs fastest at this shape on the current device (0: none needed).
 size_t mlp_workspace_bytes(int batch, int M, int N, int K, int L, bool bf16, int w_layout, int variant);
+// The ring that is enough for the flow kernel, of a call that with all of the scratch memory takes the wave kernel; 0 if that is no less.
+size_t mlp_less_workspace_bytes(int batch, int M, int N, int K, int L, bool bf16);
 
 // The four-CTA kernel with the library's own scratch array in place of a caller-provided workspace
 // (see ditto_b200_gemm_relu_gemm_static_scratch).  Allocates nothing.

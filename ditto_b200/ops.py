@@ -219,16 +219,19 @@ _VARIANT_BITS = {"auto": 0, "pair": 0x200, "quad": 0x400, "wide": 0x800, "flow":
 def _scratch(lib, op, batch, M, N, K, L, dtype, device):
     """(tensor, pointer, bytes) of the scratch memory a call runs fastest with (the C ABI itself allocates nothing).
     Taken from the caching allocator per call: in stream order, so calls on several streams and threads and
-    captured graphs each have their own.  Where there is no memory left for it the call goes without: the kernels
+    captured graphs each have their own.  Where there is no memory left for the whole hidden layer of a large call it takes
+    the ring that serves the next best kernel, and where there is none for that either it goes without: the kernels
     that keep the hidden layer inside a cluster need none."""
-    need = lib.ditto_b200_workspace_bytes(op, batch, M, N, K, L, _DTYPE_CODE[dtype])
-    if not need:
-        return None, None, 0
-    try:
-        buf = torch.empty(need, dtype=torch.uint8, device=device)
-    except torch.OutOfMemoryError:
-        return None, None, 0
-    return buf, buf.data_ptr(), need
+    for less in (0, _lib.OP_LESS_SCRATCH):
+        need = lib.ditto_b200_workspace_bytes(op | less, batch, M, N, K, L, _DTYPE_CODE[dtype])
+        if not need:
+            break
+        try:
+            buf = torch.empty(need, dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:
+            continue
+        return buf, buf.data_ptr(), need
+    return None, None, 0
 
 
 def gemm_relu_gemm(x, w1, w2, out=None, activation="relu", weight_layout="IO", variant="auto", workspace="auto"):

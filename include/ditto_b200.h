@@ -45,6 +45,7 @@ extern "C" {
 
 #define DITTO_OP_BMM_SOFTMAX_BMM 0
 #define DITTO_OP_GEMM_RELU_GEMM 1
+#define DITTO_OP_LESS_SCRATCH 0x2000 /* or-ed with the op for ditto_b200_workspace_bytes: the size to try where there is no memory for the full one */
 
 /* flags of ditto_b200_bmm_softmax_bmm */
 #define DITTO_FLAG_P_VIA_SMEM 1   /* stage the probabilities through shared memory instead of TMEM */
@@ -149,7 +150,8 @@ int ditto_b200_ffn_ws(const void* x, const void* w1, const void* b1, const void*
 
 /* Scratch bytes with which the op runs fastest at this shape on the current device (0 when none; every call
  * also works without).  `op` may be or-ed with DITTO_EPILOGUE_PAIR_MMA / _QUAD_MMA / _WIDE_MMA / _FLOW_MMA to ask for the
- * kernel that the same bits in `epilogue` select. */
+ * kernel that the same bits in `epilogue` select, or with DITTO_OP_LESS_SCRATCH: the ring of a call that would else keep its whole
+ * hidden layer in scratch memory, 0 where there is no such size below the full one. */
 size_t ditto_b200_workspace_bytes(int op, int batch, int M, int N, int K, int L, int dtype);
 
 /* How many thread-block clusters of the MLP chain kernel the current device holds at once
