@@ -16,7 +16,7 @@ LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libditto_b200.so")
 SOURCES = ["api.cu", "host_util.cu", "attention_sm100.cu", "attention_persistent_sm100.cu", "attention_narrow_sm100.cu", "attention_short_sm100.cu", "mlp_sm100.cu", "mlp_wide_sm100.cu", "mlp_pair_sm100.cu", "mlp_flow_sm100.cu", "mlp_tiles_sm100.cu", "mlp_waves_sm100.cu", "selftest_sm100.cu"]
 # sources that are compiled in parts, an object and a GPU module each: (file, macro, number of parts)
-IN_PARTS = [("mlp_tiles_kernel_sm100.cu", "DITTO_TILES_PART", 8)]
+IN_PARTS = [("mlp_tiles_kernel_sm100.cu", "DITTO_TILES_PART", 8), ("mlp_waves_kernel_sm100.cu", "DITTO_WAVES_PART", 8)]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "--use_fast_math",

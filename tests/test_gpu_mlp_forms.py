@@ -18,13 +18,13 @@ pytestmark = pytest.mark.gpu
 TILES, WAVES, FLOW = ["mlp_tiles_kernel"] * 2, ["mlp_waves_kernel"] * 2, ["mlp_flow_reset_kernel", "mlp_flow_kernel"]
 
 
-def _kernels(call):
-    """The kernels that a call launches, in order of launch."""
+def _kernels(call, sizes=None):
+    """The kernels that a call launches, in order of launch (and in `sizes` how many kernels the module of each holds)."""
     call()
     graph = torch.cuda.CUDAGraph(keep_graph=True)
     with torch.cuda.graph(graph):
         call()
-    cuda, names = ctypes.CDLL("libcuda.so.1"), []
+    cuda, names, module, held = ctypes.CDLL("libcuda.so.1"), [], ctypes.c_void_p(), ctypes.c_uint(0)
     handle, count = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(0)
     assert cuda.cuGraphGetNodes(handle, None, ctypes.byref(count)) == 0
     nodes = (ctypes.c_void_p * count.value)()
@@ -34,8 +34,16 @@ def _kernels(call):
         assert cuda.cuGraphKernelNodeGetParams_v2(ctypes.c_void_p(node), ctypes.byref(params)) == 0
         if params.func:
             assert cuda.cuFuncGetName(ctypes.byref(name), ctypes.c_void_p(params.func)) == 0
+            if sizes is not None:
+                assert cuda.cuFuncGetModule(ctypes.byref(module), ctypes.c_void_p(params.func)) == 0
+                assert cuda.cuModuleGetFunctionCount(ctypes.byref(held), module) == 0
         else:
             assert cuda.cuKernelGetName(ctypes.byref(name), ctypes.c_void_p(params.kernel)) == 0
+            if sizes is not None:
+                assert cuda.cuKernelGetLibrary(ctypes.byref(module), ctypes.c_void_p(params.kernel)) == 0
+                assert cuda.cuLibraryGetKernelCount(ctypes.byref(held), module) == 0
+        if sizes is not None:
+            sizes.append(held.value)
         names.append(re.search(r"\d(mlp_\w*?kernel)", name.value.decode()).group(1))
     return names
 
@@ -123,3 +131,13 @@ def test_a_workspace_with_room_for_the_ring_alone(cuda, dtype):
         got.append(ops.gemm_relu_gemm(x, w1, w2, workspace=ws))
     assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
     _assert_close(got[2], torch.relu(x.float() @ w1.float()).to(dtype).float() @ w2.float(), dtype, shape, cuda)
+
+
+@pytest.mark.parametrize("shape,kernels,most", [((1, 4096, 768, 768, 3072), WAVES, 9), ((1, 512, 768, 768, 3072), TILES, 60)])
+def test_a_first_call_loads_no_more_than_its_form(cuda, shape, kernels, most):
+    """A program's first call loads the module of its kernels: the instances are compiled by type, layout and bias, a module each."""
+    _, x, w1, w2 = tiles._operands(cuda, *shape, torch.bfloat16, 65)
+    out = torch.empty(shape[:3], dtype=torch.bfloat16, device=cuda)
+    sizes = []
+    assert _kernels(lambda: ops.gemm_relu_gemm(x, w1, w2, out=out), sizes) == kernels
+    assert len(sizes) == 2 and max(sizes) <= most, sizes

@@ -6,7 +6,7 @@ import subprocess
 
 import pytest
 
-SOURCE = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "ditto_b200", "csrc", "mlp_waves_sm100.cu")
+SOURCE = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "ditto_b200", "csrc", "mlp_waves_kernel_sm100.cu")
 
 MAIN = r"""
 int main(int argc, char** argv) {
@@ -35,10 +35,10 @@ int main(int argc, char** argv) {
 @pytest.fixture(scope="module")
 def program(tmp_path_factory):
     text = open(SOURCE).read()
-    code = re.search(r"constexpr int kGroup.*?\n(?=\}  // namespace)", text, re.S).group(0)
+    code = re.search(r"struct Tile \{.*?\n(?=\}  // namespace)", text, re.S).group(0)
     assert "Tile tile_at(const WavesParams& p, int t)" in code
     path = tmp_path_factory.mktemp("order")
-    (path / "order.cpp").write_text("#include <algorithm>\n#include <cstdlib>\n#include <vector>\nusing std::max;\nusing std::min;\n#define __device__\n#define __forceinline__ inline\n"
+    (path / "order.cpp").write_text("#include <algorithm>\n#include <cstdlib>\n#include <vector>\nusing std::max;\nusing std::min;\n#define __device__\n#define __forceinline__ inline\nconstexpr int kGroup = 8;\n"
                                     "struct WavesParams { int blocks_per_batch, blocks, tiles, per_group, second; };\n" + code + MAIN)
     subprocess.run(["g++", "-std=c++17", "-O0", str(path / "order.cpp"), "-o", str(path / "order")], check=True)
     return str(path / "order")
