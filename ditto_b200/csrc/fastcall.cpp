@@ -13,10 +13,13 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <climits>
 #include <cstring>
 #include <initializer_list>
@@ -250,6 +253,35 @@ struct ChainShape {
   explicit ChainShape(const Chain& r) : d{r.b, r.M, r.N}, flat(r.flat) {}
   operator at::IntArrayRef() const { return flat ? at::IntArrayRef(d + 1, 2) : at::IntArrayRef(d, 3); }
 };
+// Whether the caching allocator can be expected to have `bytes` more in one piece: cached, or free on the device and within the process's share.
+// Asked before a large request, because one that fails is dear: the allocator gives all its cached blocks back first, waiting for the device
+// (16384 x 1024 -> 4096 -> 1024 with 100 MB left and no such question: 1073 us a call, 209 with it).
+// An allocator that cannot tell is asked for the memory itself.
+bool room_for(int device, size_t bytes) {
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return true;
+  try {
+    const auto index = static_cast<c10::DeviceIndex>(device);
+    size_t largest = 1;                            // (0 would ask the device)
+    c10::cuda::CUDACachingAllocator::cacheInfo(index, &largest);
+    if (largest >= bytes) return true;
+    // what the allocator can give back: cached segments of which no part is in use
+    const auto s = c10::cuda::CUDACachingAllocator::getDeviceStats(index);
+    const size_t reserved = static_cast<size_t>(s.reserved_bytes[0].current);
+    const size_t whole = reserved - static_cast<size_t>(s.allocated_bytes[0].current) - static_cast<size_t>(s.inactive_split_bytes[0].current);
+    size_t free = 0, total = 0;
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+      cudaGetLastError();
+      return true;
+    }
+    const double share = c10::cuda::CUDACachingAllocator::getMemoryFraction(index) * static_cast<double>(total);
+    const size_t allowed = share > static_cast<double>(reserved) ? static_cast<size_t>(share) - reserved : 0;
+    return whole + std::min(free, allowed) >= bytes;
+  } catch (const std::exception&) {
+    return true;
+  }
+}
+constexpr size_t kLargeScratch = 48u << 20;      // (what the question costs counts in small calls)
+
 // Scratch memory of a call, in stream order from the caching allocator: its own for every stream, thread and captured graph.
 // Where there is no memory left for the whole hidden layer of a large call, the ring of the next best form; none where there is
 // none for that: the call then takes the form that needs none.
@@ -257,11 +289,13 @@ at::Tensor scratch_for(const Common& c, int64_t b, int64_t M, int64_t N, int64_t
   for (const int op : {kOpGemmReluGemm, kOpGemmReluGemm | kOpLessScratch}) {
     *bytes = g_bytes(op, b, M, N, K, L, c.code);
     if (*bytes == 0) break;
-    try {
-      return make({static_cast<int64_t>(*bytes)}, at::kByte, c.device);
-    } catch (const c10::OutOfMemoryError&) {
-      *bytes = 0;
+    if (*bytes <= kLargeScratch || room_for(c.device, *bytes)) {
+      try {
+        return make({static_cast<int64_t>(*bytes)}, at::kByte, c.device);
+      } catch (const c10::OutOfMemoryError&) {
+      }
     }
+    *bytes = 0;
   }
   return at::Tensor();
 }

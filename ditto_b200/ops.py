@@ -216,6 +216,28 @@ def multi_head_attention(qkv, num_heads, out=None, scale=1.0, flags=0):
 _VARIANT_BITS = {"auto": 0, "pair": 0x200, "quad": 0x400, "wide": 0x800, "flow": 0x1000}
 
 
+_LARGE_SCRATCH = 48 << 20       # (what the question costs counts in small calls)
+
+
+def _room_for(need, device):
+    """Whether the caching allocator can be expected to have `need` bytes more: cached, or free on the device and within the process's
+    share.  Asked before a large request, because for one that fails the allocator first gives all its cached blocks back, waiting for the
+    device.  An allocator that cannot tell is asked for the memory itself."""
+    if torch.cuda.is_current_stream_capturing():
+        return True
+    try:
+        stats = torch.cuda.memory_stats(device)
+        reserved, parts = stats["reserved_bytes.all.current"], stats["inactive_split_bytes.all.current"]
+        whole = reserved - stats["allocated_bytes.all.current"] - parts        # (what the allocator can give back)
+        if max(whole, parts) >= need:
+            return True
+        free, total = torch.cuda.mem_get_info(device)
+        allowed = int(torch.cuda.get_per_process_memory_fraction(device) * total) - reserved
+    except (RuntimeError, KeyError):
+        return True
+    return whole + min(free, max(allowed, 0)) >= need
+
+
 def _scratch(lib, op, batch, M, N, K, L, dtype, device):
     """(tensor, pointer, bytes) of the scratch memory a call runs fastest with (the C ABI itself allocates nothing).
     Taken from the caching allocator per call: in stream order, so calls on several streams and threads and
@@ -226,6 +248,8 @@ def _scratch(lib, op, batch, M, N, K, L, dtype, device):
         need = lib.ditto_b200_workspace_bytes(op | less, batch, M, N, K, L, _DTYPE_CODE[dtype])
         if not need:
             break
+        if need > _LARGE_SCRATCH and not _room_for(need, device):
+            continue
         try:
             buf = torch.empty(need, dtype=torch.uint8, device=device)
         except torch.OutOfMemoryError:

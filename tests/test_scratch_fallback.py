@@ -56,8 +56,8 @@ def test_less_scratch_is_the_ring(cuda):
 
 @pytest.mark.gpu
 def test_large_calls_take_the_ring_where_memory_is_short(cuda):
-    """On the native and on the checked path, with room for the ring and not for the hidden layer: the ring is what is asked for (seen by the
-    allocator's peak), and the result is that of a caller's workspace of that size."""
+    """On the native and on the checked path, with room for the ring and not for the hidden layer: the ring is what is taken (the
+    allocator counts it), and the result is that of a caller's workspace of that size."""
     x, w1, b1, w2 = _operands(cuda)
     need = _lib.load().ditto_b200_workspace_bytes
     full, ring = need(_lib.OP_GEMM_RELU_GEMM, *SHAPE, 0), need(_lib.OP_GEMM_RELU_GEMM | _lib.EPILOGUE_FLOW_MMA, *SHAPE, 0)
@@ -67,7 +67,7 @@ def test_large_calls_take_the_ring_where_memory_is_short(cuda):
     out, block = torch.empty_like(want), torch.empty_like(want)
     fast, total = ops._fast, torch.cuda.get_device_properties(cuda).total_memory
     assert fast is not None
-    peaks = []
+    taken = []
     try:
         for path in (fast, None):
             ops._fast = path
@@ -76,10 +76,13 @@ def test_large_calls_take_the_ring_where_memory_is_short(cuda):
                 torch.cuda.synchronize()
                 torch.cuda.empty_cache()
                 torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + ring + (24 << 20)) / total)
-                torch.cuda.reset_peak_memory_stats()
-                held = torch.cuda.memory_allocated()
+                before = torch.cuda.memory_stats()
                 call()
-                peaks.append(torch.cuda.max_memory_allocated() - held)
+                call()
+                after = torch.cuda.memory_stats()
+                taken.append(after["allocated_bytes.all.allocated"] - before["allocated_bytes.all.allocated"])
+                # no request failed: the allocator would have given its cached blocks back, waiting for the device, in every call
+                assert (after["num_ooms"], after["num_alloc_retries"]) == (before["num_ooms"], before["num_alloc_retries"])
             assert torch.equal(out, want)
             h = torch.relu(x[:4096].float() @ w1.float() + b1.float()).half().float()
             torch.testing.assert_close(block[:4096].float(), h @ w2.float(), rtol=2 ** -9, atol=2e-3)
@@ -88,4 +91,4 @@ def test_large_calls_take_the_ring_where_memory_is_short(cuda):
         ops._fast = fast
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert ops.device_status(cuda) == 0
-    assert all(ring <= p < ring + (4 << 20) for p in peaks), (ring, full, peaks)
+    assert all(2 * ring <= n < 2 * ring + (8 << 20) for n in taken), (ring, full, taken)
