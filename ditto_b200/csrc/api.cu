@@ -62,7 +62,7 @@ cudaError_t launch_attention_form(const ditto_b200::AttnParams& p, int slices, i
     const int asked = (flags & DITTO_FLAG_SPLIT_MASK) / DITTO_FLAG_SPLIT_UNIT, blocks = (p.L + 127) / 128;
     ditto_b200::AttnFew few = {1, false, false};
     if (asked == 0 && !(flags & DITTO_FLAG_FEW)) {
-      few = ditto_b200::attention_few(slices, p.M, p.L, d, mode);
+      few = ditto_b200::attention_few(slices, p.M, p.L, d, p.d + p.dv, mode);
     } else {
       if (asked > 1) few.parts = 1 << (asked - 1);
       while (few.parts > blocks) few.parts /= 2;

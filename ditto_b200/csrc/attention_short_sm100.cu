@@ -727,21 +727,34 @@ bool by_row(int parts, int own, int m, bool shared) { return own >= (parts == 8 
 // More than 148 items at head dimension 128: two CTAs an SM, each with a K and a V stage and P in the place of S, work beside each other, where the kernel
 // with two tiles a CTA needs two tiles of one sequence.  One tile a sequence, us, before -> now: 150 x 4 17.7 -> 13.3, 296 x 1 9.0 -> 6.9, 450 x 8 61.3 -> 52.2, 600 x 3 38.4
 // -> 35.9, 1000 x 8 136 -> 113, 2000 x 4 144 -> 116, without a softmax 150 x 4 14.0 -> 10.2, 600 x 4 46.5 -> 39.2; many items of one or two blocks are bound by what
-// is loaded, which the other kernel asks for an item ahead (1000 x 1 28.9 -> 31.3, x 2 41.9 -> 43.7).  More tiles a sequence, up to 296 items: 296 x 1 8.0 -> 6.6, x 4 15.0 -> 14.0,
-// with a softmax only as long as there are few blocks (160 x 8 21.1 -> 22.9, 150 x 16 35.9 -> 38.4; of 208 or 256 rows, 80 wide, x 4 12.4 -> 12.9; at worst x 2 of 208
-// keys 9.15 -> 9.40), without one always (150 x 64 122 -> 111); more items without a softmax
+// is loaded, which the other kernel asks for an item ahead (1000 x 1 28.9 -> 31.3, x 2 41.9 -> 43.7).  At 297 to 444 items, a second round of these CTAs, both builds in turn: chains
+// of one block are slower here but for few rows (320 of 128 wide 8.97 -> 9.24, 400 10.6 -> 12.3, 80 wide 444 8.85 -> 9.14; of 48 rows and 64 keys 400 8.52 -> 8.21); with a softmax, and of
+// two blocks, it depends on what an item brings: 128 wide with softmax 371 x 1 12.7 -> 12.1, 425 x 1 13.7 -> 15.5, without 400 of 160 keys 1.01, 425
+// 17.0 -> 17.8; of 96 keys with softmax 425 0.95, 444 14.2 -> 15.0, of 64 444 13.7 -> 12.5; 96 wide 425 x 1 0.92 to 0.95, chains 444 x 2 1.00.  Two blocks with a softmax stay here, 371 x 2 19.7 -> 19.5, 425 x 2
+// 20.3 -> 21.3: the other kernel's error is 3 to 13 % larger there (one block: the same).
+// More tiles a sequence, up to 296 items: 296 x 1 8.0 -> 6.6, x 4 15.0 -> 14.0,
+// with a softmax only as long as there are few blocks (160 x 8 21.1 -> 22.9, 150 x 16 35.9 -> 38.4; of 208 or 256 rows, 80 wide, x 4 12.4 -> 12.9; x 2 of 208
+// keys 9.14 -> 9.01), without one always (150 x 64 122 -> 111); more items without a softmax
 // where a sequence has two tiles and four blocks (512 x 16 of 208 rows 75.0 -> 69.3, 600 x 4 37.1 -> 33.6; x 2 19.3 -> 21.1; of 2048 rows 1024 x 4 37.0 -> 39.3).
-// Its error against float64 is 1 to 3 % smaller: the other kernel keeps its references within 2^8 only.
-AttnFew attention_few(int batch, int M, int L, int d, int mode) {
+// Its error against float64 is 1 to 3 % smaller at scale d^-0.5, up to 14 % where the scores spread further: the other kernel keeps its references within 2^8 only.
+AttnFew attention_few(int batch, int M, int L, int d, int widths, int mode) {
   constexpr int kSms = 148;
   const long long items = static_cast<long long>((M + kBM - 1) / kBM) * batch;
   const int blocks = (L + kBN - 1) / kBN;
   const int m = mode == kModeSoftmax ? 0 : 1, wide = d == 64 ? 0 : 1;
   AttnFew best = {1, false, false};
   if (items > kSms && d == 128) {
-    if (M <= kBM) best.two = items <= 3 * kSms || blocks >= 3;
-    else if (items <= 2 * kSms) best.two = m == 1 || blocks <= (M <= 2 * kBM ? 3 : 4);
-    else best.two = m == 1 && M <= 2 * kBM && blocks >= 4;
+    const bool full = widths > 192;                        // of 256
+    if (M <= kBM) {
+      int most = 3 * kSms;
+      if (m == 1 && blocks == 1) most = M <= 48 && L <= 96 ? 3 * kSms : 2 * kSms;
+      else if (full && M > 80 && L > 64 && (m == 1 || blocks == 1)) most = L <= 96 ? 425 : L == kBN ? 380 : 400;
+      best.two = items <= most || blocks >= 3;
+    } else if (items <= 2 * kSms) {
+      best.two = m == 1 || blocks <= (M <= 2 * kBM ? 3 : 4);
+    } else {
+      best.two = m == 1 && M <= 2 * kBM && blocks >= 4;
+    }
     best.here = best.two;
     return best;
   }

@@ -44,7 +44,8 @@ struct AttnFew {
   bool here;
   bool two;            // in the form of which two CTAs fit an SM at head dimension 128
 };
-AttnFew attention_few(int batch, int M, int L, int d, int mode);
+// (widths: the sum of the two, d of which are at most the multiple of 64 that the kernels are compiled for)
+AttnFew attention_few(int batch, int M, int L, int d, int widths, int mode);
 
 // Head dimensions up to 64 and many items (attention_narrow_sm100.cu): a small CTA an item, 64-key blocks (map_k / map_v
 // boxes of 64 rows).  mode as above.
