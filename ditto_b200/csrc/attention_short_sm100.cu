@@ -735,7 +735,9 @@ bool by_row(int parts, int own, int m, bool shared) { return own >= (parts == 8 
 // More tiles a sequence, up to 296 items: 296 x 1 8.0 -> 6.6, x 4 15.0 -> 14.0,
 // with a softmax only as long as there are few blocks (160 x 8 21.1 -> 22.9, 150 x 16 35.9 -> 38.4; of 208 or 256 rows, 80 wide, x 4 12.4 -> 12.9; x 2 of 208
 // keys 9.14 -> 9.01), without one always (150 x 64 122 -> 111); more items without a softmax
-// where a sequence has two tiles and four blocks (512 x 16 of 208 rows 75.0 -> 69.3, 600 x 4 37.1 -> 33.6; x 2 19.3 -> 21.1; of 2048 rows 1024 x 4 37.0 -> 39.3).
+// where a sequence has two tiles and four blocks (512 x 16 of 208 rows 75.0 -> 69.3, 600 x 4 37.1 -> 33.6; x 2 19.3 -> 21.1; of 2048 rows 1024 x 4 37.0 -> 39.3) as long as the items are
+// few or long: of 208 rows, 128 wide, 890 x 4 46.0 -> 44.6, 1000 x 4 50.0 -> 50.4, 2000 x 4 89.0 -> 95.8, x 8 158.6 -> 164.9, 2000 of 1200 keys 202 -> 195; 96 wide 1300 x 4 55.4 -> 55.8, 2000 x 4
+// 78.5 -> 82.8, x 8 140 -> 141.
 // Its error against float64 is 1 to 3 % smaller at scale d^-0.5, up to 14 % where the scores spread further: the other kernel keeps its references within 2^8 only.
 AttnFew attention_few(int batch, int M, int L, int d, int widths, int mode) {
   constexpr int kSms = 148;
@@ -753,7 +755,7 @@ AttnFew attention_few(int batch, int M, int L, int d, int widths, int mode) {
     } else if (items <= 2 * kSms) {
       best.two = m == 1 || blocks <= (M <= 2 * kBM ? 3 : 4);
     } else {
-      best.two = m == 1 && M <= 2 * kBM && blocks >= 4;
+      best.two = m == 1 && M <= 2 * kBM && blocks >= 4 && (items <= (full ? 7 : 9) * kSms || blocks >= (full ? 9 : 8));
     }
     best.here = best.two;
     return best;

@@ -47,3 +47,13 @@ def test_one_tile_a_sequence(b, M, N, K, L, act, form):
     call, out, want = _case(b, M, N, K, L, act)
     _check(call, out, want)
     assert _launched(call)[0] == form
+
+
+# chains of two tiles a sequence
+@pytest.mark.parametrize("b,N,K,L,form", [
+    (518, 128, 128, 512, "few"), (519, 128, 128, 512, "whole"), (519, 128, 128, 1040, "few"), (519, 128, 128, 1024, "whole"), (666, 96, 96, 512, "few"),
+    (667, 96, 96, 512, "whole"), (667, 80, 80, 1024, "few"), (667, 64, 128, 912, "few"), (667, 64, 128, 896, "whole"), (300, 128, 128, 384, "whole")])
+def test_chains_of_two_tiles_a_sequence(b, N, K, L, form):
+    call, out, want = _case(b, 208, N, K, L, "relu")
+    _check(call, out, want)
+    assert _launched(call)[0] == form
