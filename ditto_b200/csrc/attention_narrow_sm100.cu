@@ -325,8 +325,11 @@ static cudaError_t launch_n(const AttnParams& p, long long items, cudaStream_t s
   // Up to three items an SM: no place for a fourth.  The CTAs of a call go to the places that the call before it leaves free, while that one still runs (the
   // launch is programmatic): with four an SM they end up four on some SMs and two on others, and the call lasts as long as one of 592
   // items.  us, four places -> three, calls one after another: 300 items of 128 / 512 / 1024 keys 7.0 -> 6.3, 16.6 -> 14.3, 29.1 -> 25.1, 384 of 512 17.5 -> 14.4,
-  // 444 of 512 17.0 -> 14.7; behind another kernel the placing is even and nothing changes (17.1 -> 17.0).
-  cfg.dynamicSmemBytes = items > 296 && items <= 444 ? kSmemBytesThree : kSmemBytes;
+  // 444 of 512 17.0 -> 14.7; behind another kernel the placing is even and nothing changes (17.1 -> 17.0).  Items of one 64-key block are over so soon that the fourth place, where
+  // the next call's CTAs are set up, is worth more once the three are nearly full (in a graph, both builds in turn, chains 365 0.87 to 0.95, 395 0.92 to 1.05, 444 4.16 -> 4.54; softmax
+  // 425 0.90 to 0.95, 444 5.18 -> 5.34).
+  const int three = p.L > 64 ? 444 : MODE == kModeSoftmax ? 425 : 370;
+  cfg.dynamicSmemBytes = items > 296 && items <= three ? kSmemBytesThree : kSmemBytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see grid_dependency_wait in the kernel

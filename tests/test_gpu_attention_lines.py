@@ -1,10 +1,12 @@
-"""Where calls go over from one form of attention and of small chains to another at two to nine items an SM: the kernel, read from a captured graph, on
-either side of each line; and that the results of either side are those of float64 products."""
+"""Where calls go over from one form of attention and of small chains to another at two to nine items an SM: the kernel, its CTAs and the shared memory they ask
+for, read from a captured graph, on either side of each line; and that the results of either side are those of float64 products."""
+import ctypes
+
 import pytest
 import torch
 
 from ditto_b200 import ops
-from tests.test_gpu_attention_short import _launched, _operands
+from tests.test_gpu_attention_short import _KernelNode, _launched, _operands
 from tests.test_gpu_attention_split import _close, _reference
 
 pytestmark = pytest.mark.gpu
@@ -57,3 +59,26 @@ def test_chains_of_two_tiles_a_sequence(b, N, K, L, form):
     call, out, want = _case(b, 208, N, K, L, "relu")
     _check(call, out, want)
     assert _launched(call)[0] == form
+
+
+def _shared(call):
+    """Kernel, CTAs and shared memory of the one launch of a call."""
+    form, ctas = _launched(call)
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    cuda, count, node, params = ctypes.CDLL("libcuda.so.1"), ctypes.c_size_t(1), ctypes.c_void_p(), _KernelNode()
+    assert cuda.cuGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.byref(node), ctypes.byref(count)) == 0
+    assert cuda.cuGraphKernelNodeGetParams_v2(node, ctypes.byref(params)) == 0
+    return form, ctas, params.shared
+
+
+# head dimension 64, three items an SM at most: places for three CTAs an SM, or for four where one block of 64 keys is the whole item
+@pytest.mark.parametrize("b,L,act,places", [
+    (444, 80, "identity", 3), (445, 80, "identity", 4), (370, 64, "identity", 3), (371, 64, "identity", 4), (444, 16, "relu", 4), (425, 64, None, 3),
+    (426, 64, None, 4), (444, 80, None, 3), (297, 64, None, 3), (297, 16, "identity", 3)])
+def test_places_of_the_kernel_with_64_key_blocks(b, L, act, places):
+    call, out, want = _case(b, 128, 64, 64, L, act)
+    _check(call, out, want)
+    form, ctas, shared = _shared(call)
+    assert form == "narrow" and ctas == b and (228 << 10) // (shared + 1024) == places
