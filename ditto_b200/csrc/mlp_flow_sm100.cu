@@ -27,7 +27,8 @@
 // that a store instruction writes whole 128-byte rows.
 //
 // Two launches over tiles (mlp_tiles_sm100.cu, mlp_waves_sm100.cu) are the faster form wherever they are possible; this one serves hidden layers
-// of 512 MB and more, first GEMMs of one k-step, results that are not aligned to 32 bytes, and callers who ask for it.
+// of 512 MB and more, first GEMMs over fewer than 128 columns, results or scratch memory not aligned to 32 bytes, calls without memory for their hidden layer, and
+// callers who ask for it.
 //
 // What bounds it: the tensor pipe under the power cap for large inputs; the chain first load -> GEMM1 tile -> hidden
 // tile announced -> GEMM2 tile (about 13 us) and tile quantisation for short ones.  Measured, cluster kernel -> this one (two launches: 214 and 203, 33, 13 and 72):

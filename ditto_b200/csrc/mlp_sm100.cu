@@ -722,6 +722,8 @@ static int resolve_variant(int variant, int N, int K, int L, int w_layout) {
 // clusters.  Measured, us, cluster / flow / tile kernel, 1024 -> 4096 -> 1024: 64 entries of 128 rows 185 / 253 / 211; 256 of 16
 // 655 / 905 / 684; 33 of 336 217 / 232 / 235; 40 of 128 169 / 165 / 142; 24 of 384 239 / 183 / 157; 100 of 400 895 / 697 / 918;
 // 768 -> 3072 -> 768: 64 of 128 120 / 154 / 132, 100 of 128 219 / 231 / 246.
+// (The line between clusters and 256-row tiles is the flow kernel's.  Of the calls beyond it most now take the wave kernel, which does 1.27 to 1.35 PFLOP/s;
+// those on the clusters' side, 33 of 336 for one, have not been timed against that.)
 // Other widths: the cluster kernel does 0.3 to 0.6 PFLOP/s and the tile kernel is the better form of 128-row blocks
 // (256 -> 1024 -> 256, 1024 of 128: 430 / 425 / 307; 1280 -> 5120 -> 1280, 64 of 128: 481 / 376 / 361) up to hidden layers that
 // are no longer read out of L2 (512 -> 2048 -> 512, hidden layers of 105, 134 and 268 MB: 200 of 128 219 / 231 / 214, 512 of 64
@@ -743,11 +745,14 @@ static MlpForm form_with_scratch(int batch, int M, int N, int K, int L, bool bf1
 
 // Whether the wave kernel takes a call that would else go to the tile or the flow kernel.
 //
-// In place of the flow kernel, always; measured, us, operands new call after call under the power cap, flow -> waves: 16384 x 1024 -> 4096 -> 1024 235 -> 214,
-// 3328 x 1280 -> 5120 -> 1280 with GELU 86.3 -> 74.0, 4096 x 2048 -> 8192 -> 2048 224 -> 217, 16384 x 256 -> 8192 -> 256 191 -> 155, 65536 x 1024 928 -> 830; 16
-// entries of 512 x 1024 -> 4096 -> 1024 135 -> 120, 24 of 384 x 768 135 -> 97; the other way 4656 x 256 -> 8192 -> 2048 with GELU, whose GEMM1 is all
-// epilogue, 183 -> 190.  Not with a hidden layer of 512 MB or more (4096 x 2048 -> 65536 -> 2048 1570 -> 1640), of which the flow kernel
-// only holds a ring, and not with fewer than two k-steps in GEMM1: those calls keep the flow kernel, whose epilogues with biases nothing else reaches.
+// In place of the flow kernel; measured, us, operands new call after call under the power cap, flow -> waves: 16384 x 1024 -> 4096 -> 1024 235 -> 214,
+// 3328 x 1280 -> 5120 -> 1280 with GELU 86.3 -> 74.0, 4096 x 2048 -> 8192 -> 2048 224 -> 217, 16384 x 256 -> 8192 -> 256 191 -> 155; 16
+// entries of 512 x 1024 -> 4096 -> 1024 135 -> 120, 24 of 384 x 768 135 -> 97.  Of 300 more (first GEMMs of 128 to 1024 columns, results of 256 to 2048, hidden layers of 2048
+// to 8192, 1e11 and 2.5e11 operations, ReLU and GELU with biases) it is slower by more than 1 % in two, 4768 x 256 -> 8192 -> 1024 110 -> 114 and 9920 x 512 ->
+// 8192 -> 1024 214 -> 217.
+// Hidden layers of 512 MB and more, of which the flow kernel only holds a ring, stay with that one for the memory they would take: of two of
+// exactly 512 MB one is faster here and one there (65536 x 1024 -> 4096 -> 1024 928 -> 830, 4096 x 2048 -> 65536 -> 2048 1570 -> 1640).  So do first GEMMs over
+// fewer than 128 columns, which have not been timed.
 // In place of the tile kernel where its modelled time is less than 0.87 of that one's, which is scaled to what it measures (198 shapes, 1.64 t - 2.5): nearer to a
 // draw the tile kernel was the faster one by up to 25 % (1024 x 1024 -> 4096 -> 1024 21.6 against 26.7).  What the rule picks is 0.6 % (in bursts) to 1.2 % (under the power
 // cap) slower than the best form on average.  Tiles -> waves: 2048 x 1024 36.6 -> 33.5, 4096 x 768 -> 3072 -> 768 with GELU 46.3 -> 38.6, 1632 x 768 28.2 -> 23.6,

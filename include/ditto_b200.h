@@ -92,10 +92,12 @@ int ditto_b200_multi_head_attention(const void* qkv, void* out, int batch, int M
  *   undefined on return).  With it calls keep the whole hidden layer there between two launches, up to 512 MB of it; larger
  *   hidden layers, and with K < 128 or a `y` or workspace that is not aligned to 32 bytes calls of more than about 48 GFLOP, pass through a
  *   ring of row blocks between the tiles of the two GEMMs, behind a launch that clears the ring's counters.  The ring holds the row
- *   blocks that are on their way: at most 64 MB up to a hidden size of about 5000, more where a row block is longer or the other
- *   widths are small (512 MB for 2048 -> 65536 -> 2048), never more than the hidden layer.  Where batch entries of few rows make
+ *   blocks of 256 rows that are on their way: at most 64 MB up to a hidden size of about 5000, more where a row block is longer or the other
+ *   widths are small (512 MB for 2048 -> 65536 -> 2048), all of them at most, and beside them counters and the sums of divided tiles.  What is asked for is
+ *   enough for the ring as well, which can be more than the hidden layer (entries whose rows are no multiple of 256): size the
+ *   buffer by ditto_b200_workspace_bytes, not by a bound.  Where batch entries of few rows make
  *   another form the faster one, and when a cluster kernel is forced, it is used to share row blocks between clusters.  Enough for the
- *   ring alone: the ring.  NULL or too small: the hidden activations stay inside a cluster, one cluster
+ *   ring alone (DITTO_OP_LESS_SCRATCH): the ring.  NULL or too small: the hidden activations stay inside a cluster, one cluster
  *   per row block, in one launch for up to 1024 result columns: 1.2 to 3 times the time, more for wider results.
  * Shapes: N <= 128 and K <= 128 (any multiples of 16, either weight layout): the reference's own shape family;
  * otherwise L % 128 == 0, K % 64 == 0, N in {256, 512, 768, 1024}, or -- on the default kernel -- L % 64 == 0,
