@@ -261,21 +261,21 @@ bool room_for(int device, size_t bytes) {
   if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return true;
   try {
     const auto index = static_cast<c10::DeviceIndex>(device);
-    size_t largest = 1;                            // (0 would ask the device)
-    c10::cuda::CUDACachingAllocator::cacheInfo(index, &largest);
-    if (largest >= bytes) return true;
-    // what the allocator can give back: cached segments of which no part is in use
     const auto s = c10::cuda::CUDACachingAllocator::getDeviceStats(index);
     const size_t reserved = static_cast<size_t>(s.reserved_bytes[0].current);
+    // what the allocator can give back: cached segments of which no part is in use
     const size_t whole = reserved - static_cast<size_t>(s.allocated_bytes[0].current) - static_cast<size_t>(s.inactive_split_bytes[0].current);
-    size_t free = 0, total = 0;
+    if (whole >= bytes) return true;
+    size_t free = 0, total = 0, largest = 1;       // (a largest block of 0 would ask the device)
     if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
       cudaGetLastError();
       return true;
     }
     const double share = c10::cuda::CUDACachingAllocator::getMemoryFraction(index) * static_cast<double>(total);
     const size_t allowed = share > static_cast<double>(reserved) ? static_cast<size_t>(share) - reserved : 0;
-    return whole + std::min(free, allowed) >= bytes;
+    if (whole + std::min(free, allowed) >= bytes) return true;
+    c10::cuda::CUDACachingAllocator::cacheInfo(index, &largest);       // (walks all cached blocks)
+    return largest >= bytes;
   } catch (const std::exception&) {
     return true;
   }
